@@ -2410,11 +2410,9 @@ __attribute__((visibility("default"))) int tg_plan_create(const tg_segment *segs
         p->launches += 1;
     }
     // Kinds side by side (the latency-bound regime, every kind in one wave):
-    // the FP64 scalar grid is halved, each warp taking two tiles.  The scalar kind
-    // then still finishes inside the block kinds' time, and the block warps,
-    // the long pole, get more of the SMs' issue slots (2.5 deg grid, 10368
-    // columns: 84 -> 78 us).  Decided here, with the overlap setting of the
-    // plan's creation.
+    // each warp of the FP64 scalar grid takes at least two tiles, so that the
+    // block warps get more of the SMs' issue slots.  Decided here, with the
+    // overlap setting of the plan's creation.
     {
         auto &g0 = p->groups[0];
         bool split = g0.nseg > 0 && (p->groups[1].nseg > 0 || p->groups[2].nseg > 0);
@@ -2424,8 +2422,10 @@ __attribute__((visibility("default"))) int tg_plan_create(const tg_segment *segs
             for (const auto &g : p->groups)
                 if (g.nseg > 0 && !g.shape.one_wave) split = false;
         p->side_by_side = split;
-        if (split && precision == TG_PREC_F64 && g0.shape.stages > 0 && g0.shape.blocks > 1)
-            g0.shape.blocks = (g0.shape.blocks + 1) / 2;
+        if (split && precision == TG_PREC_F64 && g0.shape.stages > 0) {
+            const int half = (g0.ntiles + 1) / 2 / (g0.shape.threads / 32);
+            if (g0.shape.blocks > half && half > 0) g0.shape.blocks = half;
+        }
     }
     for (auto &g : p->groups) {
         if (!g.nseg) continue;
@@ -2698,6 +2698,7 @@ __attribute__((visibility("default"))) int tg_plan_describe(const tg_plan *p, ch
             else if (!f64) snprintf(name, sizeof name, "k_block_refine<%d>", g.kind);
             else if (h.stages && h.rows) snprintf(name, sizeof name, "k_block_f64_rows<%d,%d>", g.kind, h.stages);
             else if (h.stages && h.res) snprintf(name, sizeof name, "k_block_f64_ring<%d,%d,%d,1>", g.kind, h.stages, h.bw);
+            else if (h.stages && h.bw == 32) snprintf(name, sizeof name, "k_block_f64_chunk<%d,%d>", g.kind, h.stages);
             else if (h.stages) snprintf(name, sizeof name, "k_block_f64_ring<%d,%d,%d>", g.kind, h.stages, h.bw);
             else snprintf(name, sizeof name, "k_block_f64<%d>", g.kind);
         }

@@ -19,6 +19,7 @@
 #include "tg_internal.h"
 #include "tg_arith.cuh"
 #include "tg_bulk.cuh"
+#include "tg_stage.cuh"
 
 namespace tg {
 
@@ -438,77 +439,92 @@ __global__ void __launch_bounds__(256) k_scalar_f64_ring(SegTable tab, double *s
     }
 }
 
+// L2-resident scratch store; no memory clobber, so that the loads of the next
+// level may be scheduled above it (the back sweep is behind a barrier).
+__device__ __forceinline__ void st_scratch(double *p, double v, unsigned long long pol)
+{
+    asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;" ::"l"(p), "d"(v), "l"(pol));
+}
+__device__ __forceinline__ void st_scratch2(double *p, double v0, double v1, unsigned long long pol)
+{
+    asm volatile("st.global.L2::cache_hint.v2.f64 [%0], {%1, %2}, %3;" ::"l"(p), "d"(v0), "d"(v1), "l"(pol));
+}
+// 16-byte asynchronous copy past L1 with an L2 policy
+__device__ __forceinline__ void cp_async16(double *dst, const double *src, unsigned long long pol)
+{
+    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src),
+                 "l"(pol)
+                 : "memory");
+}
 // ---------------------------------------------------------------------------
-// Scalar Thomas, FP64, bulk-copy ring of chunks: each of C stages holds L
-// consecutive levels of the four coefficient arrays (4L copies of 256 B), so
-// the mbarrier wait, proxy fence and copy issue happen once per L levels
-// instead of once per level.  w2 in the L2 scratch slot of the lane, w3
-// parked in x, as in k_scalar_f64_ring; same arithmetic, same bits.
+// Scalar Thomas, FP64, one warp per 32-column tile, the coefficients through a
+// shared-memory ring of C stages of L levels filled by 16-byte asynchronous
+// copies (two of a level's four 256-byte rows per instruction), so that the
+// wait and the refill happen once per L levels.  A level's (w2, w3) pair goes
+// to the warp's own scratch slice, (level, column, pair): one 16-byte store at
+// a constant offset, read back by the same lane through the same ring for the
+// back sweep.  x is written once.  Level k does both divisions by its pivot:
+// w3(k) and the next level's w2 = c(k)/w1(k) (the reference's operands, so the
+// same correctly rounded quotients), under one range test.  Row 0's a is
+// replaced by zero (x - 0*0 = x for every x), so no level is special.
+// With few columns the recurrence bounds it: 10,368 columns x 57 levels 26.9
+// -> 18.8 us (the four 256-byte bulk copies a level cost the issuing lanes
+// about 200 cycles).  With many, HBM and the scratch's share of L2: 909,356
+// columns 449 -> 382 us (5.4 TB/s), 290,304 x 113 349 -> 284 (4.6).
 // ---------------------------------------------------------------------------
 template <int C, int L>
 __global__ void __launch_bounds__(256) k_scalar_f64_chunk(SegTable tab, double *scratch, unsigned *status)
 {
-    constexpr int NE = 4 * L;
-    static_assert(NE <= 32, "one copy per lane");
-    __shared__ __align__(8) unsigned long long bars[8 * C];
+    constexpr int LB = L, CB = 2 * C;   // back sweep: 16 bytes per level and column, twice the levels
     extern __shared__ __align__(128) double smem_r[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    double *buf = smem_r + (long)warp * C * NE * 32;
-    unsigned long long *bar = bars + warp * C;
+    double *buf = smem_r + (long)warp * C * L * 128;
     const unsigned long long pol = l2_policy(tab.hints, false), keep = l2_policy(tab.hints, true);
-    const long ws = (long)gridDim.x * blockDim.x;
-    double *w2s = scratch + (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (lane == 0) {
-#pragma unroll 1
-        for (int i = 0; i < C; ++i) mbar_init(&bar[i], 1);
-        fence_mbar_init();
-    }
-    __syncwarp();
-    unsigned q = 0;
+    double *wz = scratch + ((long)blockIdx.x * nwarps + warp) * ((long)tab.k2max * 64) + lane * 2;
+    const int half = lane >> 4, c2 = (lane & 15) * 2;   // this lane's row of a pair and its two columns
     for (int t = blockIdx.x * nwarps + warp; t < tab.ntiles; t += gridDim.x * nwarps) {
         const Seg s = tab.segs ? tab.segs[find_seg(tab, t)] : tab.one;
-        const long col0 = (long)(t - s.tile0) * 32;
-        const long ld = s.ld;
-        const int k2 = s.k2;
+        const long col0 = (long)(t - s.tile0) * 32, ld = s.ld;
+        const int k2 = s.k2, nch = (k2 + L - 1) / L;
         const bool valid = col0 + lane < s.ncol;
-        const int arr = lane & 3;
-        const double *src = (arr == 0 ? s.a : arr == 1 ? s.b : arr == 2 ? s.c : s.f) + col0 + (long)(lane >> 2) * ld;
-        double *px = s.x + col0 + lane;
-        const int nch = (k2 + L - 1) / L;
-        // chunk j: levels j*L .. j*L+L-1 (those < k2) into stage (q + j) % C
-        auto issue = [&](unsigned qc, int j) {
-            const int st = (int)(qc % C), l0 = j * L;
-            const int nl = k2 - l0 < L ? k2 - l0 : L;
-            if (lane == 0) mbar_expect(&bar[st], (uint32_t)(4 * nl * 256));
-            __syncwarp();
-            if (lane < 4 * nl) bulk_load_hint(buf + (st * NE + lane) * 32, src + (long)l0 * ld, 256u, &bar[st], pol);
-        };
-        const int pre = nch < C ? nch : C;
-        for (int j = 0; j < pre; ++j) issue(q + j, j);
-        bool ok = true, fin = true;
-        double w1 = 0.0, y1 = 0.0, w3 = 0.0, w2 = 0.0;   // w2: the next level's, from this pivot
-        for (int j = 0; j < nch; ++j) {
-            const unsigned qc = q + j;
-            if (!mbar_wait_warp(&bar[qc % C], (qc / C) & 1u)) {
-                const unsigned qe = q + (j + C < nch ? j + C : nch);
-#pragma unroll 1
-                for (unsigned r = qc; r < qe; ++r) mbar_wait_warp(&bar[r % C], (r / C) & 1u);
-                if (lane == 0) report(status, s.status_idx, FLAG_TIMEOUT);
-                return;
+        const double *p0 = (half ? s.b : s.a) + col0 + c2, *p1 = (half ? s.f : s.c) + col0 + c2;
+        int knext = 0;
+        double *dst = buf + half * 32 + c2;
+        auto issue = [&](int st) {   // L levels from knext into stage st; empty above the top
+            double *d = dst + st * L * 128;
+            if (knext + L <= k2) {
+#pragma unroll
+                for (int l = 0; l < L; ++l) {
+                    cp_async16(d + l * 128, p0 + l * ld, pol);
+                    cp_async16(d + l * 128 + 64, p1 + l * ld, pol);
+                }
+            } else {
+                for (int l = 0; knext + l < k2; ++l) {
+                    cp_async16(d + l * 128, p0 + l * ld, pol);
+                    cp_async16(d + l * 128 + 64, p1 + l * ld, pol);
+                }
             }
-            // the stage is read in place and handed back to the copy engine
-            // after the L levels are done (registers stay low: more warps/SM)
-            const double *stg = buf + (int)(qc % C) * NE * 32 + lane;
-            // Level k from stage row l.  Both divisions by the pivot w1(k) are
-            // done here: w3(k) = (f - a*w3(k-1))/w1(k) and the next level's
-            // w2 = c(k)/w1(k) (the same operands as the reference's, so the
-            // same correctly rounded quotients), under one range test.
-            auto step = [&](int l, int k, bool first, bool last) {
-                const double ak = stg[(4 * l + 0) * 32], bk = stg[(4 * l + 1) * 32], fk = stg[(4 * l + 3) * 32],
-                             ck = stg[(4 * l + 2) * 32];
-                w1 = first ? bk : xsub(bk, xmul(ak, w2));
-                y1 = __drcp_rn(w1);
-                const double num = first ? fk : xsub(fk, xmul(ak, w3));
+            knext = knext + L < k2 ? knext + L : k2;
+            p0 += L * ld;
+            p1 += L * ld;
+            cp_async_commit();
+        };
+        for (int j = 0; j < C; ++j) issue(j);
+        bool ok = true;
+        double w2 = 0.0, w3 = 0.0;
+        double *wk = wz;
+        int st = 0;
+        for (int j = 0; j < nch; ++j) {
+            cp_async_wait<C - 1>();
+            __syncwarp();
+            double *stg = buf + st * L * 128 + lane;
+            if (j == 0) stg[0] = 0.0;
+            auto step = [&](int l) {
+                const double ak = stg[l * 128], bk = stg[l * 128 + 32], ck = stg[l * 128 + 64],
+                             fk = stg[l * 128 + 96];
+                const double w1 = xsub(bk, xmul(ak, w2));
+                const double y1 = __drcp_rn(w1);
+                const double num = xsub(fk, xmul(ak, w3));
                 if (max(exp_dist(w1), max(exp_dist(num), exp_dist(ck))) < kExpSpan) {
                     w3 = div_markstein(num, w1, y1);
                     w2 = div_markstein(ck, w1, y1);
@@ -519,65 +535,71 @@ __global__ void __launch_bounds__(256) k_scalar_f64_chunk(SegTable tab, double *
                     // a pivot in the safe range is finite and nonzero
                     if (!w1s) ok = ok && finite_nz(w1);
                 }
-                if (!last) st_hint(&w2s[k * ws], w2, keep);
-                st_hint(&px[k * ld], w3, keep);
+                st_scratch2(wk + l * 64, w2, w3, keep);
             };
             if (valid) {
-                if (j > 0 && (j + 1) * L < k2) {   // a full chunk, neither level 0 nor the top
+                if ((j + 1) * L <= k2) {
 #pragma unroll
-                    for (int l = 0; l < L; ++l) step(l, j * L + l, false, false);
+                    for (int l = 0; l < L; ++l) step(l);
                 } else {
-#pragma unroll
-                    for (int l = 0; l < L; ++l) {
-                        const int k = j * L + l;
-                        if (k < k2) step(l, k, k == 0, k + 1 == k2);
-                    }
+                    for (int l = 0; j * L + l < k2; ++l) step(l);
                 }
             }
+            wk += L * 64;
             __syncwarp();
-            fence_proxy_async();
-            if (j + C < nch) issue(qc + C, j + C);
+            issue(st);
+            st = st + 1 == C ? 0 : st + 1;
         }
-        q += nch;
-        if (valid) {
-            // A non-finite x(k+1) makes x(k) = w3 - w2*x(k+1) non-finite (inf
-            // or NaN), down to x(0): x(0) finite <=> every x finite.
-            double xn = w3;
-            double rw[4], r2[4];
+        // back sweep: levels kh - LB + 1 .. kh of stage d, kh = k2 - 2 - d*LB;
+        // each lane copies and reads its own pairs
+        cp_async_wait<0>();
+        asm volatile("" ::: "memory");
+        __syncwarp();
+        const int KB = k2 - 1, nbk = (KB + LB - 1) / LB;
+        auto issue_b = [&](int sb, int d) {
+            const int kh = KB - 1 - d * LB;
+            double *db = buf + sb * LB * 64 + lane * 2;
+            const double *src = wz + (long)kh * 64;
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (k2 - 2 - u >= 0) {
-                    rw[u] = px[(k2 - 2 - u) * ld];
-                    r2[u] = w2s[(k2 - 2 - u) * ws];
-                }
-            int kb = k2 - 2;
-            for (; kb - 7 >= 0; kb -= 4) {   // four levels and their refills all in range
+            for (int l = 0; l < LB; ++l)
+                if (kh - l >= 0) cp_async16(db + l * 64, src - l * 64, keep);
+            cp_async_commit();
+        };
+        for (int d = 0; d < CB; ++d) issue_b(d, d);
+        // A non-finite x(k+1) makes x(k) = w3 - w2*x(k+1) non-finite (inf or
+        // NaN), down to x(0): x(0) finite <=> every x finite.
+        double xn = w3;
+        double *px = s.x + col0 + lane + (long)KB * ld;
+        if (valid) *px = xn;
+        int sb = 0;
+        for (int d = 0; d < nbk; ++d) {
+            cp_async_wait<CB - 1>();
+            const double2 *g = reinterpret_cast<const double2 *>(buf + sb * LB * 64) + lane;
+            const int nl = KB - d * LB;
+            if (valid) {
+                if (nl >= LB) {
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int k = kb - u;
-                    xn = xsub(rw[u], xmul(r2[u], xn));
-                    rw[u] = px[(k - 4) * ld];
-                    r2[u] = w2s[(k - 4) * ws];
-                    px[k * ld] = xn;
-                }
-            }
-            for (; kb >= 0; kb -= 4) {
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int k = kb - u;
-                    if (k >= 0) {
-                        xn = xsub(rw[u], xmul(r2[u], xn));
-                        if (k - 4 >= 0) {
-                            rw[u] = px[(k - 4) * ld];
-                            r2[u] = w2s[(k - 4) * ws];
-                        }
-                        px[k * ld] = xn;
+                    for (int l = 0; l < LB; ++l) {
+                        const double2 w = g[l * 32];
+                        xn = xsub(w.y, xmul(w.x, xn));
+                        px -= ld;
+                        *px = xn;
+                    }
+                } else {
+                    for (int l = 0; l < nl; ++l) {
+                        const double2 w = g[l * 32];
+                        xn = xsub(w.y, xmul(w.x, xn));
+                        px -= ld;
+                        *px = xn;
                     }
                 }
             }
-            fin = finite(xn);
-            report(status, s.status_idx, (ok ? 0u : FLAG_PIVOT) | (fin ? 0u : FLAG_NONFINITE));
+            issue_b(sb, d + CB);
+            sb = sb + 1 == CB ? 0 : sb + 1;
         }
+        cp_async_wait<0>();
+        __syncwarp();
+        if (valid) report(status, s.status_idx, (ok ? 0u : FLAG_PIVOT) | (finite(xn) ? 0u : FLAG_NONFINITE));
     }
 }
 
@@ -1723,7 +1745,8 @@ __global__ void __launch_bounds__(128) k_block_f64(SegTable tab, double *scratch
 
 // ---------------------------------------------------------------------------
 // Block-tridiagonal Thomas, FP64, bit-exact, coefficients staged by bulk
-// copies: one warp per CTA, 32 columns; the 3*B*B + B entries of a level
+// copies (opt-in: narrow tiles and Gamma in shared memory; the default is
+// k_block_f64_chunk): one warp per CTA, W columns; the 3*B*B + B entries of a level
 // (P, Q, R, f) arrive in a D-stage shared-memory ring, one 256-byte copy per
 // entry issued by one lane.  Same arithmetic as blk_f64_col.
 // ---------------------------------------------------------------------------
@@ -1899,6 +1922,210 @@ __global__ void __launch_bounds__(256) k_block_f64_ring(SegTable tab, double *sc
                 if (s.ubc_add) tv = xadd(tv, __ldg(s.ubc_add + i * ld + col0 + cl));
                 fin = fin && finite(tv);
                 pU[((long)k2 * B + i) * ld] = tv;
+            }
+        }
+        report(status, s.status_idx, (ok ? 0u : FLAG_PIVOT) | (fin ? 0u : FLAG_NONFINITE));
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Block-tridiagonal Thomas, FP64, bit-exact, one warp per 32-column tile, the
+// coefficients and the back sweep's operands through one shared-memory ring
+// filled by 16-byte asynchronous copies (two 256-byte rows per instruction;
+// a 256-byte bulk copy costs its issuing lane about 50 cycles, 30 of them a
+// level for B = 3).  In the forward sweep a stage holds L levels, so the wait
+// and the refill happen once per L levels.  Gamma and z of a level go to the
+// warp's own scratch slice, (level, entry, column) with the column fastest:
+// every store has a constant offset, and a run of levels is one contiguous
+// piece for the back sweep.  u is written once.  The forward level is the
+// arithmetic of blk_f64_col; row 0's P is replaced by zeros in shared memory
+// (x - 0*0 = x for every x), so no level is special.
+// What bounds it: with few columns the level's dependency chain (2x2, 57
+// levels: 390 cycles a level; it was 1,270 with bulk copies, 710 of them the
+// copies' issue); 10,368 columns 59.7 -> 27.8 us, 3x3 6,969 columns 106.8 ->
+// 43.9.  With many, HBM and the scratch's share of L2: 130,000 columns 2x2
+// 267 -> 205 us (4.6 TB/s of the systems' bytes), 3x3 536 -> 443 (4.4).
+// ---------------------------------------------------------------------------
+template <int B, int C, int L>
+__global__ void __launch_bounds__(256, 1) k_block_f64_chunk(SegTable tab, double *scratch, unsigned *status)
+{
+    constexpr int BB = B * B, NE = 3 * BB + B, NB = BB + B;
+    constexpr int CB = 4, LB = C * L * NE / (CB * NB);   // back sweep: CB stages of LB levels in the same ring
+    static_assert(LB >= 1, "back stage");
+    extern __shared__ __align__(128) double smem_c[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    double *buf = smem_c + (long)warp * C * L * NE * 32;
+    const unsigned long long pol = l2_policy(tab.hints, false), keep = l2_policy(tab.hints, true);
+    double *gz = scratch + ((long)blockIdx.x * nwarps + warp) * ((long)tab.k2max * NB * 32);
+    const int half = lane >> 4, c2 = (lane & 15) * 2;   // this lane's row of a pair and its two columns
+    for (int t = blockIdx.x * nwarps + warp; t < tab.ntiles; t += gridDim.x * nwarps) {
+        const Seg s = tab.segs ? tab.segs[find_seg(tab, t)] : tab.one;
+        const long col0 = (long)(t - s.tile0) * 32, ld = s.ld;
+        const int k2 = s.k2, nch = (k2 + L - 1) / L;
+        const bool valid = col0 + lane < s.ncol;
+        // n rows of one array of one level, p at its first row
+        auto rows = [&](double *dst, const double *p, int n) {
+#pragma unroll
+            for (int e = 0; e < n; e += 2)
+                if (e + 1 < n || half == 0) cp_async16(dst + (e + half) * 32 + c2, p + (long)e * ld, pol);
+        };
+        const long o0 = col0 + c2 + half * ld;
+        const double *pP = s.a + o0, *pQ = s.b + o0, *pR = s.c + o0, *pF = s.f + o0;
+        int knext = 0;                       // the next level to request
+        auto issue = [&](int st) {           // up to L levels from knext into stage st
+            double *d = buf + st * L * NE * 32;
+#pragma unroll
+            for (int l = 0; l < L; ++l, ++knext, d += NE * 32)
+                if (knext < k2) {
+                    rows(d, pP, BB);
+                    rows(d + BB * 32, pQ, BB);
+                    rows(d + 2 * BB * 32, pR, BB);
+                    rows(d + 3 * BB * 32, pF, B);
+                    pP += BB * ld;
+                    pQ += BB * ld;
+                    pR += BB * ld;
+                    pF += B * ld;
+                }
+            cp_async_commit();
+        };
+        for (int j = 0; j < C; ++j) issue(j);
+        bool ok = true;
+        double G[BB], z[B];
+#pragma unroll
+        for (int e = 0; e < BB; ++e) G[e] = 0.0;
+#pragma unroll
+        for (int i = 0; i < B; ++i) z[i] = 0.0;
+        int st = 0;
+        for (int j = 0; j < nch; ++j) {
+            cp_async_wait<C - 1>();
+            __syncwarp();
+            double *stg = buf + st * L * NE * 32 + lane;
+            if (j == 0)
+#pragma unroll
+                for (int e = 0; e < BB; ++e) stg[e * 32] = 0.0;
+            auto level = [&](int l) {
+                const double *r = stg + l * NE * 32;
+                double Qp[BB], W[BB], v[B];
+#pragma unroll
+                for (int m = 0; m < B; ++m)
+#pragma unroll
+                    for (int i = 0; i < B; ++i) {
+                        double qv = r[(BB + i + B * m) * 32];
+#pragma unroll
+                        for (int n = 0; n < B; ++n) qv = xsub(qv, xmul(r[(i + B * n) * 32], G[n + B * m]));
+                        Qp[i + B * m] = qv;
+                    }
+#pragma unroll
+                for (int i = 0; i < B; ++i) {
+                    double tv = r[(3 * BB + i) * 32];
+#pragma unroll
+                    for (int m = 0; m < B; ++m) tv = xsub(tv, xmul(r[(i + B * m) * 32], z[m]));
+                    v[i] = tv;
+                }
+                double Rv[BB];
+#pragma unroll
+                for (int e = 0; e < BB; ++e) Rv[e] = r[(2 * BB + e) * 32];
+                ok = inv_exact<B>(Qp, W) && ok;
+                double *g = gz + (long)(j * L + l) * (NB * 32) + lane;
+#pragma unroll
+                for (int i = 0; i < B; ++i) {
+                    double tv = xmul(W[i], v[0]);
+#pragma unroll
+                    for (int m = 1; m < B; ++m) tv = xadd(tv, xmul(W[i + B * m], v[m]));
+                    z[i] = tv;
+                    st_scratch(g + (BB + i) * 32, tv, keep);
+                }
+#pragma unroll
+                for (int m = 0; m < B; ++m)
+#pragma unroll
+                    for (int i = 0; i < B; ++i) {
+                        double gv = xmul(W[i], Rv[B * m]);
+#pragma unroll
+                        for (int n = 1; n < B; ++n) gv = xadd(gv, xmul(W[i + B * n], Rv[n + B * m]));
+                        G[i + B * m] = gv;
+                        st_scratch(g + (i + B * m) * 32, gv, keep);
+                    }
+            };
+            if (valid) {
+                if ((j + 1) * L <= k2) {
+#pragma unroll
+                    for (int l = 0; l < L; ++l) level(l);
+                } else {
+                    for (int l = 0; j * L + l < k2; ++l) level(l);
+                }
+            }
+            __syncwarp();
+            issue(st);
+            st = st + 1 == C ? 0 : st + 1;
+        }
+        // back sweep: rows kh - LB + 1 .. kh of stage d, kh = k2 - 2 - d*LB,
+        // one contiguous piece of the scratch slice
+        cp_async_wait<0>();
+        asm volatile("" ::: "memory");
+        __syncwarp();
+        const int KB = k2 - 1, nbk = (KB + LB - 1) / LB;
+        auto issue_b = [&](int sb, int d) {
+            if (d < nbk) {
+                const int kh = KB - 1 - d * LB, kl = kh - LB + 1 > 0 ? kh - LB + 1 : 0;
+                const double *src = gz + (long)kl * (NB * 32) + lane * 2;
+                double *dst = buf + sb * LB * NB * 32 + lane * 2;
+                const int n = (kh - kl + 1) * NB / 2;   // NB is even: two rows per copy
+#pragma unroll
+                for (int i = 0; i < LB * NB / 2; ++i)
+                    if (i < n) cp_async16(dst + i * 64, src + i * 64, keep);
+            }
+            cp_async_commit();
+        };
+        for (int d = 0; d < CB; ++d) issue_b(d, d);
+        bool fin = true;
+        double un[B], top[B];
+#pragma unroll
+        for (int i = 0; i < B; ++i) {
+            un[i] = top[i] = z[i];
+            fin = fin && finite(z[i]);
+        }
+        double *pu = s.x + col0 + lane + (long)KB * B * ld;
+        if (valid)
+#pragma unroll
+            for (int i = 0; i < B; ++i) pu[i * ld] = un[i];
+        for (int d = 0; d < nbk; ++d) {
+            cp_async_wait<CB - 1>();
+            __syncwarp();
+            const int kh = KB - 1 - d * LB, kl = kh - LB + 1 > 0 ? kh - LB + 1 : 0;
+            const double *g = buf + (d & (CB - 1)) * LB * NB * 32 + (kh - kl) * (NB * 32) + lane;
+            if (valid) {
+#pragma unroll(LB)
+                for (int k = kh; k >= kl; --k, g -= NB * 32) {
+                    double nu[B];
+#pragma unroll
+                    for (int i = 0; i < B; ++i) {
+                        double tv = g[(BB + i) * 32];
+#pragma unroll
+                        for (int m = 0; m < B; ++m) tv = xsub(tv, xmul(g[(i + B * m) * 32], un[m]));
+                        nu[i] = tv;
+                        fin = fin && finite(tv);
+                    }
+                    pu -= B * ld;
+#pragma unroll
+                    for (int i = 0; i < B; ++i) {
+                        un[i] = nu[i];
+                        pu[i * ld] = nu[i];
+                    }
+                }
+            }
+            __syncwarp();
+            issue_b(d & (CB - 1), d + CB);
+        }
+        cp_async_wait<0>();
+        __syncwarp();
+        if (!valid) continue;
+        if (s.ubc_ratio) {
+#pragma unroll
+            for (int i = 0; i < B; ++i) {
+                double tv = xmul(__ldg(s.ubc_ratio + i * ld + col0 + lane), top[i]);
+                if (s.ubc_add) tv = xadd(tv, __ldg(s.ubc_add + i * ld + col0 + lane));
+                fin = fin && finite(tv);
+                s.x[col0 + lane + ((long)k2 * B + i) * ld] = tv;
             }
         }
         report(status, s.status_idx, (ok ? 0u : FLAG_PIVOT) | (fin ? 0u : FLAG_NONFINITE));
@@ -2971,20 +3198,20 @@ struct TileCfg {
                            // shared memory, w3 parked in x, 2 w2 and w3 resident (k_scalar_f64_res)
 };
 // [kind index: scalar, block2, block3][precision]
-// Defaults: the fastest shapes on a B200 (autotune.py sweeps of the 2.5 deg
-// column step, 10368 x 57, and of the nested 2.5 deg + 3-nest batch): scalar
-// FP64 chunked bulk-copy ring of 2 stages x 4 levels, one warp per CTA, w2 in
-// global scratch; 2x2 and 3x3 block rings of depth 4, one warp per CTA (the
-// 3x3 ring beat the 128-thread register kernel on the nested batch with
-// 3x3 blocks, 2.14 against 2.32 ms); scalar refinement ring of 2 stages and
-// 2x2 block refinement ring of depth 4, one warp per CTA each; 3x3 block
-// refinement register kernel of 128 threads.
-const TileCfg kDefaultTile[3][2] = {{{256, 1, 2, 1, 4, 1, 0, 32, 4, 0}, {64, 1, 2, 0, 8, 1, 0, 32, 1, 0}},
-                                     {{64, 1, 4, 0, 4, 1, 0, 32, 1, 0}, {64, 1, 4, 0, 4, 1, 0, 32, 1, 0}},
-                                     {{128, 1, 4, 0, 4, 1, 0, 32, 1, 0}, {128, 1, 0, 0, 4, 4, 0, 32, 1, 0}}};
-TileCfg g_tile[3][2] = {{{256, 1, 2, 1, 4, 1, 0, 32, 4, 0}, {64, 1, 2, 0, 8, 1, 0, 32, 1, 0}},
-                        {{64, 1, 4, 0, 4, 1, 0, 32, 1, 0}, {64, 1, 4, 0, 4, 1, 0, 32, 1, 0}},
-                        {{128, 1, 4, 0, 4, 1, 0, 32, 1, 0}, {128, 1, 0, 0, 4, 4, 0, 32, 1, 0}}};
+// Defaults: the fastest shapes measured on a B200: scalar FP64 ring of 3
+// stages x 4 levels, one warp per CTA (909,356 columns x 57 levels at 10
+// warps per SM: 382 us, 2 x 4 levels 401, 4 x 4 379; 10,368 columns 19 us for
+// all three); 2x2 and 3x3 block rings of 8 levels, one warp per CTA (2x2,
+// 10,368 columns: 27.8 us, 4 levels 31.4; 3x3, 6,969 columns: 43.9 against
+// 48.1); scalar refinement ring of 2 stages and 2x2 block refinement ring of
+// depth 4, one warp per CTA each; 3x3 block refinement register kernel of 128
+// threads.
+const TileCfg kDefaultTile[3][2] = {{{256, 1, 3, 1, 4, 1, 0, 32, 4, 0}, {64, 1, 2, 0, 8, 1, 0, 32, 1, 0}},
+                                     {{64, 1, 8, 0, 4, 1, 0, 32, 1, 0}, {64, 1, 4, 0, 4, 1, 0, 32, 1, 0}},
+                                     {{128, 1, 8, 0, 4, 1, 0, 32, 1, 0}, {128, 1, 0, 0, 4, 4, 0, 32, 1, 0}}};
+TileCfg g_tile[3][2] = {{{256, 1, 3, 1, 4, 1, 0, 32, 4, 0}, {64, 1, 2, 0, 8, 1, 0, 32, 1, 0}},
+                        {{64, 1, 8, 0, 4, 1, 0, 32, 1, 0}, {64, 1, 4, 0, 4, 1, 0, 32, 1, 0}},
+                        {{128, 1, 8, 0, 4, 1, 0, 32, 1, 0}, {128, 1, 0, 0, 4, 4, 0, 32, 1, 0}}};
 int kind_index(int kind) { return kind == TG_KIND_SCALAR ? 0 : (kind == TG_KIND_BLOCK2 ? 1 : 2); }
 constexpr int kMaxDevIdx = 64;
 int g_num_sms[kMaxDevIdx] = {};
@@ -3085,10 +3312,17 @@ cudaError_t with_scalar_res(int C, int L, int w3s, F f)
 template <typename F>
 cudaError_t with_block_ring(int B, int D, int W, F f)
 {
+    // 32 columns per warp: D levels as stages of L levels (k_block_f64_chunk)
+    if (W == 32) {
+#define TG_CHUNK(b, d, c, l) \
+    if (B == b && D == d) return f(k_block_f64_chunk<b, c, l>);
+        TG_CHUNK(2, 4, 2, 2) TG_CHUNK(2, 8, 4, 2) TG_CHUNK(2, 16, 8, 2)
+        TG_CHUNK(3, 4, 4, 1) TG_CHUNK(3, 8, 4, 2) TG_CHUNK(3, 16, 8, 2)
+#undef TG_CHUNK
+    }
 #define TG_RING(b, d, w) \
     if (B == b && D == d && W == w) return f(k_block_f64_ring<b, d, w>);
-    TG_RING(2, 4, 32) TG_RING(2, 8, 32) TG_RING(2, 16, 32) TG_RING(2, 4, 16) TG_RING(2, 8, 16) TG_RING(2, 4, 8)
-    TG_RING(2, 8, 8) TG_RING(3, 4, 32) TG_RING(3, 8, 32) TG_RING(3, 16, 32) TG_RING(3, 4, 16) TG_RING(3, 8, 16)
+    TG_RING(2, 4, 16) TG_RING(2, 8, 16) TG_RING(2, 4, 8) TG_RING(2, 8, 8) TG_RING(3, 4, 16) TG_RING(3, 8, 16)
     TG_RING(3, 4, 8) TG_RING(3, 8, 8)
 #undef TG_RING
     return cudaErrorInvalidValue;
@@ -3231,17 +3465,27 @@ cudaError_t occupancy(K kernel, int threads, size_t smem, int *per_sm)
     return e;
 }
 
-// Resident threads allowed for the block kernels: their Gamma scratch (k2 *
-// B*B doubles per resident thread) of all of them within this budget.  160 MB
-// lets more columns into flight than L2 holds, and that wins: 3x3 blocks on
-// the nested batch took 2.15 ms at 96 MB and 1.72 ms at 128 and 192 MB (2x2
-// blocks are occupancy-bound from 128 MB on: 2.19 -> 2.17 ms).
-constexpr double kBlockBudgetMB = 160.0;
-double g_block_scratch_budget = kBlockBudgetMB * 1024 * 1024;
-// Scalar ring kernels: L2 bytes of w2 scratch and parked w3 of all resident
-// columns.  Past the L2's capacity the back sweep's re-reads go to DRAM.
-constexpr double kScalarBudgetMB = 128.0;
-double g_scalar_scratch_budget = kScalarBudgetMB * 1024 * 1024;
+// L2 budget of the chunk kernels' resident warps.  A warp's share is its sweep
+// scratch (k_scalar_f64_chunk: w2 and w3, 16 B per level and column;
+// k_block_f64_chunk: Gamma and z) and, for the scalar kernel, kStreamKB for
+// what it streams (rows in flight, the x rows on their way out).  Past the
+// budget the scratch spills: scalar, 909,356 columns x 57 levels, 382 us at 10
+// warps per SM, 431 at 13, 469 at 16; 290,304 x 113, 283 us at 7, 310 at 9,
+// 332 at 10.  126 MB of L2 with 56 KB a warp puts the line at 10 and 7.5.
+// Block, 2x2, 130,000 x 57: 200 us at 4 warps per SM, 208 at 5, 231 at 8, but
+// 20,000 columns (4.2 tiles per SM) 51 us at 4 and 38 at 5: 4.5, rounded.
+constexpr double kChunkBudgetMB[2] = {120.0, 57.0};   // scalar, block
+constexpr double kStreamKB = 56.0;
+// The register and narrow block kernels' Gamma, and the other scalar rings'
+// w2 and parked w3, which bound their grids more loosely: more columns in
+// flight win there (3x3 blocks on the nested batch, register kernel: 2.15 ms
+// at 96 MB and 1.72 ms at 128 and 192 MB).
+constexpr double kBlockRegBudgetMB = 160.0, kRingBudgetMB = 128.0;
+constexpr double kMB = 1024.0 * 1024.0;
+double g_scalar_scratch_budget = kChunkBudgetMB[0] * kMB, g_block_scratch_budget = kChunkBudgetMB[1] * kMB;
+bool g_scalar_budget_set = false, g_block_budget_set = false;
+double g_block_reg_budget() { return g_block_budget_set ? g_block_scratch_budget : kBlockRegBudgetMB * kMB; }
+double g_ring_budget() { return g_scalar_budget_set ? g_scalar_scratch_budget : kRingBudgetMB * kMB; }
 std::atomic<int> g_kind_overlap{-1};
 }  // namespace
 
@@ -3279,7 +3523,8 @@ void set_w2g(int kind, int precision, int on)
     t.w2g = on >= 0 ? on : kDefaultTile[kind_index(kind)][precision ? 1 : 0].w2g;
 }
 
-size_t scalar_scratch_bytes(long slots, int k2max) { return (size_t)slots * (size_t)(k2max > 1 ? k2max - 1 : 1) * 8; }
+// w2 and, in k_scalar_f64_chunk, w3 of every level
+size_t scalar_scratch_bytes(long slots, int k2max) { return (size_t)slots * (size_t)k2max * 16; }
 size_t refine_scratch_bytes(long slots, int k2max) { return (size_t)slots * 3 * (size_t)k2max * 4; }
 
 int cols_per_block(int kind, int precision) { return g_tile[kind_index(kind)][precision ? 1 : 0].cpb; }
@@ -3306,10 +3551,15 @@ void set_block_rows(int kind, int on)
     TileCfg &t = g_tile[kind_index(kind)][0];
     t.rows = on < 0 ? kDefaultTile[kind_index(kind)][0].rows : (on ? 1 : 0);
 }
-void set_block_scratch_budget(double mb) { g_block_scratch_budget = (mb > 0 ? mb : kBlockBudgetMB) * 1024 * 1024; }
+void set_block_scratch_budget(double mb)
+{
+    g_block_budget_set = mb > 0;
+    g_block_scratch_budget = (mb > 0 ? mb : kChunkBudgetMB[1]) * kMB;
+}
 void set_scalar_scratch_budget(double mb)
 {
-    g_scalar_scratch_budget = (mb > 0 ? mb : kScalarBudgetMB) * 1024 * 1024;
+    g_scalar_budget_set = mb > 0;
+    g_scalar_scratch_budget = (mb > 0 ? mb : kChunkBudgetMB[0]) * kMB;
 }
 void set_kind_overlap(int mode) { g_kind_overlap.store(mode == 0 || mode == 1 ? mode : -1); }
 int kind_overlap() { return g_kind_overlap.load(); }
@@ -3371,7 +3621,8 @@ size_t block_smem_bytes(int B, int stages, int threads, int rows, int bw, int pr
 
 size_t block_scratch_bytes(int B, int precision, long slots, int k2max)
 {
-    if (precision == TG_PREC_F64) return (size_t)slots * B * B * (size_t)k2max * 8;
+    // Gamma and, in k_block_f64_chunk, z of every level
+    if (precision == TG_PREC_F64) return (size_t)slots * (B * B + B) * (size_t)k2max * 8;
     return (size_t)slots * (2 * B * B + B) * (size_t)k2max * 4;
 }
 
@@ -3416,7 +3667,9 @@ cudaError_t plan_shape(int kind, int precision, int k2max, int ntiles, int cpb, 
         g_tile[kind_index(kind)][0].res > 0) {
         sh->res = 1;
         if (stages > 8) stages = sh->stages = 8;
-        if (with_block_ring_gsm(kind, stages, sh->bw, [](auto) { return cudaSuccess; }) != cudaSuccess) sh->res = 0;
+        auto built = [&](int d) { return with_block_ring_gsm(kind, d, sh->bw, [](auto) { return cudaSuccess; }) == cudaSuccess; };
+        if (!built(stages) && built(4)) stages = sh->stages = 4;
+        if (!built(stages)) sh->res = 0;
     }
     if (sh->rows && stages > 8) stages = sh->stages = 8;
     if (kind == TG_KIND_SCALAR && sh->cpt == 2 && sh->pf > 8) sh->pf = 8;
@@ -3495,14 +3748,35 @@ cudaError_t plan_shape(int kind, int precision, int k2max, int ntiles, int cpb, 
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     long blocks = (long)per_sm * nsm;
-    if (kind != TG_KIND_SCALAR && precision == TG_PREC_F64 && !sh->res) {
-        // keep the Gamma scratch of all resident blocks within the L2 budget
+    const long vt = sh->rows ? (long)ntiles * rows_group(kind)
+                             : (kind != TG_KIND_SCALAR ? (long)ntiles * (32 / sh->bw) : ntiles);   // warp tiles
+    const long units = stages > 0 ? (vt + sh->threads / 32 - 1) / (sh->threads / 32) : ntiles;
+    sh->one_wave = blocks >= units;
+    const bool chunk = precision == TG_PREC_F64 && stages > 0 && !sh->res &&
+                       (kind == TG_KIND_SCALAR ? sh->lps > 1 : !sh->rows && sh->bw == 32);
+    if (chunk) {
+        // k_scalar_f64_chunk, k_block_f64_chunk: the resident warps within
+        // the budget (at least three per SM), then the tiles dealt evenly over
+        // the nearest whole number of passes, so that none is nearly empty
+        const int wpb = sh->threads / 32;
+        const double per_warp = kind == TG_KIND_SCALAR ? 512.0 * k2max + kStreamKB * 1024.0
+                                                       : 32.0 * k2max * (kind * kind + kind) * 8.0;
+        const double budget = kind == TG_KIND_SCALAR ? g_scalar_scratch_budget : g_block_scratch_budget;
+        long cap = (long)(budget / (per_warp * wpb));
+        if (cap < 3L * nsm / wpb) cap = 3L * nsm / wpb;
+        if (cap < 1) cap = 1;
+        long passes = (2 * units + cap) / (2 * cap);
+        if (passes < 1) passes = 1;
+        if (passes * blocks < units) passes = (units + blocks - 1) / blocks;   // what fits on the SMs at all
+        blocks = (units + passes - 1) / passes;
+    } else if (kind != TG_KIND_SCALAR && precision == TG_PREC_F64 && !sh->res) {
+        // keep the Gamma scratch of all resident blocks within the budget
         // (a cap on the total, not per SM, so that a grid that fits in one
         // wave is not split into two).  The block refinement kernel is not
         // capped: its loads are latency-bound, and more columns in flight
         // win over the planes' L2 spill (6.2 vs 7.4 ms on the nested batch).
-        const double per_thread = (double)block_scratch_bytes(kind, precision, 1, k2max);
-        const long cap = (long)(g_block_scratch_budget / (per_thread * sh->threads));
+        const double per_thread = (double)kind * kind * k2max * 8.0;
+        const long cap = (long)(g_block_reg_budget() / (per_thread * sh->threads));
         if (blocks > cap) blocks = cap > 0 ? cap : 1;
     } else if (stages > 0 && sh->res != 2 && sh->res != 3) {
         // ring kernels: w2 scratch plus the w3 parked in x, 8 B each per level
@@ -3513,13 +3787,9 @@ cudaError_t plan_shape(int kind, int precision, int k2max, int ntiles, int cpb, 
         const double per_col = sh->res == 1 ? (double)k2max * 8.0
                                : precision == TG_PREC_F64 ? (double)(2 * k2max - 1) * 8.0
                                                           : (double)k2max * (cache_hints() >= 2 ? 52.0 : 20.0);
-        const long cap = (long)(g_scalar_scratch_budget / (per_col * sh->threads * sh->cpt));
+        const long cap = (long)(g_ring_budget() / (per_col * sh->threads * sh->cpt));
         if (blocks > cap) blocks = cap > 0 ? cap : 1;
     }
-    const long vt = sh->rows ? (long)ntiles * rows_group(kind)
-                             : (kind != TG_KIND_SCALAR ? (long)ntiles * (32 / sh->bw) : ntiles);   // warp tiles
-    const long units = stages > 0 ? (vt + sh->threads / 32 - 1) / (sh->threads / 32) : ntiles;
-    sh->one_wave = blocks >= units;
     if (blocks > units) blocks = units;
     sh->blocks = (int)(blocks > 0 ? blocks : 1);
     return cudaSuccess;
