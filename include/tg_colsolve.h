@@ -708,16 +708,16 @@ int tg_set_assembly_mode(int mode);
  * waiting on memory otherwise, 1 above.  Same results. */
 int tg_set_walk_prefetch(int levels);
 
-/* Block kinds, FP64: the budget for the Gamma scratch of all resident warps
- * of the block kernels, in MB (default 160; <= 0 restores it).  It caps
- * how many columns are in flight at once on large batches (the refinement
- * kernel is not capped). */
+/* Block kinds: the budget for the sweep scratch (FP64: Gamma and z;
+ * refinement: the FP32 planes) of all resident warps, in MB (<= 0 restores
+ * the kernels' own limits).  It caps how many columns are in flight at once
+ * on large batches. */
 int tg_set_block_scratch_budget(double megabytes);
 
-/* Scalar kind, FP64 ring kernels: the L2 budget for the w2 scratch and the
- * parked forward-sweep results (16 B per level and column) of all resident
- * columns, in MB (default 128; <= 0 restores it).  It caps how many columns
- * are in flight at once on large batches. */
+/* Scalar kind, ring kernels: the L2 budget for the sweep scratch of all
+ * resident columns and what they stream, in MB (<= 0 restores the kernels'
+ * own limits).  It caps how many columns are in flight at once on large
+ * batches. */
 int tg_set_scalar_scratch_budget(double megabytes);
 
 /* How the kinds of one plan share the GPU, read when a plan is created: 1 the

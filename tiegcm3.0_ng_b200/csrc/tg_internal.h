@@ -311,7 +311,7 @@ void set_stage_levels(int kind, int precision, int l);
 void set_column_residency(int kind, int precision, int mode);
 int column_residency();
 // L2 budget (MB) for the Gamma scratch of all resident block-kernel warps;
-// <= 0 restores the default 96 MB.
+// <= 0 restores the default.
 void set_block_scratch_budget(double mb);
 void set_scalar_scratch_budget(double mb);
 // Kinds of one plan: 1 concurrently (block kinds on a side stream), 0 one

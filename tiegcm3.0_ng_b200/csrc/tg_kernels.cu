@@ -456,6 +456,14 @@ __device__ __forceinline__ void cp_async16(double *dst, const double *src, unsig
                  "l"(pol)
                  : "memory");
 }
+// 4- or 8-byte asynchronous copy of a lane's own value with an L2 policy
+template <int N>
+__device__ __forceinline__ void cp_async_own(void *dst, const void *src, unsigned long long pol)
+{
+    asm volatile("cp.async.ca.shared.global.L2::cache_hint [%0], [%1], %2, %3;" ::"r"(smem_addr(dst)), "l"(src), "n"(N),
+                 "l"(pol)
+                 : "memory");
+}
 // ---------------------------------------------------------------------------
 // Scalar Thomas, FP64, one warp per 32-column tile, the coefficients through a
 // shared-memory ring of C stages of L levels filled by 16-byte asynchronous
@@ -1005,63 +1013,53 @@ __global__ void __launch_bounds__(256) k_scalar_refine(SegTable tab, Refine rf, 
 }
 
 // ---------------------------------------------------------------------------
-// Scalar Thomas, FP32 sweeps + FP64 refinement, coefficients staged by the
-// bulk-copy ring (one warp per 32 columns, its own ring and barriers).
+// Scalar Thomas, FP32 sweeps + FP64 refinement, one warp per 32-column tile,
+// everything a sweep reads staged through one shared-memory ring.
 //
-// Sweep 0 reads a, b, c, f rows through the ring (4L copies of 256 B per
-// stage of L levels), factors in FP32 and solves.  The FP32 factors (w2,
-// 1/w1) and the forward result y go to three float planes of a global
-// scratch slot per resident lane ([plane][level][slot], kept in L2 by
-// eviction hints), so shared memory holds only the ring.  Each correction
-// sweep streams a, b, c, f, the x rows one level above and the 1/w1 rows
-// (5L copies of 256 B and L of 128 B per stage), forms the FP64 residual,
-// eliminates with the FP32 factors and back-substitutes x += d.  Stopping
-// rule, cap, bit-exact FP64 fallback and flags as in k_scalar_refine.
-// x and 1/w1 rows written by this warp's generic stores are read back by bulk
-// copies: a proxy fence orders the two before each correction sweep.
+// Sweep 0 streams the a, b, c, f rows (16-byte asynchronous copies, stages of
+// L levels), factors in FP32 and solves.  The FP32 (w2, y) pairs and 1/w1 of
+// every level go to the warp's own scratch slice ([level][lane] pairs, then
+// [lane] reciprocals), so shared memory holds only the ring.  Each correction
+// sweep streams a, b, c, f again, with x one level above and 1/w1 (each lane
+// its own values), forms the FP64 residual, eliminates with the FP32 factors
+// and back-substitutes x += d; the back sweeps stream x and the pairs top
+// down.  Stopping rule, cap, bit-exact FP64 fallback and flags as in
+// k_scalar_refine.
+// Against the ring of bulk copies it replaced (40 copies issued a stage, back
+// sweeps reading L2 four levels ahead): 10,368 columns x 57 levels 78 -> 48
+// us, 267,708 425 -> 349, 290,304 x 113 1,114 -> 906.  Three passes over the
+// coefficients bound it (evict-first fills; keeping them in L2 measured
+// slower: 438 us at 267,708 columns).
 // Requires ld % 32 == 0 and 16-byte aligned a, b, c, f, x.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void fence_proxy_async_global()
-{
-    asm volatile("fence.proxy.async.global;" ::: "memory");
-}
 __device__ __forceinline__ void st_hint_f(float *p, float v, unsigned long long pol)
 {
     asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(p), "f"(v), "l"(pol) : "memory");
 }
+__device__ __forceinline__ void st_hint_f2(float *p, float v0, float v1, unsigned long long pol)
+{
+    asm volatile("st.global.L2::cache_hint.v2.f32 [%0], {%1, %2}, %3;" ::"l"(p), "f"(v0), "f"(v1), "l"(pol) : "memory");
+}
 
-constexpr int kRefineStageLevels = 4;   // levels per ring stage of the refinement ring
+constexpr int kRefineStageLevels = 4;      // levels per ring stage of the refinement ring
+constexpr int kRefineRowDoubles = 176;     // a level in a stage: a, b, c, f, x rows of 32 doubles, 1/w1 of 32 floats
 
 template <int C>
 __global__ void __launch_bounds__(256) k_scalar_refine_ring(SegTable tab, Refine rf, float *scratch, unsigned *status,
                                                             unsigned long long *hist)
 {
-    constexpr int L = kRefineStageLevels, NC = 4 * L, NE = 5 * L;
-    constexpr int SD = NE * 32 + L * 16;   // doubles per stage: NE double rows, L float rows
-    static_assert(NE + L <= 32, "one copy per lane");
-    __shared__ __align__(8) unsigned long long bars[8 * C];
+    constexpr int L = kRefineStageLevels, RD = kRefineRowDoubles;
+    constexpr int LB = 4, BD = 64, CB = C * L * RD / (LB * BD);   // back sweep: x and the (w2, y) pairs
     extern __shared__ __align__(128) double smem_r[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const long K = tab.k2max;
-    double *buf = smem_r + (long)warp * C * SD;
-    const long S = (long)gridDim.x * blockDim.x;            // slots: level stride of a plane
-    const long slot0 = (long)blockIdx.x * blockDim.x + warp * 32;
-    float *gw2 = scratch + slot0 + lane;                    // plane 0: w2(k)
-    float *gri = gw2 + K * S;                               // plane 1: 1/w1(k)
-    float *gy = gri + K * S;                                // plane 2: y(k)
-    const float *rirow = scratch + K * S + slot0;           // row k of plane 1 for this warp
-    unsigned long long *bar = bars + warp * C;
+    double *buf = smem_r + (long)warp * C * L * RD;
+    float *gwy = scratch + ((long)blockIdx.x * nwarps + warp) * ((long)tab.k2max * 96) + 2 * lane;   // level k at 96*k
+    float *gri = gwy - lane + 64;
     const unsigned long long pol = refine_fill_policy(tab.hints), keep = l2_policy(tab.hints, true);
-    if (lane == 0) {
-#pragma unroll 1
-        for (int i = 0; i < C; ++i) mbar_init(&bar[i], 1);
-        fence_mbar_init();
-    }
-    __syncwarp();
+    const int half = lane >> 4, c2 = (lane & 15) * 2;
     unsigned long long hl[kMaxSweepBins];
 #pragma unroll
     for (int i = 0; i < kMaxSweepBins; ++i) hl[i] = 0ull;
-    unsigned q = 0;
     for (int t = blockIdx.x * nwarps + warp; t < tab.ntiles; t += gridDim.x * nwarps) {
         const Seg s = tab.segs ? tab.segs[find_seg(tab, t)] : tab.one;
         const long col0 = (long)(t - s.tile0) * 32;
@@ -1070,112 +1068,101 @@ __global__ void __launch_bounds__(256) k_scalar_refine_ring(SegTable tab, Refine
         const bool valid = col0 + lane < s.ncol;
         double *px = s.x + col0 + lane;
         const int nch = (k2 + L - 1) / L;
-        // lanes 0..4L-1: row (level lane/4) of array lane%4; lanes 4L..5L-1:
-        // x row (lane - 4L + 1) above the chunk's first level; lanes
-        // 5L..6L-1: 1/w1 row (lane - 5L)
-        const int arr = lane & 3;
-        const double *src = lane < NC ? (arr == 0 ? s.a : arr == 1 ? s.b : arr == 2 ? s.c : s.f) + col0 +
-                                            (long)(lane >> 2) * ld
-                                      : s.x + col0 + (long)(lane - NC + 1) * ld;
-        auto issue = [&](unsigned qc, int j, bool corr) {
-            const int st = (int)(qc % C), l0 = j * L;
-            const int nl = k2 - l0 < L ? k2 - l0 : L;
-            const int nx = corr ? (k2 - 1 - l0 < L ? k2 - 1 - l0 : L) : 0;
-            if (lane == 0) mbar_expect(&bar[st], (uint32_t)(4 * nl + nx) * 256u + (corr ? (uint32_t)nl * 128u : 0u));
-            __syncwarp();
-            double *stg = buf + (long)st * SD;
-            if (lane < NC) {
-                if ((lane >> 2) < nl) bulk_load_hint(stg + lane * 32, src + (long)l0 * ld, 256u, &bar[st], pol);
-            } else if (lane < NE) {
-                if (lane - NC < nx) bulk_load_hint(stg + lane * 32, src + (long)l0 * ld, 256u, &bar[st], pol);
-            } else if (lane < NE + L) {
-                const int i = lane - NE;
-                if (corr && i < nl)
-                    bulk_load_hint(stg + NE * 32 + i * 16, rirow + (long)(l0 + i) * S, 128u, &bar[st], keep);
+        const double *c0 = (half ? s.b : s.a) + col0 + c2, *c1 = (half ? s.f : s.c) + col0 + c2;
+        // chunk j: levels j*L .. of those below k2, into stage st
+        auto issue = [&](int st, int j, bool corr) {
+            double *d = buf + st * L * RD;
+#pragma unroll
+            for (int l = 0; l < L; ++l) {
+                const int k = j * L + l;
+                if (k < k2) {
+                    cp_async16(d + l * RD + half * 32 + c2, c0 + (long)k * ld, pol);
+                    cp_async16(d + l * RD + 64 + half * 32 + c2, c1 + (long)k * ld, pol);
+                    if (corr) {
+                        if (k + 1 < k2) cp_async_own<8>(d + l * RD + 128 + lane, px + (long)(k + 1) * ld, keep);
+                        cp_async_own<4>(reinterpret_cast<float *>(d + l * RD + 160) + lane, gri + k * 96, keep);
+                    }
+                }
             }
+            cp_async_commit();
         };
-        // bounded wait for chunk j; on timeout drain the fills in flight
-        auto wait = [&](unsigned q0, int j, int n) -> bool {
-            const unsigned qc = q0 + j;
-            if (mbar_wait_warp(&bar[qc % C], (qc / C) & 1u)) return true;
-            const unsigned qe = q0 + (j + C < n ? j + C : n);
-#pragma unroll 1
-            for (unsigned r = qc; r < qe; ++r) mbar_wait_warp(&bar[r % C], (r / C) & 1u);
-            if (lane == 0) report(status, s.status_idx, FLAG_TIMEOUT);
-            return false;
+        // back stage d: levels kh - LB + 1 .. kh, kh = k2 - 2 - d*LB; every lane its own values
+        const int KB = k2 - 1, nbk = (KB + LB - 1) / LB;
+        auto issue_b = [&](int sb, int d, bool corr) {
+            const int kh = KB - 1 - d * LB;
+            double *db = buf + sb * LB * BD;
+#pragma unroll
+            for (int l = 0; l < LB; ++l)
+                if (kh - l >= 0) {
+                    if (corr) cp_async_own<8>(db + l * BD + lane, px + (long)(kh - l) * ld, keep);
+                    cp_async_own<8>(db + l * BD + 32 + lane, gwy + (kh - l) * 96, keep);
+                }
+            cp_async_commit();
         };
 
         // ---- sweep 0: FP32 factor + solve
         bool ok = true;
         float xm0 = 0.f;
         {
-            const int pre = nch < C ? nch : C;
-            for (int j = 0; j < pre; ++j) issue(q + j, j, false);
-            float w1 = 0.f, ri = 0.f, y = 0.f, cprev = 0.f;
+#pragma unroll 1
+            for (int j = 0; j < C; ++j) issue(j, j, false);
+            float w2 = 0.f, y = 0.f;
+            int st = 0;
+#pragma unroll 1
             for (int j = 0; j < nch; ++j) {
-                if (!wait(q, j, nch)) return;
-                const double *stg = buf + (long)((q + j) % C) * SD + lane;
-                auto step0 = [&](int l, int k, bool first) {
-                    const float af = (float)stg[(4 * l) * 32], bf = (float)stg[(4 * l + 1) * 32],
-                                ff = (float)stg[(4 * l + 3) * 32];
-                    if (first) {
-                        w1 = bf;
-                        ri = __frcp_rn(w1);
-                        y = ff * ri;
-                    } else {
-                        const float w2 = cprev * ri;
-                        st_hint_f(&gw2[(k - 1) * S], w2, keep);
-                        w1 = bf - af * w2;
-                        ri = __frcp_rn(w1);
-                        y = (ff - af * y) * ri;
-                    }
+                cp_async_wait<C - 1>();
+                __syncwarp();
+                double *stg = buf + st * L * RD + lane;
+                if (j == 0) stg[0] = 0.0;   // row 0 has no a: x - 0*0 = x
+                auto step0 = [&](int l, int k) {
+                    const float af = (float)stg[l * RD], bf = (float)stg[l * RD + 32], cf = (float)stg[l * RD + 64],
+                                ff = (float)stg[l * RD + 96];
+                    const float w1 = bf - af * w2;
+                    const float ri = __frcp_rn(w1);
+                    y = (ff - af * y) * ri;
+                    w2 = cf * ri;
                     ok = ok && (fabsf(w1) <= FLT_MAX) && (w1 != 0.f);
-                    st_hint_f(&gri[k * S], ri, keep);
-                    st_hint_f(&gy[k * S], y, keep);
-                    cprev = (float)stg[(4 * l + 2) * 32];
+                    st_hint_f2(gwy + k * 96, w2, y, keep);
+                    st_hint_f(gri + k * 96, ri, keep);
                 };
                 if (valid) {
-                    if (j > 0 && (j + 1) * L <= k2) {   // a full chunk past level 0: no per-level tests
+                    if ((j + 1) * L <= k2) {
 #pragma unroll
-                        for (int l = 0; l < L; ++l) step0(l, j * L + l, false);
+                        for (int l = 0; l < L; ++l) step0(l, j * L + l);
                     } else {
-#pragma unroll
-                        for (int l = 0; l < L; ++l)
-                            if (j * L + l < k2) step0(l, j * L + l, j * L + l == 0);
+                        for (int l = 0; j * L + l < k2; ++l) step0(l, j * L + l);
                     }
                 }
                 __syncwarp();
-                fence_proxy_async();
-                if (j + C < nch) issue(q + j + C, j + C, false);
+                issue(st, j + C, false);
+                st = st + 1 == C ? 0 : st + 1;
             }
-            q += nch;
-            if (valid) {
-                // back substitution; y and w2 re-read 4 levels ahead
-                float xk = y;
-                xm0 = fabsf(y);
-                px[(k2 - 1) * ld] = (double)xk;
-                float ry[4], rw[4];
+            // back substitution
+            cp_async_wait<0>();
+            __syncwarp();
+#pragma unroll 1
+            for (int d = 0; d < CB; ++d) issue_b(d, d, false);
+            float xk = y;
+            xm0 = fabsf(y);
+            if (valid) st_hint(&px[(long)KB * ld], (double)xk, keep);
+            int sb = 0;
+#pragma unroll 1
+            for (int d = 0; d < nbk; ++d) {
+                cp_async_wait<CB - 1>();
+                const double *g = buf + sb * LB * BD;
+                const int kh = KB - 1 - d * LB;
+                if (valid) {
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (k2 - 2 - u >= 0) {
-                        ry[u] = gy[(k2 - 2 - u) * S];
-                        rw[u] = gw2[(k2 - 2 - u) * S];
-                    }
-                for (int kb = k2 - 2; kb >= 0; kb -= 4) {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int k = kb - u;
-                        if (k >= 0) {
-                            xk = ry[u] - rw[u] * xk;
-                            if (k - 4 >= 0) {
-                                ry[u] = gy[(k - 4) * S];
-                                rw[u] = gw2[(k - 4) * S];
-                            }
+                    for (int l = 0; l < LB; ++l)
+                        if (kh - l >= 0) {
+                            const float2 w = reinterpret_cast<const float2 *>(g + l * BD + 32)[lane];
+                            xk = w.y - w.x * xk;
                             xm0 = fmaxf(xm0, fabsf(xk));
-                            st_hint(&px[k * ld], (double)xk, keep);
+                            st_hint(&px[(long)(kh - l) * ld], (double)xk, keep);
                         }
-                    }
                 }
+                issue_b(sb, d + CB, false);
+                sb = sb + 1 == CB ? 0 : sb + 1;
             }
         }
 
@@ -1184,27 +1171,30 @@ __global__ void __launch_bounds__(256) k_scalar_refine_ring(SegTable tab, Refine
         int sw = 0, taken = rf.max_sweeps + 1;   // sweep of convergence, else cap + 1
         double dprev = (double)xm0;
         for (sw = 1; sw <= rf.max_sweeps && __any_sync(0xffffffffu, active); ++sw) {
-            fence_proxy_async_global();
+            cp_async_wait<0>();
             __syncwarp();
-            const int pre = nch < C ? nch : C;
-            for (int j = 0; j < pre; ++j) issue(q + j, j, true);
+#pragma unroll 1
+            for (int j = 0; j < C; ++j) issue(j, j, true);
             double xm1 = 0.0, x0 = active ? px[0] : 0.0;
             float y = 0.f;
+            int st = 0;
+#pragma unroll 1
             for (int j = 0; j < nch; ++j) {
-                if (!wait(q, j, nch)) return;
-                const double *stg = buf + (long)((q + j) % C) * SD + lane;
-                const float *stf = reinterpret_cast<const float *>(buf + (long)((q + j) % C) * SD + NE * 32) + lane;
+                cp_async_wait<C - 1>();
+                __syncwarp();
+                const double *stg = buf + st * L * RD + lane;
                 // level k from stage row l; `first` for level 0, `last` for k2-1
                 auto step = [&](int l, int k, bool first, bool last) {
-                    const double xp1 = last ? 0.0 : stg[(NC + l) * 32];
+                    const double xp1 = last ? 0.0 : stg[l * RD + 128];
                     if (active) {
-                        const double ak = stg[(4 * l) * 32];
-                        double r = fma(-stg[(4 * l + 1) * 32], x0, stg[(4 * l + 3) * 32]);
+                        const double ak = stg[l * RD];
+                        double r = fma(-stg[l * RD + 32], x0, stg[l * RD + 96]);
                         if (!first) r = fma(-ak, xm1, r);
-                        if (!last) r = fma(-stg[(4 * l + 2) * 32], xp1, r);
-                        const float rr = (float)r, rik = stf[l * 32];
+                        if (!last) r = fma(-stg[l * RD + 64], xp1, r);
+                        const float rr = (float)r;
+                        const float rik = reinterpret_cast<const float *>(buf + (st * L + l) * RD + 160)[lane];
                         y = first ? rr * rik : (rr - (float)ak * y) * rik;
-                        st_hint_f(&gy[k * S], y, keep);
+                        st_hint_f(gwy + k * 96 + 1, y, keep);
                     }
                     xm1 = x0;
                     x0 = xp1;
@@ -1220,44 +1210,40 @@ __global__ void __launch_bounds__(256) k_scalar_refine_ring(SegTable tab, Refine
                     }
                 }
                 __syncwarp();
-                fence_proxy_async();
-                if (j + C < nch) issue(q + j + C, j + C, true);
+                issue(st, j + C, true);
+                st = st + 1 == C ? 0 : st + 1;
             }
-            q += nch;
-            if (active) {
-                // back substitution, x += d; x(k2-1) is in xm1; x, y and w2
-                // of lower levels re-read 4 levels ahead
-                float d = y;
-                double xv = xm1 + (double)d;
-                st_hint(&px[(k2 - 1) * ld], xv, keep);
-                double dmax = fabs((double)d), xmax = fabs(xv);
-                double rx[4];
-                float ry[4], rw[4];
+            // back substitution, x += d; x(k2-1) is in xm1
+            cp_async_wait<0>();
+            __syncwarp();
+#pragma unroll 1
+            for (int d = 0; d < CB; ++d) issue_b(d, d, true);
+            float dk = y;
+            double xv = xm1 + (double)dk;
+            if (active) st_hint(&px[(long)KB * ld], xv, keep);
+            double dmax = fabs((double)dk), xmax = fabs(xv);
+            int sb = 0;
+#pragma unroll 1
+            for (int d = 0; d < nbk; ++d) {
+                cp_async_wait<CB - 1>();
+                const double *g = buf + sb * LB * BD;
+                const int kh = KB - 1 - d * LB;
+                if (active) {
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (k2 - 2 - u >= 0) {
-                        rx[u] = px[(k2 - 2 - u) * ld];
-                        ry[u] = gy[(k2 - 2 - u) * S];
-                        rw[u] = gw2[(k2 - 2 - u) * S];
-                    }
-                for (int kb = k2 - 2; kb >= 0; kb -= 4) {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int k = kb - u;
-                        if (k >= 0) {
-                            d = ry[u] - rw[u] * d;
-                            xv = rx[u] + (double)d;
-                            if (k - 4 >= 0) {
-                                rx[u] = px[(k - 4) * ld];
-                                ry[u] = gy[(k - 4) * S];
-                                rw[u] = gw2[(k - 4) * S];
-                            }
-                            st_hint(&px[k * ld], xv, keep);
-                            dmax = fmax(dmax, fabs((double)d));
+                    for (int l = 0; l < LB; ++l)
+                        if (kh - l >= 0) {
+                            const float2 w = reinterpret_cast<const float2 *>(g + l * BD + 32)[lane];
+                            dk = w.y - w.x * dk;
+                            xv = g[l * BD + lane] + (double)dk;
+                            st_hint(&px[(long)(kh - l) * ld], xv, keep);
+                            dmax = fmax(dmax, fabs((double)dk));
                             xmax = fmax(xmax, fabs(xv));
                         }
-                    }
                 }
+                issue_b(sb, d + CB, true);
+                sb = sb + 1 == CB ? 0 : sb + 1;
+            }
+            if (active) {
                 if (!(xmax <= DBL_MAX) || !(dmax <= DBL_MAX)) {
                     active = false;
                 } else if (refine_done(dmax, xmax, dprev, rf.rel_tol, sw == 1)) {
@@ -1269,10 +1255,11 @@ __global__ void __launch_bounds__(256) k_scalar_refine_ring(SegTable tab, Refine
                 }
             }
         }
+        cp_async_wait<0>();
+        __syncwarp();
         unsigned flags = 0u;
         if (valid && !conv) {
-            // ---- fallback: bit-exact FP64 re-solve; w2 as two 32-bit halves
-            // in this lane's w2 and 1/w1 plane slots, w3 parked in x
+            // ---- fallback: bit-exact FP64 re-solve; w2 in this lane's pair slots, w3 parked in x
             const double *pa = s.a + col0 + lane, *pb = s.b + col0 + lane, *pc = s.c + col0 + lane,
                          *pf = s.f + col0 + lane;
             bool okd = true, fin = true;
@@ -1283,8 +1270,8 @@ __global__ void __launch_bounds__(256) k_scalar_refine_ring(SegTable tab, Refine
             for (int k = 1; k < k2; ++k) {
                 const double ak = pa[k * ld], bk = pb[k * ld], fk = pf[k * ld];
                 const double w2 = xdiv(cprev, w1);
-                gw2[(k - 1) * S] = __int_as_float(__double2hiint(w2));
-                gri[(k - 1) * S] = __int_as_float(__double2loint(w2));
+                gwy[(k - 1) * 96] = __int_as_float(__double2hiint(w2));
+                gwy[(k - 1) * 96 + 1] = __int_as_float(__double2loint(w2));
                 w1 = xsub(bk, xmul(ak, w2));
                 w3 = xdiv(xsub(fk, xmul(ak, w3)), w1);
                 okd = okd && finite_nz(w1);
@@ -1294,7 +1281,7 @@ __global__ void __launch_bounds__(256) k_scalar_refine_ring(SegTable tab, Refine
             double xn = w3;
             fin = finite(xn);
             for (int k = k2 - 2; k >= 0; --k) {
-                const double w2 = __hiloint2double(__float_as_int(gw2[k * S]), __float_as_int(gri[k * S]));
+                const double w2 = __hiloint2double(__float_as_int(gwy[k * 96]), __float_as_int(gwy[k * 96 + 1]));
                 xn = xsub(px[k * ld], xmul(w2, xn));
                 fin = fin && finite(xn);
                 px[k * ld] = xn;
@@ -2653,113 +2640,124 @@ __device__ __forceinline__ unsigned blk_refine_col(const Seg &s, long col, float
 }
 
 // ---------------------------------------------------------------------------
-// Block-tridiagonal FP32 sweeps + FP64 refinement with the coefficients
-// staged by the bulk-copy ring: one warp per 32 columns, a D-level ring of
-// the 3*B*B + B coefficient rows per level (and, in the correction sweeps,
-// the B rows of u one level above), one 256-byte copy per row.  Same
-// arithmetic, planes, stopping rule, fallback and flags as blk_refine_col;
-// the FP32 planes W | G | z of level k sit at (k*NS + e)*gs of the lane's
-// scratch slot.  u rows written by this warp's generic stores are read back
-// by bulk copies: a proxy fence orders the two before each correction sweep.
+// 2x2 block-tridiagonal FP32 sweeps + FP64 refinement, one warp per 32-column
+// tile, everything a sweep reads staged through one shared-memory ring of D
+// levels: the 14 coefficient rows (16-byte asynchronous copies, two rows per
+// instruction) and, in the correction sweeps, u one level above and the FP32
+// inverse W (each lane its own values); the back sweeps stream u, Gamma and z
+// top down.  The FP32 planes of a level lie in the warp's own scratch slice as
+// [lane] W (4), [lane] Gamma (4), [lane] z (2).  Same arithmetic, stopping
+// rule, fallback and flags as blk_refine_col.  Against the ring of
+// bulk copies with back sweeps straight from L2 it replaced: 10,368 columns x
+// 57 levels 172 -> 71 us, 38,244 275 -> 134, 41,472 x 113 564 -> 295.
 // Requires ld % 32 == 0 and 16-byte aligned P, Q, R, f, u.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void st_hint_f4(float *p, float4 v, unsigned long long pol)
+{
+    asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z),
+                 "f"(v.w), "l"(pol)
+                 : "memory");
+}
+constexpr int kBlkRefineRowDoubles = 18 * 32;   // a level in the ring: P, Q, R, f, u and W
+
 template <int B, int D>
 __global__ void __launch_bounds__(256) k_block_refine_ring(SegTable tab, Refine rf, float *scratch, unsigned *status,
                                                            unsigned long long *hist)
 {
-    constexpr int BB = B * B, NE = 3 * BB + B, NX = NE + B, NS = 2 * BB + B;
-    static_assert(NX <= 32, "one copy per lane");
-    __shared__ __align__(8) unsigned long long bars[8 * D];
+    static_assert(B == 2, "2x2 blocks");
+    constexpr int BB = B * B, NE = 3 * BB + B, RD = kBlkRefineRowDoubles, NS = 10 * 32;
+    constexpr int BD = 160, LB = 2, CB = D * RD / (LB * BD);   // back sweep: u, Gamma and z
     extern __shared__ __align__(128) double smem_b[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    double *buf = smem_b + (long)warp * D * NX * 32;
-    unsigned long long *bar = bars + warp * D;
+    double *buf = smem_b + (long)warp * D * RD;
     const unsigned long long pol = refine_fill_policy(tab.hints), keep = l2_policy(tab.hints, true);
-    const long gs = (long)gridDim.x * blockDim.x;
-    float *scr = scratch + (long)blockIdx.x * blockDim.x + threadIdx.x;
-    auto S = [&](int k, int e) -> float & { return scr[((long)k * NS + e) * gs]; };
-    if (lane == 0) {
-#pragma unroll 1
-        for (int i = 0; i < D; ++i) mbar_init(&bar[i], 1);
-        fence_mbar_init();
-    }
-    __syncwarp();
+    float *gw = scratch + ((long)blockIdx.x * nwarps + warp) * ((long)tab.k2max * NS) + 4 * lane;   // level k at NS*k
+    float *gg = gw + 128, *gz = gw - 2 * lane + 256;
+    // the fallback's Gamma halves: element e of level k
+    auto S = [&](int k, int e) -> float & { return gw[(long)k * NS + (e >> 2) * 128 + (e & 3)]; };
+    const int half = lane >> 4, c2 = (lane & 15) * 2;
     unsigned long long hl[kMaxSweepBins];
 #pragma unroll
     for (int i = 0; i < kMaxSweepBins; ++i) hl[i] = 0ull;
-    unsigned q = 0;
     for (int t = blockIdx.x * nwarps + warp; t < tab.ntiles; t += gridDim.x * nwarps) {
         const Seg s = tab.segs ? tab.segs[find_seg(tab, t)] : tab.one;
         const long col0 = (long)(t - s.tile0) * 32;
         const long ld = s.ld;
         const int k2 = s.k2;
         const bool valid = col0 + lane < s.ncol;
-        // row e of level k: P/Q/R element e at (k*BB + e)*ld, f and u
-        // component i at (k*B + i)*ld; lanes NE.. copy u of level k+1
-        const double *src = s.a + col0;
-        long lstride = 0;
-        if (lane < BB) {
-            src = s.a + col0 + lane * ld;
-            lstride = BB * ld;
-        } else if (lane < 2 * BB) {
-            src = s.b + col0 + (lane - BB) * ld;
-            lstride = BB * ld;
-        } else if (lane < 3 * BB) {
-            src = s.c + col0 + (lane - 2 * BB) * ld;
-            lstride = BB * ld;
-        } else if (lane < NE) {
-            src = s.f + col0 + (lane - 3 * BB) * ld;
-            lstride = B * ld;
-        } else if (lane < NX) {
-            src = s.x + col0 + (lane - NE + B) * ld;
-            lstride = B * ld;
-        }
         double *pU = s.x + col0 + lane;
-        auto issue = [&](unsigned qk, int k, bool withu) {
-            const int st = (int)(qk % D);
-            const bool u = withu && k + 1 < k2;
-            if (lane == 0) mbar_expect(&bar[st], (uint32_t)(NE + (u ? B : 0)) * 256u);
-            __syncwarp();
-            if (lane < NE || (u && lane < NX))
-                bulk_load_hint(buf + (st * NX + lane) * 32, src + (long)k * lstride, 256u, &bar[st], pol);
+        const long o0 = col0 + c2 + half * ld;
+        // level k into stage st
+        auto issue = [&](int st, int k, bool corr) {
+            if (k < k2) {
+                double *d = buf + st * RD + half * 32 + c2;
+                const long om = (long)k * BB * ld + o0;
+#pragma unroll
+                for (int e = 0; e < BB; e += 2) {
+                    cp_async16(d + e * 32, s.a + om + e * ld, pol);
+                    cp_async16(d + (BB + e) * 32, s.b + om + e * ld, pol);
+                    cp_async16(d + (2 * BB + e) * 32, s.c + om + e * ld, pol);
+                }
+                cp_async16(d + 3 * BB * 32, s.f + (long)k * B * ld + o0, pol);
+                if (corr) {
+                    double *u = buf + st * RD + NE * 32;
+                    if (k + 1 < k2)
+#pragma unroll
+                        for (int i = 0; i < B; ++i)
+                            cp_async_own<8>(u + i * 32 + lane, pU + ((long)(k + 1) * B + i) * ld, keep);
+                    cp_async16(u + 64 + lane * 2, reinterpret_cast<const double *>(gw + (long)k * NS), keep);
+                }
+            }
+            cp_async_commit();
         };
-        auto wait = [&](unsigned q0, int k) -> bool {
-            const unsigned qk = q0 + k;
-            if (mbar_wait_warp(&bar[qk % D], (qk / D) & 1u)) return true;
-            const unsigned qe = q0 + (k + D < k2 ? k + D : k2);
-#pragma unroll 1
-            for (unsigned r = qk; r < qe; ++r) mbar_wait_warp(&bar[r % D], (r / D) & 1u);
-            if (lane == 0) report(status, s.status_idx, FLAG_TIMEOUT);
-            return false;
+        // back stage d: levels kh - LB + 1 .. kh, kh = k2 - 2 - d*LB
+        const int KB = k2 - 1, nbk = (KB + LB - 1) / LB;
+        auto issue_b = [&](int sb, int d, bool corr) {
+            const int kh = KB - 1 - d * LB;
+            double *db = buf + sb * LB * BD;
+#pragma unroll
+            for (int l = 0; l < LB; ++l)
+                if (kh - l >= 0) {
+                    const int k = kh - l;
+                    if (corr)
+#pragma unroll
+                        for (int i = 0; i < B; ++i)
+                            cp_async_own<8>(db + l * BD + i * 32 + lane, pU + ((long)k * B + i) * ld, keep);
+                    cp_async16(db + l * BD + 64 + lane * 2, reinterpret_cast<const double *>(gg + (long)k * NS), keep);
+                    cp_async_own<8>(db + l * BD + 128 + lane, gz + (long)k * NS, keep);
+                }
+            cp_async_commit();
         };
-        auto at = [&](unsigned qk, int e) { return buf[((int)(qk % D) * NX + e) * 32 + lane]; };
 
         // ---- sweep 0: FP64 pivots and inverses, FP32 planes and sweeps
         bool ok = true;
         float xm = 0.f;
         {
-            const int pre = k2 < D ? k2 : D;
-            for (int j = 0; j < pre; ++j) issue(q + j, j, false);
+#pragma unroll 1
+            for (int j = 0; j < D; ++j) issue(j, j, false);
             float G[BB], z[B];
 #pragma unroll
             for (int e = 0; e < BB; ++e) G[e] = 0.f;
 #pragma unroll
             for (int i = 0; i < B; ++i) z[i] = 0.f;
+            int st = 0;
+#pragma unroll 1
             for (int k = 0; k < k2; ++k) {
-                const unsigned qk = q + k;
-                if (!wait(q, k)) return;
+                cp_async_wait<D - 1>();
+                __syncwarp();
                 double P[BB], Q[BB], R[BB], F[B];
+                const double *r = buf + st * RD + lane;
 #pragma unroll
                 for (int e = 0; e < BB; ++e) {
-                    P[e] = k > 0 ? at(qk, e) : 0.0;
-                    Q[e] = at(qk, BB + e);
-                    R[e] = k < k2 - 1 ? at(qk, 2 * BB + e) : 0.0;
+                    P[e] = k > 0 ? r[e * 32] : 0.0;
+                    Q[e] = r[(BB + e) * 32];
+                    R[e] = k < k2 - 1 ? r[(2 * BB + e) * 32] : 0.0;
                 }
 #pragma unroll
-                for (int i = 0; i < B; ++i) F[i] = at(qk, 3 * BB + i);
+                for (int i = 0; i < B; ++i) F[i] = r[(3 * BB + i) * 32];
                 __syncwarp();
-                fence_proxy_async();
-                if (k + D < k2) issue(qk + D, k + D, false);
+                issue(st, k + D, false);
+                st = st + 1 == D ? 0 : st + 1;
                 if (!valid) continue;
                 double Qp[BB], W[BB];
 #pragma unroll
@@ -2775,10 +2773,8 @@ __global__ void __launch_bounds__(256) k_block_refine_ring(SegTable tab, Refine 
                 ok = inv_exact<B>(Qp, W) && ok;
                 float W32[BB], v[B];
 #pragma unroll
-                for (int e = 0; e < BB; ++e) {
-                    W32[e] = (float)W[e];
-                    st_hint_f(&S(k, e), W32[e], keep);
-                }
+                for (int e = 0; e < BB; ++e) W32[e] = (float)W[e];
+                st_hint_f4(gw + (long)k * NS, make_float4(W32[0], W32[1], W32[2], W32[3]), keep);
 #pragma unroll
                 for (int i = 0; i < B; ++i) {
                     float tv = (float)F[i];
@@ -2793,7 +2789,6 @@ __global__ void __launch_bounds__(256) k_block_refine_ring(SegTable tab, Refine 
 #pragma unroll
                     for (int m = 0; m < B; ++m) tv = fmaf(W32[i + B * m], v[m], tv);
                     z[i] = tv;
-                    st_hint_f(&S(k, 2 * BB + i), tv, keep);
                 }
 #pragma unroll
                 for (int m = 0; m < B; ++m)
@@ -2804,34 +2799,46 @@ __global__ void __launch_bounds__(256) k_block_refine_ring(SegTable tab, Refine 
 #pragma unroll
                             for (int n = 0; n < B; ++n) g = fmaf(W32[i + B * n], (float)R[n + B * m], g);
                         G[i + B * m] = g;
-                        st_hint_f(&S(k, BB + i + B * m), g, keep);
                     }
+                st_hint_f4(gg + (long)k * NS, make_float4(G[0], G[1], G[2], G[3]), keep);
+                st_hint_f2(gz + (long)k * NS, z[0], z[1], keep);
             }
-            q += k2;
-            if (valid) {
-                float un[B];
+            cp_async_wait<0>();
+            __syncwarp();
+#pragma unroll 1
+            for (int d = 0; d < CB; ++d) issue_b(d, d, false);
+            float un[B];
 #pragma unroll
-                for (int i = 0; i < B; ++i) {
-                    un[i] = z[i];
-                    xm = fmaxf(xm, fabsf(z[i]));
-                    st_hint(&pU[((long)(k2 - 1) * B + i) * ld], (double)z[i], keep);
+            for (int i = 0; i < B; ++i) {
+                un[i] = z[i];
+                xm = fmaxf(xm, fabsf(z[i]));
+                if (valid) st_hint(&pU[((long)KB * B + i) * ld], (double)z[i], keep);
+            }
+            int sb = 0;
+#pragma unroll 1
+            for (int d = 0; d < nbk; ++d) {
+                cp_async_wait<CB - 1>();
+                const double *g = buf + sb * LB * BD;
+                const int kh = KB - 1 - d * LB;
+                if (valid) {
+#pragma unroll
+                    for (int l = 0; l < LB; ++l)
+                        if (kh - l >= 0) {
+                            const float4 gv = reinterpret_cast<const float4 *>(g + l * BD + 64)[lane];
+                            const float2 zv = reinterpret_cast<const float2 *>(g + l * BD + 128)[lane];
+                            const float nu0 = fmaf(-gv.z, un[1], fmaf(-gv.x, un[0], zv.x));
+                            const float nu1 = fmaf(-gv.w, un[1], fmaf(-gv.y, un[0], zv.y));
+                            un[0] = nu0;
+                            un[1] = nu1;
+#pragma unroll
+                            for (int i = 0; i < B; ++i) {
+                                xm = fmaxf(xm, fabsf(un[i]));
+                                st_hint(&pU[((long)(kh - l) * B + i) * ld], (double)un[i], keep);
+                            }
+                        }
                 }
-                for (int k = k2 - 2; k >= 0; --k) {
-                    float nu[B];
-#pragma unroll
-                    for (int i = 0; i < B; ++i) {
-                        float tv = S(k, 2 * BB + i);
-#pragma unroll
-                        for (int m = 0; m < B; ++m) tv = fmaf(-S(k, BB + i + B * m), un[m], tv);
-                        nu[i] = tv;
-                    }
-#pragma unroll
-                    for (int i = 0; i < B; ++i) {
-                        un[i] = nu[i];
-                        xm = fmaxf(xm, fabsf(nu[i]));
-                        st_hint(&pU[((long)k * B + i) * ld], (double)nu[i], keep);
-                    }
-                }
+                issue_b(sb, d + CB, false);
+                sb = sb + 1 == CB ? 0 : sb + 1;
             }
         }
 
@@ -2840,10 +2847,10 @@ __global__ void __launch_bounds__(256) k_block_refine_ring(SegTable tab, Refine 
         int sw = 0, taken = rf.max_sweeps + 1;
         double dprev = (double)xm;
         for (sw = 1; sw <= rf.max_sweeps && __any_sync(0xffffffffu, active); ++sw) {
-            fence_proxy_async_global();
+            cp_async_wait<0>();
             __syncwarp();
-            const int pre = k2 < D ? k2 : D;
-            for (int j = 0; j < pre; ++j) issue(q + j, j, true);
+#pragma unroll 1
+            for (int j = 0; j < D; ++j) issue(j, j, true);
             double um[B], u0[B];
             float zc[B];
 #pragma unroll
@@ -2852,31 +2859,35 @@ __global__ void __launch_bounds__(256) k_block_refine_ring(SegTable tab, Refine 
                 u0[i] = active ? pU[i * ld] : 0.0;
                 zc[i] = 0.f;
             }
+            int st = 0;
+#pragma unroll 1
             for (int k = 0; k < k2; ++k) {
-                const unsigned qk = q + k;
-                if (!wait(q, k)) return;
+                cp_async_wait<D - 1>();
+                __syncwarp();
+                const double *rw = buf + st * RD + lane;
                 double up[B], r[B];
 #pragma unroll
                 for (int i = 0; i < B; ++i) {
-                    up[i] = k + 1 < k2 ? at(qk, NE + i) : 0.0;
-                    r[i] = at(qk, 3 * BB + i);
+                    up[i] = k + 1 < k2 ? rw[(NE + i) * 32] : 0.0;
+                    r[i] = rw[(3 * BB + i) * 32];
                 }
                 float P32[BB];
 #pragma unroll
                 for (int e = 0; e < BB; ++e) {
                     const int i = e % B, m = e / B;
-                    r[i] = fma(-at(qk, BB + e), u0[m], r[i]);
+                    r[i] = fma(-rw[(BB + e) * 32], u0[m], r[i]);
                     double p = 0.0;
                     if (k > 0) {
-                        p = at(qk, e);
+                        p = rw[e * 32];
                         r[i] = fma(-p, um[m], r[i]);
                     }
                     P32[e] = (float)p;
-                    if (k + 1 < k2) r[i] = fma(-at(qk, 2 * BB + e), up[m], r[i]);
+                    if (k + 1 < k2) r[i] = fma(-rw[(2 * BB + e) * 32], up[m], r[i]);
                 }
+                const float4 wv = reinterpret_cast<const float4 *>(buf + st * RD + (NE + B) * 32)[lane];
                 __syncwarp();
-                fence_proxy_async();
-                if (k + D < k2) issue(qk + D, k + D, true);
+                issue(st, k + D, true);
+                st = st + 1 == D ? 0 : st + 1;
                 if (active) {
                     float v[B];
 #pragma unroll
@@ -2886,14 +2897,15 @@ __global__ void __launch_bounds__(256) k_block_refine_ring(SegTable tab, Refine 
                         for (int m = 0; m < B; ++m) tv = fmaf(-P32[i + B * m], zc[m], tv);
                         v[i] = tv;
                     }
+                    const float W32[BB] = {wv.x, wv.y, wv.z, wv.w};
 #pragma unroll
                     for (int i = 0; i < B; ++i) {
                         float tv = 0.f;
 #pragma unroll
-                        for (int m = 0; m < B; ++m) tv = fmaf(S(k, i + B * m), v[m], tv);
+                        for (int m = 0; m < B; ++m) tv = fmaf(W32[i + B * m], v[m], tv);
                         zc[i] = tv;
-                        st_hint_f(&S(k, 2 * BB + i), tv, keep);
                     }
+                    st_hint_f2(gz + (long)k * NS, zc[0], zc[1], keep);
                 }
 #pragma unroll
                 for (int i = 0; i < B; ++i) {
@@ -2901,37 +2913,49 @@ __global__ void __launch_bounds__(256) k_block_refine_ring(SegTable tab, Refine 
                     u0[i] = up[i];
                 }
             }
-            q += k2;
+            cp_async_wait<0>();
+            __syncwarp();
+#pragma unroll 1
+            for (int d = 0; d < CB; ++d) issue_b(d, d, true);
+            double dmax = 0.0, xmax = 0.0;
+            float dn[B];
+#pragma unroll
+            for (int i = 0; i < B; ++i) {
+                dn[i] = zc[i];
+                const double xv = um[i] + (double)dn[i];   // um holds u(k2-1)
+                if (active) st_hint(&pU[((long)KB * B + i) * ld], xv, keep);
+                dmax = fmax(dmax, fabs((double)dn[i]));
+                xmax = fmax(xmax, fabs(xv));
+            }
+            int sb = 0;
+#pragma unroll 1
+            for (int d = 0; d < nbk; ++d) {
+                cp_async_wait<CB - 1>();
+                const double *g = buf + sb * LB * BD;
+                const int kh = KB - 1 - d * LB;
+                if (active) {
+#pragma unroll
+                    for (int l = 0; l < LB; ++l)
+                        if (kh - l >= 0) {
+                            const float4 gv = reinterpret_cast<const float4 *>(g + l * BD + 64)[lane];
+                            const float2 zv = reinterpret_cast<const float2 *>(g + l * BD + 128)[lane];
+                            const float nd0 = fmaf(-gv.z, dn[1], fmaf(-gv.x, dn[0], zv.x));
+                            const float nd1 = fmaf(-gv.w, dn[1], fmaf(-gv.y, dn[0], zv.y));
+                            dn[0] = nd0;
+                            dn[1] = nd1;
+#pragma unroll
+                            for (int i = 0; i < B; ++i) {
+                                const double xv = g[l * BD + i * 32 + lane] + (double)dn[i];
+                                st_hint(&pU[((long)(kh - l) * B + i) * ld], xv, keep);
+                                dmax = fmax(dmax, fabs((double)dn[i]));
+                                xmax = fmax(xmax, fabs(xv));
+                            }
+                        }
+                }
+                issue_b(sb, d + CB, true);
+                sb = sb + 1 == CB ? 0 : sb + 1;
+            }
             if (active) {
-                double dmax = 0.0, xmax = 0.0;
-                float dn[B];
-#pragma unroll
-                for (int i = 0; i < B; ++i) {
-                    dn[i] = zc[i];
-                    const double xv = um[i] + (double)dn[i];   // um holds u(k2-1)
-                    st_hint(&pU[((long)(k2 - 1) * B + i) * ld], xv, keep);
-                    dmax = fmax(dmax, fabs((double)dn[i]));
-                    xmax = fmax(xmax, fabs(xv));
-                }
-                for (int k = k2 - 2; k >= 0; --k) {
-                    float nd[B];
-#pragma unroll
-                    for (int i = 0; i < B; ++i) {
-                        float tv = S(k, 2 * BB + i);
-#pragma unroll
-                        for (int m = 0; m < B; ++m) tv = fmaf(-S(k, BB + i + B * m), dn[m], tv);
-                        nd[i] = tv;
-                    }
-#pragma unroll
-                    for (int i = 0; i < B; ++i) {
-                        dn[i] = nd[i];
-                        double *p = pU + ((long)k * B + i) * ld;
-                        const double xv = *p + (double)nd[i];
-                        st_hint(p, xv, keep);
-                        dmax = fmax(dmax, fabs((double)nd[i]));
-                        xmax = fmax(xmax, fabs(xv));
-                    }
-                }
                 if (!(xmax <= DBL_MAX) || !(dmax <= DBL_MAX)) {
                     active = false;
                 } else if (refine_done(dmax, xmax, dprev, rf.rel_tol, sw == 1)) {
@@ -2943,6 +2967,8 @@ __global__ void __launch_bounds__(256) k_block_refine_ring(SegTable tab, Refine 
                 }
             }
         }
+        cp_async_wait<0>();
+        __syncwarp();
         unsigned flags = 0u;
         if (valid && !conv) {
             // ---- fallback: bit-exact FP64 solve, G kept as (hi, lo) float pairs
@@ -3476,16 +3502,28 @@ cudaError_t occupancy(K kernel, int threads, size_t smem, int *per_sm)
 // 20,000 columns (4.2 tiles per SM) 51 us at 4 and 38 at 5: 4.5, rounded.
 constexpr double kChunkBudgetMB[2] = {120.0, 57.0};   // scalar, block
 constexpr double kStreamKB = 56.0;
+// Refinement rings.  Scalar (FP32 planes and the iterate, 20 B per level and
+// column): 267,708 columns x 57 levels 349 us at 11 warps per SM, 369 at 9,
+// 360 at 14; 290,304 x 113 906 us at 8, 951 at 7, 1,087 at 12.  2x2 blocks: a
+// fixed 7 warps per SM; 130,000 x 57 387 to 393 us at 5 to 7, 436 from 8 on,
+// 41,472 x 113 392 us at 3, 298 at 6, 295 at 9 (latency, not L2, decides there).
+constexpr double kRefineBudgetMB[2] = {152.0, 0.0};
+constexpr int kBlockRefineWarps = 7;
 // The register and narrow block kernels' Gamma, and the other scalar rings'
 // w2 and parked w3, which bound their grids more loosely: more columns in
 // flight win there (3x3 blocks on the nested batch, register kernel: 2.15 ms
 // at 96 MB and 1.72 ms at 128 and 192 MB).
 constexpr double kBlockRegBudgetMB = 160.0, kRingBudgetMB = 128.0;
 constexpr double kMB = 1024.0 * 1024.0;
-double g_scalar_scratch_budget = kChunkBudgetMB[0] * kMB, g_block_scratch_budget = kChunkBudgetMB[1] * kMB;
-bool g_scalar_budget_set = false, g_block_budget_set = false;
-double g_block_reg_budget() { return g_block_budget_set ? g_block_scratch_budget : kBlockRegBudgetMB * kMB; }
-double g_ring_budget() { return g_scalar_budget_set ? g_scalar_scratch_budget : kRingBudgetMB * kMB; }
+double g_scalar_scratch_budget = 0.0, g_block_scratch_budget = 0.0;   // set by the caller; 0: the defaults
+double chunk_budget(int kind, bool refine)
+{
+    const int i = kind == TG_KIND_SCALAR ? 0 : 1;
+    const double set = i ? g_block_scratch_budget : g_scalar_scratch_budget;
+    return set > 0.0 ? set : (refine ? kRefineBudgetMB[i] : kChunkBudgetMB[i]) * kMB;
+}
+double block_reg_budget() { return g_block_scratch_budget > 0.0 ? g_block_scratch_budget : kBlockRegBudgetMB * kMB; }
+double ring_budget() { return g_scalar_scratch_budget > 0.0 ? g_scalar_scratch_budget : kRingBudgetMB * kMB; }
 std::atomic<int> g_kind_overlap{-1};
 }  // namespace
 
@@ -3551,16 +3589,8 @@ void set_block_rows(int kind, int on)
     TileCfg &t = g_tile[kind_index(kind)][0];
     t.rows = on < 0 ? kDefaultTile[kind_index(kind)][0].rows : (on ? 1 : 0);
 }
-void set_block_scratch_budget(double mb)
-{
-    g_block_budget_set = mb > 0;
-    g_block_scratch_budget = (mb > 0 ? mb : kChunkBudgetMB[1]) * kMB;
-}
-void set_scalar_scratch_budget(double mb)
-{
-    g_scalar_budget_set = mb > 0;
-    g_scalar_scratch_budget = (mb > 0 ? mb : kChunkBudgetMB[0]) * kMB;
-}
+void set_block_scratch_budget(double mb) { g_block_scratch_budget = mb > 0 ? mb * kMB : 0.0; }
+void set_scalar_scratch_budget(double mb) { g_scalar_scratch_budget = mb > 0 ? mb * kMB : 0.0; }
 void set_kind_overlap(int mode) { g_kind_overlap.store(mode == 0 || mode == 1 ? mode : -1); }
 int kind_overlap() { return g_kind_overlap.load(); }
 void set_column_residency(int kind, int precision, int mode)
@@ -3602,8 +3632,8 @@ static int rows_group(int B) { return B == 2 ? 2 : 4; }
 size_t scalar_smem_bytes(int precision, int threads, int cpt, int k2max, int stages, int w2g, int lps)
 {
     const size_t lev = (size_t)(k2max > 1 ? k2max - 1 : 1);
-    if (stages > 0 && precision != TG_PREC_F64)   // refinement ring: 5L double rows + L float rows per stage
-        return (size_t)threads / 32 * stages * (5 * kRefineStageLevels * 32 + kRefineStageLevels * 16) * 8;
+    if (stages > 0 && precision != TG_PREC_F64)   // refinement ring
+        return (size_t)threads / 32 * stages * kRefineStageLevels * kRefineRowDoubles * 8;
     if (stages > 0 && lps > 1) return (size_t)threads / 32 * stages * 4 * lps * 32 * 8;
     if (stages > 0) return (size_t)threads / 32 * ((size_t)stages * 4 * 32 * 8 + (w2g ? 0 : 32 * lev * 8));
     if (w2g) return 0;
@@ -3613,8 +3643,8 @@ size_t scalar_smem_bytes(int precision, int threads, int cpt, int k2max, int sta
 
 size_t block_smem_bytes(int B, int stages, int threads, int rows, int bw, int precision)
 {
-    if (precision != TG_PREC_F64)   // refinement ring: P, Q, R, f and u rows per level
-        return stages > 0 ? (size_t)threads / 32 * stages * (3 * B * B + 2 * B) * 32 * 8 : 0;
+    if (precision != TG_PREC_F64)   // refinement ring
+        return stages > 0 ? (size_t)threads / 32 * stages * kBlkRefineRowDoubles * 8 : 0;
     const int w = rows ? 32 / rows_group(B) : bw;
     return stages > 0 ? (size_t)threads / 32 * stages * (3 * B * B + B) * w * 8 : 0;
 }
@@ -3752,17 +3782,19 @@ cudaError_t plan_shape(int kind, int precision, int k2max, int ntiles, int cpb, 
                              : (kind != TG_KIND_SCALAR ? (long)ntiles * (32 / sh->bw) : ntiles);   // warp tiles
     const long units = stages > 0 ? (vt + sh->threads / 32 - 1) / (sh->threads / 32) : ntiles;
     sh->one_wave = blocks >= units;
-    const bool chunk = precision == TG_PREC_F64 && stages > 0 && !sh->res &&
-                       (kind == TG_KIND_SCALAR ? sh->lps > 1 : !sh->rows && sh->bw == 32);
+    const bool refine = precision != TG_PREC_F64;
+    const bool chunk = stages > 0 && !sh->res &&
+                       (refine || (kind == TG_KIND_SCALAR ? sh->lps > 1 : !sh->rows && sh->bw == 32));
     if (chunk) {
-        // k_scalar_f64_chunk, k_block_f64_chunk: the resident warps within
-        // the budget (at least three per SM), then the tiles dealt evenly over
-        // the nearest whole number of passes, so that none is nearly empty
+        // the chunk kernels and the refinement rings: the resident warps
+        // within the budget (at least three per SM), then the tiles dealt
+        // evenly over the nearest whole number of passes, so that none is
+        // nearly empty
         const int wpb = sh->threads / 32;
-        const double per_warp = kind == TG_KIND_SCALAR ? 512.0 * k2max + kStreamKB * 1024.0
-                                                       : 32.0 * k2max * (kind * kind + kind) * 8.0;
-        const double budget = kind == TG_KIND_SCALAR ? g_scalar_scratch_budget : g_block_scratch_budget;
-        long cap = (long)(budget / (per_warp * wpb));
+        const double per_warp = kind == TG_KIND_SCALAR ? (refine ? 640.0 : 512.0) * k2max + kStreamKB * 1024.0
+                                                       : (refine ? 1792.0 : 256.0 * (kind * kind + kind)) * k2max;
+        const double budget = chunk_budget(kind, refine);
+        long cap = budget > 0.0 ? (long)(budget / (per_warp * wpb)) : (long)kBlockRefineWarps * nsm / wpb;
         if (cap < 3L * nsm / wpb) cap = 3L * nsm / wpb;
         if (cap < 1) cap = 1;
         long passes = (2 * units + cap) / (2 * cap);
@@ -3772,22 +3804,16 @@ cudaError_t plan_shape(int kind, int precision, int k2max, int ntiles, int cpb, 
     } else if (kind != TG_KIND_SCALAR && precision == TG_PREC_F64 && !sh->res) {
         // keep the Gamma scratch of all resident blocks within the budget
         // (a cap on the total, not per SM, so that a grid that fits in one
-        // wave is not split into two).  The block refinement kernel is not
-        // capped: its loads are latency-bound, and more columns in flight
-        // win over the planes' L2 spill (6.2 vs 7.4 ms on the nested batch).
+        // wave is not split into two)
         const double per_thread = (double)kind * kind * k2max * 8.0;
-        const long cap = (long)(g_block_reg_budget() / (per_thread * sh->threads));
+        const long cap = (long)(block_reg_budget() / (per_thread * sh->threads));
         if (blocks > cap) blocks = cap > 0 ? cap : 1;
     } else if (stages > 0 && sh->res != 2 && sh->res != 3) {
-        // ring kernels: w2 scratch plus the w3 parked in x, 8 B each per level
-        // and column (refinement: three float planes plus x; w2 on chip: the
-        // parked w3 alone), of every resident column within the L2 budget
-        // (refinement with hints 2 or 3 keeps its FP64 coefficients in L2
-        // between the sweeps: their 32 B per level count too)
-        const double per_col = sh->res == 1 ? (double)k2max * 8.0
-                               : precision == TG_PREC_F64 ? (double)(2 * k2max - 1) * 8.0
-                                                          : (double)k2max * (cache_hints() >= 2 ? 52.0 : 20.0);
-        const long cap = (long)(g_ring_budget() / (per_col * sh->threads * sh->cpt));
+        // the other scalar rings: w2 scratch plus the w3 parked in x, 8 B each
+        // per level and column (w2 on chip: the parked w3 alone), of every
+        // resident column within the L2 budget
+        const double per_col = sh->res == 1 ? (double)k2max * 8.0 : (double)(2 * k2max - 1) * 8.0;
+        const long cap = (long)(ring_budget() / (per_col * sh->threads * sh->cpt));
         if (blocks > cap) blocks = cap > 0 ? cap : 1;
     }
     if (blocks > units) blocks = units;
