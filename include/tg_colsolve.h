@@ -568,6 +568,19 @@ int tg_oplus_ng_factor_dev(const tg_oplus_fields *F, const tg_oplus_consts *C, d
                            double *factor, int nk, int ncol, long ld, int *status_dev, void *stream);
 int tg_oplus_ng_solve_dev(const tg_oplus_fields *F, const tg_oplus_consts *C, const double *factor, double *opout,
                           int nk, int ncol, long ld, const tg_post_step *P, int *status_dev, void *stream);
+/* The whole sub-cycle in one call, for a nest held as one subdomain of
+ * (nlon+4) x (nlat+4) columns: tg_oplus_ng_factor_dev, then consts->nstep_sub
+ * times tg_smooth_ng_dev(optm1, shapiro) and tg_oplus_ng_solve_dev with the
+ * post-solve steps, the same bits.  Sub-step s (0-based) writes op_a, optm1_a
+ * when s is even and op_b, optm1_b when it is odd, and reads what s-1 wrote
+ * (F->op and optm1 at s = 0).  explicit_h is the same in every sub-step;
+ * F->optm1_smooth2 is not read.  optm1_smooth (nk planes) is work space;
+ * bnd_mask and bnd as in tg_post_step (both or neither). */
+int tg_oplus_ng_subcycle_dev(const tg_oplus_fields *F, const tg_oplus_consts *C, double *xiop2p, double *xiop2d,
+                             double *factor, const double *optm1, double *optm1_smooth, double shapiro, double *op_a,
+                             double *optm1_a, double *op_b, double *optm1_b, int nk, int nlon, int nlat, long ld,
+                             const unsigned char *bnd_mask, const double *bnd, double dtsmooth, double dtsmooth_div2,
+                             int *status_dev, void *stream);
 
 /* ---- batched, GPU-resident plans ---------------------------------------------
  * A plan solves many independent systems ("segments": any mix of grids, nest

@@ -39,7 +39,7 @@ LIB_PATH = os.path.join(HERE, "libtg_colsolve.so")
 
 # Every symbol include/tg_colsolve.h declares.
 EXPORTS = ("tg_solve_host", "tg_dt_ng", "tg_dt_ng_dev", "tg_minor_ng", "tg_minor_ng_dev", "tg_comp_ng",
-           "tg_comp_ng_dev", "tg_comp_post_ng", "tg_comp_post_ng_dev", "tg_comp_diag_ng", "tg_comp_diag_ng_dev", "tg_oplus_ng_factor_doubles", "tg_oplus_diag_ng", "tg_oplus_diag_ng_dev", "tg_oplus_ng_factor_dev", "tg_oplus_ng_solve_dev", "tg_time_filter_ng", "tg_time_filter_ng_dev", "tg_advec_ng", "tg_advec_ng_dev", "tg_smooth_ng", "tg_smooth_ng_dev", "tg_settei_ng", "tg_settei_ng_dev", "tg_oplus_ng",
+           "tg_comp_ng_dev", "tg_comp_post_ng", "tg_comp_post_ng_dev", "tg_comp_diag_ng", "tg_comp_diag_ng_dev", "tg_oplus_ng_factor_doubles", "tg_oplus_diag_ng", "tg_oplus_diag_ng_dev", "tg_oplus_ng_factor_dev", "tg_oplus_ng_solve_dev", "tg_oplus_ng_subcycle_dev", "tg_time_filter_ng", "tg_time_filter_ng_dev", "tg_advec_ng", "tg_advec_ng_dev", "tg_smooth_ng", "tg_smooth_ng_dev", "tg_settei_ng", "tg_settei_ng_dev", "tg_oplus_ng",
            "tg_oplus_ng_dev", "tg_trsolv", "tg_trsolv_ng", "tg_blktri", "tg_comp_blksolve_ng", "tg_blksolve", "tg_trsolv_dev",
            "tg_blksolve_dev", "tg_blksolve_dev_noalloc", "tg_plan_create", "tg_plan_execute", "tg_plan_capture_graph",
            "tg_plan_status", "tg_plan_launches", "tg_plan_describe", "tg_set_cache_hints", "tg_set_block_rows", "tg_set_block_width", "tg_set_stage_levels", "tg_set_column_residency", "tg_set_assembly_mode", "tg_set_walk_prefetch", "tg_set_block_scratch_budget", "tg_set_scalar_scratch_budget", "tg_set_kind_overlap", "tg_set_host_pipeline", "tg_selftest_wait", "tg_plan_sweep_histogram", "tg_plan_destroy",
@@ -222,6 +222,8 @@ def lib():
                                        P],
             "tg_oplus_ng_solve_dev": [ctypes.POINTER(OplusFields), ctypes.POINTER(OplusConsts), P, P, I, I, Lg,
                                       ctypes.POINTER(PostStepArgs), P, P],
+            "tg_oplus_ng_subcycle_dev": [ctypes.POINTER(OplusFields), ctypes.POINTER(OplusConsts), P, P, P, P, P, D, P,
+                                         P, P, P, I, I, I, Lg, P, P, D, D, P, P],
             "tg_time_filter_ng": [I, P, P, D, D, I, I, P, P],
             "tg_time_filter_ng_dev": [I, P, P, D, D, I, I, Lg, P, P, P],
             "tg_advec_ng": [P, P, P, P, D, D, D, I, I, I, P],
@@ -775,6 +777,23 @@ def oplus_ng_solve_dev(fields, consts, factor, opout, nk, ncol, ld, post=None, s
     rc = lib().tg_oplus_ng_solve_dev(ctypes.byref(F), ctypes.byref(C), _dptr(factor), _dptr(opout), nk, ncol, ld,
                                      Pp, None if status is None else _int_dptr(status), _stream(stream))
     return _check(rc, "tg_oplus_ng_solve_dev", numeric_ok=False)
+
+
+def oplus_ng_subcycle_dev(fields, consts, xiop2p, xiop2d, factor, optm1, optm1_smooth, shapiro, op, optm1_out, nk,
+                          nlon, nlat, ld, dtsmooth, dtsmooth_div2, bnd_mask=None, bnd=None, status=None, stream=None):
+    """tg_oplus_ng_subcycle_dev: one step's whole O+ sub-cycle (factor, then
+    consts["nstep_sub"] smoothings and solves).  op and optm1_out are pairs of
+    (nk, ld) tensors the sub-steps write in turn; optm1_smooth is work space."""
+    F = OplusFields(*[_dptr(fields[n]) for n in OPLUS_FIELDS])
+    C = oplus_consts(consts)
+    if bnd_mask is not None and (not bnd_mask.is_cuda or str(bnd_mask.dtype) != "torch.uint8"):
+        raise TypeError("bnd_mask must be a uint8 CUDA tensor")
+    rc = lib().tg_oplus_ng_subcycle_dev(
+        ctypes.byref(F), ctypes.byref(C), _dptr(xiop2p), _dptr(xiop2d), _dptr(factor), _dptr(optm1),
+        _dptr(optm1_smooth), float(shapiro), _dptr(op[0]), _dptr(optm1_out[0]), _dptr(op[1]), _dptr(optm1_out[1]), nk,
+        nlon, nlat, ld, None if bnd_mask is None else bnd_mask.data_ptr(), _dptr(bnd), float(dtsmooth),
+        float(dtsmooth_div2), None if status is None else _int_dptr(status), _stream(stream))
+    return _check(rc, "tg_oplus_ng_subcycle_dev", numeric_ok=False)
 
 
 def settei_ng_dev(fields, consts, te_out, ti_out, qtotal, nk, ncol, ld, system_out=None, status=None, stream=None):

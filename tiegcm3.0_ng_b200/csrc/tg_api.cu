@@ -62,8 +62,8 @@ std::atomic<int> g_host_slots{kHostSlotsDefault};
 std::atomic<long> g_host_chunk_bytes{0};   // 0: chosen per call
 // Device workspace of the stream-ordered (_dev) entries, one per caller
 // stream: entries issued on different streams may run at the same time, so
-// each stream's work gets its own scratch, relayout buffers, status word and
-// sweep histogram.  Work on one stream is ordered, so it can share them.
+// each stream's work gets its own scratch, relayout buffers and status word.
+// Work on one stream is ordered, so it can share them.
 struct StreamWs {
     cudaStream_t key = nullptr;
     bool used = false;
@@ -71,7 +71,6 @@ struct StreamWs {
     Buf lvl[7];                    // level-major relayout of column-layout solves
     Buf scratch;                   // kernel scratch (Gamma, planes, w2)
     unsigned *flags = nullptr;     // device status word
-    unsigned long long *hist = nullptr;   // device, kMaxSweepBins
 };
 constexpr int kStreamWs = 16;
 
@@ -179,7 +178,6 @@ int stream_ws(DevCtx *c, cudaStream_t st, StreamWs **out)
             }
         }
         if (!hit->flags) TG_CUDA(cudaMalloc(&hit->flags, sizeof(unsigned)));
-        if (!hit->hist) TG_CUDA(cudaMalloc(&hit->hist, kMaxSweepBins * sizeof(unsigned long long)));
         hit->key = st;
         hit->used = true;
     }
@@ -187,6 +185,11 @@ int stream_ws(DevCtx *c, cudaStream_t st, StreamWs **out)
     *out = hit;
     return TG_OK;
 }
+
+// The stream's status word, for a caller that asks for the status; a call
+// without status_dev needs no word and saves the memset in front of its
+// kernels (about 2 us of a chain of small ones).
+unsigned *status_word(StreamWs *ws, const int *status_dev) { return status_dev ? ws->flags : nullptr; }
 
 int flags_to_status(unsigned f)
 {
@@ -957,10 +960,8 @@ static int dev_solve(int kind, const double *a, const double *b, const double *c
     std::lock_guard<std::mutex> lk(cx->mu);
     StreamWs *ws = nullptr;
     if ((rc = stream_ws(cx, st, &ws))) return rc;
-    unsigned *flags = ws->flags;
-    TG_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned), st));
-    if (precision != TG_PREC_F64)
-        TG_CUDA(cudaMemsetAsync(ws->hist, 0, kMaxSweepBins * sizeof(unsigned long long), st));
+    unsigned *flags = status_word(ws, status_dev);
+    if (flags) TG_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned), st));
     if (ncol > 0) {
         Seg seg{};
         seg.nk = nk;
@@ -973,7 +974,7 @@ static int dev_solve(int kind, const double *a, const double *b, const double *c
             seg.ubc_ratio = ubc_ratio;
             seg.ubc_add = ubc_ratio ? ubc_add : nullptr;
             seg.ld = ld;
-            if ((rc = solve_level(ws->scratch, ws->hist, kind, precision, seg, flags, st))) return rc;
+            if ((rc = solve_level(ws->scratch, nullptr, kind, precision, seg, flags, st))) return rc;
         } else {
             const long mrows = (long)B * B * k2, vrows = (long)B * k2;
             const long lld = round_up(ncol, 32);
@@ -999,7 +1000,7 @@ static int dev_solve(int kind, const double *a, const double *b, const double *c
             seg.ubc_add = (ubc_ratio && ubc_add) ? lv[6] : nullptr;
             seg.ld = lld;
             seg.nk = k2 + (ubc_ratio ? 1 : 0);
-            if ((rc = solve_level(ws->scratch, ws->hist, kind, precision, seg, flags, st))) return rc;
+            if ((rc = solve_level(ws->scratch, nullptr, kind, precision, seg, flags, st))) return rc;
             TG_CUDA(launch_level_to_col(lv[4], lld, x, (long)B * nk, orows, ncol, st));
         }
     }
@@ -1034,10 +1035,11 @@ __attribute__((visibility("default"))) int tg_dt_ng_dev(const tg_dt_fields *F, c
     cudaStream_t st = (cudaStream_t)stream;
     StreamWs *ws = nullptr;
     if ((rc = stream_ws(cx, st, &ws))) return rc;
-    TG_CUDA(cudaMemsetAsync(ws->flags, 0, sizeof(unsigned), st));
+    unsigned *flags = status_word(ws, status_dev);
+    if (flags) TG_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned), st));
     if ((rc = grow(ws->scratch, sizeof(double) * dt_scratch_planes() * (size_t)nk * (size_t)(ld > 0 ? ld : 1))))
         return rc;
-    TG_CUDA(launch_dt_ng(*F, *C, tn_upd, nk, ncol, ld, system_out, ws->flags, st, nullptr, (double *)ws->scratch.p));
+    TG_CUDA(launch_dt_ng(*F, *C, tn_upd, nk, ncol, ld, system_out, flags, st, nullptr, (double *)ws->scratch.p));
     if (status_dev) {
         k_finish_status<<<1, 1, 0, st>>>(ws->flags, status_dev);
         TG_CUDA(cudaGetLastError());
@@ -1125,8 +1127,9 @@ __attribute__((visibility("default"))) int tg_minor_ng_dev(const tg_minor_fields
     StreamWs *ws = nullptr;
     if ((rc = stream_ws(cx, st, &ws))) return rc;
     if ((rc = grow(ws->scratch, sizeof(double) * minor_scratch_planes() * (size_t)nk * (size_t)(ld > 0 ? ld : 1)))) return rc;
-    TG_CUDA(cudaMemsetAsync(ws->flags, 0, sizeof(unsigned), st));
-    TG_CUDA(launch_minor_ng(*F, *C, out, nk, ncol, ld, system_out, ws->flags, st, (double *)ws->scratch.p));
+    unsigned *flags = status_word(ws, status_dev);
+    if (flags) TG_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned), st));
+    TG_CUDA(launch_minor_ng(*F, *C, out, nk, ncol, ld, system_out, flags, st, (double *)ws->scratch.p));
     if (status_dev) {
         k_finish_status<<<1, 1, 0, st>>>(ws->flags, status_dev);
         TG_CUDA(cudaGetLastError());
@@ -1370,10 +1373,11 @@ __attribute__((visibility("default"))) int tg_dt_ng_post_dev(const tg_dt_fields 
     StreamWs *ws = nullptr;
     if ((rc = stream_ws(cx, st, &ws))) return rc;
     const PostStep post = post_of(P, 100.0, 0);
-    TG_CUDA(cudaMemsetAsync(ws->flags, 0, sizeof(unsigned), st));
+    unsigned *flags = status_word(ws, status_dev);
+    if (flags) TG_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned), st));
     if ((rc = grow(ws->scratch, sizeof(double) * dt_scratch_planes() * (size_t)nk * (size_t)(ld > 0 ? ld : 1))))
         return rc;
-    TG_CUDA(launch_dt_ng(*F, *C, tn_upd, nk, ncol, ld, nullptr, ws->flags, st, &post, (double *)ws->scratch.p));
+    TG_CUDA(launch_dt_ng(*F, *C, tn_upd, nk, ncol, ld, nullptr, flags, st, &post, (double *)ws->scratch.p));
     if (status_dev) {
         k_finish_status<<<1, 1, 0, st>>>(ws->flags, status_dev);
         TG_CUDA(cudaGetLastError());
@@ -1398,8 +1402,9 @@ __attribute__((visibility("default"))) int tg_minor_ng_post_dev(const tg_minor_f
     if ((rc = stream_ws(cx, st, &ws))) return rc;
     if ((rc = grow(ws->scratch, sizeof(double) * minor_scratch_planes() * (size_t)nk * (size_t)(ld > 0 ? ld : 1)))) return rc;
     const PostStep post = post_of(P, 1.e-12, 1);
-    TG_CUDA(cudaMemsetAsync(ws->flags, 0, sizeof(unsigned), st));
-    TG_CUDA(launch_minor_ng(*F, *C, fcomp_out, nk, ncol, ld, nullptr, ws->flags, st, (double *)ws->scratch.p,
+    unsigned *flags = status_word(ws, status_dev);
+    if (flags) TG_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned), st));
+    TG_CUDA(launch_minor_ng(*F, *C, fcomp_out, nk, ncol, ld, nullptr, flags, st, (double *)ws->scratch.p,
                             &post));
     if (status_dev) {
         k_finish_status<<<1, 1, 0, st>>>(ws->flags, status_dev);
@@ -1434,8 +1439,9 @@ __attribute__((visibility("default"))) int tg_comp_ng_dev(const tg_comp_fields *
     StreamWs *ws = nullptr;
     if ((rc = stream_ws(cx, st, &ws))) return rc;
     if ((rc = grow(ws->scratch, sizeof(double) * comp_scratch_doubles(nk, ld > 0 ? ld : 1)))) return rc;
-    TG_CUDA(cudaMemsetAsync(ws->flags, 0, sizeof(unsigned), st));
-    TG_CUDA(launch_comp_ng(*F, *C, out, (double *)ws->scratch.p, nk, ncol, ld, system_out, ws->flags, st));
+    unsigned *flags = status_word(ws, status_dev);
+    if (flags) TG_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned), st));
+    TG_CUDA(launch_comp_ng(*F, *C, out, (double *)ws->scratch.p, nk, ncol, ld, system_out, flags, st));
     if (status_dev) {
         k_finish_status<<<1, 1, 0, st>>>(ws->flags, status_dev);
         TG_CUDA(cudaGetLastError());
@@ -1904,8 +1910,9 @@ __attribute__((visibility("default"))) int tg_settei_ng_dev(const tg_settei_fiel
     StreamWs *ws = nullptr;
     if ((rc = stream_ws(cx, st, &ws))) return rc;
     if ((rc = grow(ws->scratch, sizeof(double) * settei_scratch_doubles(nk, ld > 0 ? ld : 1)))) return rc;
-    TG_CUDA(cudaMemsetAsync(ws->flags, 0, sizeof(unsigned), st));
-    TG_CUDA(launch_settei_ng(*F, *C, te_out, ti_out, qtotal, nk, ncol, ld, system_out, ws->flags, st,
+    unsigned *flags = status_word(ws, status_dev);
+    if (flags) TG_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned), st));
+    TG_CUDA(launch_settei_ng(*F, *C, te_out, ti_out, qtotal, nk, ncol, ld, system_out, flags, st,
                              (double *)ws->scratch.p));
     if (status_dev) {
         k_finish_status<<<1, 1, 0, st>>>(ws->flags, status_dev);
@@ -1991,9 +1998,10 @@ __attribute__((visibility("default"))) int tg_oplus_ng_dev(const tg_oplus_fields
     if ((rc = stream_ws(cx, st, &ws))) return rc;
     const size_t sbytes = sizeof(double) * oplus_scratch_planes() * (size_t)nk * (size_t)(ld > 0 ? ld : 1);
     if ((rc = grow(ws->scratch, sbytes))) return rc;
-    TG_CUDA(cudaMemsetAsync(ws->flags, 0, sizeof(unsigned), st));
+    unsigned *flags = status_word(ws, status_dev);
+    if (flags) TG_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned), st));
     TG_CUDA(launch_oplus_ng(*F, *C, opout, xiop2p, xiop2d, Fe, Fn, (double *)ws->scratch.p, nk, ncol, ld,
-                            system_out, ws->flags, st));
+                            system_out, flags, st));
     if (status_dev) {
         k_finish_status<<<1, 1, 0, st>>>(ws->flags, status_dev);
         TG_CUDA(cudaGetLastError());
@@ -2021,9 +2029,10 @@ __attribute__((visibility("default"))) int tg_oplus_ng_post_dev(const tg_oplus_f
     const size_t sbytes = sizeof(double) * oplus_scratch_planes() * (size_t)nk * (size_t)(ld > 0 ? ld : 1);
     if ((rc = grow(ws->scratch, sbytes))) return rc;
     const PostStep post = post_of(P, 0.0, 1);
-    TG_CUDA(cudaMemsetAsync(ws->flags, 0, sizeof(unsigned), st));
+    unsigned *flags = status_word(ws, status_dev);
+    if (flags) TG_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned), st));
     TG_CUDA(launch_oplus_ng(*F, *C, opout, xiop2p, xiop2d, Fe, Fn, (double *)ws->scratch.p, nk, ncol, ld, nullptr,
-                            ws->flags, st, &post));
+                            flags, st, &post));
     if (status_dev) {
         k_finish_status<<<1, 1, 0, st>>>(ws->flags, status_dev);
         TG_CUDA(cudaGetLastError());
@@ -2052,8 +2061,9 @@ __attribute__((visibility("default"))) int tg_oplus_ng_factor_dev(const tg_oplus
     cudaStream_t st = (cudaStream_t)stream;
     StreamWs *ws = nullptr;
     if ((rc = stream_ws(cx, st, &ws))) return rc;
-    TG_CUDA(cudaMemsetAsync(ws->flags, 0, sizeof(unsigned), st));
-    TG_CUDA(launch_oplus_factor(*F, *C, xiop2p, xiop2d, factor, nk, ncol, ld, ws->flags, st));
+    unsigned *flags = status_word(ws, status_dev);
+    if (flags) TG_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned), st));
+    TG_CUDA(launch_oplus_factor(*F, *C, xiop2p, xiop2d, factor, nk, ncol, ld, flags, st));
     if (status_dev) {
         k_finish_status<<<1, 1, 0, st>>>(ws->flags, status_dev);
         TG_CUDA(cudaGetLastError());
@@ -2078,13 +2088,46 @@ __attribute__((visibility("default"))) int tg_oplus_ng_solve_dev(const tg_oplus_
     cudaStream_t st = (cudaStream_t)stream;
     StreamWs *ws = nullptr;
     if ((rc = stream_ws(cx, st, &ws))) return rc;
-    TG_CUDA(cudaMemsetAsync(ws->flags, 0, sizeof(unsigned), st));
+    unsigned *flags = status_word(ws, status_dev);
+    if (flags) TG_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned), st));
     if (P) {
         const PostStep post = post_of(P, 0.0, 1);
-        TG_CUDA(launch_oplus_solve(*F, *C, factor, opout, nk, ncol, ld, ws->flags, st, &post));
+        TG_CUDA(launch_oplus_solve(*F, *C, factor, opout, nk, ncol, ld, flags, st, &post));
     } else {
-        TG_CUDA(launch_oplus_solve(*F, *C, factor, opout, nk, ncol, ld, ws->flags, st, nullptr));
+        TG_CUDA(launch_oplus_solve(*F, *C, factor, opout, nk, ncol, ld, flags, st, nullptr));
     }
+    if (status_dev) {
+        k_finish_status<<<1, 1, 0, st>>>(ws->flags, status_dev);
+        TG_CUDA(cudaGetLastError());
+    }
+    return TG_OK;
+}
+
+__attribute__((visibility("default"))) int tg_oplus_ng_subcycle_dev(
+    const tg_oplus_fields *F, const tg_oplus_consts *C, double *xiop2p, double *xiop2d, double *factor,
+    const double *optm1, double *optm1_smooth, double shapiro, double *op_a, double *optm1_a, double *op_b,
+    double *optm1_b, int nk, int nlon, int nlat, long ld, const unsigned char *bnd_mask, const double *bnd,
+    double dtsmooth, double dtsmooth_div2, int *status_dev, void *stream)
+{
+    const long ncol = nlon > 0 && nlat > 0 ? (long)(nlon + 4) * (nlat + 4) : -1;
+    if (!F || !C || !xiop2p || !xiop2d || !factor || !optm1 || !optm1_smooth || !op_a || !optm1_a || !op_b ||
+        !optm1_b || nk < 3 || ncol < 0 || ncol > 0x7fffffffL || ld < ncol || C->nstep_sub < 1 ||
+        (!bnd_mask) != (!bnd) || !oplus_fields_ok(F)) {
+        set_err("tg_oplus_ng_subcycle_dev: bad arguments (nk=%d nlon=%d nlat=%d ld=%ld)", nk, nlon, nlat, ld);
+        return TG_EINVAL;
+    }
+    DevCtx *cx = nullptr;
+    int rc = get_ctx(&cx);
+    if (rc) return rc;
+    std::lock_guard<std::mutex> lk(cx->mu);
+    cudaStream_t st = (cudaStream_t)stream;
+    StreamWs *ws = nullptr;
+    if ((rc = stream_ws(cx, st, &ws))) return rc;
+    unsigned *flags = status_word(ws, status_dev);
+    if (flags) TG_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned), st));
+    const OplusSubcycle sc{F->op, optm1, optm1_smooth, {op_a, op_b}, {optm1_a, optm1_b}, shapiro, nlon, nlat};
+    const PostStep post{nullptr, nullptr, nullptr, bnd_mask, bnd, dtsmooth, dtsmooth_div2, 0.0, 1};
+    TG_CUDA(launch_oplus_subcycle(*F, *C, xiop2p, xiop2d, factor, sc, nk, (int)ncol, ld, flags, post, st));
     if (status_dev) {
         k_finish_status<<<1, 1, 0, st>>>(ws->flags, status_dev);
         TG_CUDA(cudaGetLastError());
@@ -2762,7 +2805,6 @@ __attribute__((visibility("default"))) int tg_release_buffers(void)
                 if (b.p) cudaFree(b.p);
             if (w.scratch.p) cudaFree(w.scratch.p);
             if (w.flags) cudaFree(w.flags);
-            if (w.hist) cudaFree(w.hist);
         }
         if (c->flags) cudaFree(c->flags);
         if (c->flags_host) cudaFreeHost(c->flags_host);

@@ -83,6 +83,22 @@ __device__ __forceinline__ void qdiv2(double a, double c, double b, double y, do
     }
 }
 
+// One Shapiro pass of smooth_ng along an axis (lat :18-29, lon :31-42) at
+// index t of n points: x - sh*(2*fm2 - 8*fm1 + 6*x) inside,
+// x - sh*(-8*fm1 + 8*x) one row in from a boundary (written 8*x - 8*fm1, the
+// same rounded number), x on the outermost ghost row.  Where they are used,
+// fm1 and fm2 are the plain +-1 and +-2 means; at(d) is the value d points on.
+template <class At>
+__device__ __forceinline__ double shapiro_at(At at, int t, int n, double sh)
+{
+    const double x = at(0);
+    if (t == 0 || t == n - 1) return x;
+    const double m1 = xmul(xadd(at(1), at(-1)), 0.5);
+    if (t == 1 || t == n - 2) return xsub(x, xmul(sh, xsub(xmul(8.0, x), xmul(8.0, m1))));
+    const double m2 = xmul(xadd(at(2), at(-2)), 0.5);
+    return xsub(x, xmul(sh, xadd(xsub(xmul(2.0, m2), xmul(8.0, m1)), xmul(6.0, x))));
+}
+
 // A hint that brings the line holding p into L1 (no register, no wait).
 __device__ __forceinline__ void pf_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 

@@ -1352,7 +1352,7 @@ __device__ __forceinline__ void comp_top(const CompConsts &C, const CompLevel &L
     }
     if (!C.calc_helium)
         for (int k = 0; k < nk; ++k) out[2 * slab + (long)k * ld + col] = C.pshelb;
-    if (!ok || !fin) atomicOr(status, (ok ? 0u : FLAG_PIVOT) | (fin ? 0u : FLAG_NONFINITE));
+    if (status && (!ok || !fin)) atomicOr(status, (ok ? 0u : FLAG_PIVOT) | (fin ? 0u : FLAG_NONFINITE));
 }
 
 __device__ __forceinline__ void comp_back(const CompConsts &C, const CompLevel &Lp, double flx00, double flx_he,

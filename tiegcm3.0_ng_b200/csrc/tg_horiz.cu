@@ -76,21 +76,6 @@ __global__ void __launch_bounds__(kTx * kTy) k_advec_ng(const double *f, const d
     hadvec[o] = xadd(qdiv_by(wk1, dlamda, rc.rlam, rc.lam_safe), qdiv_by(xmul(wk2, re_inv), dphi, rc.rphi, rc.phi_safe));
 }
 
-// One Shapiro pass of smooth_ng along an axis (lat :18-29, lon :31-42) at
-// index t of n points, stride s: x - sh*(2*fm2 - 8*fm1 + 6*x) inside,
-// x - sh*(-8*fm1 + 8*x) one row in from a boundary (written 8*x - 8*fm1,
-// the same rounded number), x on the outermost ghost row.  Where they are
-// used, fm1 and fm2 are the plain +-1 and +-2 means.
-__device__ __forceinline__ double shapiro_at(const double *p, int t, int n, int s, double sh)
-{
-    const double x = p[0];
-    if (t == 0 || t == n - 1) return x;
-    const double m1 = xmul(xadd(p[s], p[-s]), 0.5);
-    if (t == 1 || t == n - 2) return xsub(x, xmul(sh, xsub(xmul(8.0, x), xmul(8.0, m1))));
-    const double m2 = xmul(xadd(p[2 * s], p[-2 * s]), 0.5);
-    return xsub(x, xmul(sh, xadd(xsub(xmul(2.0, m2), xmul(8.0, m1)), xmul(6.0, x))));
-}
-
 // The lat pass lands in a shared tile of the block's 8 rows x (32 + 4)
 // longitudes (the lon pass needs +-2 neighbours): its 288 points are dealt
 // to the 256 threads in order, so only one warp takes a second point.  Then
@@ -106,13 +91,15 @@ __global__ void __launch_bounds__(kTx * kTy) k_smooth_ng(const double *fin, doub
         const int r = q / W, c = q - r * W;
         const int i = i0 - 2 + c, j = j0 + r;
         if (i < 0 || i >= nlond || j >= nlatd) continue;
-        ft[r][c] = shapiro_at(plane + i + (long)nlond * j, j, nlatd, nlond, sh);
+        const double *p = plane + i + (long)nlond * j;
+        ft[r][c] = shapiro_at([&](int d) { return p[d * nlond]; }, j, nlatd, sh);
     }
     __syncthreads();
     const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
     if (i >= nlond || j >= nlatd) return;
     // every longitude the lon pass reads (i-2..i+2 where used) is in the tile
-    fout[(long)blockIdx.z * ld + i + (long)nlond * j] = shapiro_at(&ft[threadIdx.y][threadIdx.x + 2], i, nlond, 1, sh);
+    const double *p = &ft[threadIdx.y][threadIdx.x + 2];
+    fout[(long)blockIdx.z * ld + i + (long)nlond * j] = shapiro_at([&](int d) { return p[d]; }, i, nlond, sh);
 }
 
 dim3 plane_grid(int nk, int nlond, int nlatd)

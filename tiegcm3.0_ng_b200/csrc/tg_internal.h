@@ -276,6 +276,21 @@ cudaError_t launch_oplus_diag_ng(const OplusFields &F, const OplusConsts &C, con
 cudaError_t launch_oplus_factor_pass(double *factor, int nk, int ncol, long ld, unsigned *status, cudaStream_t st);
 cudaError_t launch_oplus_solve(const OplusFields &F, const OplusConsts &C, const double *factor, double *opout, int nk,
                                int ncol, long ld, unsigned *status, cudaStream_t st, const PostStep *post = nullptr);
+// The whole O+ sub-cycle of a step on one nest held as one subdomain: the
+// factor pass, then nstep_sub sub-steps, each smoothing optm1 (shapiro) and
+// solving; sub-step s writes op[s % 2], optm1[s % 2] and reads what s - 1
+// wrote.  post gives the lateral boundary and the filter weights; smooth (nk
+// planes) is work space of launches the fused sub-step does not take.
+struct OplusSubcycle {
+    const double *op0, *optm10;
+    double *smooth;
+    double *op[2], *optm1[2];
+    double shapiro;
+    int nlon, nlat;
+};
+cudaError_t launch_oplus_subcycle(const OplusFields &F, const OplusConsts &C, double *xiop2p, double *xiop2d,
+                                  double *factor, const OplusSubcycle &sc, int nk, int ncol, long ld,
+                                  unsigned *status, const PostStep &post, cudaStream_t st);
 int oplus_scratch_planes();   // level-major scratch planes of launch_oplus_ng (each nk*ld doubles)
 
 // Polar ring filter (tg_filter.cu): the latitudes it filters, with their

@@ -15,6 +15,7 @@
 // intrinsics.  log10, pow, sin and cos are the device library's, within a few
 // ulp of the host C library's: the kernel agrees with the CPU restatement to
 // a stated tolerance.
+#include <algorithm>
 #include <cfloat>
 
 #include "tg_internal.h"
@@ -677,6 +678,199 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_oplus_solve_tile(OplusField
     }
 }
 
+// One sub-step of the O+ sub-cycle in one kernel: the Shapiro smoothing of
+// optm1, the right-hand side, the solve from the factor and the post-solve
+// steps.  A block of five warps takes kSubCols consecutive columns.  It copies
+// p, w1, 1/w1 and w2 of every level into shared memory and reads each thread's
+// explicit_h and op_prod values (none of which the sub-step before writes);
+// then waits for that sub-step (programmatic dependent launch), so those reads
+// and the launch overlap its tail.  The lat pass of the smoothing covers the
+// tile's columns and two on each side, straight from L2 (every column a value
+// is used from lies in the same grid row); the lon pass and the right-hand
+// side follow from shared memory, one thread per level and column, so that
+// the walk of warp 0 is the recurrence alone.  prev and cur stay in registers
+// from before the walk to the post-solve steps.
+// What bounds it: the walk (56 levels forward and back, one warp) and the L2
+// latency of the reads after the wait.  The step's O+ chain (factor pass and 10
+// sub-steps), as a graph: 2,072 columns x 57 levels 169 us with smoothing and
+// solve as two kernels -> 107, 6,969 columns 297 -> 149, 11,248 columns 389 ->
+// 252 (there the solve's 130 KB tiles also left one block per SM; these take
+// 38 KB).
+// R: levels a thread holds (10 threads per column: nk <= 10 R).
+// shapiro_at at a fixed index t of n points (stride s) over many levels: the
+// neighbours it does not use are read at the point itself, so that every read
+// can be in flight at once, and the edge forms are selected.
+struct Shapiro3 {
+    int d1, m1, d2, m2;
+    bool edge, near;
+    __device__ __forceinline__ Shapiro3(int t, int n, int s)
+    {
+        edge = t == 0 || t == n - 1;
+        near = t == 1 || t == n - 2;
+        d1 = edge ? 0 : s;
+        m1 = -d1;
+        d2 = edge || near ? 0 : 2 * s;
+        m2 = -d2;
+    }
+    template <class At>
+    __device__ __forceinline__ double operator()(At at, double sh) const
+    {
+        const double x = at(0), a1 = at(d1), b1 = at(m1), a2 = at(d2), b2 = at(m2);
+        const double f1 = xm(xa(a1, b1), 0.5), f2 = xm(xa(a2, b2), 0.5);
+        const double yn = xs(x, xm(sh, xs(xm(8.0, x), xm(8.0, f1))));
+        const double yi = xs(x, xm(sh, xa(xs(xm(2.0, f2), xm(8.0, f1)), xm(6.0, x))));
+        return edge ? x : near ? yn : yi;
+    }
+};
+constexpr int kSubCols = 16, kSubThreads = 160;
+template <int R>
+__global__ void __launch_bounds__(kSubThreads) k_oplus_substep(OplusFields F, OplusConsts C, const double *scr,
+                                                               const double *op, const double *optm1, double *op_out,
+                                                               double *optm1_out, double sh, int nlond, int nlatd,
+                                                               int nk, int ncol, long ld, unsigned *status,
+                                                               PostStep post, int wide)
+{
+    constexpr int T = kSubCols, W = T + 4, NG = kSubThreads / T;
+    extern __shared__ __align__(16) double sub_tile[];
+    const int tid = threadIdx.x, t = tid % T, g = tid / T, K = nk - 1;
+    const long c0 = (long)blockIdx.x * T, col = c0 + t, slab = (long)nk * ld;
+    const bool live = col < ncol;
+    // the smoothed rows (K x W) give way to ex, then the solution (nk x T)
+    double *sp = sub_tile, *sw1 = sp + K * T, *sy1 = sw1 + K * T, *sw2 = sy1 + K * T, *se = sw2 + K * T;
+    const double *src[4] = {scr + S_P * slab + c0, scr + S_W1 * slab + c0, scr + S_Y1 * slab + c0,
+                            scr + S_W2 * slab + c0};
+    if (wide) {   // 16-byte copies, 8 lanes a row: whole rows lie below ld
+        const int c2 = (tid % 8) * 2;
+        for (int k = tid / 8; k < K; k += kSubThreads / 8)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) cp_async16_ca(sp + (v * K + k) * T + c2, src[v] + (long)k * ld + c2);
+    } else if (live) {
+        for (int k = g; k < K; k += NG)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) cp_async8(sp + (v * K + k) * T + t, src[v] + (long)k * ld + t);
+    }
+    cp_async_commit();
+    double xh[R], pr[R], bv[R];
+    const bool bcol = live && post.bnd_mask && post.bnd_mask[col];
+#pragma unroll
+    for (int m = 0; m < R; ++m) {
+        const int k = g + m * NG;
+        const long o = (long)k * ld + col;
+        xh[m] = pr[m] = bv[m] = 0.0;
+        if (live && k < K) {
+            xh[m] = __ldg(F.explicit_h + o);
+            pr[m] = __ldg(scr + S_PROD * slab + o);
+        }
+        if (bcol && k < nk) bv[m] = __ldg(post.bnd + o);
+    }
+    const double t_top = live ? __ldg(scr + S_TB * slab + col) : 0.0;
+    const double t_bot = live ? __ldg(scr + S_TB * slab + ld + col) : 0.0;
+    // everything below reads what the sub-step before wrote
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    double pv[R], cv[R];
+#pragma unroll
+    for (int m = 0; m < R; ++m) {
+        const int k = g + m * NG;
+        pv[m] = cv[m] = 0.0;
+        if (live && k < nk) {
+            pv[m] = __ldcg(optm1 + (long)k * ld + col);
+            cv[m] = __ldcg(op + (long)k * ld + col);
+        }
+    }
+    {   // lat pass: a thread takes one column of the W, every eighth level
+        const int w = tid % W;
+        const long c = c0 - 2 + w;
+        if (c >= 0 && c < ncol) {
+            const int j = (int)c / nlond;
+            const Shapiro3 lat(j, nlatd, nlond);
+            const double *p = optm1 + c;
+#pragma unroll 7
+            for (int k = tid / W; k < K; k += kSubThreads / W) {
+                const double *pk = p + (long)k * ld;
+                se[k * W + w] = lat([&](int d) { return __ldcg(pk + d); }, sh);
+            }
+        }
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    double ex[R];
+    const Shapiro3 lon(live ? (int)(col % nlond) : 0, nlond, 1);
+#pragma unroll
+    for (int m = 0; m < R; ++m) {
+        const int k = g + m * NG;
+        if (live && k < K) {
+            const double *p = se + k * W + t + 2;
+            const double om = lon([&](int d) { return p[d]; }, sh);
+            double e = xs(xh[m], xm(xm(om, C.dtx2inv), (double)C.nstep_sub));
+            if (k == nk - 2) e = xs(e, t_top);
+            e = xs(e, pr[m]);
+            if (k == 0) e = xs(e, t_bot);
+            ex[m] = e;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < R; ++m)
+        if (live && g + m * NG < K) se[(g + m * NG) * T + t] = ex[m];
+    __syncthreads();
+    if (tid < T && live) {
+        // as in k_oplus_solve_tile: Markstein quotients without a branch, the
+        // IEEE fallback from the first level whose operands leave its range
+        double w3 = 0.;
+        int bad = K;
+        auto level = [&](int k, double e, double p, double w1, double y1) {
+            const double num = k == 0 ? e : xs(e, xm(p, w3));
+            const unsigned d = max(exp_dist(num), exp_dist(w1));
+            bad = d >= kExpSpan && bad == K ? k : bad;
+            w3 = div_markstein(num, w1, y1);
+            if (bad > k) se[k * T + t] = w3;
+        };
+        double en = se[t], pn = sp[t], w1n = sw1[t], y1n = sy1[t];
+        for (int k = 0; k < K - 1; ++k) {
+            const int s = (k + 1) * T + t;
+            const double e = en, p = pn, w1 = w1n, y1 = y1n;
+            en = se[s];
+            pn = sp[s];
+            w1n = sw1[s];
+            y1n = sy1[s];
+            level(k, e, p, w1, y1);
+        }
+        level(K - 1, en, pn, w1n, y1n);
+        if (bad < K) {
+            w3 = bad > 0 ? se[(bad - 1) * T + t] : 0.;
+            for (int k = bad; k < K; ++k) {
+                const int s = k * T + t;
+                w3 = qdiv1(k == 0 ? se[s] : xs(se[s], xm(sp[s], w3)), sw1[s], sy1[s]);
+                se[s] = w3;
+            }
+        }
+        const double xtop = w3;
+        back_sweep<T>(se, sw2, K, t, w3);
+        // x(k) = w3 - w2*x(k+1) carries a non-finite value down to x(0)
+        const bool fin = finite(se[t]) && finite(xtop);
+        // opout(nk) = opout(nk-1)**2/opout(nk-2) from the unfiltered values (oplus_ng.F90:307)
+        se[K * T + t] = xd(xm(xtop, xtop), se[(K - 2) * T + t]);
+        if (status && !fin) atomicOr(status, FLAG_NONFINITE);
+    }
+    __syncthreads();
+    if (!live) return;
+    post.nm = optm1_out;
+#pragma unroll
+    for (int m = 0; m < R; ++m) {
+        const int k = g + m * NG;
+        if (k < nk) {
+            const double x = bcol ? bv[m] : se[k * T + t];
+            post_store_v(post, false, op_out, (long)k * ld + col, x, pv[m], cv[m]);
+        }
+    }
+}
+size_t substep_smem(int nk)
+{
+    const size_t K = nk - 1, W = kSubCols + 4;
+    return sizeof(double) * (4 * K * kSubCols + std::max((size_t)nk * kSubCols, K * W));
+}
+
 constexpr int kSolveThreads = 32;
 // The same solve reading the rows from global memory (launches too large for
 // the shared-memory tile), pd levels requested ahead.
@@ -835,6 +1029,55 @@ cudaError_t launch_oplus_solve(const OplusFields &F, const OplusConsts &C, const
                                                         walk_prefetch(ncol));
     }
     return cudaGetLastError();
+}
+
+cudaError_t launch_oplus_subcycle(const OplusFields &F, const OplusConsts &C, double *xiop2p, double *xiop2d,
+                                  double *factor, const OplusSubcycle &sc, int nk, int ncol, long ld,
+                                  unsigned *status, const PostStep &post, cudaStream_t st)
+{
+    if (ncol <= 0) return cudaSuccess;
+    cudaError_t e = launch_oplus_factor(F, C, xiop2p, xiop2d, factor, nk, ncol, ld, status, st);
+    const size_t smem = substep_smem(nk);
+    const int nlond = sc.nlon + 4, nlatd = sc.nlat + 4;
+    const bool fused = ncol <= kSmallWalkColumns && nk <= 130 && smem <= (size_t)smem_optin();
+    const bool wide = ld % 2 == 0 && ld >= (ncol + kSubCols - 1) / kSubCols * kSubCols && ((uintptr_t)factor & 15) == 0;
+    if (fused)
+        once_per_device([] {
+            cudaFuncSetAttribute(k_oplus_substep<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin());
+            cudaFuncSetAttribute(k_oplus_substep<13>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin());
+        });
+    const double *op = sc.op0, *optm1 = sc.optm10;
+    for (int s = 0; s < C.nstep_sub && e == cudaSuccess; ++s) {
+        double *op_out = sc.op[s % 2], *optm1_out = sc.optm1[s % 2];
+        if (fused) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)((ncol + kSubCols - 1) / kSubCols));
+            cfg.blockDim = dim3(kSubThreads);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = st;
+            // the first sub-step reads the factor pass's planes before it waits: a plain launch
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = s > 0 ? 1 : 0;
+            auto k = nk <= 60 ? k_oplus_substep<6> : k_oplus_substep<13>;
+            e = cudaLaunchKernelEx(&cfg, k, F, C, (const double *)factor, op, optm1, op_out, optm1_out, sc.shapiro,
+                                   nlond, nlatd, nk, ncol, ld, status, post, (int)wide);
+        } else {
+            e = launch_smooth_ng(optm1, sc.shapiro, nk, sc.nlon, sc.nlat, ld, sc.smooth, st);
+            OplusFields Fs = F;
+            Fs.optm1_smooth2 = sc.smooth;
+            PostStep ps = post;
+            ps.cur = op;
+            ps.prev = optm1;
+            ps.nm = optm1_out;
+            if (e == cudaSuccess) e = launch_oplus_solve(Fs, C, factor, op_out, nk, ncol, ld, status, st, &ps);
+        }
+        op = op_out;
+        optm1 = optm1_out;
+    }
+    return e;
 }
 
 cudaError_t launch_oplus_ng(const OplusFields &F, const OplusConsts &C, double *opout, double *xiop2p,

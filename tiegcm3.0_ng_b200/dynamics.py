@@ -8,8 +8,8 @@ inputs it computes itself:
                          hook + time filter (src/oplus_ng.F90:159, 125-340);
                          sub-step s reads what sub-step s-1 wrote; the rows
                          and pivots, the same in every sub-step, are formed
-                         once (tg_oplus_ng_factor_dev) and each sub-step
-                         solves from them (tg_oplus_ng_solve_dev)
+                         once and each sub-step smooths and solves from them
+                         in one kernel (tg_oplus_ng_subcycle_dev)
   minor_ng x 4           N2D, N4S, NO, Ar (comp_n2d_ng ... comp_ar_ng):
                          smooth_ng(fcomp_tm1), advec_ng(fcomp), the column
                          step + lateral hook + time filter and floors
@@ -206,18 +206,10 @@ class DynamicsStep:
                     dtsmooth_div2=self.ds[1])
 
     def _oplus(self, st):
-        # the rows and pivots once (they do not change between sub-steps),
-        # then each sub-step's smoothing and solve
         g, o = self.grid, self.oplus
-        op, optm1 = o["op0"], o["optm10"]
-        cs.oplus_ng_factor_dev(o["F"], o["C"], o["xiop2p"], o["xiop2d"], o["factor"], g.nk, g.ncol, g.ld, stream=st)
-        for s in range(self.nstep_sub):
-            nxt = s % 2
-            self._smooth(optm1, o["F"]["optm1_smooth2"], st, g.shapiro / self.nstep_sub)
-            F = dict(o["F"], op=op)
-            cs.oplus_ng_solve_dev(F, o["C"], o["factor"], o["op"][nxt], g.nk, g.ncol, g.ld,
-                                  self._post(op, optm1, o["optm1"][nxt], o["bnd"]), stream=st)
-            op, optm1 = o["op"][nxt], o["optm1"][nxt]
+        cs.oplus_ng_subcycle_dev(o["F"], o["C"], o["xiop2p"], o["xiop2d"], o["factor"], o["optm10"],
+                                 o["F"]["optm1_smooth2"], g.shapiro / self.nstep_sub, o["op"], o["optm1"], g.nk, g.nlon,
+                                 g.nlat, g.ld, self.ds[0], self.ds[1], bnd_mask=self.mask, bnd=o["bnd"], stream=st)
 
     def _minor(self, m, st):
         g = self.grid
