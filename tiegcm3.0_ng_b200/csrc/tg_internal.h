@@ -32,6 +32,10 @@ inline void once_per_device(F &&f)
 }
 // Opt-in shared memory per block of the current device (bytes).
 int smem_optin();
+int sm_count();
+// Blocks of smem dynamic bytes (1 KB more is the system's) that are resident
+// at once on the current device as far as shared memory goes.
+inline long resident_by_smem(size_t smem) { return (long)sm_count() * ((smem_optin() + 1024) / (long)(smem + 1024)); }
 
 // Per-segment status bits written by the kernels (atomicOr into a device word).
 enum : unsigned {
@@ -198,10 +202,10 @@ int assembly_mode();
 void set_assembly_mode(int m);
 // The walk of the three-pass form (tg_walk.cu): rows 0..K-1 of the p, q, r, f
 // planes into x; top 0: K = nk; top 1: K = nk-1 and x(nk-1) =
-// x(nk-2)**2/x(nk-3); stored through post when given.
-cudaError_t launch_thomas_post(const double *p, const double *q, const double *r, const double *f, double *x, int nk,
-                               int K, int top, int ncol, long ld, unsigned *status, const PostStep *post,
-                               cudaStream_t st);
+// x(nk-2)**2/x(nk-3); stored through post when given.  p and q are work space
+// afterwards.
+cudaError_t launch_thomas_post(double *p, double *q, const double *r, const double *f, double *x, int nk, int K,
+                               int top, int ncol, long ld, unsigned *status, const PostStep *post, cudaStream_t st);
 // Levels a column walk of the assembly kernels prefetches ahead of the level
 // it computes, for a launch over ncol columns: few columns leave few warps
 // per SM, and each level of the walk then waits out a memory latency unless

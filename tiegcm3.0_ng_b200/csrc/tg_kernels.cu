@@ -3451,6 +3451,7 @@ int num_sms()
     return g_num_sms[device_index()];
 }
 }  // namespace
+int sm_count() { return num_sms(); }
 int smem_optin()
 {
     device_init();

@@ -7,8 +7,8 @@
 // per SM every level then waits on its own instruction latencies.  Here the
 // rows come from planes p, q, r, f (level-major, k*ld + col) that one thread
 // per (level, column) wrote, so a walk level is the recurrence alone: two
-// divisions sharing one correctly rounded reciprocal (qdiv), a product and a
-// difference, with the planes requested pd levels ahead.
+// divisions sharing one correctly rounded reciprocal, a product and a
+// difference.
 //
 //   top = 0 (minor_ng): rows 0..K-1 with K = nk, no extrapolation;
 //   top = 1 (dt_ng, oplus_ng): rows 0..K-1 with K = nk-1 and
@@ -18,10 +18,12 @@
 // boundary overwrite, the time filter and the floors.  Same operations in the
 // same order as the fused walks, so the same bits.
 #include <cfloat>
+#include <cstdint>
 
 #include "tg_internal.h"
 #include "tg_arith.cuh"
 #include "tg_stage.cuh"
+#include "tg_tile.cuh"
 
 namespace tg {
 namespace {
@@ -29,336 +31,237 @@ __device__ __forceinline__ double xm(double a, double b) { return __dmul_rn(a, b
 __device__ __forceinline__ double xs(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double xd(double a, double b) { return __ddiv_rn(a, b); }
 
-constexpr int kWalkThreads = 32;   // one warp per block: the walk's columns spread over every SM
-
-__global__ void __launch_bounds__(kWalkThreads) k_thomas_post(const double *P, const double *Q, const double *R,
-                                                              const double *Fv, double *x, int nk, int K, int top,
-                                                              int ncol, long ld, unsigned *status, PostStep post,
-                                                              int has_post, int pd)
+// The walk with the column tile held in shared memory, for launches of
+// few columns.  A block of kWalkTileThreads threads takes kTileCols columns:
+// together they copy the p, q, r, f rows of every level (every copy in flight
+// at once) and read the post-step inputs of their own levels into registers;
+// one thread per column walks (tile_thomas); then all store the rows through
+// the post-solve steps, each its own levels.  16 columns a block spread a
+// launch of few columns over twice the SMs a 32-column tile does, and 29 KB of
+// rows (57 levels) leave seven blocks per SM (a 32-column tile that also held
+// the post-step inputs took 87 KB: two).  The walk's chain bounds it; dt_ng
+// with its rows, 11,248 columns x 57 levels 61 -> 45 us, 2,072 columns 21.5 ->
+// 18.7 (the post-step stores had waited on the boundary values one by one).
+constexpr int kWalkTileThreads = 128;
+template <bool WIDE>
+__global__ void __launch_bounds__(kWalkTileThreads) k_thomas_post_tile(const double *P, const double *Q,
+                                                                       const double *R, const double *Fv, double *x,
+                                                                       int nk, int K, int top, int ncol, long ld,
+                                                                       unsigned *status, PostStep post, int has_post)
 {
-    extern __shared__ double w2_walk[];
-    const long col = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= ncol) return;
-    const int T = blockDim.x;
-    double *w2s = w2_walk + threadIdx.x;
-    auto pf_row = [&](int k) {
-        const long o = (long)k * ld + col;
-        pf_l1(P + o);
-        pf_l1(Q + o);
-        pf_l1(R + o);
-        pf_l1(Fv + o);
-    };
-    for (int kk = 1; kk < pd && kk < K; ++kk) pf_row(kk);
-    bool ok = true;
-    double w1 = 0.0, y1 = 0.0, w3 = 0.0, rprev = 0.0;
-    for (int k = 0; k < K; ++k) {
-        if (k + pd < K) pf_row(k + pd);
-        const long o = (long)k * ld + col;
-        const double p = P[o], q = Q[o], r = R[o], f = Fv[o];
-        if (k == 0) {
-            w1 = q;
-            y1 = __drcp_rn(w1);
-            w3 = qdiv(f, w1, y1);
-        } else {
-            const double w2 = qdiv(rprev, w1, y1);
-            w2s[(long)(k - 1) * T] = w2;
-            w1 = xs(q, xm(p, w2));
-            y1 = __drcp_rn(w1);
-            w3 = qdiv(xs(f, xm(p, w3)), w1, y1);
-        }
-        ok = ok && fabs(w1) <= DBL_MAX && w1 != 0.0;
-        x[o] = w3;
-        rprev = r;
-    }
-    const bool bcol = has_post && post.bnd_mask && post.bnd_mask[col];
-    double xn = w3;
-    const double xtop = w3;
-    bool fin = fabs(xn) <= DBL_MAX;
-    double park = K >= 2 ? x[(long)(K - 2) * ld + col] : 0.0;
-    if (top == 0 && has_post) post_store(post, true, bcol, x, (long)(K - 1) * ld + col, xn);
-    for (int kk = K - 3; kk > K - 2 - pd && kk >= 0; --kk) post_prefetch(post, has_post, bcol, x, (long)kk * ld + col);
-    for (int k = K - 2; k >= 0; --k) {
-        if (k - pd >= 0) post_prefetch(post, has_post, bcol, x, (long)(k - pd) * ld + col);
-        const double wk = park;
-        if (k >= 1) park = x[(long)(k - 1) * ld + col];
-        xn = xs(wk, xm(w2s[(long)k * T], xn));
-        fin = fin && fabs(xn) <= DBL_MAX;
-        post_store(post, has_post, bcol, x, (long)k * ld + col, xn);
-        if (top == 1 && k == K - 2) {
-            // xtop = x(K-1), xn = x(K-2): the two top solved rows
-            post_store(post, has_post, bcol, x, (long)K * ld + col, xd(xm(xtop, xtop), xn));
-            if (has_post) post_store(post, true, bcol, x, (long)(K - 1) * ld + col, xtop);
-        }
-    }
-    if (status && (!ok || !fin)) atomicOr(status, (ok ? 0u : FLAG_PIVOT) | (fin ? 0u : FLAG_NONFINITE));
-}
-// The same walk with the column tile held in shared memory, for launches of
-// few columns.  The kTileWarps warps of a block share one 32-column tile:
-// together they copy the p, q, r, f rows of every level (cp.async, every
-// copy in flight at once, each warp a quarter of the levels), then warp 0
-// alone runs the recurrence from shared memory, keeping the next level's
-// w2 = r(k)/w1(k) where r(k) was and the parked w3, then the solution, where
-// q(k) was; finally all warps
-// store the rows through the post-solve steps, each its quarter of the
-// levels.  The per-column serial part is the recurrence alone.
-constexpr int kTileWarps = 4;
-__global__ void __launch_bounds__(32 * kTileWarps) k_thomas_post_tile(const double *P, const double *Q,
-                                                                      const double *R, const double *Fv, double *x,
-                                                                      int nk, int K, int top, int ncol, long ld,
-                                                                      unsigned *status, PostStep post, int has_post)
-{
-    extern __shared__ double tile_walk[];
-    const int T = 32, t = threadIdx.x & 31, w = threadIdx.x >> 5, NW = kTileWarps;
-    const long col = (long)blockIdx.x * T + t;
+    constexpr int T = kTileCols, NG = kWalkTileThreads / T;
+    extern __shared__ __align__(16) double tile_walk[];
+    const int t = threadIdx.x % T, g = threadIdx.x / T;
+    const long c0 = (long)blockIdx.x * T, col = c0 + t;
     const bool live = col < ncol;
-    // with the post-solve steps, prev and cur of every stored row (K, and the
-    // top row for top = 1) come in with the rows; q holds the KS solved rows
-    const int KS = top == 1 ? K + 1 : K;
-    double *sp = tile_walk, *sq = sp + (long)K * T, *sr = sq + (long)KS * T, *sf = sr + (long)K * T;
-    double *sprev = sf + (long)K * T, *scur = sprev + (long)KS * T;
-    if (live) {
-        for (int k = w; k < K; k += NW) {
-            const long o = (long)k * ld + col;
-            const int s = k * T + t;
-            cp_async8(sp + s, P + o);
-            cp_async8(sq + s, Q + o);
-            cp_async8(sr + s, R + o);
-            cp_async8(sf + s, Fv + o);
-        }
-        if (has_post)
-            for (int k = w; k < KS; k += NW) {
-                const long o = (long)k * ld + col;
-                cp_async8(sprev + k * T + t, post.prev + o);
-                cp_async8(scur + k * T + t, post.cur + o);
-            }
+    const int KS = top == 1 ? K + 1 : K;   // q holds the KS solved rows
+    double *sp = tile_walk, *sr = sp + K * T, *sf = sr + K * T, *sq = sf + K * T;
+    double *dst[4] = {sp, sq, sr, sf};
+    const double *src[4] = {P + c0, Q + c0, R + c0, Fv + c0};
+    if (WIDE) {   // 8 lanes a row, 16 bytes each
+        const int c2 = (threadIdx.x % (T / 2)) * 2;
+        for (int k = threadIdx.x / (T / 2); k < K; k += 2 * NG)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) cp_async16_ca(dst[v] + k * T + c2, src[v] + (long)k * ld + c2);
+    } else if (live) {
+        for (int k = g; k < K; k += NG)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) cp_async8(dst[v] + k * T + t, src[v] + (long)k * ld + t);
     }
     cp_async_commit();
+    const bool bcol = live && has_post && post.bnd_mask && post.bnd_mask[col];
+    TilePost<NG, 8> ps;
+    if (live) ps.load(post, has_post, bcol, g, KS, ld, col);
     cp_async_wait<0>();
     __syncthreads();
-    if (w == 0 && live) {
-        // Level k divides by its pivot w1(k) twice: w3(k) and the next
-        // level's w2 = r(k)/w1(k) (the reference's operands, so the same
-        // quotients), kept where r(k) was.  The walk's chain is the
-        // recurrence alone: every quotient by Markstein's sequence, no
-        // branch, each level's operands read one level ahead.  A level whose
-        // operands leave the sequence's safe range (zeros, non-finite or
-        // extreme values) stops the stores; the levels from the first such
-        // one are then walked again with the IEEE fallback (qdiv2, qdiv1).
-        bool ok = true;
-        int bad = K;
-        double w1 = 0.0, y1 = 0.0, w2 = 0.0, w3 = 0.0;
-        auto level = [&](int k, double p, double q, double r, double f, bool top_level) {
-            w1 = k == 0 ? q : xs(q, xm(p, w2));
-            y1 = __drcp_rn(w1);
-            const double num = k == 0 ? f : xs(f, xm(p, w3));
-            ok = ok && (bad < K || finite_nz(w1));
-            const unsigned d = max(exp_dist(w1), max(exp_dist(num), top_level ? 0u : exp_dist(r)));
-            bad = d >= kExpSpan && bad == K ? k : bad;
-            w3 = div_markstein(num, w1, y1);
-            w2 = div_markstein(r, w1, y1);
-            if (bad > k) {
-                sr[k * T + t] = w2;
-                sq[k * T + t] = w3;
-            }
-        };
-        double pn = sp[t], qn = sq[t], rn = sr[t], fn = sf[t];
-        for (int k = 0; k < K - 1; ++k) {
-            const int s = k * T + t;
-            const double p = pn, q = qn, r = rn, f = fn;
-            pn = sp[s + T];
-            qn = sq[s + T];
-            rn = sr[s + T];
-            fn = sf[s + T];
-            level(k, p, q, r, f, false);
-        }
-        level(K - 1, pn, qn, rn, fn, true);
-        if (bad < K) {
-            w2 = bad > 0 ? sr[(bad - 1) * T + t] : 0.0;
-            w3 = bad > 0 ? sq[(bad - 1) * T + t] : 0.0;
-            for (int k = bad; k < K; ++k) {
-                const int s = k * T + t;
-                const double p = sp[s], q = sq[s], f = sf[s];
-                w1 = k == 0 ? q : xs(q, xm(p, w2));
-                y1 = __drcp_rn(w1);
-                const double num = k == 0 ? f : xs(f, xm(p, w3));
-                if (k + 1 < K) {
-                    qdiv2(num, sr[s], w1, y1, w3, w2);
-                    sr[s] = w2;
-                } else {
-                    w3 = qdiv1(num, w1, y1);
-                }
-                ok = ok && finite_nz(w1);
-                sq[s] = w3;
-            }
-        }
-        const double xtop = w3;
-        back_sweep(sq, sr, K, t, w3);
-        // x(k) = w3 - w2*x(k+1) carries a non-finite value down to x(0)
-        const bool fin = finite(sq[t]) && finite(xtop);
-        // x(nk-1) = x(nk-2)**2/x(nk-3) from the unfiltered values
-        if (top == 1) sq[K * T + t] = xd(xm(xtop, xtop), sq[(K - 2) * T + t]);
-        if (status && (!ok || !fin)) atomicOr(status, (ok ? 0u : FLAG_PIVOT) | (fin ? 0u : FLAG_NONFINITE));
-    }
+    if (threadIdx.x < T && live) tile_thomas<T>(sp, sq, sr, sf, K, top, t, status);
     __syncthreads();
-    if (!live) return;
-    if (has_post) {
-        const bool bcol = post.bnd_mask && post.bnd_mask[col];
-        for (int k = w; k < KS; k += NW)
-            post_store_v(post, bcol, x, (long)k * ld + col, sq[k * T + t], sprev[k * T + t], scur[k * T + t]);
-    } else {
-        for (int k = w; k < KS; k += NW) x[(long)k * ld + col] = sq[k * T + t];
-    }
+    if (live) ps.template store<T>(post, has_post, bcol, sq, x, t, g, KS, ld, col);
 }
 
-// The walk for launches above the tile limit, one warp per 32-column block:
-// each lane's rows of p, q, r, f stream through a two-buffer shared-memory
-// ring of kRingLevels levels, the copies of the next chunk in flight while
-// this one is walked (a lane reads only what it copied itself: no barrier).
-// w2 of every level stays in shared memory, w3 is parked in x; the main loop
-// is branch-free Markstein with the IEEE re-walk from the first out-of-range
-// level (from the planes in global memory), as in the tile walk.  The back
-// sweep leaves the solution in shared memory where w2 was, and the stores
-// through the post steps go out last.
-constexpr int kRingLevels = 4;
-__global__ void __launch_bounds__(32) k_thomas_post_ring(const double *P, const double *Q, const double *R,
-                                                         const double *Fv, double *x, int nk, int K, int top,
-                                                         int ncol, long ld, unsigned *status, PostStep post,
-                                                         int has_post)
+// The walk for launches of more columns, one warp per 32-column block.
+// The rows stream through a shared-memory ring of kRingStages stages of
+// kRingLevels levels (WIDE: 16-byte asynchronous copies, two rows per
+// instruction).  w2 and w3 of a level replace its p and q in the planes (each
+// lane its own column, behind the copies), and come back with the post-step
+// inputs, every lane its own values, through the same ring for the back sweep,
+// which stores each row as it solves it.  Alone on 43,216 columns x 57 levels
+// the walk took 107 us with w2 in shared memory, w3 parked in x and the stores
+// waiting on their inputs level by level (issue 20%, 6.6 long-scoreboard stalls
+// per issue); dt_ng there went from 203 to 130 us, minor_ng from 252 to 186.
+// The tile walk is taken while its blocks are resident all at once (16,576
+// columns at 57 levels, 7,104 at 113): dt_ng with its rows on 16,384 columns
+// took 66 us with the tiles and 68 on 16,770 with the ring; at 113 levels 142
+// us (16,384, tiles in three passes) against 126 (17,420, ring).
+constexpr int kRingLevels = 4, kRingStages = 3;
+constexpr int kRingDoubles = 5 * 32;   // a level of the back sweep: w2, w3, prev, cur, bnd
+template <bool WIDE>
+__global__ void __launch_bounds__(32) k_thomas_post_ring(double *P, double *Q, const double *R, const double *Fv,
+                                                         double *x, int nk, int K, int top, int ncol, long ld,
+                                                         unsigned *status, PostStep post, int has_post)
 {
-    extern __shared__ double ring_walk[];
-    const int T = 32, t = threadIdx.x, L = kRingLevels;
-    const long col = (long)blockIdx.x * T + t;
-    if (col >= ncol) return;
-    const int KS = top == 1 ? K + 1 : K, nch = (K + L - 1) / L;
-    double *rb = ring_walk, *sw = ring_walk + 2 * L * 4 * T;   // ring [2][L][4][32]; w2, then x: KS rows
-    const double *src[4] = {P, Q, R, Fv};
-    auto load = [&](int c) {
-        const int k0 = c * L, nl = K - k0 < L ? K - k0 : L;
-        double *buf = rb + (c & 1) * L * 4 * T + t;
-        for (int l = 0; l < nl; ++l)
+    constexpr int L = kRingLevels, C = kRingStages, RD = kRingDoubles;
+    extern __shared__ __align__(16) double ring_walk[];
+    const int t = threadIdx.x;
+    const long c0 = (long)blockIdx.x * 32, col = c0 + t;
+    const bool live = col < ncol;
+    const int nch = (K + L - 1) / L;
+    const int half = t >> 4, c2 = (t & 15) * 2;
+    const double *a0 = WIDE ? (half ? Q : P) + c0 + c2 : P + col, *a1 = WIDE ? (half ? Fv : R) + c0 + c2 : R + col;
+    auto issue = [&](int st, int j) {
+        double *d = ring_walk + st * L * RD;
 #pragma unroll
-            for (int v = 0; v < 4; ++v) cp_async8(buf + (l * 4 + v) * T, src[v] + (long)(k0 + l) * ld + col);
+        for (int l = 0; l < L; ++l) {
+            const int k = j * L + l;
+            if (k < K) {
+                const long o = (long)k * ld;
+                if (WIDE) {
+                    cp_async16_cg(d + l * RD + half * 32 + c2, a0 + o);
+                    cp_async16_cg(d + l * RD + 64 + half * 32 + c2, a1 + o);
+                } else if (live) {
+                    cp_async8(d + l * RD + t, a0 + o);
+                    cp_async8(d + l * RD + 32 + t, Q + o + col);
+                    cp_async8(d + l * RD + 64 + t, a1 + o);
+                    cp_async8(d + l * RD + 96 + t, Fv + o + col);
+                }
+            }
+        }
         cp_async_commit();
     };
+#pragma unroll 1
+    for (int j = 0; j < C; ++j) issue(j, j);
     bool ok = true;
-    int bad = K;
-    double w1 = 0.0, y1 = 0.0, w2 = 0.0, w3 = 0.0;
-    load(0);
-    for (int c = 0; c < nch; ++c) {
-        if (c + 1 < nch) load(c + 1);
-        else cp_async_commit();
-        cp_async_wait<1>();
-        const double *buf = rb + (c & 1) * L * 4 * T + t;
-        const int k0 = c * L, nl = K - k0 < L ? K - k0 : L;
-        for (int l = 0; l < nl; ++l) {
-            const int k = k0 + l;
-            const double p = buf[(l * 4) * T], q = buf[(l * 4 + 1) * T], r = buf[(l * 4 + 2) * T],
-                         f = buf[(l * 4 + 3) * T];
-            w1 = k == 0 ? q : xs(q, xm(p, w2));
-            y1 = __drcp_rn(w1);
-            const double num = k == 0 ? f : xs(f, xm(p, w3));
-            ok = ok && (bad < K || finite_nz(w1));
-            const unsigned d = max(exp_dist(w1), max(exp_dist(num), k + 1 == K ? 0u : exp_dist(r)));
-            bad = d >= kExpSpan && bad == K ? k : bad;
-            w3 = div_markstein(num, w1, y1);
-            w2 = div_markstein(r, w1, y1);
-            if (bad > k) {
-                sw[k * T + t] = w2;
-                x[(long)k * ld + col] = w3;
+    double w2 = 0.0, w3 = 0.0;
+    int st = 0;
+#pragma unroll 1
+    for (int j = 0; j < nch; ++j) {
+        cp_async_wait<C - 1>();
+        __syncwarp();
+        double *stg = ring_walk + st * L * RD + t;
+        if (j == 0) stg[0] = 0.0;   // row 0 has no p: x - 0*0 = x
+        auto step = [&](int l) {
+            const double p = stg[l * RD], q = stg[l * RD + 32], r = stg[l * RD + 64], f = stg[l * RD + 96];
+            const double w1 = xs(q, xm(p, w2));
+            const double y1 = __drcp_rn(w1);
+            const double num = xs(f, xm(p, w3));
+            if (max(exp_dist(w1), max(exp_dist(num), exp_dist(r))) < kExpSpan) {
+                w3 = div_markstein(num, w1, y1);
+                w2 = div_markstein(r, w1, y1);
+            } else {
+                const bool w1s = exp_safe(w1);
+                w3 = qdiv_pivot(num, w1, y1, w1s);
+                w2 = qdiv_pivot(r, w1, y1, w1s);
+                if (!w1s) ok = ok && finite_nz(w1);
+            }
+            const long o = (long)(j * L + l) * ld + col;
+            P[o] = w2;
+            Q[o] = w3;
+        };
+        if (live) {
+            if ((j + 1) * L <= K) {
+#pragma unroll
+                for (int l = 0; l < L; ++l) step(l);
+            } else {
+                for (int l = 0; j * L + l < K; ++l) step(l);
             }
         }
+        __syncwarp();
+        issue(st, j + C);
+        st = st + 1 == C ? 0 : st + 1;
     }
-    if (bad < K) {
-        // from the first out-of-range level, the divisions with their IEEE
-        // fallback, the rows read again from the planes
-        w2 = bad > 0 ? sw[(bad - 1) * T + t] : 0.0;
-        w3 = bad > 0 ? x[(long)(bad - 1) * ld + col] : 0.0;
-        for (int k = bad; k < K; ++k) {
-            const long o = (long)k * ld + col;
-            const double p = P[o], q = Q[o], f = Fv[o];
-            w1 = k == 0 ? q : xs(q, xm(p, w2));
-            y1 = __drcp_rn(w1);
-            const double num = k == 0 ? f : xs(f, xm(p, w3));
-            if (k + 1 < K) qdiv2(num, R[o], w1, y1, w3, w2);
-            else w3 = qdiv1(num, w1, y1);
-            ok = ok && finite_nz(w1);
-            sw[k * T + t] = w2;
-            x[o] = w3;
-        }
-    }
-    // back sweep: x(k) = w3(k) - w2(k)*x(k+1), w3 from x four levels ahead
-    const double xtop = w3;
-    double xn = xtop, rw[4] = {0., 0., 0., 0.};
+    cp_async_wait<0>();
+    __syncwarp();
+    if (!live) return;
+    // back sweep: x(k) = w3(k) - w2(k)*x(k+1), levels kh - L + 1 .. kh of stage
+    // d, kh = K - 2 - d*L; no lane reads another's copies
+    const bool bcol = has_post && post.bnd_mask && post.bnd_mask[col];
+    const int KB = K - 1, nbk = (KB + L - 1) / L;
+    auto issue_b = [&](int sb, int d) {
+        double *db = ring_walk + sb * L * RD + t;
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-        if (K - 2 - u >= 0) rw[u] = x[(long)(K - 2 - u) * ld + col];
-    sw[(K - 1) * T + t] = xtop;
-    int kb = K - 2;
-    for (; kb - 7 >= 0; kb -= 4) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int k = kb - u;
-            xn = xs(rw[u], xm(sw[k * T + t], xn));
-            rw[u] = x[(long)(k - 4) * ld + col];
-            sw[k * T + t] = xn;
-        }
-    }
-    for (; kb >= 0; kb -= 4) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int k = kb - u;
+        for (int l = 0; l < L; ++l) {
+            const int k = KB - 1 - d * L - l;
             if (k >= 0) {
-                xn = xs(rw[u], xm(sw[k * T + t], xn));
-                if (k - 4 >= 0) rw[u] = x[(long)(k - 4) * ld + col];
-                sw[k * T + t] = xn;
+                const long o = (long)k * ld + col;
+                cp_async8(db + l * RD, P + o);
+                cp_async8(db + l * RD + 32, Q + o);
+                if (has_post) {
+                    cp_async8(db + l * RD + 64, post.prev + o);
+                    cp_async8(db + l * RD + 96, post.cur + o);
+                    if (bcol) cp_async8(db + l * RD + 128, post.bnd + o);
+                }
             }
         }
+        cp_async_commit();
+    };
+#pragma unroll 1
+    for (int d = 0; d < C; ++d) issue_b(d, d);
+    // the rows above the ring: K-1 now, for top = 1 row K when x(K-2) is known
+    const long ot = (long)(K - 1) * ld + col;
+    const double xtop = w3;
+    double pk = 0.0, ck = 0.0, xn = w3;
+    if (top == 1 && has_post) {
+        pk = post.prev[ot + ld];
+        ck = post.cur[ot + ld];
     }
+    post_store(post, has_post, bcol, x, ot, xtop);
+    st = 0;
+#pragma unroll 1
+    for (int d = 0; d < nbk; ++d) {
+        cp_async_wait<C - 1>();
+        const double *g = ring_walk + st * L * RD + t;
+#pragma unroll
+        for (int l = 0; l < L; ++l) {
+            const int k = KB - 1 - d * L - l;
+            if (k >= 0) {
+                xn = xs(g[l * RD + 32], xm(g[l * RD], xn));
+                const long o = (long)k * ld + col;
+                if (has_post)
+                    post_store_v(post, false, x, o, bcol ? g[l * RD + 128] : xn, g[l * RD + 64], g[l * RD + 96]);
+                else
+                    x[o] = xn;
+                if (top == 1 && d == 0 && l == 0) {   // x(nk-1) = x(nk-2)**2/x(nk-3) from the unfiltered values
+                    const double xe = xd(xm(xtop, xtop), xn);
+                    if (has_post) post_store_v(post, bcol, x, ot + ld, xe, pk, ck);
+                    else x[ot + ld] = xe;
+                }
+            }
+        }
+        issue_b(st, d + C);
+        st = st + 1 == C ? 0 : st + 1;
+    }
+    cp_async_wait<0>();
     // x(k) = w3 - w2*x(k+1) carries a non-finite value down to x(0)
-    const bool fin = finite(sw[t]) && finite(xtop);
-    // x(nk-1) = x(nk-2)**2/x(nk-3) from the unfiltered values
-    if (top == 1) sw[K * T + t] = xd(xm(xtop, xtop), sw[(K - 2) * T + t]);
+    const bool fin = finite(xn) && finite(xtop);
     if (status && (!ok || !fin)) atomicOr(status, (ok ? 0u : FLAG_PIVOT) | (fin ? 0u : FLAG_NONFINITE));
-    if (has_post) {
-        const bool bcol = post.bnd_mask && post.bnd_mask[col];
-        for (int k = 0; k < KS; ++k) post_store(post, true, bcol, x, (long)k * ld + col, sw[k * T + t]);
-    } else {
-        for (int k = 0; k < KS; ++k) x[(long)k * ld + col] = sw[k * T + t];
-    }
 }
 }  // namespace
 
-cudaError_t launch_thomas_post(const double *p, const double *q, const double *r, const double *f, double *x, int nk,
-                               int K, int top, int ncol, long ld, unsigned *status, const PostStep *post,
-                               cudaStream_t st)
+cudaError_t launch_thomas_post(double *p, double *q, const double *r, const double *f, double *x, int nk, int K,
+                               int top, int ncol, long ld, unsigned *status, const PostStep *post, cudaStream_t st)
 {
     if (ncol <= 0) return cudaSuccess;
     if (K < 1 || K > nk || (top == 1 && (K != nk - 1 || K < 2))) return cudaErrorInvalidValue;
-    const int KS = top == 1 ? K + 1 : K;
-    const size_t tile = (size_t)32 * (3 * K + KS + (post ? 2 * KS : 0)) * sizeof(double);
-    if (ncol <= kSmallWalkColumns && tile <= (size_t)smem_optin()) {
+    const PostStep pv = post ? *post : PostStep{};
+    const int hp = post != nullptr, KS = top == 1 ? K + 1 : K;
+    auto aligned = [](const double *v) { return ((uintptr_t)v & 15) == 0; };
+    auto wide = [&](int T) {   // whole 16-byte pieces of rows of T columns lie in the planes
+        return ld % 2 == 0 && ld >= (long)(ncol + T - 1) / T * T && aligned(p) && aligned(q) && aligned(r) && aligned(f);
+    };
+    const size_t tile = (size_t)kTileCols * (3 * K + KS) * sizeof(double);
+    if (tile <= (size_t)smem_optin() && (ncol + kTileCols - 1) / kTileCols <= resident_by_smem(tile)) {
         once_per_device([] {
-            cudaFuncSetAttribute(k_thomas_post_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin());
+            cudaFuncSetAttribute(k_thomas_post_tile<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin());
+            cudaFuncSetAttribute(k_thomas_post_tile<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin());
         });
-        k_thomas_post_tile<<<(ncol + 31) / 32, 32 * kTileWarps, tile, st>>>(
-            p, q, r, f, x, nk, K, top, ncol, ld, status, post ? *post : PostStep{}, post != nullptr);
+        auto k = wide(kTileCols) ? k_thomas_post_tile<true> : k_thomas_post_tile<false>;
+        k<<<(ncol + kTileCols - 1) / kTileCols, kWalkTileThreads, tile, st>>>(p, q, r, f, x, nk, K, top, ncol, ld,
+                                                                             status, pv, hp);
         return cudaGetLastError();
     }
-    const size_t ring = (size_t)32 * (2 * kRingLevels * 4 + KS) * sizeof(double);
-    if (ring <= (size_t)smem_optin()) {
-        once_per_device([] {
-            cudaFuncSetAttribute(k_thomas_post_ring, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin());
-        });
-        k_thomas_post_ring<<<(ncol + 31) / 32, 32, ring, st>>>(p, q, r, f, x, nk, K, top, ncol, ld, status,
-                                                               post ? *post : PostStep{}, post != nullptr);
-        return cudaGetLastError();
-    }
-    const size_t smem = (size_t)kWalkThreads * (K > 1 ? K - 1 : 1) * sizeof(double);
-    once_per_device([] { cudaFuncSetAttribute(k_thomas_post, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin()); });
-    if (smem > (size_t)smem_optin()) return cudaErrorInvalidValue;
-    k_thomas_post<<<(ncol + kWalkThreads - 1) / kWalkThreads, kWalkThreads, smem, st>>>(
-        p, q, r, f, x, nk, K, top, ncol, ld, status, post ? *post : PostStep{}, post != nullptr,
-        walk_prefetch(ncol));
+    auto k = wide(32) ? k_thomas_post_ring<true> : k_thomas_post_ring<false>;
+    k<<<(ncol + 31) / 32, 32, sizeof(double) * kRingStages * kRingLevels * kRingDoubles, st>>>(
+        p, q, r, f, x, nk, K, top, ncol, ld, status, pv, hp);
     return cudaGetLastError();
 }
 }  // namespace tg
