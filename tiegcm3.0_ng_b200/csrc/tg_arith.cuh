@@ -1,6 +1,7 @@
 // Exact FP64 arithmetic helpers shared by the solver and assembly kernels.
 #pragma once
 #include <cfloat>
+#include <cmath>
 #include <cuda_runtime.h>
 
 namespace tg {
@@ -97,6 +98,44 @@ __device__ __forceinline__ double shapiro_at(At at, int t, int n, double sh)
     if (t == 1 || t == n - 2) return xsub(x, xmul(sh, xsub(xmul(8.0, x), xmul(8.0, m1))));
     const double m2 = xmul(xadd(at(2), at(-2)), 0.5);
     return xsub(x, xmul(sh, xadd(xsub(xmul(2.0, m2), xmul(8.0, m1)), xmul(6.0, x))));
+}
+
+// Division by a value every thread shares (the level spacing dz, a constant),
+// correctly rounded, y its correctly rounded reciprocal from the host.  EXACT:
+// b is a power of two with a normal reciprocal (the model's dz are 1/2, 1/4
+// and 1/8), where a*y and a/b round the same exact number for every a: one
+// multiplication in place of about ten operations.
+template <bool EXACT>
+struct DivBy {
+    static constexpr bool exact = EXACT;
+    double b, y;
+    __device__ __forceinline__ double operator()(double a) const { return EXACT ? xmul(a, y) : qdiv1(a, b, y); }
+};
+inline bool exact_reciprocal(double b)
+{
+    int e;
+    const double m = frexp(b, &e);
+    return (m == 0.5 || m == -0.5) && e > -1000 && e < 1000;
+}
+
+// exp(z) of a small argument: for |z| <= 1/8 the Taylor polynomial of degree
+// 11 (the first dropped term is below 3e-20 of the result), else the device
+// exp.  Rounding: the last step adds 1 to less than 1/8 of an ulp's error.
+__device__ __forceinline__ double exp_small(double z)
+{
+    if (!(fabs(z) <= 0.125)) return exp(z);
+    double p = 1.0 / 39916800.0;
+    p = fma(p, z, 1.0 / 3628800.0);
+    p = fma(p, z, 1.0 / 362880.0);
+    p = fma(p, z, 1.0 / 40320.0);
+    p = fma(p, z, 1.0 / 5040.0);
+    p = fma(p, z, 1.0 / 720.0);
+    p = fma(p, z, 1.0 / 120.0);
+    p = fma(p, z, 1.0 / 24.0);
+    p = fma(p, z, 1.0 / 6.0);
+    p = fma(p, z, 0.5);
+    p = fma(p, z, 1.0);
+    return fma(p, z, 1.0);
 }
 
 // A hint that brings the line holding p into L1 (no register, no wait).

@@ -14,6 +14,7 @@
 // level constants expz and dift at k.
 #include <atomic>
 #include <cfloat>
+#include <type_traits>
 
 #include "tg_internal.h"
 #include "tg_arith.cuh"
@@ -556,17 +557,18 @@ struct MinorIface {
     double pso1, pso2, pshe, do1dz, do2dz, dhedz, dmdz;
 };
 
-__device__ __forceinline__ MinorIface minor_iface(const MinorConsts &C, double o1, double o1m, double o2, double o2m,
+template <class Dz>
+__device__ __forceinline__ MinorIface minor_iface(const Dz &dz, double o1, double o1m, double o2, double o2m,
                                                   double he, double hem, double mb, double mbm)
 {
     MinorIface r;
-    r.dmdz = xd(xs(mb, mbm), C.dzp);
+    r.dmdz = dz(xs(mb, mbm));
     r.pso1 = xm(0.5, xa(o1, o1m));
     r.pso2 = xm(0.5, xa(o2, o2m));
     r.pshe = xm(0.5, xa(he, hem));
-    r.do1dz = xd(xs(o1, o1m), C.dzp);
-    r.do2dz = xd(xs(o2, o2m), C.dzp);
-    r.dhedz = xd(xs(he, hem), C.dzp);
+    r.do1dz = dz(xs(o1, o1m));
+    r.do2dz = dz(xs(o2, o2m));
+    r.dhedz = dz(xs(he, hem));
     return r;
 }
 
@@ -574,12 +576,13 @@ __device__ __forceinline__ MinorIface minor_iface(const MinorConsts &C, double o
 // of the three species and (t00/tni)**0.25, as exp(y*ln(tni/t00)).  With
 // |y*ln(tni/t00)| below 1 the argument's rounding adds about 2 ulp to exp's
 // own error, within the tolerance the device pow already needs against the
-// host library (the reference writes these as ** powers).
+// host library (the reference writes these as ** powers).  The species'
+// exponents 1.75-ss are 0.04 and below, so their arguments stay small.
 __device__ __forceinline__ void diffusion_powers(double tni, double (&df)[3], double &p25)
 {
-    const double lx = log(xd(tni, 273.0));
+    const double lx = log(qdiv1(tni, 273.0, 1.0 / 273.0));
 #pragma unroll
-    for (int n = 0; n < 3; ++n) df[n] = exp(xm(xs(1.75, kMSs[n]), lx));
+    for (int n = 0; n < 3; ++n) df[n] = exp_small(xm(xs(1.75, kMSs[n]), lx));
     p25 = exp(xm(-0.25, lx));
 }
 
@@ -609,12 +612,14 @@ __device__ __forceinline__ MinorLevel minor_level(const MinorConsts &C, const Mi
     const double sa1 = xa(xa(xm(s0, W[0]), xm(s1, W[1])), xm(s2, W[2]));
     const double sa2 = xa(xa(xm(s0, W[3]), xm(s1, W[4])), xm(s2, W[5]));
     const double sa3 = xa(xa(xm(s0, W[6]), xm(s1, W[7])), xm(s2, W[8]));
-    double ex = xs(1.0, xd(xa(C.rmx, I.dmdz), barm));
-    ex = xa(ex, xm(sa1, xs(I.do2dz, xm(xs(1.0, xd(xa(C.rmass_o2, I.dmdz), barm)), I.pso2))));
-    ex = xa(ex, xm(sa2, xs(I.do1dz, xm(xs(1.0, xd(xa(C.rmass_o1, I.dmdz), barm)), I.pso1))));
-    ex = xa(ex, xm(sa3, xs(I.dhedz, xm(xs(1.0, xd(xa(C.rmass_he, I.dmdz), barm)), I.pshe))));
+    // five quotients by barm share its reciprocal
+    const double yb = __drcp_rn(barm);
+    double ex = xs(1.0, qdiv1(xa(C.rmx, I.dmdz), barm, yb));
+    ex = xa(ex, xm(sa1, xs(I.do2dz, xm(xs(1.0, qdiv1(xa(C.rmass_o2, I.dmdz), barm, yb)), I.pso2))));
+    ex = xa(ex, xm(sa2, xs(I.do1dz, xm(xs(1.0, qdiv1(xa(C.rmass_o1, I.dmdz), barm, yb)), I.pso1))));
+    ex = xa(ex, xm(sa3, xs(I.dhedz, xm(xs(1.0, qdiv1(xa(C.rmass_he, I.dmdz), barm, yb)), I.pshe))));
     MinorLevel L;
-    L.dmdzs = xd(I.dmdz, barm);
+    L.dmdzs = qdiv1(I.dmdz, barm, yb);
     const double den = xa(xa(xa(C.phix[2], xm(s0, I.pso2)), xm(s1, I.pso1)), xm(s2, I.pshe));
     L.ax = -xd(xm(xd(barm, xm(tau, C.rmass_n2)), p25), den);
     L.thdiff = xs(ex, xd(xm(C.alfax, dtnidz), xm(C.dzp, tni)));
@@ -632,6 +637,7 @@ __global__ void __launch_bounds__(128) k_minor_ng(MinorFields F, MinorConsts C, 
     const int T = blockDim.x;
     auto at = [&](const double *p, int k) { return __ldg(p + k * ld + col); };
     const double dzp = C.dzp;
+    const DivBy<false> dzq{dzp, xd(1.0, dzp)};
     // lower-boundary mixing ratios and mean mass (:72-75)
     const double o2_0 = at(F.o2, 0), o1_0 = at(F.o1, 0), he_0 = at(F.he, 0), mb_0 = at(F.mbar, 0);
     const double bo2 = xa(xa(xa(xm(C.b[0], o2_0), xm(C.b[3], o1_0)), xm(C.b[6], he_0)), C.fb[0]);
@@ -674,7 +680,7 @@ __global__ void __launch_bounds__(128) k_minor_ng(MinorFields F, MinorConsts C, 
         if (k < nk - 1) {
             // level k+1 quantities
             const double o1k = at(F.o1, k + 1), o2k = at(F.o2, k + 1), hek = at(F.he, k + 1), mbk = at(F.mbar, k + 1);
-            const MinorIface I1 = minor_iface(C, o1k, o1_p, o2k, o2_p, hek, he_p, mbk, mb_p);
+            const MinorIface I1 = minor_iface(dzq, o1k, o1_p, o2k, o2_p, hek, he_p, mbk, mb_p);
             o1_p = o1k; o2_p = o2k; he_p = hek; mb_p = mbk;
             // tni of k+2 for dtnidz(k+1)
             double tni_pp = 0.0;
@@ -769,11 +775,12 @@ __device__ __forceinline__ double minor_tni(const MinorFields &F, int j, int nk,
 }
 
 // ax, thdiff, dmdz/barm of level j of one column (minor_ng.F90:72-153).
-__device__ __forceinline__ MinorLevel minor_level_at(const MinorFields &F, const MinorConsts &C, int j, int nk, long ld,
-                                                     long col)
+template <class Dz>
+__device__ __forceinline__ MinorLevel minor_level_at(const MinorFields &F, const MinorConsts &C, const Dz &dz, int j,
+                                                     int nk, long ld, long col)
 {
     auto at = [&](const double *p, int k) { return __ldg(p + k * ld + col); };
-    const double dzp = C.dzp, tlbc = __ldg(F.tlbc + col);
+    const double tlbc = __ldg(F.tlbc + col);
     MinorIface I;
     if (j == 0) {
         const double o2_0 = at(F.o2, 0), o1_0 = at(F.o1, 0), he_0 = at(F.he, 0), mb_0 = at(F.mbar, 0);
@@ -784,32 +791,33 @@ __device__ __forceinline__ MinorLevel minor_level_at(const MinorFields &F, const
             xd(1.0, xa(xa(xa(xm(bo2, C.rmassinv_o2), xm(bo1, C.rmassinv_o1)),
                           xm(xs(xs(xs(1.0, bo2), bo1), bhe), C.rmassinv_n2)),
                        xm(bhe, C.rmassinv_he)));
-        I.dmdz = xd(xs(mb_0, xmbari), dzp);
+        I.dmdz = dz(xs(mb_0, xmbari));
         I.pso1 = xm(0.5, xa(bo1, o1_0));
         I.pso2 = xm(0.5, xa(bo2, o2_0));
         I.pshe = xm(0.5, xa(bhe, he_0));
-        I.do1dz = xd(xs(o1_0, bo1), dzp);
-        I.do2dz = xd(xs(o2_0, bo2), dzp);
-        I.dhedz = xd(xs(he_0, bhe), dzp);
+        I.do1dz = dz(xs(o1_0, bo1));
+        I.do2dz = dz(xs(o2_0, bo2));
+        I.dhedz = dz(xs(he_0, bhe));
     } else {
-        I = minor_iface(C, at(F.o1, j), at(F.o1, j - 1), at(F.o2, j), at(F.o2, j - 1), at(F.he, j), at(F.he, j - 1),
+        I = minor_iface(dz, at(F.o1, j), at(F.o1, j - 1), at(F.o2, j), at(F.o2, j - 1), at(F.he, j), at(F.he, j - 1),
                         at(F.mbar, j), at(F.mbar, j - 1));
     }
     const double t0 = minor_tni(F, j, nk, ld, col, tlbc);
     double dt;
     if (j == 0) dt = xs(minor_tni(F, 1, nk, ld, col, tlbc), t0);
     else if (j == nk - 1) dt = xs(t0, minor_tni(F, nk - 2, nk, ld, col, tlbc));
-    else dt = xd(xs(minor_tni(F, j + 1, nk, ld, col, tlbc), minor_tni(F, j - 1, nk, ld, col, tlbc)), 2.0);
+    else dt = xm(xs(minor_tni(F, j + 1, nk, ld, col, tlbc), minor_tni(F, j - 1, nk, ld, col, tlbc)), 0.5);
     return minor_level(C, I, at(F.barm, j), t0, dt);
 }
 
-__global__ void __launch_bounds__(128) k_minor_levels(MinorFields F, MinorConsts C, double *lv, int nk, int ncol,
-                                                      long ld)
+template <bool EX>
+__global__ void __launch_bounds__(128) k_minor_levels(MinorFields F, MinorConsts C, DivBy<EX> dz, double *lv, int nk,
+                                                      int ncol, long ld)
 {
     const long col = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
     if (col >= ncol) return;
-    const MinorLevel L = minor_level_at(F, C, j, nk, ld, col);
+    const MinorLevel L = minor_level_at(F, C, dz, j, nk, ld, col);
     const long slab = (long)nk * ld;
     lv[(long)j * ld + col] = L.ax;
     lv[slab + (long)j * ld + col] = L.thdiff;
@@ -823,11 +831,12 @@ struct MinorRowIn {
     double sprod, xnmbar, ftm1, hadvec, sloss, w0, w1;
     MinorLevel L0, L1;
 };
-__device__ __forceinline__ void minor_row(const MinorFields &F, const MinorConsts &C, long col, int k, int nk,
-                                          double dfac, const MinorRowIn &in, double &p, double &q, double &r,
+template <class Dz>
+__device__ __forceinline__ void minor_row(const MinorFields &F, const MinorConsts &C, const Dz &dz, long col, int k,
+                                          int nk, double dfac, const MinorRowIn &in, double &p, double &q, double &r,
                                           double &f)
 {
-    const double dzp = C.dzp, rdz = xd(1.0, dzp);
+    const double dzp = C.dzp, rdz = dz.y;
     const MinorLevel &L0 = in.L0, &L1 = in.L1;
     const double expz = __ldg(F.expz + k);
     const double sp = xd(xm(in.sprod, C.rmx), in.xnmbar);
@@ -843,9 +852,9 @@ __device__ __forceinline__ void minor_row(const MinorFields &F, const MinorConst
         const double eddyq = xa(xm(xm(C.expzmid_inv, difk0), xa(rdz, xm(0.5, L0.dmdzs))),
                                 xm(xm(C.expzmid, difk1), xs(rdz, xm(0.5, L1.dmdzs))));
         const double wi = xm(0.5, xa(in.w0, in.w1));
-        p = xs(xd(molp, dzp), xd(xm(expz, xa(xm(eddyp, dfac), xm(0.5, wi))), dzp));
-        r = xs(xd(molr, dzp), xd(xm(expz, xs(xm(eddyr, dfac), xm(0.5, wi))), dzp));
-        q = xa(-xd(molq, dzp), xm(expz, xs(xa(xd(xm(eddyq, dfac), dzp), C.dtx2inv), in.sloss)));
+        p = xs(dz(molp), dz(xm(expz, xa(xm(eddyp, dfac), xm(0.5, wi)))));
+        r = xs(dz(molr), dz(xm(expz, xs(xm(eddyr, dfac), xm(0.5, wi)))));
+        q = xa(-dz(molq), xm(expz, xs(xa(dz(xm(eddyq, dfac)), C.dtx2inv), in.sloss)));
         if (k == 0) {
             const double l1 = __ldg(F.flbc1 + col), l2 = __ldg(F.flbc2 + col), l3 = __ldg(F.flbc3 + col);
             const double den = xs(l1, xm(xm(0.5, l2), dzp));
@@ -863,8 +872,9 @@ __device__ __forceinline__ void minor_row(const MinorFields &F, const MinorConst
 
 // Three-pass form, pass 2: row k of every column, one thread per (row,
 // column), into the planes pqrf (p, q, r, f, each nk*ld).
-__global__ void __launch_bounds__(128) k_minor_coefs(MinorFields F, MinorConsts C, const double *lv, double *pqrf,
-                                                     int nk, int ncol, long ld, double *sys_out)
+template <bool EX>
+__global__ void __launch_bounds__(128) k_minor_coefs(MinorFields F, MinorConsts C, DivBy<EX> dz, const double *lv,
+                                                     double *pqrf, int nk, int ncol, long ld, double *sys_out)
 {
     const long col = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= ncol) return;
@@ -902,7 +912,7 @@ __global__ void __launch_bounds__(128) k_minor_coefs(MinorFields F, MinorConsts 
         in.L1.dmdzs = __ldg(lv + 2 * slab + o + ld);
     }
     double p, q, r, f;
-    minor_row(F, C, col, k, nk, __ldg(F.dfactor + col), in, p, q, r, f);
+    minor_row(F, C, dz, col, k, nk, __ldg(F.dfactor + col), in, p, q, r, f);
     pqrf[o] = p;
     pqrf[slab + o] = q;
     pqrf[2 * slab + o] = r;
@@ -924,6 +934,7 @@ __global__ void __launch_bounds__(128) k_minor_rows(MinorFields F, MinorConsts C
                                                     int nk, int ncol, long ld, double *sys_out, unsigned *status,
                                                     PostStep post, int has_post, int pd)
 {
+    const DivBy<false> dz{C.dzp, xd(1.0, C.dzp)};
     extern __shared__ double smem_mr[];
     const long col = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= ncol) return;
@@ -984,7 +995,7 @@ __global__ void __launch_bounds__(128) k_minor_rows(MinorFields F, MinorConsts C
             in.L1.dmdzs = sg.at(b, 9);
         }
         double p, q, r, f;
-        minor_row(F, C, col, k, nk, dfac, in, p, q, r, f);
+        minor_row(F, C, dz, col, k, nk, dfac, in, p, q, r, f);
         const MinorLevel L1 = in.L1;
         if (sys_out) {
             sys_out[k * ld + col] = p;
@@ -1058,11 +1069,19 @@ cudaError_t launch_minor_ng(const MinorFields &F, const MinorConsts &C, double *
     while (T > 32 && (size_t)T * (nk - 1) * sizeof(double) > (size_t)optin) T /= 2;
     const size_t smem = (size_t)T * (nk - 1 > 0 ? nk - 1 : 1) * sizeof(double);
     if (smem > (size_t)optin) return cudaErrorInvalidValue;
+    const DivBy<false> dzq{C.dzp, 1.0 / C.dzp};
     if (scratch && assembly_mode() == 2) {
         const long slab = (long)nk * ld;
         double *pqrf = scratch + 3 * slab;
-        k_minor_levels<<<dim3((ncol + 127) / 128, nk), 128, 0, st>>>(F, C, scratch, nk, ncol, ld);
-        k_minor_coefs<<<dim3((ncol + 127) / 128, nk), 128, 0, st>>>(F, C, scratch, pqrf, nk, ncol, ld, sys_out);
+        const dim3 grid((ncol + 127) / 128, nk);
+        if (exact_reciprocal(C.dzp)) {
+            const DivBy<true> dz{C.dzp, 1.0 / C.dzp};
+            k_minor_levels<true><<<grid, 128, 0, st>>>(F, C, dz, scratch, nk, ncol, ld);
+            k_minor_coefs<true><<<grid, 128, 0, st>>>(F, C, dz, scratch, pqrf, nk, ncol, ld, sys_out);
+        } else {
+            k_minor_levels<false><<<grid, 128, 0, st>>>(F, C, dzq, scratch, nk, ncol, ld);
+            k_minor_coefs<false><<<grid, 128, 0, st>>>(F, C, dzq, scratch, pqrf, nk, ncol, ld, sys_out);
+        }
         return launch_thomas_post(pqrf, pqrf + slab, pqrf + 2 * slab, pqrf + 3 * slab, out, nk, nk, 0, ncol, ld,
                                   status, post, st);
     }
@@ -1072,7 +1091,7 @@ cudaError_t launch_minor_ng(const MinorFields &F, const MinorConsts &C, double *
         int TR = 128;
         while (TR > 32 && (size_t)TR * per_r > (size_t)optin) TR /= 2;
         if ((size_t)TR * per_r > (size_t)optin) return cudaErrorInvalidValue;
-        k_minor_levels<<<dim3((ncol + 127) / 128, nk), 128, 0, st>>>(F, C, scratch, nk, ncol, ld);
+        k_minor_levels<false><<<dim3((ncol + 127) / 128, nk), 128, 0, st>>>(F, C, dzq, scratch, nk, ncol, ld);
         k_minor_rows<<<(ncol + TR - 1) / TR, TR, (size_t)TR * per_r, st>>>(F, C, scratch, out, nk, ncol, ld, sys_out,
                                                                           status, pv, hp, walk_prefetch(ncol));
         return cudaGetLastError();
@@ -1107,8 +1126,10 @@ __global__ void __launch_bounds__(128) k_minor_diag_ng(MinorFields F, MinorConst
     d[6 * slab] = -__ldg(F.hadvec + o);
     double mol = 0.0, eddy = 0.0, vadv = 0.0;
     if (k >= 1 && k <= nk - 2) {
-        const MinorLevel L0 = minor_level_at(F, C, k, nk, ld, col), L1 = minor_level_at(F, C, k + 1, nk, ld, col);
         const double rdz = xd(1.0, dzp);
+        const DivBy<false> dzq{dzp, rdz};
+        const MinorLevel L0 = minor_level_at(F, C, dzq, k, nk, ld, col),
+                         L1 = minor_level_at(F, C, dzq, k + 1, nk, ld, col);
         const double molp = xm(L0.ax, xa(rdz, xm(0.5, L0.thdiff)));
         const double molr = xm(L1.ax, xs(rdz, xm(0.5, L1.thdiff)));
         const double molq = xa(xm(L0.ax, xs(rdz, xm(0.5, L0.thdiff))), xm(L1.ax, xa(rdz, xm(0.5, L1.thdiff))));
@@ -1160,7 +1181,7 @@ __device__ __forceinline__ void comp_level(const CompConsts &C, double o2i, doub
     const double tau = 1.86e+3, thdiffalpha = -0.38;
     double df[3], p25;
     diffusion_powers(tni, df, p25);
-    const double rinv = xd(1.0, embari);
+    const double rinv = __drcp_rn(embari);
     L.ep[0] = xs(1.0, xm(rinv, xa(C.rmass_o2, dembardz)));
     L.ep[1] = xs(1.0, xm(rinv, xa(C.rmass_o1, dembardz)));
     L.ep[2] = xs(1.0, xm(rinv, xa(C.rmass_he, dembardz)));
@@ -1183,10 +1204,10 @@ __device__ __forceinline__ void comp_level(const CompConsts &C, double o2i, doub
     L.a23 = A[7];
     L.a32 = A[5];
     inv3_ieee(A, W);
-    const double wks1 = xd(xm(xm(embari, C.rmassinv_n2), p25), tau);
+    const double wks1 = qdiv1(xm(xm(embari, C.rmassinv_n2), p25), tau, 1.0 / tau);
 #pragma unroll
     for (int e = 0; e < 9; ++e) L.ak[e] = xm(W[e], wks1);
-    L.wks4 = xd(dembardz, xm(embari, 2.0));
+    L.wks4 = qdiv1(dembardz, xm(embari, 2.0), xm(rinv, 0.5));   // half the reciprocal, exactly
 }
 }  // namespace
 }  // namespace tg
@@ -1195,15 +1216,16 @@ namespace tg {
 // Row k of the comp_ng block system (comp_ng.F90:213-279): P, Q, R and f
 // from the level quantities of levels k (Lk) and k+1 (Lp) and the fields of
 // level k (through Src), with both boundary folds; flx00 is set at the top row.
-template <class Src>
-__device__ __forceinline__ void comp_row(const CompFields &F, const CompConsts &C, const Src &src, const CompLevel &Lk,
+template <class Src, class Dz>
+__device__ __forceinline__ void comp_row(const CompFields &F, const CompConsts &C, const Dz &dv, const Src &src,
+                                         const CompLevel &Lk,
                                          const CompLevel &Lp, int k, int nk, long ld, long col, double dfac,
                                          double flx_he, double (&P)[9], double (&Q)[9], double (&R)[9],
                                          double (&f)[3], double &flx00)
 {
     auto at = [&](const double *p, int kk) { return __ldg(p + kk * ld + col); };
     const double tau = 1.86e+3, t00 = 273.;
-    const double dz = C.dz, rdz = xd(1.0, dz);
+    const double dz = C.dz, rdz = dv.y;
     const double wi = xm(0.5, xa(src.w(k), src.w1(k)));
     const double difk0 = __ldg(F.difk + k), difk1 = __ldg(F.difk + k + 1), ez = __ldg(F.expz + k);
     // mol / eddy coefficients and the rows (comp_ng.F90:213-244)
@@ -1211,13 +1233,13 @@ __device__ __forceinline__ void comp_row(const CompFields &F, const CompConsts &
     const double eddyr = xm(xm(C.expzmid, difk1), xa(rdz, Lp.wks4));
     const double eddyq =
         xa(xm(xm(C.expzmid_inv, difk0), xa(rdz, Lk.wks4)), xm(xm(C.expzmid, difk1), xs(rdz, Lp.wks4)));
-    const double ezdz = xd(ez, dz);
+    const double ezdz = dv(ez);
     const double tp = xm(ezdz, xa(xm(eddyp, dfac), xm(0.5, wi)));
     const double tr = xm(ezdz, xs(xm(eddyr, dfac), xm(0.5, wi)));
-    const double tq = xm(ez, xa(xd(xm(eddyq, dfac), dz), C.dtx2inv));
+    const double tq = xm(ez, xa(dv(xm(eddyq, dfac)), C.dtx2inv));
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
-        const double hk = xd(Lk.ep[m], 2.0), hp = xd(Lp.ep[m], 2.0);
+        const double hk = xm(Lk.ep[m], 0.5), hp = xm(Lp.ep[m], 0.5);
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             const int e = i + 3 * m;
@@ -1225,9 +1247,9 @@ __device__ __forceinline__ void comp_row(const CompFields &F, const CompConsts &
             const double molr = xm(Lp.ak[e], xs(rdz, hp));
             const double molq = xa(xm(Lk.ak[e], xs(rdz, hk)), xm(Lp.ak[e], xa(rdz, hp)));
             const double fsl = xm(ez, src.fs((m + 1) * 3 + i, k));
-            P[e] = i == m ? xs(xd(molp, dz), tp) : xd(molp, dz);
-            R[e] = i == m ? xs(xd(molr, dz), tr) : xd(molr, dz);
-            Q[e] = i == m ? xs(xa(-xd(molq, dz), tq), fsl) : xs(-xd(molq, dz), fsl);
+            P[e] = i == m ? xs(dv(molp), tp) : dv(molp);
+            R[e] = i == m ? xs(dv(molr), tr) : dv(molr);
+            Q[e] = i == m ? xs(xa(-dv(molq), tq), fsl) : xs(-dv(molq), fsl);
         }
     }
 #pragma unroll
@@ -1403,6 +1425,7 @@ __device__ __forceinline__ void comp_walk(const CompFields &F, const CompConsts 
     const long slab = (long)nk * ld;
     const double dfac = __ldg(F.dfactor + col);
     const double flx_he = C.calc_helium ? __ldg(F.flx_he + col) : 0.0;
+    const DivBy<false> dv{C.dz, xd(1.0, C.dz)};
     CompLevel Lk, Lp;
     src.first(Lp);
     double G[9], z[3];
@@ -1417,7 +1440,7 @@ __device__ __forceinline__ void comp_walk(const CompFields &F, const CompConsts 
         Lk = Lp;
         src.next(k, Lp);
         double P[9], Q[9], R[9], f[3];
-        comp_row(F, C, src, Lk, Lp, k, nk, ld, col, dfac, flx_he, P, Q, R, f, flx00);
+        comp_row(F, C, dv, src, Lk, Lp, k, nk, ld, col, dfac, flx_he, P, Q, R, f, flx00);
         if (sys_out) {
             double *so = sys_out + (long)k * ld + col;
 #pragma unroll
@@ -1508,7 +1531,9 @@ __global__ void __launch_bounds__(128) k_comp_ng(CompFields F, CompConsts C, dou
 // col; the top level's a22, a33, a23, a32 in 4 rows of ld after them.
 constexpr int kCompPlanes = 13;
 
-__global__ void __launch_bounds__(128) k_comp_levels(CompFields F, CompConsts C, double *lv, int nk, int ncol, long ld)
+template <bool EX>
+__global__ void __launch_bounds__(128) k_comp_levels(CompFields F, CompConsts C, DivBy<EX> dv, double *lv, int nk,
+                                                     int ncol, long ld)
 {
     const long col = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
@@ -1519,11 +1544,10 @@ __global__ void __launch_bounds__(128) k_comp_levels(CompFields F, CompConsts C,
         src.first(L);
     } else {
         auto at = [&](const double *p, int k) { return __ldg(p + k * ld + col); };
-        const double dz = C.dz;
         const double mb0 = at(F.mbar, j - 1), mb1 = at(F.mbar, j), tn0 = at(F.tn, j - 1), tn1 = at(F.tn, j);
         comp_level(C, xm(0.5, xa(at(F.o2, j - 1), at(F.o2, j))), xm(0.5, xa(at(F.o1, j - 1), at(F.o1, j))),
                    xm(0.5, xa(at(F.he, j - 1), at(F.he, j))), xm(0.5, xa(mb0, mb1)), xm(0.5, xa(tn0, tn1)),
-                   xd(xs(mb1, mb0), dz), xd(xs(tn1, tn0), dz), j != nk - 1, L);
+                   dv(xs(mb1, mb0)), dv(xs(tn1, tn0)), j != nk - 1, L);
     }
     const long slab = (long)nk * ld, o = (long)j * ld + col;
 #pragma unroll
@@ -1671,157 +1695,189 @@ __global__ void __launch_bounds__(kCompRowThreads, 5) k_comp_rows(CompFields F, 
     comp_walk(F, C, src, out, scr, nk, ld, col, sys_out, status, pd);
 }
 
-// Three-pass form, pass 2: row k of every column, one thread per (row,
-// column), into 30 row planes (P, Q, R by entry i + 3m, then f); the top row
-// also leaves flx00 in its column's slot.
-__global__ void __launch_bounds__(128) k_comp_coefs(CompFields F, CompConsts C, const double *lv, double *rows,
-                                                    double *flx00_row, int nk, int ncol, long ld, double *sys_out)
+// Three-pass form, passes 2 and 3 in one kernel, a 32-column tile per block:
+// warp 0 runs the block recurrence, NP warps form its rows.  While
+// warp 0 walks one chunk of NP levels, each producer forms one
+// level of the next from the level planes and the fields (comp_row) straight
+// into the other half of a two-buffer shared-memory ring, so the 30 row planes
+// never leave the SM.  Gamma and z of every level go to the tile's own scratch
+// slice, (level, entry, column) with the column fastest, and come back through
+// the same memory for the back sweep.  Same arithmetic as comp_walk.
+// What bounds it: the recurrence's dependency chain (one warp per tile, about
+// 800 cycles a level) on few columns; on many the reads (846 MB of 43,216 x 57
+// in 252 us before the next level's lines were requested into L2 ahead, which
+// took the routine from 330 to 279 us).  It replaced rows formed by their own
+// kernel and a 16-column walk up to 16,384 columns, and a walk that formed its
+// rows above: comp_ng 2,072 columns x 57 levels 83 -> 51 us, 11,248 229 -> 91,
+// 43,216 451 -> 279, 43,216 x 113 880 -> 540.
+constexpr size_t comp_solve_bytes(int np) { return sizeof(double) * 2 * np * 30 * 32; }
+template <bool EX, int NP>
+__global__ void __launch_bounds__(32 * (1 + NP), NP == 4 ? 3 : 5) k_comp_solve(
+    CompFields F, CompConsts C, DivBy<EX> dv, const double *lv, double *out, double *scr, int nk, int ncol, long ld,
+    double *sys_out, unsigned *status)
 {
-    const long col = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= ncol) return;
-    const int k = blockIdx.y;
-    const long slab = (long)nk * ld, o = (long)k * ld + col;
+    extern __shared__ __align__(16) double comp_ring[];
+    __shared__ double flx00_s[32];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long col = (long)blockIdx.x * 32 + lane, slab = (long)nk * ld;
+    const bool live = col < ncol;
+    const int K = nk - 1, nch = (K + NP - 1) / NP;
+    double *gz = scr + (long)blockIdx.x * 12 * nk * 32;
     CompPlaneSrc src{{F, ld, col, nk}, lv};
-    CompLevel Lk, Lp;
-    src.load(k, Lk);
-    src.load(k + 1, Lp);
-    double P[9], Q[9], R[9], f[3], flx00 = 1.0;
-    comp_row(F, C, src, Lk, Lp, k, nk, ld, col, __ldg(F.dfactor + col),
-             C.calc_helium ? __ldg(F.flx_he + col) : 0.0, P, Q, R, f, flx00);
+    const double flx_he = live && C.calc_helium ? __ldg(F.flx_he + col) : 0.0;
+    if (w > 0) {
+        const double dfac = live ? __ldg(F.dfactor + col) : 0.0;
+#pragma unroll 1
+        for (int c = 0; c <= nch; ++c) {
+            const int k = c * NP + w - 1;
+            if (k + NP < K && live && (lane & 15) == 0) {   // the lines this warp's next level reads, into L2
+                const long o = (long)(k + NP) * ld + col;
+                auto pf = [&](const double *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); };
 #pragma unroll
-    for (int e = 0; e < 9; ++e) {
-        rows[(long)e * slab + o] = P[e];
-        rows[(long)(9 + e) * slab + o] = Q[e];
-        rows[(long)(18 + e) * slab + o] = R[e];
-    }
+                for (int e = 0; e < kCompPlanes; ++e) pf(lv + e * slab + o + ld);
 #pragma unroll
-    for (int i = 0; i < 3; ++i) rows[(long)(27 + i) * slab + o] = f[i];
-    if (k == nk - 2) flx00_row[col] = flx00;
-    if (sys_out) {
-        double *so = sys_out + o;
+                for (int e = 0; e < 12; ++e) pf(F.fs + e * slab + o);
+                const double *one[] = {F.o2nm_smooth, F.o1nm_smooth, F.henm_smooth, F.o2_advec, F.o1_advec, F.he_advec,
+                                       F.hdo2, F.hdo1, F.hdhe, F.w};
 #pragma unroll
-        for (int e = 0; e < 9; ++e) {
-            so[(long)e * slab] = P[e];
-            so[(long)(9 + e) * slab] = Q[e];
-            so[(long)(18 + e) * slab] = R[e];
+                for (int e = 0; e < 10; ++e) pf(one[e] + o);
+            }
+            if (k < K && live) {
+                CompLevel Lk, Lp;
+                src.load(k, Lk);
+                src.load(k + 1, Lp);
+                double P[9], Q[9], R[9], f[3], flx00 = 1.0;
+                comp_row(F, C, dv, src, Lk, Lp, k, nk, ld, col, dfac, flx_he, P, Q, R, f, flx00);
+                double *r = comp_ring + ((c & 1) * NP + w - 1) * 30 * 32 + lane;
+#pragma unroll
+                for (int e = 0; e < 9; ++e) {
+                    r[e * 32] = P[e];
+                    r[(9 + e) * 32] = Q[e];
+                    r[(18 + e) * 32] = R[e];
+                }
+#pragma unroll
+                for (int i = 0; i < 3; ++i) r[(27 + i) * 32] = f[i];
+                if (k == K - 1) flx00_s[lane] = flx00;
+                if (sys_out) {
+                    double *so = sys_out + (long)k * ld + col;
+#pragma unroll
+                    for (int e = 0; e < 9; ++e) {
+                        so[(long)e * slab] = P[e];
+                        so[(long)(9 + e) * slab] = Q[e];
+                        so[(long)(18 + e) * slab] = R[e];
+                    }
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) so[(long)(27 + i) * slab] = f[i];
+                }
+            }
+            __syncthreads();
         }
-#pragma unroll
-        for (int i = 0; i < 3; ++i) so[(long)(27 + i) * slab] = f[i];
+        return;
     }
-}
-
-// Three-pass form, pass 3: the block recurrence over the row planes, on a
-// 16-column tile per block of kCompTileWarps warps.  The 30 row planes
-// stream through a two-buffer shared-memory ring, kCompChunk levels per
-// buffer: all warps copy the next
-// chunk (cp.async) while warp 0 runs the recurrence over this one.  Gamma
-// and z of every level go to the global scratch (L2) and come back through
-// the same ring, top down, for the back sweep.  Same arithmetic
-// (comp_forward, comp_back_level, comp_top), same bits.
-constexpr int kCompTileCols = 16, kCompChunk = 8, kCompTileWarps = 4;
-constexpr size_t kCompTileBytes = sizeof(double) * 2 * kCompChunk * 30 * kCompTileCols;
-__global__ void __launch_bounds__(32 * kCompTileWarps) k_comp_walk_tile(CompFields F, CompConsts C, const double *lv,
-                                                                        const double *rows, const double *flx00_row,
-                                                                        double *out, double *scr, int nk, int ncol,
-                                                                        long ld, unsigned *status)
-{
-    extern __shared__ double comp_tile[];
-    constexpr int TC = kCompTileCols, L = kCompChunk, NT = 32 * kCompTileWarps;
-    double *ring = comp_tile;
-    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    const long col0 = (long)blockIdx.x * TC, col = col0 + lane;
-    const long slab = (long)nk * ld;
-    const int K = nk - 1, nch = (K + L - 1) / L;
-    // chunk c (levels c*L .. c*L+L-1 below K) into buffer c & 1, laid out
-    // [level][plane][column]
-    auto load = [&](int c) {
-        const int k0 = c * L, nl = K - k0 < L ? K - k0 : L;
-        double *buf = ring + (c & 1) * L * 30 * TC;
-        for (int i = tid; i < nl * 30 * TC; i += NT) {
-            const int j = i % TC, lv30 = i / TC, l = lv30 / 30, v = lv30 - 30 * l;
-            if (col0 + j < ncol) cp_async8(buf + i, rows + (long)v * slab + (long)(k0 + l) * ld + col0 + j);
-        }
-        cp_async_commit();
-    };
-    const bool walker = w == 0 && lane < TC && col < ncol;
     double G[9], z[3];
 #pragma unroll
     for (int e = 0; e < 9; ++e) G[e] = 0.0;
 #pragma unroll
     for (int i = 0; i < 3; ++i) z[i] = 0.0;
     bool ok = true;
-    load(0);
+    __syncthreads();   // chunk 0 is formed
+#pragma unroll 1
     for (int c = 0; c < nch; ++c) {
-        if (c + 1 < nch) load(c + 1);
-        else cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        if (walker) {
-            const double *buf = ring + (c & 1) * L * 30 * TC + lane;
-            const int k0 = c * L, nl = K - k0 < L ? K - k0 : L;
-            for (int l = 0; l < nl; ++l) {
-                const double *r = buf + l * 30 * TC;
-                double P[9], Q[9], R[9], f[3];
+        if (live)
+#pragma unroll 1
+            for (int l = 0; l < NP && c * NP + l < K; ++l) {
+                const int k = c * NP + l;
+                const double *r = comp_ring + ((c & 1) * NP + l) * 30 * 32 + lane;
+                double Q[9], W[9], v[3], Rv[9];
+                // row 0's P is zero: x - 0*0 = x
 #pragma unroll
-                for (int e = 0; e < 9; ++e) {
-                    P[e] = r[e * TC];
-                    Q[e] = r[(9 + e) * TC];
-                    R[e] = r[(18 + e) * TC];
+                for (int m = 0; m < 3; ++m)
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) {
+                        double q = r[(9 + i + 3 * m) * 32];
+#pragma unroll
+                        for (int n = 0; n < 3; ++n) q = xs(q, xm(r[(i + 3 * n) * 32], G[n + 3 * m]));
+                        Q[i + 3 * m] = q;
+                    }
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    double q = r[(27 + i) * 32];
+#pragma unroll
+                    for (int m = 0; m < 3; ++m) q = xs(q, xm(r[(i + 3 * m) * 32], z[m]));
+                    v[i] = q;
                 }
 #pragma unroll
-                for (int i = 0; i < 3; ++i) f[i] = r[(27 + i) * TC];
-                comp_forward(P, Q, R, f, k0 + l, nk, ld, col, scr, G, z, ok);
+                for (int e = 0; e < 9; ++e) Rv[e] = r[(18 + e) * 32];
+                inv3_ieee(Q, W);
+#pragma unroll
+                for (int e = 0; e < 9; ++e) ok = ok && fabs(W[e]) <= DBL_MAX;
+                double *g = gz + (long)k * (12 * 32) + lane;
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    z[i] = xa(xa(xm(W[i], v[0]), xm(W[i + 3], v[1])), xm(W[i + 6], v[2]));
+                    g[(9 + i) * 32] = z[i];
+                }
+#pragma unroll
+                for (int m = 0; m < 3; ++m)
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) {
+                        G[i + 3 * m] = xa(xa(xm(W[i], Rv[3 * m]), xm(W[i + 3], Rv[1 + 3 * m])), xm(W[i + 6], Rv[2 + 3 * m]));
+                        g[(i + 3 * m) * 32] = G[i + 3 * m];
+                    }
             }
-        }
         __syncthreads();
     }
-    // back sweep (comp_ng.F90:317-324): level k from the Gamma/z row k+1,
-    // k = nk-3 .. 0, chunk d holding levels kh(d) - l, l < L
-    const int KB = nk - 2, nb = (KB + L - 1) / L;
-    auto load_b = [&](int d) {
-        const int kh = nk - 3 - d * L, nl = KB - d * L < L ? KB - d * L : L;
-        double *buf = ring + (d & 1) * L * 30 * TC;
-        for (int i = tid; i < nl * 12 * TC; i += NT) {
-            const int j = i % TC, le = i / TC, l = le / 12, e = le - 12 * l;
-            if (col0 + j < ncol) cp_async8(buf + i, scr + (long)(kh - l + 1) * 12 * ld + (long)e * ld + col0 + j);
+    // back sweep (comp_ng.F90:317-324): level k from z(k+1), Gamma(k+1), which
+    // row k of the slice holds; stage d holds levels kh - LB + 1 .. kh, kh = nk-3 - d*LB
+    constexpr int CB = 4, LB = 2 * NP * 30 / (CB * 12);
+    const int KB = nk - 2, nbk = (KB + LB - 1) / LB;
+    auto issue_b = [&](int sb, int d) {
+        if (d < nbk) {
+            const int kh = KB - 1 - d * LB, kl = kh - LB + 1 > 0 ? kh - LB + 1 : 0;
+            const double *s = gz + (long)kl * (12 * 32) + lane * 2;
+            double *dst = comp_ring + sb * LB * 12 * 32 + lane * 2;
+            const int n = (kh - kl + 1) * 6;   // two rows per copy
+#pragma unroll 6
+            for (int i = 0; i < n; ++i) cp_async16_cg(dst + i * 64, s + i * 64);
         }
         cp_async_commit();
     };
+    asm volatile("" ::: "memory");
+    __syncwarp();
+#pragma unroll 1
+    for (int d = 0; d < CB; ++d) issue_b(d, d);
     bool fin = true;
     double x[3], xb[3];
-    if (walker)
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            x[i] = xb[i] = z[i];
-            out[(long)i * slab + (long)(nk - 2) * ld + col] = x[i];
-            fin = fin && fabs(x[i]) <= DBL_MAX;
-        }
-    load_b(0);
-    for (int d = 0; d < nb; ++d) {
-        if (d + 1 < nb) load_b(d + 1);
-        else cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        if (walker) {
-            const double *buf = ring + (d & 1) * L * 30 * TC + lane;
-            const int kh = nk - 3 - d * L, nl = KB - d * L < L ? KB - d * L : L;
-            for (int l = 0; l < nl; ++l) {
-                double g[9], zk[3];
-#pragma unroll
-                for (int e = 0; e < 9; ++e) g[e] = buf[(l * 12 + e) * TC];
-#pragma unroll
-                for (int i = 0; i < 3; ++i) zk[i] = buf[(l * 12 + 9 + i) * TC];
-                comp_back_level(g, zk, x, fin, out, slab, (long)(kh - l) * ld + col);
-            }
-        }
-        __syncthreads();
+    for (int i = 0; i < 3; ++i) {
+        x[i] = xb[i] = z[i];
+        if (live) out[(long)i * slab + (long)(nk - 2) * ld + col] = x[i];
+        fin = fin && fabs(x[i]) <= DBL_MAX;
     }
-    if (!walker) return;
-    CompPlaneSrc src{{F, ld, col, nk}, lv};
+#pragma unroll 1
+    for (int d = 0; d < nbk; ++d) {
+        cp_async_wait<CB - 1>();
+        __syncwarp();
+        const int kh = KB - 1 - d * LB, kl = kh - LB + 1 > 0 ? kh - LB + 1 : 0;
+        const double *g = comp_ring + (d & (CB - 1)) * LB * 12 * 32 + (kh - kl) * (12 * 32) + lane;
+        if (live)
+#pragma unroll 1
+            for (int k = kh; k >= kl; --k, g -= 12 * 32) {
+                double ga[9], zk[3];
+#pragma unroll
+                for (int e = 0; e < 9; ++e) ga[e] = g[e * 32];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) zk[i] = g[(9 + i) * 32];
+                comp_back_level(ga, zk, x, fin, out, slab, (long)k * ld + col);
+            }
+        __syncwarp();
+        issue_b(d & (CB - 1), d + CB);
+    }
+    cp_async_wait<0>();
+    if (!live) return;
     CompLevel Lp;
     src.load(nk - 1, Lp);
-    comp_top(C, Lp, flx00_row[col], C.calc_helium ? __ldg(F.flx_he + col) : 0.0, xb, ok, fin, out, nk, ld, col,
-             status);
+    comp_top(C, Lp, flx00_s[lane], flx_he, xb, ok, fin, out, nk, ld, col, status);
 }
 
 // ---------------------------------------------------------------------------
@@ -1911,14 +1967,16 @@ __global__ void __launch_bounds__(128) k_comp_diag_ng(CompFields F, CompConsts C
     }
 }
 
+size_t comp_gz_doubles(int nk, long ld);
 cudaError_t launch_comp_diag_ng(const CompFields &F, const CompConsts &C, const double *x, int nk, int ncol, long ld,
                                 double *diag, double *scratch, cudaStream_t st)
 {
     if (ncol <= 0) return cudaSuccess;
     if (nk < 3) return cudaErrorInvalidValue;
     const int T = 128;
-    double *lv = scratch + 12 * (long)nk * ld;
-    k_comp_levels<<<dim3((ncol + T - 1) / T, nk), T, 0, st>>>(F, C, lv, nk, ncol, ld);
+    double *lv = scratch + comp_gz_doubles(nk, ld);
+    k_comp_levels<false><<<dim3((ncol + T - 1) / T, nk), T, 0, st>>>(F, C, DivBy<false>{C.dz, 1.0 / C.dz}, lv, nk, ncol,
+                                                                     ld);
     k_comp_diag_ng<<<dim3((ncol + T - 1) / T, nk), T, 0, st>>>(F, C, lv, x, nk, ncol, ld, diag);
     return cudaGetLastError();
 }
@@ -1929,25 +1987,38 @@ cudaError_t launch_comp_ng(const CompFields &F, const CompConsts &C, double *out
     if (ncol <= 0) return cudaSuccess;
     if (nk < 3) return cudaErrorInvalidValue;
     const int T = 128;
-    // the 30 row planes cost more traffic than they save above a few thousand
-    // columns per SM-wave (41472 columns: 625 against 449 us)
-    if (assembly_mode() == 2 && ncol <= kSmallWalkColumns) {
-        const long slab = (long)nk * ld;
-        double *lv = scratch + 12 * slab;                   // after the Gamma/z scratch
-        double *flx00_row = lv + kCompPlanes * slab + 4 * ld;
-        double *rows = flx00_row + ld;
-        k_comp_levels<<<dim3((ncol + T - 1) / T, nk), T, 0, st>>>(F, C, lv, nk, ncol, ld);
-        k_comp_coefs<<<dim3((ncol + T - 1) / T, nk - 1), T, 0, st>>>(F, C, lv, rows, flx00_row, nk, ncol, ld, sys_out);
-        once_per_device([] {
-            cudaFuncSetAttribute(k_comp_walk_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCompTileBytes);
-        });
-        k_comp_walk_tile<<<(ncol + kCompTileCols - 1) / kCompTileCols, 32 * kCompTileWarps, kCompTileBytes, st>>>(
-            F, C, lv, rows, flx00_row, out, scratch, nk, ncol, ld, status);
-        return cudaGetLastError();
-    }
     if (assembly_mode() >= 1) {
-        double *lv = scratch + 12 * (long)nk * ld;   // after the Gamma/z scratch
-        k_comp_levels<<<dim3((ncol + T - 1) / T, nk), T, 0, st>>>(F, C, lv, nk, ncol, ld);
+        double *lv = scratch + comp_gz_doubles(nk, ld);   // after the Gamma/z scratch
+        const dim3 grid((ncol + T - 1) / T, nk);
+        const bool ex = exact_reciprocal(C.dz);
+        const DivBy<true> de{C.dz, 1.0 / C.dz};
+        const DivBy<false> dq{C.dz, 1.0 / C.dz};
+        if (ex) k_comp_levels<true><<<grid, T, 0, st>>>(F, C, de, lv, nk, ncol, ld);
+        else k_comp_levels<false><<<grid, T, 0, st>>>(F, C, dq, lv, nk, ncol, ld);
+        if (assembly_mode() == 2) {
+            const int blocks = (ncol + 31) / 32;
+            auto go = [&](auto dv, auto np) {
+                constexpr int NP = decltype(np)::value;
+                auto k = k_comp_solve<decltype(dv)::exact, NP>;
+                once_per_device([k] {
+                    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)comp_solve_bytes(NP));
+                });
+                k<<<blocks, 32 * (1 + NP), comp_solve_bytes(NP), st>>>(F, C, dv, lv, out, scratch, nk, ncol, ld, sys_out,
+                                                                      status);
+            };
+            // while every tile is resident with four producers (three blocks
+            // per SM) the tile's own time decides; past that, more tiles at
+            // once (two producers, five blocks per SM): 11,248 columns x 57
+            // levels 91 us with 4 and 108 with 2, 21,216 165 and 151, 43,216
+            // 292 and 279
+            auto pick = [&](auto dv) {
+                if (blocks <= 3 * sm_count()) go(dv, std::integral_constant<int, 4>{});
+                else go(dv, std::integral_constant<int, 2>{});
+            };
+            if (ex) pick(de);
+            else pick(dq);
+            return cudaGetLastError();
+        }
         const int TR = kCompRowThreads;
         k_comp_rows<<<(ncol + TR - 1) / TR, TR, 2 * CompStagedSrc::NS * TR * sizeof(double), st>>>(
             F, C, lv, out, scratch, nk, ncol, ld, sys_out, status, walk_prefetch(ncol));
@@ -1957,9 +2028,13 @@ cudaError_t launch_comp_ng(const CompFields &F, const CompConsts &C, double *out
     return cudaGetLastError();
 }
 
-// Gamma/z (12 planes), the level planes and their 4 top rows, then (three-pass
-// form) the flx00 row and the 30 row planes
-size_t comp_scratch_doubles(int nk, long ld) { return (size_t)(12 + kCompPlanes + 30) * nk * ld + 5 * (size_t)ld; }
+// Gamma and z of every level (12 planes of whole 32-column tiles)
+size_t comp_gz_doubles(int nk, long ld) { return (size_t)12 * nk * ((ld + 31) / 32 * 32); }
+// those, then the level planes and their 4 top rows
+size_t comp_scratch_doubles(int nk, long ld)
+{
+    return comp_gz_doubles(nk, ld) + (size_t)kCompPlanes * nk * ld + 4 * (size_t)ld;
+}
 }  // namespace tg
 
 // comp_ng post-solve steps (src/comp_ng.F90:394-457): the lateral-boundary
