@@ -784,7 +784,7 @@ def main():
     horizontal = None
     if not args.skip_assembly:
         horizontal = {}
-        for which, name, kern in (("advec", "advec_ng", "k_advec_ng"), ("smooth", "smooth_ng", "k_smooth_ng"),
+        for which, name, kern in (("advec", "advec_ng", "k_horiz_ng<1>"), ("smooth", "smooth_ng", "k_horiz_ng<2>"),
                                   ("filter", "time_filter_ng", "k_time_filter"), ("ring", "filter_o2o", "k_ringfilter")):
             launch, npts, nbytes = horizontal_setup(pkg, which, dev)
             for _ in range(args.warmup):

@@ -405,6 +405,14 @@ int tg_advec_ng_dev(const double *f, const double *un, const double *vn, const d
                     void *stream);
 int tg_smooth_ng_dev(const double *fin, double shapiro, double *fout, int nk, int nlon, int nlat, long ld,
                      void *stream);
+/* Several fields of one grid in one launch: tg_advec_ng_dev of f[0..n_advec)
+ * into hadvec[] with the same winds, and tg_smooth_ng_dev of fin[0..n_smooth)
+ * into fout[], the same bits.  The pointer lists are host arrays; no output
+ * may alias any input of the call. */
+int tg_horiz_ng_dev(int n_advec, const double *const *f, double *const *hadvec, int n_smooth,
+                    const double *const *fin, double *const *fout, const double *un, const double *vn,
+                    const double *racs, double dlamda, double dphi, double re_inv, double shapiro, int nk, int nlon,
+                    int nlat, long ld, void *stream);
 
 /* Device arrays, level-major (k*ld + col), stream-ordered; nk <= 65535. */
 int tg_time_filter_ng_dev(int which, const double *cur, const double *prev, double dtsmooth,

@@ -39,7 +39,7 @@ LIB_PATH = os.path.join(HERE, "libtg_colsolve.so")
 
 # Every symbol include/tg_colsolve.h declares.
 EXPORTS = ("tg_solve_host", "tg_dt_ng", "tg_dt_ng_dev", "tg_minor_ng", "tg_minor_ng_dev", "tg_comp_ng",
-           "tg_comp_ng_dev", "tg_comp_post_ng", "tg_comp_post_ng_dev", "tg_comp_diag_ng", "tg_comp_diag_ng_dev", "tg_oplus_ng_factor_doubles", "tg_oplus_diag_ng", "tg_oplus_diag_ng_dev", "tg_oplus_ng_factor_dev", "tg_oplus_ng_solve_dev", "tg_oplus_ng_subcycle_dev", "tg_time_filter_ng", "tg_time_filter_ng_dev", "tg_advec_ng", "tg_advec_ng_dev", "tg_smooth_ng", "tg_smooth_ng_dev", "tg_settei_ng", "tg_settei_ng_dev", "tg_oplus_ng",
+           "tg_comp_ng_dev", "tg_comp_post_ng", "tg_comp_post_ng_dev", "tg_comp_diag_ng", "tg_comp_diag_ng_dev", "tg_oplus_ng_factor_doubles", "tg_oplus_diag_ng", "tg_oplus_diag_ng_dev", "tg_oplus_ng_factor_dev", "tg_oplus_ng_solve_dev", "tg_oplus_ng_subcycle_dev", "tg_time_filter_ng", "tg_time_filter_ng_dev", "tg_advec_ng", "tg_advec_ng_dev", "tg_smooth_ng", "tg_smooth_ng_dev", "tg_horiz_ng_dev", "tg_settei_ng", "tg_settei_ng_dev", "tg_oplus_ng",
            "tg_oplus_ng_dev", "tg_trsolv", "tg_trsolv_ng", "tg_blktri", "tg_comp_blksolve_ng", "tg_blksolve", "tg_trsolv_dev",
            "tg_blksolve_dev", "tg_blksolve_dev_noalloc", "tg_plan_create", "tg_plan_execute", "tg_plan_capture_graph",
            "tg_plan_status", "tg_plan_launches", "tg_plan_describe", "tg_set_cache_hints", "tg_set_block_rows", "tg_set_block_width", "tg_set_stage_levels", "tg_set_column_residency", "tg_set_assembly_mode", "tg_set_walk_prefetch", "tg_set_block_scratch_budget", "tg_set_scalar_scratch_budget", "tg_set_kind_overlap", "tg_set_host_pipeline", "tg_selftest_wait", "tg_plan_sweep_histogram", "tg_plan_destroy",
@@ -230,6 +230,8 @@ def lib():
             "tg_advec_ng_dev": [P, P, P, P, D, D, D, P, I, I, I, Lg, P],
             "tg_smooth_ng": [P, D, I, I, I, P],
             "tg_smooth_ng_dev": [P, D, P, I, I, I, Lg, P],
+            "tg_horiz_ng_dev": [I, ctypes.POINTER(P), ctypes.POINTER(P), I, ctypes.POINTER(P), ctypes.POINTER(P), P, P, P,
+                                D, D, D, D, I, I, I, Lg, P],
             "tg_minor_ng_dev": [ctypes.POINTER(MinorFields), ctypes.POINTER(MinorConsts), P, I, I, Lg, P, P, P],
             "tg_dt_ng_dev": [ctypes.POINTER(DtFields), ctypes.POINTER(DtConsts), P, I, I, Lg, P, P, P],
             "tg_trsolv_ng": [P, P, P, P, P, I, I, I],
@@ -909,6 +911,19 @@ def smooth_ng_dev(fin, shapiro, fout, nk, nlon, nlat, ld, stream=None):
     """Device form of smooth_ng on level-major planes (k*ld + i + (nlon+4)*j)."""
     rc = lib().tg_smooth_ng_dev(_dptr(fin), float(shapiro), _dptr(fout), nk, nlon, nlat, ld, _stream(stream))
     return _check(rc, "tg_smooth_ng_dev", numeric_ok=False)
+
+
+def horiz_ng_dev(f, hadvec, fin, fout, un, vn, racs, dlamda, dphi, re_inv, shapiro, nk, nlon, nlat, ld, stream=None):
+    """tg_horiz_ng_dev: advec_ng of the fields f into hadvec and smooth_ng of
+    the fields fin into fout (lists of (nk, ld) tensors) in one launch."""
+    def ptrs(ts):
+        return (ctypes.c_void_p * max(len(ts), 1))(*[_dptr(t) for t in ts])
+    if len(f) != len(hadvec) or len(fin) != len(fout):
+        raise ValueError("horiz_ng_dev: one output per field")
+    rc = lib().tg_horiz_ng_dev(len(f), ptrs(f), ptrs(hadvec), len(fin), ptrs(fin), ptrs(fout), _dptr(un), _dptr(vn),
+                               _dptr(racs), float(dlamda), float(dphi), float(re_inv), float(shapiro), nk, nlon, nlat,
+                               ld, _stream(stream))
+    return _check(rc, "tg_horiz_ng_dev", numeric_ok=False)
 
 
 def minor_ng_dev(fields, consts, out, nk, ncol, ld, system_out=None, status=None, stream=None):

@@ -1681,6 +1681,33 @@ __attribute__((visibility("default"))) int tg_advec_ng_dev(const double *f, cons
     return TG_OK;
 }
 
+__attribute__((visibility("default"))) int tg_horiz_ng_dev(
+    int n_advec, const double *const *f, double *const *hadvec, int n_smooth, const double *const *fin,
+    double *const *fout, const double *un, const double *vn, const double *racs, double dlamda, double dphi,
+    double re_inv, double shapiro, int nk, int nlon, int nlat, long ld, void *stream)
+{
+    bool ok = n_advec >= 0 && n_smooth >= 0 && (!n_advec || (f && hadvec && un && vn && racs)) &&
+              (!n_smooth || (fin && fout));
+    auto is_input = [&](const double *p) {
+        if (!p || (n_advec && (p == un || p == vn))) return true;
+        for (int i = 0; i < n_advec; ++i)
+            if (p == f[i]) return true;
+        for (int i = 0; i < n_smooth; ++i)
+            if (p == fin[i]) return true;
+        return false;
+    };
+    for (int i = 0; ok && i < n_advec; ++i) ok = f[i] && !is_input(hadvec[i]);
+    for (int i = 0; ok && i < n_smooth; ++i) ok = fin[i] && !is_input(fout[i]);
+    if (!ok) {
+        set_err("tg_horiz_ng_dev: a pointer is NULL or an output aliases an input");
+        return TG_EINVAL;
+    }
+    if (!horiz_args_ok("tg_horiz_ng_dev", nk, nlon, nlat, ld, true)) return TG_EINVAL;
+    TG_CUDA(launch_horiz_ng(n_advec, f, hadvec, n_smooth, fin, fout, un, vn, racs, dlamda, dphi, re_inv, shapiro, nk,
+                            nlon, nlat, ld, (cudaStream_t)stream));
+    return TG_OK;
+}
+
 __attribute__((visibility("default"))) int tg_smooth_ng_dev(const double *fin, double shapiro, double *fout, int nk,
                                                             int nlon, int nlat, long ld, void *stream)
 {

@@ -62,14 +62,17 @@ __device__ __forceinline__ double advec_dir(const double *p, const double *u, in
     return xsub(lhs, rhs);
 }
 
-__global__ void __launch_bounds__(kTx * kTy) k_advec_ng(const double *f, const double *un, const double *vn,
-                                                       const double *racs, double dlamda, double dphi,
-                                                       double re_inv, AdvecRcp rc, int nlond, int nlatd, long ld,
-                                                       double *hadvec)
+// Several fields in one launch: blockIdx.z counts planes, nk of each field.
+constexpr int kMaxBatch = 8;
+struct HorizBatch {
+    const double *in[kMaxBatch];
+    double *out[kMaxBatch];
+};
+
+__device__ __forceinline__ void advec_point(const double *f, const double *un, const double *vn, const double *racs,
+                                            double dlamda, double dphi, double re_inv, const AdvecRcp &rc, int i, int j,
+                                            int nlond, int nlatd, long o, double *hadvec)
 {
-    const int i = blockIdx.x * kTx + threadIdx.x, j = blockIdx.y * kTy + threadIdx.y;
-    if (i >= nlond || j >= nlatd) return;
-    const long o = (long)blockIdx.z * ld + i + (long)nlond * j;
     const double wk1 = xmul(advec_dir(f + o, un + o, i, nlond, 1, rc), __ldg(racs + j));
     const double wk2 = advec_dir(f + o, vn + o, j, nlatd, nlond, rc);
     // hadvec = wk1/dlamda + wk2*re_inv/dphi (:50)
@@ -80,18 +83,16 @@ __global__ void __launch_bounds__(kTx * kTy) k_advec_ng(const double *f, const d
 // longitudes (the lon pass needs +-2 neighbours): its 288 points are dealt
 // to the 256 threads in order, so only one warp takes a second point.  Then
 // the lon pass reads the tile.
-__global__ void __launch_bounds__(kTx * kTy) k_smooth_ng(const double *fin, double sh, int nlond, int nlatd,
-                                                        long ld, double *fout)
+__device__ __forceinline__ void smooth_point(const double *fin, double sh, int i0, int j0, int nlond, int nlatd,
+                                             long plane, double *fout)
 {
     constexpr int W = kTx + 4;
     __shared__ double ft[kTy][W + 1];
-    const int i0 = blockIdx.x * kTx, j0 = blockIdx.y * kTy;
-    const double *plane = fin + (long)blockIdx.z * ld;
     for (int q = threadIdx.y * kTx + threadIdx.x; q < W * kTy; q += kTx * kTy) {
         const int r = q / W, c = q - r * W;
         const int i = i0 - 2 + c, j = j0 + r;
         if (i < 0 || i >= nlond || j >= nlatd) continue;
-        const double *p = plane + i + (long)nlond * j;
+        const double *p = fin + plane + i + (long)nlond * j;
         ft[r][c] = shapiro_at([&](int d) { return p[d * nlond]; }, j, nlatd, sh);
     }
     __syncthreads();
@@ -99,7 +100,38 @@ __global__ void __launch_bounds__(kTx * kTy) k_smooth_ng(const double *fin, doub
     if (i >= nlond || j >= nlatd) return;
     // every longitude the lon pass reads (i-2..i+2 where used) is in the tile
     const double *p = &ft[threadIdx.y][threadIdx.x + 2];
-    fout[(long)blockIdx.z * ld + i + (long)nlond * j] = shapiro_at([&](int d) { return p[d]; }, i, nlond, sh);
+    fout[plane + i + (long)nlond * j] = shapiro_at([&](int d) { return p[d]; }, i, nlond, sh);
+}
+
+// KIND 1: advec_ng of n_adv fields, 2: smooth_ng, 3: both, the advected fields
+// first.  One field of a small grid is a launch gap and a quarter of a wave
+// (56 x 37 x 57: 4.2 us for 3 MB), so a routine's fields share a launch: one
+// advec + one smooth 6.2 us against 8.4, three of each 10.3 against 25 (147 x
+// 76 x 57: 14.4 against 18.5, 35 against 56).  Bound by the loads' latency and
+// the issue slots, hence 8 blocks per SM: at 32 registers instead of 38 to 40
+// advec_ng of 580 x 292 x 20 falls from 42.9 to 37.0 us and three of each of
+// 147 x 76 x 57 from 38 to 35; 4 levels per thread with every load in flight
+// took 60.  ONE: one field, whose plane needs no loop (smooth_ng of 580 x 292 x
+// 20: 22.6 us, 23.7 with it).  The lists stay in the parameter bank (__grid_constant__): indexed as a plain
+// parameter they are copied to the stack, and advec_ng takes 71 us.
+template <int KIND, bool ONE>
+__global__ void __launch_bounds__(kTx * kTy, 8)
+    k_horiz_ng(const __grid_constant__ HorizBatch hb, int n_adv, const double *un, const double *vn, const double *racs,
+               double dlamda, double dphi, double re_inv, AdvecRcp rc, double sh, int nk, int nlond, int nlatd, long ld)
+{
+    int n = 0, k = blockIdx.z;
+    if (!ONE)
+        for (; k >= nk; k -= nk) ++n;
+    const long plane = (long)k * ld;
+    const int i0 = blockIdx.x * kTx, j0 = blockIdx.y * kTy;
+    if (KIND == 1 || (KIND == 3 && n < n_adv)) {
+        const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
+        if (i < nlond && j < nlatd)
+            advec_point(hb.in[n], un, vn, racs, dlamda, dphi, re_inv, rc, i, j, nlond, nlatd,
+                        plane + i + (long)nlond * j, hb.out[n]);
+    } else {
+        smooth_point(hb.in[n], sh, i0, j0, nlond, nlatd, plane, hb.out[n]);
+    }
 }
 
 dim3 plane_grid(int nk, int nlond, int nlatd)
@@ -109,25 +141,49 @@ dim3 plane_grid(int nk, int nlond, int nlatd)
 
 }  // namespace
 
-cudaError_t launch_advec_ng(const double *f, const double *un, const double *vn, const double *racs, double dlamda,
-                            double dphi, double re_inv, int nk, int nlon, int nlat, long ld, double *hadvec,
-                            cudaStream_t st)
+cudaError_t launch_horiz_ng(int n_adv, const double *const *f, double *const *hadvec, int n_smooth,
+                            const double *const *fin, double *const *fout, const double *un, const double *vn,
+                            const double *racs, double dlamda, double dphi, double re_inv, double shapiro, int nk,
+                            int nlon, int nlat, long ld, cudaStream_t st)
 {
     const int nlond = nlon + 4, nlatd = nlat + 4;
     // host IEEE division: the correctly rounded reciprocals the Markstein step needs
     auto in_range = [](double b) { return std::fabs(b) >= 0x1p-500 && std::fabs(b) < 0x1p500; };
     const AdvecRcp rc{1.0 / 3.0, 1.0 / 12.0, 1.0 / dlamda, 1.0 / dphi, in_range(dlamda), in_range(dphi)};
-    k_advec_ng<<<plane_grid(nk, nlond, nlatd), dim3(kTx, kTy), 0, st>>>(f, un, vn, racs, dlamda, dphi, re_inv, rc,
-                                                                        nlond, nlatd, ld, hadvec);
+    // grid.z counts planes: at most 65535
+    const int most = nk > 65535 / kMaxBatch ? 65535 / nk : kMaxBatch;
+    for (int a = 0, s = 0; a < n_adv || s < n_smooth;) {
+        HorizBatch hb{};
+        int n = 0, na = 0;
+        for (; a < n_adv && n < most; ++a, ++n, ++na) {
+            hb.in[n] = f[a];
+            hb.out[n] = hadvec[a];
+        }
+        for (; s < n_smooth && n < most; ++s, ++n) {
+            hb.in[n] = fin[s];
+            hb.out[n] = fout[s];
+        }
+        auto k = n == 1 ? na ? k_horiz_ng<1, true> : k_horiz_ng<2, true>
+                 : na == n ? k_horiz_ng<1, false> : na ? k_horiz_ng<3, false> : k_horiz_ng<2, false>;
+        k<<<plane_grid(nk * n, nlond, nlatd), dim3(kTx, kTy), 0, st>>>(hb, na, un, vn, racs, dlamda, dphi, re_inv, rc,
+                                                                       shapiro, nk, nlond, nlatd, ld);
+    }
     return cudaGetLastError();
+}
+
+cudaError_t launch_advec_ng(const double *f, const double *un, const double *vn, const double *racs, double dlamda,
+                            double dphi, double re_inv, int nk, int nlon, int nlat, long ld, double *hadvec,
+                            cudaStream_t st)
+{
+    return launch_horiz_ng(1, &f, &hadvec, 0, nullptr, nullptr, un, vn, racs, dlamda, dphi, re_inv, 0.0, nk, nlon, nlat,
+                           ld, st);
 }
 
 cudaError_t launch_smooth_ng(const double *fin, double shapiro, int nk, int nlon, int nlat, long ld, double *fout,
                              cudaStream_t st)
 {
-    const int nlond = nlon + 4, nlatd = nlat + 4;
-    k_smooth_ng<<<plane_grid(nk, nlond, nlatd), dim3(kTx, kTy), 0, st>>>(fin, shapiro, nlond, nlatd, ld, fout);
-    return cudaGetLastError();
+    return launch_horiz_ng(0, nullptr, nullptr, 1, &fin, &fout, nullptr, nullptr, nullptr, 1.0, 1.0, 1.0, shapiro, nk,
+                           nlon, nlat, ld, st);
 }
 
 }  // namespace tg

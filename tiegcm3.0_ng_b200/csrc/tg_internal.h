@@ -238,6 +238,12 @@ cudaError_t launch_comp_post_ng(const double *const *in7, const double *zpmid, d
                                 double dtsmooth_div2, int nk, int ncol, long ld, double *const *upd6,
                                 cudaStream_t st, const unsigned char *bnd_mask = nullptr,
                                 const double *const *bnd3 = nullptr);
+// advec_ng of n_adv fields and smooth_ng of n_smooth in one launch (of up to 8
+// each), all with the same winds and grid.
+cudaError_t launch_horiz_ng(int n_adv, const double *const *f, double *const *hadvec, int n_smooth,
+                            const double *const *fin, double *const *fout, const double *un, const double *vn,
+                            const double *racs, double dlamda, double dphi, double re_inv, double shapiro, int nk,
+                            int nlon, int nlat, long ld, cudaStream_t st);
 // advec_ng / smooth_ng on one nest held as a single subdomain (tg_horiz.cu):
 // level-major planes (k, i, j) at k*ld + i + (nlon+4)*j
 cudaError_t launch_advec_ng(const double *f, const double *un, const double *vn, const double *racs, double dlamda,

@@ -192,14 +192,10 @@ class DynamicsStep:
         self.graph = None
 
     # ---- the routines, each on one stream --------------------------------
-    def _advec(self, f, out, st):
+    def _horiz(self, f, hadvec, fin, fout, st):
         g = self.grid
-        cs.advec_ng_dev(f, self.un, self.vn, self.racs, g.dlamda, g.dphi, g.re_inv, out, g.nk, g.nlon, g.nlat, g.ld,
-                        stream=st)
-
-    def _smooth(self, fin, out, st, shapiro=None):
-        g = self.grid
-        cs.smooth_ng_dev(fin, g.shapiro if shapiro is None else shapiro, out, g.nk, g.nlon, g.nlat, g.ld, stream=st)
+        cs.horiz_ng_dev(f, hadvec, fin, fout, self.un, self.vn, self.racs, g.dlamda, g.dphi, g.re_inv, g.shapiro, g.nk,
+                        g.nlon, g.nlat, g.ld, stream=st)
 
     def _post(self, cur, prev, nm, bnd):
         return dict(cur=cur, prev=prev, nm_upd=nm, bnd_mask=self.mask, bnd=bnd, dtsmooth=self.ds[0],
@@ -211,17 +207,17 @@ class DynamicsStep:
                                  o["F"]["optm1_smooth2"], g.shapiro / self.nstep_sub, o["op"], o["optm1"], g.nk, g.nlon,
                                  g.nlat, g.ld, self.ds[0], self.ds[1], bnd_mask=self.mask, bnd=o["bnd"], stream=st)
 
-    def _minor(self, m, st):
+    def _minors(self, ms, st):
         g = self.grid
-        self._smooth(m["fcomp_tm1"], m["F"]["ftm1_smooth"], st)
-        self._advec(m["fcomp"], m["F"]["hadvec"], st)
-        cs.minor_ng_post_dev(m["F"], m["C"], m["out"], g.nk, g.ncol, g.ld,
-                             self._post(m["fcomp"], m["fcomp_tm1"], m["nm"], m["bnd"]), stream=st)
+        self._horiz([m["fcomp"] for m in ms], [m["F"]["hadvec"] for m in ms], [m["fcomp_tm1"] for m in ms],
+                    [m["F"]["ftm1_smooth"] for m in ms], st)
+        for m in ms:
+            cs.minor_ng_post_dev(m["F"], m["C"], m["out"], g.nk, g.ncol, g.ld,
+                                 self._post(m["fcomp"], m["fcomp_tm1"], m["nm"], m["bnd"]), stream=st)
 
     def _settei_dt(self, st):
         g, s, d = self.grid, self.settei, self.dt
-        self._advec(d["F"]["tn"], d["F"]["horadv"], st)
-        self._smooth(d["tn_nm"], d["F"]["tnsmooth"], st)
+        self._horiz([d["F"]["tn"]], [d["F"]["horadv"]], [d["tn_nm"]], [d["F"]["tnsmooth"]], st)
         s["qtotal"].copy_(s["qtotal0"])
         cs.settei_ng_dev(s["F"], s["C"], s["te"], s["ti"], s["qtotal"], g.nk, g.ncol, g.ld, stream=st)
         cs.dt_ng_post_dev(d["F"], d["C"], d["out"], g.nk, g.ncol, g.ld,
@@ -230,9 +226,9 @@ class DynamicsStep:
     def _comp(self, st):
         g, c = self.grid, self.comp
         F = c["F"]
-        for sp in ("o2", "o1", "he"):
-            self._advec(F[sp], F[sp + "_advec"], st)
-            self._smooth(c["post_in"][sp + "_nm"], F[sp + "nm_smooth"], st)
+        sps = ("o2", "o1", "he")
+        self._horiz([F[sp] for sp in sps], [F[sp + "_advec"] for sp in sps], [c["post_in"][sp + "_nm"] for sp in sps],
+                    [F[sp + "nm_smooth"] for sp in sps], st)
         cs.comp_ng_dev(F, c["C"], c["out"], g.nk, g.ncol, g.ld, stream=st)
         if self.ring is not None:
             # filter_o2o on the interior latitudes: rows 2 .. nlat+1 of the subdomain
@@ -251,8 +247,7 @@ class DynamicsStep:
         if not self.fan_out:
             with torch.cuda.stream(stream):
                 self._oplus(stream)
-                for m in self.minor:
-                    self._minor(m, stream)
+                self._minors(self.minor, stream)
                 self._settei_dt(stream)
                 self._comp(stream)
             return
@@ -262,11 +257,9 @@ class DynamicsStep:
         with torch.cuda.stream(s_op):
             self._oplus(s_op)
         with torch.cuda.stream(s_m0):
-            self._minor(self.minor[0], s_m0)
-            self._minor(self.minor[1], s_m0)
+            self._minors(self.minor[:2], s_m0)
         with torch.cuda.stream(s_m1):
-            self._minor(self.minor[2], s_m1)
-            self._minor(self.minor[3], s_m1)
+            self._minors(self.minor[2:], s_m1)
         with torch.cuda.stream(s_c):
             self._comp(s_c)
         with torch.cuda.stream(stream):
