@@ -50,11 +50,11 @@ __device__ __forceinline__ Lev load_lev(const SetteiFields &F, long o)
 
 // tek0/h_int of an interface from its raw averages (settei_ng.F90:116-139)
 struct Iface {
-    double tek0, th, tn_int;
+    double tek0, th;
 };
 
 __device__ __forceinline__ Iface iface(const SetteiConsts &C, double te_int, double o2n, double o1n, double hen,
-                                       double n2n, double tn_int, double xnmbari, double ne, double h_int)
+                                       double n2n, double xnmbari, double ne, double h_int)
 {
     n2n = dmax(n2n, 0.);
     o2n = xm(xm(xnmbari, o2n), C.rmassinv_o2);
@@ -70,7 +70,6 @@ __device__ __forceinline__ Iface iface(const SetteiConsts &C, double te_int, dou
     Iface I;
     I.tek0 = xm(xd(7.5e5, xa(1.0, X)), C.evergs);
     I.th = xd(I.tek0, h_int);
-    I.tn_int = tn_int;
     return I;
 }
 
@@ -87,6 +86,34 @@ __device__ __forceinline__ double qsum(const SetteiFields &F, long o)
 }  // namespace
 
 namespace {
+// x^e of e = RN(2/7), the power that turns Te^3.5 back into Te, within 0.51
+// ulp.  y, the single-precision root, is off by a few 1e-6: its exact seventh
+// power against x*x (both as sums of two doubles) gives e7 = x^2/y^7 - 1, the
+// binomial series of (1 + e7)^(1/7) the correction (Newton's step and its next
+// two terms; the first dropped term is below 1e-20), and x^(e - 2/7) =
+// 1 + (e - 2/7)*log(x) the difference of the exponents, e - 2/7 =
+// -2/7*2^-54.  About 40 operations for pow's two hundred.  Outside the range
+// that single precision holds with room to spare (zeros, negative values and
+// NaN included) the device pow.
+__device__ __forceinline__ double pow27(double x)
+{
+    if (!(x >= 0x1p-60 && x <= 0x1p110)) return pow(x, xd(2., 7.));
+    const float l = __log2f((float)x);
+    const double y = (double)exp2f(l * (2.0f / 7.0f));
+    const double y2 = xm(y, y);   // exact: 48 bits
+    const double p3 = xm(y2, y), c3 = __fma_rn(y2, y, -p3);
+    const double p4 = xm(y2, y2), c4 = __fma_rn(y2, y2, -p4);
+    const double p7 = xm(p4, p3);
+    const double c7 = xa(__fma_rn(p4, p3, -p7), __fma_rn(p4, c3, xm(c4, p3)));
+    const double px = xm(x, x), cx = __fma_rn(x, x, -px);
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(p7));
+    r = __fma_rn(r, __fma_rn(-p7, r, 1.0), r);
+    const double e7 = xm(xa(xs(px, p7), xs(cx, c7)), r);
+    const double t = xm(e7, __fma_rn(e7, __fma_rn(e7, 13. / 343., -3. / 49.), 1. / 7.));
+    return __fma_rn(y, __fma_rn(-2. / 7. * 0x1p-54 * 0.6931471805599453, (double)l, t), y);
+}
+
 // Heating, cooling and exchange of one level (settei_ng.F90:157-246).
 struct Loss {
     double dq;      // subtracted from q: (loss_en+loss_ei)/te**2.5
@@ -96,6 +123,20 @@ struct Loss {
     double lei_ti;  // loss_ei*ti
     double lei, lin, q_eni;
 };
+
+// t^2.5 from t and rt = sqrt(t): the product t*t*rt with the rounding errors
+// of its three factors carried along (two FMA residuals, and t - rt*rt =
+// (sqrt(t) - rt)*2*rt for the root's), within 0.51 ulp; about ten operations
+// for pow's two hundred.  Outside the range that keeps the residuals normal
+// (and for zeros, negative values and NaN) the device pow.
+__device__ __forceinline__ double pow25(double t, double rt)
+{
+    if (!(t >= 0x1p-200 && t <= 0x1p200)) return pow(t, 2.5);
+    const double h = xm(t, t), eh = __fma_rn(t, t, -h);
+    const double es = __fma_rn(-rt, rt, t);
+    const double p = xm(h, rt), ep = __fma_rn(h, rt, -p);
+    return xa(p, __fma_rn(xm(0.5, xm(t, rt)), es, __fma_rn(eh, rt, ep)));
+}
 
 __device__ __forceinline__ Loss level_loss(const SetteiFields &F, const SetteiConsts &C, long o, const Lev &L,
                                            double rne_raw, double qtot)
@@ -129,23 +170,35 @@ __device__ __forceinline__ Loss level_loss(const SetteiFields &F, const SetteiCo
     R.qe_h = xm(xm(qe, qtot), ev);
     R.et_h = C.et ? xm(xa(__ldg(F.Q1 + o), __ldg(F.Q2 + o)), 10.0) : 0.0;
     const double te = L.te, tn = L.tn, rt = sqrt(te);
-    double coll = te >= 1000. ? xm(2.e-7, exp(xd(-4605.2, te))) : xm(5.71e-8, exp(xd(-3352.6, te)));
-    if (te > 2000.) coll = xm(xm(2.53e-6, rt), exp(xd(-17620., te)));
+    // te and rt each divide two constants (all normal): one reciprocal each
+    const bool safe = exp_safe(te);
+    const double yte = __drcp_rn(te), yrt = __drcp_rn(rt);
+    auto by_te = [&](double a) { return safe ? div_markstein(a, te, yte) : xd(a, te); };
+    auto by_rt = [&](double a) { return safe ? div_markstein(a, rt, yrt) : xd(a, rt); };
+    // the excitation rate's three ranges of te differ in two constants: one
+    // exp for all of a warp's lanes
+    const double coll = xm(te > 2000. ? xm(2.53e-6, rt) : te >= 1000. ? 2.e-7 : 5.71e-8,
+                           exp(by_te(te > 2000. ? -17620. : te >= 1000. ? -4605.2 : -3352.6)));
     double l2v;
     if (fabs(xs(te, tn)) < del) l2v = xd(3200., xm(tn, tn));
     else l2v = xm(xd(1., xs(te, tn)), xs(1., exp(xd(xm(-3200., xs(te, tn)), xm(te, tn)))));
     l2v = xm(xm(1.3e-4, l2v), coll);
-    const double leo2 = xm(o2n, xa(xa(xm(xm(1.21e-18, xa(1., xm(3.6e-2, rt))), rt), xd(6.9e-14, rt)),
+    const double leo2 = xm(o2n, xa(xa(xm(xm(1.21e-18, xa(1., xm(3.6e-2, rt))), rt), by_rt(6.9e-14)),
                                    xm(3.125e-21, xm(te, te))));
     const double leo1d = 0.;
     const double leo1 = xm(o1n, xa(xm(xm(7.9e-19, xa(1., xm(5.7e-4, te))), rt),
-                                   xm(xd(xm(3.4e-12, xs(1., xm(7.e-5, te))), tn), xa(xd(150., te), 0.4))));
+                                   xm(xd(xm(3.4e-12, xs(1., xm(7.e-5, te))), tn), xa(by_te(150.), 0.4))));
     const double lehe = xm(xm(hen, 2.46e-17), rt);
-    const double len2 = xm(n2n, xa(xa(xm(xm(1.77E-19, xs(1., xm(1.21E-4, te))), te), xd(2.9e-14, rt)), l2v));
+    const double len2 = xm(n2n, xa(xa(xm(xm(1.77E-19, xs(1., xm(1.21E-4, te))), te), by_rt(2.9e-14)), l2v));
     double len = xa(xa(xa(leo2, leo1), lehe), len2);
     if (C.et && te > 500.0 && __ldg(F.Q2 + o) > 0.0) len = xm(len, exp(xm(-7.54E-4, xs(te, 500.0))));
-    const double lxen = xm(xm(xa(len, xm(xm(o1n, xs(1., xd(alam, xa(ad, xm(sd, n2n))))), leo1d)), rne), ev);
-    len = xm(xm(xa(len, xm(o1n, leo1d)), rne), ev);
+    // lxen weights leo1d = 0 with 1 - alam/(ad + sd*n2n): the same zero as
+    // len's while that factor is positive and o1n finite
+    const double d1n = xa(ad, xm(sd, n2n)), len0 = len;
+    len = xm(xm(xa(len0, xm(o1n, leo1d)), rne), ev);
+    double lxen = len;
+    if (!(d1n >= 0.007 && finite(o1n)))
+        lxen = xm(xm(xa(len0, xm(xm(o1n, xs(1., xd(alam, d1n))), leo1d)), rne), ev);
     double ions = xm(__ldg(F.op + o), C.rmassinv_o1);
     ions = xa(ions, xm(__ldg(F.o2p + o), C.rmassinv_o2));
     ions = xa(ions, xm(__ldg(F.nplus + o), C.rmassinv_n4s));
@@ -161,7 +214,7 @@ __device__ __forceinline__ Loss level_loss(const SetteiFields &F, const SetteiCo
     s = xa(s, xm(n2p, xa(xa(xa(xm(5.54, o2n), xm(4.65, o1n)), xm(1.82, hen)), xm(xm(0.27, n2n), rtn))));
     s = xa(s, xm(nop, xa(xa(xa(xm(5.45, o2n), xm(4.5, o1n)), xm(1.72, hen)), xm(5.92, n2n))));
     const double lin = xm(xm(1e-14, ev), s);
-    R.dq = xd(xa(len, lei), pow(te, 2.5));
+    R.dq = xd(xa(len, lei), pow25(te, rt));
     R.len_tn = xm(len, tn);
     R.lei_ti = xm(lei, ti);
     R.lei = lei;
@@ -225,7 +278,7 @@ __global__ void __launch_bounds__(128) k_settei_ng(SetteiFields F, SetteiConsts 
         const double o1n = xm(.5, xa(xa(xa(fb[0], xm(b[0], L0.o2)), xm(xa(b[3], 1.), L0.o1)), xm(b[6], L0.he)));
         const double hen = xm(.5, xa(xa(xa(fb[0], xm(b[0], L0.o2)), xm(b[3], L0.o1)), xm(xa(b[6], 1.), L0.he)));
         const double n2n = dmax(xs(xs(xs(1., o2n), o1n), hen), 0.);
-        I0 = iface(C, te_int, o2n, o1n, hen, n2n, t_lbc, at(F.xnmbari, 0), at(F.ne, 0), at(F.schti, 0));
+        I0 = iface(C, te_int, o2n, o1n, hen, n2n, at(F.xnmbari, 0), at(F.ne, 0), at(F.schti, 0));
     }
     double qs0 = qsum(F, col), qs1 = qsum(F, ld + col);
     double ne0 = at(F.ne, 0), ne1 = at(F.ne, 1);
@@ -252,13 +305,13 @@ __global__ void __launch_bounds__(128) k_settei_ng(SetteiFields F, SetteiConsts 
             Iface I1;
             if (k + 1 < nk - 1) {
                 I1 = iface(C, xm(.5, xa(Lp.te, L0.te)), xm(.5, xa(Lp.o2, L0.o2)), xm(.5, xa(Lp.o1, L0.o1)),
-                           xm(.5, xa(Lp.he, L0.he)), xm(.5, xa(Lp.n2, L0.n2)), xm(.5, xa(Lp.tn, L0.tn)),
+                           xm(.5, xa(Lp.he, L0.he)), xm(.5, xa(Lp.n2, L0.n2)),
                            at(F.xnmbari, k + 1), at(F.ne, k + 1), at(F.schti, k + 1));
             } else {
-                // top interface: te_int and tn_int extrapolated from levels nk-2, nk-3
-                const double te_im = k >= 1 ? Lm.te : 0., tn_im = k >= 1 ? Lm.tn : 0.;
+                // top interface: te_int extrapolated from levels nk-2, nk-3
+                const double te_im = k >= 1 ? Lm.te : 0.;
                 I1 = iface(C, xs(xm(1.5, L0.te), xm(.5, te_im)), xm(.5, xa(Lp.o2, L0.o2)), xm(.5, xa(Lp.o1, L0.o1)),
-                           xm(.5, xa(Lp.he, L0.he)), xm(.5, xa(Lp.n2, L0.n2)), xs(xm(1.5, L0.tn), xm(.5, tn_im)),
+                           xm(.5, xa(Lp.he, L0.he)), xm(.5, xa(Lp.n2, L0.n2)),
                            at(F.xnmbari, k + 1), at(F.ne, k + 1), at(F.schti, k + 1));
             }
             // row k (settei_ng.F90:131-155, 183, 240-242)
@@ -269,7 +322,7 @@ __global__ void __launch_bounds__(128) k_settei_ng(SetteiFields F, SetteiConsts 
             double rhs = 0.;
             if (k == 0) {
                 q = xs(q, p);
-                rhs = xs(rhs, xm(xm(2., p), pow(I0.tn_int, 3.5)));
+                rhs = xs(rhs, xm(xm(2., p), pow(t_lbc, 3.5)));
                 p = 0.;
             }
             if (k == nk - 2) {
@@ -319,7 +372,7 @@ __global__ void __launch_bounds__(128) k_settei_ng(SetteiFields F, SetteiConsts 
     // back sweep, x = Te^3.5 -> Te, top level, Ti (settei_ng.F90:256-261)
     const int K = nk - 1;
     double xn = w3;
-    double tk = pow(xn, xd(2., 7.));
+    double tk = pow27(xn);
     double t_top1 = tk, t_top2 = 0.;
     bool fin = fabs(xn) <= DBL_MAX;
     auto finish = [&](int k, double t) {
@@ -335,7 +388,7 @@ __global__ void __launch_bounds__(128) k_settei_ng(SetteiFields F, SetteiConsts 
     for (int k = K - 2; k >= 0; --k) {
         xn = xs(te_out[(long)k * ld + col], xm(w2s[(long)k * T], xn));
         fin = fin && fabs(xn) <= DBL_MAX;
-        tk = pow(xn, xd(2., 7.));
+        tk = pow27(xn);
         if (k == K - 2) t_top2 = tk;
         finish(k, tk);
     }
@@ -397,20 +450,13 @@ __global__ void __launch_bounds__(128) k_settei_levels(SetteiFields F, SetteiCon
         const double o1n = xm(.5, xa(xa(xa(fb[0], xm(b[0], L.o2)), xm(xa(b[3], 1.), L.o1)), xm(b[6], L.he)));
         const double hen = xm(.5, xa(xa(xa(fb[0], xm(b[0], L.o2)), xm(b[3], L.o1)), xm(xa(b[6], 1.), L.he)));
         const double n2n = dmax(xs(xs(xs(1., o2n), o1n), hen), 0.);
-        I = iface(C, te_int, o2n, o1n, hen, n2n, t_lbc, at(F.xnmbari, 0), at(F.ne, 0), at(F.schti, 0));
+        I = iface(C, te_int, o2n, o1n, hen, n2n, at(F.xnmbari, 0), at(F.ne, 0), at(F.schti, 0));
     } else {
         const Lev Lm = load_lev(F, o - ld);
-        double te_int, tn_int;
-        if (j == nk - 1) {
-            const Lev Lmm = load_lev(F, o - 2 * ld);
-            te_int = xs(xm(1.5, Lm.te), xm(.5, Lmm.te));
-            tn_int = xs(xm(1.5, Lm.tn), xm(.5, Lmm.tn));
-        } else {
-            te_int = xm(.5, xa(L.te, Lm.te));
-            tn_int = xm(.5, xa(L.tn, Lm.tn));
-        }
+        const double te_int = j == nk - 1 ? xs(xm(1.5, Lm.te), xm(.5, __ldg(F.te + o - 2 * ld)))
+                                          : xm(.5, xa(L.te, Lm.te));
         I = iface(C, te_int, xm(.5, xa(L.o2, Lm.o2)), xm(.5, xa(L.o1, Lm.o1)), xm(.5, xa(L.he, Lm.he)),
-                  xm(.5, xa(L.n2, Lm.n2)), tn_int, at(F.xnmbari, j), at(F.ne, j), at(F.schti, j));
+                  xm(.5, xa(L.n2, Lm.n2)), at(F.xnmbari, j), at(F.ne, j), at(F.schti, j));
     }
     // heating, cooling and exchange of level j (settei_ng.F90:157-246)
     const double ne0 = at(F.ne, j);
@@ -565,7 +611,7 @@ __global__ void __launch_bounds__(128) k_settei_rows(SetteiFields F, SetteiConst
         if (lev(i) >= 1 && i < K) pf_l1(te_out + (long)(lev(i) - 1) * ld + col);
     };
     double xn = w3;
-    double tk = pow(xn, xd(2., 7.));
+    double tk = pow27(xn);
     double t_top1 = tk, t_top2 = 0.;
     bool fin = fabs(xn) <= DBL_MAX;
     double park = K >= 2 ? te_out[(long)(K - 2) * ld + col] : 0.;
@@ -586,7 +632,7 @@ __global__ void __launch_bounds__(128) k_settei_rows(SetteiFields F, SetteiConst
             if (k >= 1) park = te_out[(long)(k - 1) * ld + col];
             xn = xs(wk, xm(w2s[(long)k * T], xn));
             fin = fin && fabs(xn) <= DBL_MAX;
-            tk = pow(xn, xd(2., 7.));
+            tk = pow27(xn);
             if (k == K - 2) t_top2 = tk;
             t = tk;
         } else {
@@ -606,57 +652,100 @@ __global__ void __launch_bounds__(128) k_settei_rows(SetteiFields F, SetteiConst
 // ---------------------------------------------------------------------------
 // settei_ng in three passes (the default), so that the column walk is the
 // recurrence alone instead of forming its rows and raising every solved
-// level to the 2/7 power level by level.  After k_settei_levels:
-//   k_settei_coefs: one thread per (level, column) forms row k (p, q, r and
-//     rhs, as the walk forms them) into four planes and adds q_eni to qtotal
-//     at the interfaces;
+// level to the 2/7 power level by level:
+//   k_settei_system: one thread per (level, column) forms the row (p, q, r and
+//     rhs) and keeps three rates of the level;
 //   the Thomas walk of the assembly routines (launch_thomas_post) solves the
 //     rows 0..nk-2 for x = Te^3.5 into a scratch plane;
 //   k_settei_post: one thread per (level, column) turns x into Te, the top
-//     level from its two neighbours, and forms Ti.
+//     level from its two neighbours, forms Ti and adds q_eni to qtotal at the
+//     interfaces.
 // The same operations on the same operands as k_settei_rows: the same bits.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_settei_coefs(SetteiFields F, SetteiConsts C, const double *lv,
-                                                      double *rows, double *qtotal, int nk, int ncol, long ld,
-                                                      double *sys_out)
+namespace {
+enum { K_LEI = 0, K_LIN, K_QENI, K_N };
+constexpr int kSysLevels = 4, kSysBlocks = 8;
+}
+
+// A block holds 4 levels of 32 columns, one warp each, and a fifth warp for the
+// interface above them: each interface's conductivity and each level's heating
+// sum is formed once and handed on in shared memory, where a first form wrote
+// ten level planes and read nine of them again in a kernel of its own (46 + 19
+// us on 11,248 columns x 57; this one 50).  About 1,400 instructions per point,
+// a third of them FP64, behind 33 reads: bound by the reads' latency and the
+// issue slots (59% busy, 124 MB read), so it runs 8 blocks per SM at 48
+// registers and 60 bytes of spills (80 us the routine, 84 at 5 blocks and no
+// spills, 98 with 8 levels per block at 2 blocks), with the losses' lines
+// requested before the interface is formed (84 without).  Threads that walk 2
+// to 8 levels and keep the window in registers need 126 of them: 86 to 125 us.
+// The routine, before and now: 37.0 and 29.0 us on 2,072 columns x 57, 92.9
+// and 78.0 on 11,248, 292 and 233 on 43,216, 28.0 and 22.7 on 2,816 x 29.
+__global__ void __launch_bounds__(32 * (kSysLevels + 1), kSysBlocks)
+    k_settei_system(SetteiFields F, SetteiConsts C, double *rows, double *keep, int nk, int ncol, long ld,
+                    double *sys_out)
 {
-    const long col = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= ncol) return;
-    const int k = blockIdx.y;
+    __shared__ double s_th[kSysLevels + 1][32], s_tek0[kSysLevels + 1][32], s_qs[kSysLevels + 1][32];
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const long col = (long)blockIdx.x * 32 + tx;
+    const int k = blockIdx.y * kSysLevels + ty;
+    if (col >= ncol || k >= nk) return;   // a barrier counts the threads that are left
     const long slab = (long)nk * ld, o = (long)k * ld + col;
-    auto pl = [&](int e, int kk) { return __ldg(lv + e * slab + (long)kk * ld + col); };
-    {
-        // every line the row reads, requested into L1 at once
-        const int km = k > 0 ? k - 1 : 0, kp = k + 1 < nk ? k + 1 : nk - 1;
-        pf_l1(lv + P_QENI * slab + (long)km * ld + col);
-        pf_l1(lv + P_QENI * slab + o);
-        pf_l1(lv + P_QENI * slab + (long)kp * ld + col);
-        pf_l1(lv + P_TH * slab + (long)kp * ld + col);
-#pragma unroll
-        for (int e = P_TH; e <= P_LEITI; ++e) pf_l1(lv + e * slab + o);
-        pf_l1(qtotal + o);
+    const Lev L = load_lev(F, o);
+    const double ne0 = __ldg(F.ne + o);
+    // the lines of the losses, requested ahead of the interface
+    if (ty < kSysLevels) {
+        pf_l1(F.xnmbar + o);
+        pf_l1(F.ti + o);
+        pf_l1(F.op + o);
+        pf_l1(F.o2p + o);
+        pf_l1(F.nplus + o);
+        pf_l1(F.n2p + o);
+        pf_l1(F.nop + o);
         pf_l1(F.scht + o);
     }
-    // qtotal += q_eni at the interfaces (settei_ng.F90:248-254); level k
-    // reads and writes only its own qtotal
-    const double qe_k = pl(P_QENI, k);
-    if (k == 0)
-        qtotal[o] = xa(qtotal[o], xs(xm(1.5, qe_k), xm(0.5, pl(P_QENI, 1))));
-    else if (k <= nk - 2)
-        qtotal[o] = xa(qtotal[o], xm(.5, xa(pl(P_QENI, k - 1), qe_k)));
-    else
-        qtotal[o] = xa(qtotal[o], xs(xm(1.5, pl(P_QENI, nk - 2)), xm(0.5, nk >= 3 ? pl(P_QENI, nk - 3) : 0.)));
-    if (k > nk - 2) return;
-    const double dz = C.dz;
+    {
+        // interface k (settei_ng.F90:89-139)
+        double te_int, o2n, o1n, hen, n2n;
+        if (k == 0) {
+            const double *b = C.b, *fb = C.fb;
+            te_int = dmax(xs(xm(1.5, L.te), xm(.5, __ldg(F.te + o + ld))), __ldg(F.t_lbc + col));
+            o2n = xm(.5, xa(xa(xa(fb[0], xm(xa(b[0], 1.), L.o2)), xm(b[3], L.o1)), xm(b[6], L.he)));
+            o1n = xm(.5, xa(xa(xa(fb[0], xm(b[0], L.o2)), xm(xa(b[3], 1.), L.o1)), xm(b[6], L.he)));
+            hen = xm(.5, xa(xa(xa(fb[0], xm(b[0], L.o2)), xm(b[3], L.o1)), xm(xa(b[6], 1.), L.he)));
+            n2n = dmax(xs(xs(xs(1., o2n), o1n), hen), 0.);
+        } else {
+            const Lev Lm = load_lev(F, o - ld);
+            te_int = k == nk - 1 ? xs(xm(1.5, Lm.te), xm(.5, __ldg(F.te + o - 2 * ld))) : xm(.5, xa(L.te, Lm.te));
+            o2n = xm(.5, xa(L.o2, Lm.o2));
+            o1n = xm(.5, xa(L.o1, Lm.o1));
+            hen = xm(.5, xa(L.he, Lm.he));
+            n2n = xm(.5, xa(L.n2, Lm.n2));
+        }
+        const Iface I = iface(C, te_int, o2n, o1n, hen, n2n, __ldg(F.xnmbari + o), ne0, __ldg(F.schti + o));
+        s_th[ty][tx] = I.th;
+        s_tek0[ty][tx] = I.tek0;
+        s_qs[ty][tx] = qsum(F, o);
+    }
+    __syncthreads();
+    if (ty == kSysLevels) return;   // the group's upper interface
+    // heating, cooling and exchange of level k (:157-246)
+    const bool top = k == nk - 1;
+    const double rne_raw = top ? xd(xm(xm(ne0, ne0), ne0), __ldg(F.ne + o - ld)) : xm(ne0, __ldg(F.ne + o + ld));
+    const Loss T = level_loss(F, C, o, L, rne_raw, top ? 0. : sqrt(xm(s_qs[ty][tx], s_qs[ty + 1][tx])));
+    keep[K_LEI * slab + o] = T.lei;
+    keep[K_LIN * slab + o] = T.lin;
+    keep[K_QENI * slab + o] = T.q_eni;
+    if (top) return;
     double sindip;
     {
         const double dm = fabs(__ldg(F.dipmag + col));
         const double sn = sin(dm > C.dipmin ? dm : C.dipmin);
         sindip = dmax(xm(sn, sn), .10);
     }
-    const double pb = xm(xd(xd(2., 7.), xm(__ldg(F.scht + o), xm(dz, dz))), sindip);
-    double r = xm(pb, pl(P_TH, k + 1));
-    double p = xm(pb, pl(P_TH, k));
+    // row k (:131-155, :183, :240-242)
+    const double pb = xm(xd(xd(2., 7.), xm(__ldg(F.scht + o), xm(C.dz, C.dz))), sindip);
+    double r = xm(pb, s_th[ty + 1][tx]);
+    double p = xm(pb, s_th[ty][tx]);
     double q = -xa(p, r);
     double rhs = 0.;
     if (k == 0) {
@@ -666,14 +755,14 @@ __global__ void __launch_bounds__(128) k_settei_coefs(SetteiFields F, SetteiCons
     }
     if (k == nk - 2) {
         q = xa(q, r);
-        rhs = xa(rhs, xd(xm(xm(xm(xm(r, dz), 3.5), __ldg(F.schti + (long)(nk - 1) * ld + col)), settei_fe(F, C, col)),
-                         pl(P_TEK0, nk - 1)));
+        rhs = xa(rhs, xd(xm(xm(xm(xm(r, C.dz), 3.5), __ldg(F.schti + o + ld)), settei_fe(F, C, col)),
+                         s_tek0[ty + 1][tx]));
         r = 0.;
     }
-    rhs = xs(rhs, pl(P_QE, k));
-    if (C.et) rhs = xs(rhs, pl(P_ET, k));
-    q = xs(q, pl(P_DQ, k));
-    rhs = xs(xs(rhs, pl(P_LENTN, k)), pl(P_LEITI, k));
+    rhs = xs(rhs, T.qe_h);
+    if (C.et) rhs = xs(rhs, T.et_h);
+    q = xs(q, T.dq);
+    rhs = xs(xs(rhs, T.len_tn), T.lei_ti);
     rows[o] = p;
     rows[slab + o] = q;
     rows[2 * slab + o] = r;
@@ -686,32 +775,39 @@ __global__ void __launch_bounds__(128) k_settei_coefs(SetteiFields F, SetteiCons
     }
 }
 
-__global__ void __launch_bounds__(128) k_settei_post(SetteiFields F, SetteiConsts C, const double *lv, const double *x,
-                                                     double *te_out, double *ti_out, int nk, int ncol, long ld)
+// pow27 in place of the device pow took it from 14.5 to 11.6 us on 11,248
+// columns x 57; 41 MB are read in that time, the rest is the reads' latency.
+__global__ void __launch_bounds__(128) k_settei_post(SetteiFields F, SetteiConsts C, const double *keep, const double *x,
+                                                     double *te_out, double *ti_out, double *qtotal, int nk, int ncol,
+                                                     long ld)
 {
     const long col = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= ncol) return;
     const int k = blockIdx.y, K = nk - 1;
     const long slab = (long)nk * ld, o = (long)k * ld + col;
-    const double e27 = xd(2., 7.);
+    auto qe = [&](int kk) { return __ldg(keep + K_QENI * slab + (long)kk * ld + col); };
+    // qtotal += q_eni at the interfaces (settei_ng.F90:248-254)
+    const double dqt = k == 0 ? xs(xm(1.5, qe(0)), xm(0.5, qe(1)))
+                       : k < K ? xm(.5, xa(qe(k - 1), qe(k))) : xs(xm(1.5, qe(K - 1)), xm(0.5, qe(K - 2)));
+    qtotal[o] = xa(qtotal[o], dqt);
     double t;
     if (k < K) {
-        t = pow(x[o], e27);
+        t = pow27(x[o]);
     } else {
         // te(nk) = te(nk-1)**2/te(nk-2) from the unfloored values
-        const double t1 = pow(x[(long)(K - 1) * ld + col], e27), t2 = pow(x[(long)(K - 2) * ld + col], e27);
+        const double t1 = pow27(x[(long)(K - 1) * ld + col]), t2 = pow27(x[(long)(K - 2) * ld + col]);
         t = xd(xm(t1, t1), t2);
     }
     const double tn = __ldg(F.tn + o);
     const double te = dmax(t, tn);
-    const double lei = __ldg(lv + P_LEI * slab + o), lin = __ldg(lv + P_LIN * slab + o);
+    const double lei = __ldg(keep + K_LEI * slab + o), lin = __ldg(keep + K_LIN * slab + o);
     te_out[o] = te;
     const double num = xa(xa(xd(xm(__ldg(F.qji_ti + o), __ldg(F.xnmbar + o)), C.avo), xm(lei, te)), xm(lin, tn));
     ti_out[o] = dmax(xd(num, xa(lei, lin)), tn);
 }
 
-// the level planes, then (three-pass form) the four row planes and x
-size_t settei_scratch_doubles(int nk, long ld) { return (size_t)(P_N + 5) * nk * ld; }
+// ten level planes (two-pass form), or four row planes, x and three rates
+size_t settei_scratch_doubles(int nk, long ld) { return (size_t)P_N * nk * ld; }
 
 cudaError_t launch_settei_ng(const SetteiFields &F, const SetteiConsts &C, double *te_out, double *ti_out,
                              double *qtotal, int nk, int ncol, long ld, double *sys_out, unsigned *status,
@@ -729,17 +825,18 @@ cudaError_t launch_settei_ng(const SetteiFields &F, const SetteiConsts &C, doubl
     const size_t per = (size_t)(2 * nk - 1) * sizeof(double);
     while (T > 32 && (size_t)T * per > (size_t)optin) T /= 2;
     if ((size_t)T * per > (size_t)optin) return cudaErrorInvalidValue;
-    // three-pass (on 41472 columns 271 against 280 us for the two-pass walk)
+    // three-pass (on 43,216 columns x 57 233 against 280 us for the two-pass walk)
     if (scratch && assembly_mode() == 2) {
         const long slab = (long)nk * ld;
-        double *rows = scratch + P_N * slab, *x = rows + 4 * slab;
-        const dim3 grid((ncol + 127) / 128, nk);
-        k_settei_levels<<<grid, 128, 0, st>>>(F, C, scratch, nk, ncol, ld);
-        k_settei_coefs<<<grid, 128, 0, st>>>(F, C, scratch, rows, qtotal, nk, ncol, ld, sys_out);
+        double *rows = scratch, *x = rows + 4 * slab, *keep = x + slab;
+        static_assert(5 + K_N <= P_N, "scratch planes");
+        const dim3 grid((ncol + 31) / 32, (nk + kSysLevels - 1) / kSysLevels);
+        k_settei_system<<<grid, dim3(32, kSysLevels + 1), 0, st>>>(F, C, rows, keep, nk, ncol, ld, sys_out);
         cudaError_t e = launch_thomas_post(rows, rows + slab, rows + 2 * slab, rows + 3 * slab, x, nk, nk - 1, 0, ncol,
                                            ld, status, nullptr, st);
         if (e != cudaSuccess) return e;
-        k_settei_post<<<grid, 128, 0, st>>>(F, C, scratch, x, te_out, ti_out, nk, ncol, ld);
+        k_settei_post<<<dim3((ncol + 127) / 128, nk), 128, 0, st>>>(F, C, keep, x, te_out, ti_out, qtotal, nk, ncol,
+                                                                    ld);
         return cudaGetLastError();
     }
     if (scratch && assembly_mode() >= 1) {
