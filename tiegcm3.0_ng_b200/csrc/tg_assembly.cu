@@ -245,6 +245,13 @@ __global__ void __launch_bounds__(128) k_dt_ng(DtFields F, DtConsts C, double *t
 // Three-pass form of dt_ng: row k (0..nk-2) of every column, one thread per
 // (row, column), from the fields of levels k-1..k+1 read directly: the same
 // operations as k_dt_ng's walk, which keeps those levels in a sliding window.
+// Bound by its 28 reads per point (43,216 columns x 57: the routine 131 us for
+// 490 MB that it must move, 4.3 TB/s in this kernel): divisions by dz, exact
+// where dz is a power of two, one reciprocal for the two by mbar, and 10 blocks
+// per SM (48 registers) take it from 136 to 131 us, 47.3 to 45.4 on 11,248;
+// 8 blocks 133, 12 blocks 147.  Forming each level's g and f once for the rows
+// on both sides, handed on in shared memory, is slower (141 and 49.3): the
+// barrier holds the reads back.
 namespace {
 // g, f of level j: tni(0) is the previous lower boundary, tni(j) the
 // interface mean of tn(j-1), tn(j) up to nk-2 and tn(j-1) above
@@ -266,18 +273,18 @@ __device__ __forceinline__ double dt_v0(const DtFields &F, int j, int nk, long l
     return 0.0;
 }
 // wind shear of row k (dt_ng.F90:86-95); the top rows divide the row below by 3
-__device__ __forceinline__ void dt_shear_at(const DtFields &F, const DtConsts &C, int k, int nk, long ld, long col,
+template <bool EX>
+__device__ __forceinline__ void dt_shear_at(const DtFields &F, const DivBy<EX> &dz, const DivBy<EX> &dz2, int k, int nk, long ld, long col,
                                             double &dudz, double &dvdz)
 {
     auto at = [&](const double *p, int kk) { return __ldg(p + kk * ld + col); };
-    const double dz = C.dz;
     const int kc = k <= nk - 3 ? k : nk - 3;
     if (kc <= 0) {
-        dudz = xd(xs(xa(at(F.un, 0), xm(1.0 / 3.0, at(F.un, 1))), xm(4.0 / 3.0, __ldg(F.ulbc + col))), dz);
-        dvdz = xd(xs(xa(at(F.vn, 0), xm(1.0 / 3.0, at(F.vn, 1))), xm(4.0 / 3.0, __ldg(F.vlbc + col))), dz);
+        dudz = dz(xs(xa(at(F.un, 0), xm(1.0 / 3.0, at(F.un, 1))), xm(4.0 / 3.0, __ldg(F.ulbc + col))));
+        dvdz = dz(xs(xa(at(F.vn, 0), xm(1.0 / 3.0, at(F.vn, 1))), xm(4.0 / 3.0, __ldg(F.vlbc + col))));
     } else {
-        dudz = xd(xs(at(F.un, kc + 1), at(F.un, kc - 1)), xm(2.0, dz));
-        dvdz = xd(xs(at(F.vn, kc + 1), at(F.vn, kc - 1)), xm(2.0, dz));
+        dudz = dz2(xs(at(F.un, kc + 1), at(F.un, kc - 1)));
+        dvdz = dz2(xs(at(F.vn, kc + 1), at(F.vn, kc - 1)));
     }
     for (int kk = kc + 1; kk <= k; ++kk) {
         dudz = xd(dudz, 3.0);
@@ -286,8 +293,9 @@ __device__ __forceinline__ void dt_shear_at(const DtFields &F, const DtConsts &C
 }
 }  // namespace
 
-__global__ void __launch_bounds__(128) k_dt_coefs(DtFields F, DtConsts C, double *pqrf, int nk, int ncol, long ld,
-                                                  double *sys_out)
+template <bool EX>
+__global__ void __launch_bounds__(128, 10) k_dt_coefs(DtFields F, DtConsts C, DivBy<EX> dz, DivBy<EX> dz2, double *pqrf,
+                                                  int nk, int ncol, long ld, double *sys_out)
 {
     const long col = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= ncol) return;
@@ -315,7 +323,6 @@ __global__ void __launch_bounds__(128) k_dt_coefs(DtFields F, DtConsts C, double
 #pragma unroll
         for (int i = 0; i < 11; ++i) pf_l1(one[i] + o);
     }
-    const double dz = C.dz;
     const double expz = __ldg(F.expz + k);
     const GF gf0 = dt_gf_at(F, C, k, nk, ld, col), gfp = dt_gf_at(F, C, k + 1, nk, ld, col);
     double p = xs(gf0.g, gf0.f);
@@ -327,26 +334,26 @@ __global__ void __launch_bounds__(128) k_dt_coefs(DtFields F, DtConsts C, double
         q = xs(-gf0.g, gf0.f);
         r = 0.0;
     }
-    const double vad = xd(xm(xa(dt_v0(F, k, nk, ld, col), dt_v0(F, k + 1, nk, ld, col)), 0.5), dz);
+    const double vad = dz(xm(xa(dt_v0(F, k, nk, ld, col), dt_v0(F, k + 1, nk, ld, col)), 0.5));
     const double cp_0 = at(F.cp, k), cp_p = at(F.cp, k + 1);
     const double cpi = xm(0.5, xa(cp_0, cp_p));
     const double kmi = xm(0.5, xa(at(F.km, k), at(F.km, k + 1)));
     const double wi = xm(0.5, xa(at(F.w, k), at(F.w, k + 1)));
     double dudz, dvdz;
-    dt_shear_at(F, C, k, nk, ld, col, dudz, dvdz);
+    dt_shear_at(F, dz, dz2, k, nk, ld, col, dudz, dvdz);
     const double qsolar = xm(0.5, xa(at(F.qtotal, k), at(F.qtotal, k + 1)));
     const double advec = xa(at(F.horadv, k), vad);
     double cptn = xm(cpi, xs(advec, xm(C.dtx2inv, at(F.tnsmooth, k))));
     cptn = xm(cptn, expz);
-    const double mbar = at(F.mbar, k);
+    const double mbar = at(F.mbar, k), ymbar = __drcp_rn(mbar);
     const double xo = xm(xm(at(F.xnmbar, k), at(F.o1, k)), C.rmassinv_o1);
-    const double qrecomb = xd(xm(xm(xm(C.tsurplus, at(F.rkm12, k)), xm(xo, xo)), C.avo), mbar);
+    const double qrecomb = qdiv1(xm(xm(xm(C.tsurplus, at(F.rkm12, k)), xm(xo, xo)), C.avo), mbar, ymbar);
     double qm = xm(xd(xm(C.grav, kmi), xm(C.p0, at(F.scht, k))), xa(xm(dudz, dudz), xm(dvdz, dvdz)));
     qm = xd(qm, expz);
     const double th = xa(xa(xa(xa(qsolar, at(F.hdt, k)), qrecomb), at(F.qji_tn, k)), qm);
     cptn = xs(cptn, xm(th, expz));
     double rhs = xa(cptn, at(F.cool_exp, k));
-    const double qpart = xa(xm(cpi, xa(C.dtx2inv, at(F.cool_imp, k))), xd(xm(wi, C.gask), mbar));
+    const double qpart = xa(xm(cpi, xa(C.dtx2inv, at(F.cool_imp, k))), qdiv1(xm(wi, C.gask), mbar, ymbar));
     q = xs(q, xm(qpart, expz));
     if (k == 0) {   // lower boundary fold (:159-163)
         q = xs(q, p);
@@ -376,7 +383,14 @@ cudaError_t launch_dt_ng(const DtFields &F, const DtConsts &C, double *tn_upd, i
     // 41472 columns 143 against 151 us for the fused walk)
     if (scratch && assembly_mode() == 2 && nk >= 3) {
         const long slab = (long)nk * ld;
-        k_dt_coefs<<<dim3((ncol + 127) / 128, nk - 1), 128, 0, st>>>(F, C, scratch, nk, ncol, ld, sys_out);
+        const dim3 grid((ncol + 127) / 128, nk - 1);
+        const double dz2 = 2.0 * C.dz;
+        if (exact_reciprocal(C.dz))
+            k_dt_coefs<true><<<grid, 128, 0, st>>>(F, C, DivBy<true>{C.dz, 1.0 / C.dz}, DivBy<true>{dz2, 1.0 / dz2},
+                                                   scratch, nk, ncol, ld, sys_out);
+        else
+            k_dt_coefs<false><<<grid, 128, 0, st>>>(F, C, DivBy<false>{C.dz, 1.0 / C.dz},
+                                                    DivBy<false>{dz2, 1.0 / dz2}, scratch, nk, ncol, ld, sys_out);
         return launch_thomas_post(scratch, scratch + slab, scratch + 2 * slab, scratch + 3 * slab, tn_upd, nk, nk - 1,
                                   1, ncol, ld, status, post, st);
     }
