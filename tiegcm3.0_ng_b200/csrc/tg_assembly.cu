@@ -2052,20 +2052,22 @@ size_t comp_scratch_doubles(int nk, long ld)
 }  // namespace tg
 
 // comp_ng post-solve steps (src/comp_ng.F90:394-457): the lateral-boundary
-// overwrite of the columns flagged in bmask (when given), the time filter,
-// the N2 extrapolation, floors and normalisation.  A block takes 32 columns
-// with sixteen warps (about four levels each, so that few-column launches
-// do not wait on a long run of levels per warp); a warp works on the 32
-// columns of one level at a time, so
-// every phase runs over all levels at once: the overwrite, the search for the
-// first level with N2 < 0.01 (the least level any warp finds), the
-// extrapolation constants (one thread per column), then the per-level steps.
+// values of the columns flagged in bmask (when given), the time filter, the N2
+// extrapolation, floors and normalisation.  A block takes 16 columns with 32
+// threads each, so that two levels per thread cover a 57-level column and few
+// columns still spread over the chip; every phase runs over all levels at
+// once: the search for the first level with N2 < 0.01 (the least level any
+// thread finds), the extrapolation constants (one thread per column), then the
+// per-level steps.  Bound by the reads' latency: the search reads its levels
+// without leaving off at the first and requests the last phase's lines.
+// 2,072 columns x 57 levels 10.4 us with 32-column blocks that stopped at the
+// first such level, 6.3 now; 6,969 12.4 and 10.7; 11,248 17.7 and 16.5.
 // The N2 extrapolation uses the device log/exp, so it agrees with the CPU
 // restatement to a tolerance in the extrapolated levels.
 namespace tg {
-constexpr int kPostCols = 32, kPostWarps = 16;
+constexpr int kPostCols = 16, kPostGroups = 32;
 
-__global__ void __launch_bounds__(kPostCols * kPostWarps) k_comp_post_ng(
+__global__ void __launch_bounds__(kPostCols * kPostGroups) k_comp_post_ng(
     const double *o2, const double *o1, const double *he, const double *o2_nm, const double *o1_nm,
     const double *he_nm, const double *xnmbar, const double *zpmid, double dz, double ds, double ds2, int nk, int ncol,
     long ld, double *o2u, double *o1u, double *heu, double *o2n, double *o1n, double *hen, const unsigned char *bmask,
@@ -2078,24 +2080,29 @@ __global__ void __launch_bounds__(kPostCols * kPostWarps) k_comp_post_ng(
     const bool live = col < ncol;
     const double small = 1.e-9;
     if (w == 0) ktop_s[c] = nk;
-    // the Dirichlet lateral-boundary hook (comp_ng.F90:394-413)
-    if (live && bmask && bmask[col])
-        for (int k = w; k < nk; k += kPostWarps) {
-            const long o = (long)k * ld + col;
-            o2u[o] = b2[o];
-            o1u[o] = b1[o];
-            heu[o] = bh[o];
-        }
     __syncthreads();
+    // the Dirichlet lateral-boundary hook (comp_ng.F90:394-413): a flagged
+    // column's solution is its boundary value
+    const bool bcol = live && bmask && bmask[col];
+    const double *x2 = bcol ? b2 : o2u, *x1 = bcol ? b1 : o1u, *xh = bcol ? bh : heu;
+    auto n2_at = [&](long o) { return xs(xs(xs(1.0, x2[o]), x1[o]), xh[o]); };
     // first level with N2 < 0.01 (comp_ng.F90:425-429)
-    if (live)
-        for (int k = w; k < nk; k += kPostWarps) {
+    if (live) {
+        int kt = nk;
+#pragma unroll 4
+        for (int k = w; k < nk; k += kPostGroups) {
             const long o = (long)k * ld + col;
-            if (xs(xs(xs(1.0, o2u[o]), o1u[o]), heu[o]) < 0.01) {
-                atomicMin(&ktop_s[c], k);
-                break;
-            }
+            pf_l1(o2_nm + o);
+            pf_l1(o1_nm + o);
+            pf_l1(he_nm + o);
+            pf_l1(o2 + o);
+            pf_l1(o1 + o);
+            pf_l1(he + o);
+            pf_l1(xnmbar + o);
+            if (n2_at(o) < 0.01) kt = min(kt, k);
         }
+        if (kt < nk) atomicMin(&ktop_s[c], kt);
+    }
     __syncthreads();
     if (w == 0 && live) {
         const int ktop = ktop_s[c];
@@ -2103,8 +2110,8 @@ __global__ void __launch_bounds__(kPostCols * kPostWarps) k_comp_post_ng(
         if (ktop > 0 && ktop < nk - 1) {
             const long o = (long)ktop * ld + col, om = o - ld;
             zmtop = zpmid[ktop];
-            n2top = log(xm(xs(xs(xs(1.0, o2u[o]), o1u[o]), heu[o]), xnmbar[o]));
-            const double n2top1 = log(xm(xs(xs(xs(1.0, o2u[om]), o1u[om]), heu[om]), xnmbar[om]));
+            n2top = log(xm(n2_at(o), xnmbar[o]));
+            const double n2top1 = log(xm(n2_at(om), xnmbar[om]));
             dn2dz = xd(xs(n2top, n2top1), dz);
         }
         n2top_s[c] = n2top;
@@ -2116,9 +2123,9 @@ __global__ void __launch_bounds__(kPostCols * kPostWarps) k_comp_post_ng(
     const int ktop = ktop_s[c];
     const bool extrap = ktop > 0 && ktop < nk - 1;
     const double n2top = n2top_s[c], dn2dz = dn2dz_s[c], zmtop = zmtop_s[c];
-    for (int k = w; k < nk; k += kPostWarps) {
+    for (int k = w; k < nk; k += kPostGroups) {
         const long o = (long)k * ld + col;
-        const double a0 = o2u[o], b0 = o1u[o], c0 = heu[o];
+        const double a0 = x2[o], b0 = x1[o], c0 = xh[o];
         const double an = xa(xm(ds2, xa(o2_nm[o], a0)), xm(ds, o2[o]));
         const double bn = xa(xm(ds2, xa(o1_nm[o], b0)), xm(ds, o1[o]));
         const double cn = xa(xm(ds2, xa(he_nm[o], c0)), xm(ds, he[o]));
@@ -2148,7 +2155,7 @@ cudaError_t launch_comp_post_ng(const double *const *in7, const double *zpmid, d
                                 const unsigned char *bnd_mask, const double *const *bnd3)
 {
     if (ncol <= 0) return cudaSuccess;
-    k_comp_post_ng<<<(ncol + kPostCols - 1) / kPostCols, kPostCols * kPostWarps, 0, st>>>(
+    k_comp_post_ng<<<(ncol + kPostCols - 1) / kPostCols, kPostCols * kPostGroups, 0, st>>>(
         in7[0], in7[1], in7[2], in7[3], in7[4], in7[5], in7[6], zpmid, dz, dtsmooth, dtsmooth_div2, nk, ncol, ld,
         upd6[0], upd6[1], upd6[2], upd6[3], upd6[4], upd6[5], bnd_mask, bnd_mask ? bnd3[0] : nullptr,
         bnd_mask ? bnd3[1] : nullptr, bnd_mask ? bnd3[2] : nullptr);

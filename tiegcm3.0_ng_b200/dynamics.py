@@ -231,11 +231,11 @@ class DynamicsStep:
                     [F[sp + "nm_smooth"] for sp in sps], st)
         cs.comp_ng_dev(F, c["C"], c["out"], g.nk, g.ncol, g.ld, stream=st)
         if self.ring is not None:
-            # filter_o2o on the interior latitudes: rows 2 .. nlat+1 of the subdomain
+            # filter_o2o on the interior latitudes, rows 2 .. nlat+1 of the subdomain; the three species
+            # are one array, 3*nk levels apart by ld: one launch
             off = 8 * 2 * (g.nlon + 4)
-            for i in range(3):
-                cs.ringfilter_dev(c["out"][i].data_ptr() + off, g.nk, g.nlon, g.nlat, 1, 0, self.ring, g.dlamda,
-                                  g.ld, stream=st)
+            cs.ringfilter_dev(c["out"].data_ptr() + off, 3 * g.nk, g.nlon, g.nlat, 1, 0, self.ring, g.dlamda, g.ld,
+                              stream=st)
         cs.comp_post_ng_dev(c["post_in"], c["zpmid"], c["pc"], [c["out"][i] for i in range(3)],
                             [c["nm"][i] for i in range(3)], g.nk, g.ncol, g.ld, bnd_mask=self.mask, bnd=c["bnd"],
                             stream=st)
