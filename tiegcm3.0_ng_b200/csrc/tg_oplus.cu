@@ -154,14 +154,27 @@ struct OplusRowsAt {
     }
 };
 
+// What every row needs of them; the rest is the top row's.
+__device__ __forceinline__ OplusCol oplus_col_rows(const OplusFields &F, const OplusConsts &C, long col, double gmr)
+{
+    OplusCol c;
+    c.bz = __ldg(F.bz + col);
+    c.dvbz = xd(__ldg(F.dvb + col), c.bz);
+    c.bz2 = xm(c.bz, c.bz);
+    c.gmr = gmr;
+    c.dtn = xm(C.dtx2inv, (double)C.nstep_sub);
+    c.opflux = c.ubca = c.ubcb = 0.;
+    return c;
+}
+// g*m/(2R) of O+ (the same IEEE operations on the host and the device)
+__host__ __device__ inline double oplus_gmr(const OplusConsts &C) { return C.grav * C.rmass_op / (2. * C.gask); }
 __device__ __forceinline__ OplusCol oplus_col(const OplusFields &F, const OplusConsts &C, const OplusRowsAt &A)
 {
     const long col = A.col;
     // pi = 4*atan(1) of the reference, correctly rounded
     const double pi = 3.141592653589793, rtd = 180. / pi;
     const double phid = 2.0e8, phin = -2.0e8, ppolar = 0.;
-    OplusCol c;
-    c.bz = __ldg(F.bz + col);
+    OplusCol c = oplus_col_rows(F, C, col, oplus_gmr(C));
     {
         const double arl = fabs(__ldg(F.rlatm + col)), chi = __ldg(F.chi + col);
         double a = 0.;
@@ -176,10 +189,6 @@ __device__ __forceinline__ OplusCol oplus_col(const OplusFields &F, const OplusC
         if (arl >= xd(pi, 3.)) opflux = xa(opflux, ppolar);
         c.opflux = opflux;
     }
-    c.dvbz = xd(__ldg(F.dvb + col), c.bz);
-    c.bz2 = xm(c.bz, c.bz);
-    c.gmr = xd(xm(C.grav, C.rmass_op), xm(2., C.gask));
-    c.dtn = xm(C.dtx2inv, (double)C.nstep_sub);
     OplusRowsAt B = A;
     B.gmr = c.gmr;
     const int nk = A.nk;
@@ -383,47 +392,78 @@ __global__ void __launch_bounds__(128) k_oplus_rows(OplusFields F, OplusConsts C
     oplus_walk(F, C, opout, scr, smem_or + threadIdx.x, blockDim.x, nk, ld, col, sys_out, status, post, has_post, pd);
 }
 
-// Three-pass form, pass 2: row k of every column, one thread per (row, column).
-// A block covers kCoefCols columns x kCoefRows rows; the column quantities
-// (oplus_col: the O+ flux boundary with its cosine, the upper-boundary
-// coefficients, several divisions) are formed once per column and block by
-// the block's first row of threads and shared.
-constexpr int kCoefCols = 32, kCoefRows = 8;
-dim3 coef_grid(int nk, int ncol)
+// oplus_row of a row that no boundary touches (0 < k < nk-2): the same
+// operations on level values read once; re by its reciprocal.
+__device__ __forceinline__ void oplus_row_mid(const OplusFields &F, const OplusConsts &C, const double *scr, long slab,
+                                              long o, long ld, const OplusCol &cc, double yre, double &p, double &q,
+                                              double &r, double &ex)
 {
-    return dim3((unsigned)((ncol + kCoefCols - 1) / kCoefCols), (unsigned)((nk - 1 + kCoefRows - 1) / kCoefRows));
+    auto S = [&](int e, long d) { return __ldg(scr + (long)e * slab + o + d); };
+    const double djm = S(S_DJ, -ld), dj0 = S(S_DJ, 0), djp = S(S_DJ, ld);
+    const double hzm = S(S_HDZ, -ld), hz0 = S(S_HDZ, 0), hzp = S(S_HDZ, ld);
+    const double tpm = S(S_TP1, -ld), tp0 = S(S_TP1, 0), tpp = S(S_TP1, ld);
+    const double bum = S(S_BDOTU, -ld), bu0 = S(S_BDOTU, 0), bup = S(S_BDOTU, ld);
+    const double wii = xm(.5, xa(__ldg(F.wi + o), __ldg(F.wi + o + ld)));
+    const double hi0 = xm(0.5, xa(hzm, hz0)), hi1 = xm(0.5, xa(hz0, hzp));
+    const double dji_k = xm(0.5, xa(djm, dj0)), dji_1 = xm(0.5, xa(dj0, djp));
+    const double divbz = xa(cc.dvbz, xd(__ldg(F.bdotdh_djbz + o), xm(dj0, cc.bz2)));
+    const double hdzm_k = xm(xs(hz0, xm(0.5, divbz)), cc.bz2), hdzp_k = xm(xa(hz0, xm(0.5, divbz)), cc.bz2);
+    const double t0k = xs(xm(xm(2., tpm), hi0), cc.gmr), t1k = xa(xm(xm(2., tp0), hi0), cc.gmr);
+    const double t01 = xs(xm(xm(2., tp0), hi1), cc.gmr), t11 = xa(xm(xm(2., tpp), hi1), cc.gmr);
+    p = xa(xa(xm(xm(hdzm_k, dji_k), t0k), xm(xm(wii, 0.5), hz0)), xm(xm(xm(cc.bz, bum), 0.5), hz0));
+    q = -xa(xm(xm(hdzp_k, dji_1), t01), xm(xm(hdzm_k, dji_k), t1k));
+    q = xa(xa(q, qdiv1(xm(-wii, 6.), C.re, yre)), xm(xm(-bu0, cc.dvbz), cc.bz));
+    q = xs(xs(q, cc.dtn), S(S_OL, 0));
+    r = xa(xa(xm(xm(hdzp_k, dji_1), t11), xm(xm(-wii, 0.5), hz0)), xm(xm(xm(-cc.bz, bup), 0.5), hz0));
+    ex = xs(__ldg(F.explicit_h + o), xm(xm(__ldg(F.optm1_smooth2 + o), C.dtx2inv), (double)C.nstep_sub));
+    ex = xs(ex, S(S_PROD, 0));
 }
-__global__ void __launch_bounds__(kCoefCols * kCoefRows) k_oplus_coefs(OplusFields F, OplusConsts C, double *scr,
-                                                                       int nk, int ncol, long ld, double *sys_out)
+
+// Three-pass form, pass 2: row k of every column, one thread per (row, column).
+// The O+ flux boundary (a cosine, several divisions) and the upper-boundary
+// ratios are formed by the top row alone, and rows that no boundary touches
+// take oplus_row_mid, whose 20 reads are all in flight before its first
+// operation.  Bound by those reads (43,216 columns x 57: the routine 258 us
+// with the column quantities formed by one warp of eight behind a barrier and
+// every level value read through its boundary cases, 224 with them formed by
+// the rows, 202 now; 11,248 82.7, 75.2 and 69.8; 2,072 30.0 and 28.7).  The
+// lines are requested into L1 first (208 without); 8 blocks per SM, 64
+// registers without spills (10 blocks 208, 12 blocks 212).
+__global__ void __launch_bounds__(128, 8) k_oplus_coefs(OplusFields F, OplusConsts C, double gmr, double yre,
+                                                        double *scr, int nk, int ncol, long ld, double *sys_out)
 {
-    __shared__ OplusCol col_q[kCoefCols];
-    const long col = (long)blockIdx.x * kCoefCols + threadIdx.x;
-    const int k = blockIdx.y * kCoefRows + threadIdx.y;
+    const long col = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (col >= ncol) return;
+    const int k = blockIdx.y;
     const long slab = (long)nk * ld, o = (long)k * ld + col;
     OplusRowsAt A{scr, slab, ld, col, nk, 0., 0., 0.};
     // every line row k reads, requested into L1 at once: the loads below
     // sit between divisions and would otherwise wait one at a time
-    if (col < ncol && k < nk - 1) {
+    {
         const int km = k > 0 ? k - 1 : 0;
-        for (int e = S_DJ; e <= S_PROD; ++e)
+#pragma unroll
+        for (int e = S_DJ; e <= S_BDOTU; ++e)
 #pragma unroll
             for (int j = 0; j < 3; ++j) pf_l1(scr + (long)e * slab + (long)(km + j) * ld + col);
+        pf_l1(scr + (long)S_OL * slab + o);
+        pf_l1(scr + (long)S_PROD * slab + o);
         pf_l1(F.bdotdh_djbz + o);
-        pf_l1(F.bdotdh_djbz + o + ld);
         pf_l1(F.wi + o);
         pf_l1(F.wi + o + ld);
         pf_l1(F.explicit_h + o);
         pf_l1(F.optm1_smooth2 + o);
     }
-    if (threadIdx.y == 0 && col < ncol) col_q[threadIdx.x] = oplus_col(F, C, A);
-    __syncthreads();
-    if (col >= ncol || k >= nk - 1) return;
-    const OplusCol cc = col_q[threadIdx.x];
-    A.gmr = cc.gmr;
-    double p, q, r, ex, t_top = 0., t_bot = 0.;
-    oplus_row(F, C, A, cc, k, p, q, r, ex, &t_top, &t_bot);
-    if (k == nk - 2) scr[S_TB * slab + col] = t_top;
-    if (k == 0) scr[S_TB * slab + ld + col] = t_bot;
+    double p, q, r, ex;
+    if (k > 0 && k < nk - 2) {
+        oplus_row_mid(F, C, scr, slab, o, ld, oplus_col_rows(F, C, col, gmr), yre, p, q, r, ex);
+    } else {
+        const OplusCol cc = oplus_col(F, C, A);
+        A.gmr = cc.gmr;
+        double t_top = 0., t_bot = 0.;
+        oplus_row(F, C, A, cc, k, p, q, r, ex, &t_top, &t_bot);
+        if (k == nk - 2) scr[S_TB * slab + col] = t_top;
+        if (k == 0) scr[S_TB * slab + ld + col] = t_bot;
+    }
     scr[S_P * slab + o] = p;
     scr[S_Q * slab + o] = q;
     scr[S_R * slab + o] = r;
@@ -989,7 +1029,8 @@ cudaError_t launch_oplus_factor(const OplusFields &F, const OplusConsts &C, doub
     if (nk < 3) return cudaErrorInvalidValue;
     k_oplus_levels<<<dim3((ncol + 127) / 128, nk), 128, 0, st>>>(F, C, xiop2p, xiop2d, nullptr, nullptr, factor, nk,
                                                                  ncol, ld);
-    k_oplus_coefs<<<coef_grid(nk, ncol), dim3(kCoefCols, kCoefRows), 0, st>>>(F, C, factor, nk, ncol, ld, nullptr);
+    k_oplus_coefs<<<dim3((ncol + 127) / 128, nk - 1), 128, 0, st>>>(F, C, oplus_gmr(C), 1.0 / C.re, factor, nk, ncol,
+                                                                    ld, nullptr);
     return launch_oplus_factor_pass(factor, nk, ncol, ld, status, st);
 }
 
@@ -1102,8 +1143,8 @@ cudaError_t launch_oplus_ng(const OplusFields &F, const OplusConsts &C, double *
         const long slab = (long)nk * ld;
         k_oplus_levels<<<dim3((ncol + 127) / 128, nk), 128, 0, st>>>(F, C, xiop2p, xiop2d, Fe, Fn, scratch, nk, ncol,
                                                                      ld);
-        k_oplus_coefs<<<coef_grid(nk, ncol), dim3(kCoefCols, kCoefRows), 0, st>>>(F, C, scratch, nk, ncol, ld,
-                                                                                  sys_out);
+        k_oplus_coefs<<<dim3((ncol + 127) / 128, nk - 1), 128, 0, st>>>(F, C, oplus_gmr(C), 1.0 / C.re, scratch, nk,
+                                                                        ncol, ld, sys_out);
         return launch_thomas_post(scratch + S_P * slab, scratch + S_Q * slab, scratch + S_R * slab,
                                   scratch + S_EX * slab, opout, nk, nk - 1, 1, ncol, ld, status, post, st);
     }
