@@ -245,13 +245,14 @@ __global__ void __launch_bounds__(128) k_dt_ng(DtFields F, DtConsts C, double *t
 // Three-pass form of dt_ng: row k (0..nk-2) of every column, one thread per
 // (row, column), from the fields of levels k-1..k+1 read directly: the same
 // operations as k_dt_ng's walk, which keeps those levels in a sliding window.
-// Bound by its 28 reads per point (43,216 columns x 57: the routine 131 us for
-// 490 MB that it must move, 4.3 TB/s in this kernel): divisions by dz, exact
+// Bound by its 28 reads per point (43,216 columns x 57: the routine 126 us for
+// 490 MB that it must move, 4.6 TB/s in this kernel): divisions by dz, exact
 // where dz is a power of two, one reciprocal for the two by mbar, and 10 blocks
-// per SM (48 registers) take it from 136 to 131 us, 47.3 to 45.4 on 11,248;
-// 8 blocks 133, 12 blocks 147.  Forming each level's g and f once for the rows
-// on both sides, handed on in shared memory, is slower (141 and 49.3): the
-// barrier holds the reads back.
+// per SM (48 registers) take it from 136 to 130 us (8 blocks 133, 12 blocks
+// 147), rows that no boundary touches reading their levels once, all reads in
+// flight, from 130 to 126 (11,248 columns: 47.3, 45.3 and 43.7).  Forming each
+// level's g and f once for the rows on both sides, handed on in shared memory,
+// is slower (141 and 49.3): the barrier holds the reads back.
 namespace {
 // g, f of level j: tni(0) is the previous lower boundary, tni(j) the
 // interface mean of tn(j-1), tn(j) up to nk-2 and tn(j-1) above
@@ -324,9 +325,30 @@ __global__ void __launch_bounds__(128, 10) k_dt_coefs(DtFields F, DtConsts C, Di
         for (int i = 0; i < 11; ++i) pf_l1(one[i] + o);
     }
     const double expz = __ldg(F.expz + k);
-    const GF gf0 = dt_gf_at(F, C, k, nk, ld, col), gfp = dt_gf_at(F, C, k + 1, nk, ld, col);
-    double p = xs(gf0.g, gf0.f);
-    double q, r;
+    GF gf0, gfp;
+    double vad, dudz, dvdz;
+    double p, q, r;
+    const bool mid = k > 0 && k < nk - 3;
+    if (mid) {   // no boundary case: the levels' values read once, at once
+        const long o = (long)k * ld + col;
+        const double tnm = __ldg(F.tn + o - ld), tn0 = __ldg(F.tn + o), tnp = __ldg(F.tn + o + ld);
+        const double um = __ldg(F.un + o - ld), up_ = __ldg(F.un + o + ld);
+        const double vm = __ldg(F.vn + o - ld), vp = __ldg(F.vn + o + ld);
+        const double h0 = __ldg(F.schti + o), hp = __ldg(F.schti + o + ld);
+        const double kt0 = __ldg(F.kt + o), ktp = __ldg(F.kt + o + ld);
+        const double c0 = __ldg(F.cp + o), c1 = __ldg(F.cp + o + ld), w0 = __ldg(F.w + o), w1 = __ldg(F.w + o + ld);
+        gf0 = dt_gf(C, h0, c0, kt0, xm(0.5, xa(tnm, tn0)), expz, __ldg(F.dift + k));
+        gfp = dt_gf(C, hp, c1, ktp, xm(0.5, xa(tn0, tnp)), __ldg(F.expz + k + 1), __ldg(F.dift + k + 1));
+        vad = dz(xm(xa(xm(xs(tn0, tnm), w0), xm(xs(tnp, tn0), w1)), 0.5));
+        dudz = dz2(xs(up_, um));
+        dvdz = dz2(xs(vp, vm));
+    } else {
+        gf0 = dt_gf_at(F, C, k, nk, ld, col);
+        gfp = dt_gf_at(F, C, k + 1, nk, ld, col);
+        vad = dz(xm(xa(dt_v0(F, k, nk, ld, col), dt_v0(F, k + 1, nk, ld, col)), 0.5));
+        dt_shear_at(F, dz, dz2, k, nk, ld, col, dudz, dvdz);
+    }
+    p = xs(gf0.g, gf0.f);
     if (k < K - 1) {
         q = -xa(xa(xs(gfp.g, gfp.f), gf0.g), gf0.f);
         r = xa(gfp.g, gfp.f);
@@ -334,13 +356,10 @@ __global__ void __launch_bounds__(128, 10) k_dt_coefs(DtFields F, DtConsts C, Di
         q = xs(-gf0.g, gf0.f);
         r = 0.0;
     }
-    const double vad = dz(xm(xa(dt_v0(F, k, nk, ld, col), dt_v0(F, k + 1, nk, ld, col)), 0.5));
     const double cp_0 = at(F.cp, k), cp_p = at(F.cp, k + 1);
     const double cpi = xm(0.5, xa(cp_0, cp_p));
     const double kmi = xm(0.5, xa(at(F.km, k), at(F.km, k + 1)));
     const double wi = xm(0.5, xa(at(F.w, k), at(F.w, k + 1)));
-    double dudz, dvdz;
-    dt_shear_at(F, dz, dz2, k, nk, ld, col, dudz, dvdz);
     const double qsolar = xm(0.5, xa(at(F.qtotal, k), at(F.qtotal, k + 1)));
     const double advec = xa(at(F.horadv, k), vad);
     double cptn = xm(cpi, xs(advec, xm(C.dtx2inv, at(F.tnsmooth, k))));
