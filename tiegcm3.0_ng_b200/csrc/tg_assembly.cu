@@ -793,7 +793,8 @@ __global__ void __launch_bounds__(128) k_minor_ng(MinorFields F, MinorConsts C, 
 }
 
 // ---------------------------------------------------------------------------
-// minor_ng in two passes.  The level quantities (ax, thdiff, dmdz/barm: four
+// minor_ng in two passes (in three, the default, see k_minor_system).  The
+// level quantities (ax, thdiff, dmdz/barm: four
 // fractional powers and a 3x3 inverse per level) are independent across
 // levels, so the first kernel computes them with one thread per (level,
 // column), i.e. nk times the parallelism of the column walk, into a 3-plane
@@ -843,8 +844,7 @@ __device__ __forceinline__ MinorLevel minor_level_at(const MinorFields &F, const
     return minor_level(C, I, at(F.barm, j), t0, dt);
 }
 
-template <bool EX>
-__global__ void __launch_bounds__(128) k_minor_levels(MinorFields F, MinorConsts C, DivBy<EX> dz, double *lv, int nk,
+__global__ void __launch_bounds__(128) k_minor_levels(MinorFields F, MinorConsts C, DivBy<false> dz, double *lv, int nk,
                                                       int ncol, long ld)
 {
     const long col = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -903,46 +903,55 @@ __device__ __forceinline__ void minor_row(const MinorFields &F, const MinorConst
     }
 }
 
-// Three-pass form, pass 2: row k of every column, one thread per (row,
-// column), into the planes pqrf (p, q, r, f, each nk*ld).
+// Three-pass form, passes 1 and 2 in one kernel: row k of every column into the
+// planes pqrf (p, q, r, f, each nk*ld).  A block holds 8 levels of 32 columns,
+// one warp each, and a ninth warp for the level above them, whose quantities
+// the rows below need: every level hands its three on in shared memory.  As two
+// kernels with three planes between them the level pass (FP64 pipe 54% busy)
+// and the row pass (4.6 TB/s) took 47 + 22 us on 21,216 columns x 57; in one
+// the reads pass under the arithmetic.  What it needs is warps in flight: 4
+// blocks per SM at 56 registers and 100 bytes of spills (154 us the routine on
+// 43,216 columns x 57, 165 at 3 blocks, 200 at 2 without spills, 162 at 5);
+// 4 levels per block 159, 15 levels 158.  minor_ng before and now: 22.8 and
+// 20.8 us on 2,072 columns x 57, 53.4 and 50.5 on 11,248, 170 and 153 on 43,216,
+// 328 and 293 on 43,216 x 113.
+constexpr int kMinorLevels = 8, kMinorBlocks = 4;
 template <bool EX>
-__global__ void __launch_bounds__(128) k_minor_coefs(MinorFields F, MinorConsts C, DivBy<EX> dz, const double *lv,
-                                                     double *pqrf, int nk, int ncol, long ld, double *sys_out)
+__global__ void __launch_bounds__(32 * (kMinorLevels + 1), kMinorBlocks)
+    k_minor_system(MinorFields F, MinorConsts C, DivBy<EX> dz, double *pqrf, int nk, int ncol, long ld, double *sys_out)
 {
-    const long col = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= ncol) return;
-    const int k = blockIdx.y;
+    __shared__ double sh[3][kMinorLevels + 1][32];
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const long col = (long)blockIdx.x * 32 + tx;
+    const int k = blockIdx.y * kMinorLevels + ty;
+    if (col >= ncol || k >= nk) return;   // a barrier counts the threads that are left
     const long slab = (long)nk * ld, o = (long)k * ld + col;
-    {
-        // every line the row reads, requested into L1 at once
-        const long op = k < nk - 1 ? o + ld : o;
+    if (ty < kMinorLevels) {
+        // the lines of the row's own reads, requested ahead of the level's
         const double *one[] = {F.sprod, F.xnmbar, F.ftm1_smooth, F.hadvec, F.sloss, F.w};
 #pragma unroll
         for (int i = 0; i < 6; ++i) pf_l1(one[i] + o);
-        pf_l1(F.w + op);
-#pragma unroll
-        for (int e = 0; e < 3; ++e) {
-            pf_l1(lv + e * slab + o);
-            pf_l1(lv + e * slab + op);
-        }
     }
     MinorRowIn in;
+    in.L0 = minor_level_at(F, C, dz, k, nk, ld, col);
+    sh[0][ty][tx] = in.L0.ax;
+    sh[1][ty][tx] = in.L0.thdiff;
+    sh[2][ty][tx] = in.L0.dmdzs;
+    __syncthreads();
+    if (ty == kMinorLevels) return;   // the level above the group's
     in.sprod = __ldg(F.sprod + o);
     in.xnmbar = __ldg(F.xnmbar + o);
     in.ftm1 = __ldg(F.ftm1_smooth + o);
     in.hadvec = __ldg(F.hadvec + o);
-    in.L0.ax = __ldg(lv + o);
-    in.L0.thdiff = __ldg(lv + slab + o);
-    in.L0.dmdzs = __ldg(lv + 2 * slab + o);
     in.L1 = in.L0;
     in.sloss = in.w0 = in.w1 = 0.0;
     if (k < nk - 1) {
         in.sloss = __ldg(F.sloss + o);
         in.w0 = __ldg(F.w + o);
         in.w1 = __ldg(F.w + o + ld);
-        in.L1.ax = __ldg(lv + o + ld);
-        in.L1.thdiff = __ldg(lv + slab + o + ld);
-        in.L1.dmdzs = __ldg(lv + 2 * slab + o + ld);
+        in.L1.ax = sh[0][ty + 1][tx];
+        in.L1.thdiff = sh[1][ty + 1][tx];
+        in.L1.dmdzs = sh[2][ty + 1][tx];
     }
     double p, q, r, f;
     minor_row(F, C, dz, col, k, nk, __ldg(F.dfactor + col), in, p, q, r, f);
@@ -1073,8 +1082,8 @@ static std::atomic<int> g_assembly_mode{2};
 int assembly_mode() { return g_assembly_mode.load(); }
 void set_assembly_mode(int m) { g_assembly_mode.store(m < 0 ? 2 : (m > 2 ? 2 : m)); }
 
-// level planes (ax, thdiff, dmdz/barm) and the rows p, q, r, f
-int minor_scratch_planes() { return 7; }
+// three level planes (two passes) or four row planes (three)
+int minor_scratch_planes() { return 4; }
 
 static std::atomic<int> g_walk_prefetch{-1};
 int walk_prefetch(long ncol)
@@ -1105,16 +1114,11 @@ cudaError_t launch_minor_ng(const MinorFields &F, const MinorConsts &C, double *
     const DivBy<false> dzq{C.dzp, 1.0 / C.dzp};
     if (scratch && assembly_mode() == 2) {
         const long slab = (long)nk * ld;
-        double *pqrf = scratch + 3 * slab;
-        const dim3 grid((ncol + 127) / 128, nk);
-        if (exact_reciprocal(C.dzp)) {
-            const DivBy<true> dz{C.dzp, 1.0 / C.dzp};
-            k_minor_levels<true><<<grid, 128, 0, st>>>(F, C, dz, scratch, nk, ncol, ld);
-            k_minor_coefs<true><<<grid, 128, 0, st>>>(F, C, dz, scratch, pqrf, nk, ncol, ld, sys_out);
-        } else {
-            k_minor_levels<false><<<grid, 128, 0, st>>>(F, C, dzq, scratch, nk, ncol, ld);
-            k_minor_coefs<false><<<grid, 128, 0, st>>>(F, C, dzq, scratch, pqrf, nk, ncol, ld, sys_out);
-        }
+        double *pqrf = scratch;
+        const DivBy<true> dz{C.dzp, 1.0 / C.dzp};
+        const dim3 grid((ncol + 31) / 32, (nk + kMinorLevels - 1) / kMinorLevels), block(32, kMinorLevels + 1);
+        if (exact_reciprocal(C.dzp)) k_minor_system<true><<<grid, block, 0, st>>>(F, C, dz, pqrf, nk, ncol, ld, sys_out);
+        else k_minor_system<false><<<grid, block, 0, st>>>(F, C, dzq, pqrf, nk, ncol, ld, sys_out);
         return launch_thomas_post(pqrf, pqrf + slab, pqrf + 2 * slab, pqrf + 3 * slab, out, nk, nk, 0, ncol, ld,
                                   status, post, st);
     }
@@ -1124,7 +1128,7 @@ cudaError_t launch_minor_ng(const MinorFields &F, const MinorConsts &C, double *
         int TR = 128;
         while (TR > 32 && (size_t)TR * per_r > (size_t)optin) TR /= 2;
         if ((size_t)TR * per_r > (size_t)optin) return cudaErrorInvalidValue;
-        k_minor_levels<false><<<dim3((ncol + 127) / 128, nk), 128, 0, st>>>(F, C, dzq, scratch, nk, ncol, ld);
+        k_minor_levels<<<dim3((ncol + 127) / 128, nk), 128, 0, st>>>(F, C, dzq, scratch, nk, ncol, ld);
         k_minor_rows<<<(ncol + TR - 1) / TR, TR, (size_t)TR * per_r, st>>>(F, C, scratch, out, nk, ncol, ld, sys_out,
                                                                           status, pv, hp, walk_prefetch(ncol));
         return cudaGetLastError();
