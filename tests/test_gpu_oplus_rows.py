@@ -1,5 +1,7 @@
-"""oplus_ng's row kernel (its rows between the boundaries have a form of their
-own) against the column walk, bit for bit, from the smallest column on."""
+"""oplus_ng's row kernels (rows between the boundaries have a form of their own;
+launches of few blocks form level quantities and rows in one kernel) against
+the column walk, bit for bit, from the smallest column on and on both sides of
+the rule that chooses."""
 import numpy as np
 import pytest
 
@@ -7,7 +9,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("nk,ncol,pad,cap", [(3, 1, 0, 0.), (4, 127, 1, 1e5), (5, 128, 0, 0.), (6, 129, 0, 1e7),
-                                             (29, 257, 3, 0.), (57, 300, 0, 0.), (113, 64, 0, 1e6)])
+                                             (11, 31, 0, 0.), (12, 33, 1, 0.), (29, 257, 3, 0.), (57, 300, 0, 0.),
+                                             (113, 64, 0, 1e6), (12, 21300, 2, 0.), (12, 21400, 0, 0.),
+                                             (3, 42700, 1, 1e5), (22, 21400, 0, 0.)])
 @pytest.mark.parametrize("bz", [1., 1e-140])
 def test_rows_are_the_walks(pkg, nk, ncol, pad, cap, bz):
     import torch

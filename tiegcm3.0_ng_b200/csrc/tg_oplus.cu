@@ -46,22 +46,25 @@ __device__ __forceinline__ double up(const double *p, int j, int nk, long ld, lo
 }  // namespace
 
 // Level quantities of level j of one column (oplus_ng.F90:112-169, 285-299):
-// dj, hdz, tp1, b.u, op_loss and op_prod into the scratch planes, xiop2p,
-// xiop2d and (if requested) Fe, Fn into the outputs.
-__device__ __forceinline__ void oplus_level(const OplusFields &F, const OplusConsts &C, double *scr, double *xiop2p,
-                                            double *xiop2d, double *Fe, double *Fn, int nk, long ld, long col, int j)
+// dj, hdz, tp1 and b.u; with chem also op_loss and op_prod, and xiop2p, xiop2d
+// and (if requested) Fe, Fn into the outputs.
+struct OplusLevel {
+    double dj, hdz, tp1, bdotu, ol, prod;
+};
+__device__ __forceinline__ OplusLevel oplus_level_at(const OplusFields &F, const OplusConsts &C, double *xiop2p,
+                                                     double *xiop2d, double *Fe, double *Fn, int nk, long ld, long col,
+                                                     int j, bool chem)
 {
     auto at = [&](const double *p, int k) { return __ldg(p + k * ld + col); };
-    auto S = [&](int e, int k) -> double & { return scr[(long)e * nk * ld + (long)k * ld + col]; };
+    OplusLevel L;
     const double dz = C.dz;
     const double bx = __ldg(F.bx + col), by = __ldg(F.by + col), bz = __ldg(F.bz + col);
     const bool capped = !(fabs(xs(C.opdiffcap, 0.)) < 1e-9);
-    const double sncs = Fe ? xm(sin(__ldg(F.dipmag + col)), cos(__ldg(F.dipmag + col))) : 0.;
+    const double sncs = Fe && chem ? xm(sin(__ldg(F.dipmag + col)), cos(__ldg(F.dipmag + col))) : 0.;
     const double ogg = xd(xm(C.rmass_op, C.grav), C.gask);
 
     const double tn = at(F.tn, j), te = at(F.te, j), ti = at(F.ti, j), o2 = at(F.o2, j), o1 = at(F.o1, j),
-                 n2 = at(F.n2, j), he = at(F.he, j), xn = at(F.xnmbar, j), hj = at(F.scht, j),
-                 ne = at(F.ne, j);
+                 n2 = at(F.n2, j), he = at(F.he, j), xn = at(F.xnmbar, j), hj = at(F.scht, j);
     const double tr = xm(0.5, xa(tn, ti));
     const double lg = xs(1., xm(0.064, log10(tr)));
     double vni = xm(xm(18.1, o2), C.rmassinv_o2);
@@ -75,10 +78,12 @@ __device__ __forceinline__ void oplus_level(const OplusFields &F, const OplusCon
         dj = dj < cap ? dj : cap;
     }
     const double wni = up(F.w, j, nk, ld, col);
-    S(S_DJ, j) = dj;
-    S(S_HDZ, j) = xd(1., xm(hj, dz));
-    S(S_TP1, j) = xm(0.5, xa(ti, te));
-    S(S_BDOTU, j) = xa(xa(xm(bx, at(F.u, j)), xm(by, at(F.v, j))), xm(xm(hj, bz), wni));
+    L.dj = dj;
+    L.hdz = xd(1., xm(hj, dz));
+    L.tp1 = xm(0.5, xa(ti, te));
+    L.bdotu = xa(xa(xm(bx, at(F.u, j)), xm(by, at(F.v, j))), xm(xm(hj, bz), wni));
+    L.ol = L.prod = 0.;
+    if (!chem) return L;
     if (Fe) {
         auto tpop = [&](int i) { return xm(xa(at(F.te, i), at(F.ti, i)), at(F.op, i)); };
         double d;
@@ -92,7 +97,7 @@ __device__ __forceinline__ void oplus_level(const OplusFields &F, const OplusCon
         Fn[j * ld + col] = xm(xm(wd, sncs), __ldg(F.csdec + col));
     }
     // chemistry (oplus_ng.F90:285-299)
-    const double rk19 = at(F.rk19, j), rk20 = at(F.rk20, j), rk25 = at(F.rk25, j);
+    const double ne = at(F.ne, j), rk19 = at(F.rk19, j), rk20 = at(F.rk20, j), rk25 = at(F.rk25, j);
     const double den2p = xa(xa(xa(xm(xn, xa(xm(xm(xa(C.rk16, C.rk17), n2), C.rmassinv_n2),
                                             xm(xm(C.rk18, o1), C.rmassinv_o1))),
                                   xm(xa(rk19, rk20), ne)),
@@ -107,12 +112,27 @@ __device__ __forceinline__ void oplus_level(const OplusFields &F, const OplusCon
     const double x2d = xd(xa(up(F.qop2d, j, nk, ld, col), xm(xa(xm(rk20, ne), C.rk22), x2p)), den2d);
     xiop2p[j * ld + col] = x2p;
     xiop2d[j * ld + col] = x2d;
-    S(S_OL, j) = xm(xn, xa(xa(xm(xm(at(F.rk1, j), o2), C.rmassinv_o2), xm(xm(at(F.rk2, j), n2), C.rmassinv_n2)),
+    L.ol = xm(xn, xa(xa(xm(xm(at(F.rk1, j), o2), C.rmassinv_o2), xm(xm(at(F.rk2, j), n2), C.rmassinv_n2)),
                             xm(xm(C.rk10, at(F.n2d, j)), C.rmassinv_n2d)));
     double prod = xa(up(F.qop, j, nk, ld, col), xm(xa(xm(rk19, ne), C.rk21), x2p));
     prod = xa(prod, xm(xa(xm(rk25, ne), C.rk27), x2d));
     prod = xa(prod, xm(xm(xm(xa(xm(C.rk18, x2p), xm(C.rk24, x2d)), o1), C.rmassinv_o1), xn));
-    S(S_PROD, j) = prod;
+    L.prod = prod;
+    return L;
+}
+
+// Those of one level into the scratch planes.
+__device__ __forceinline__ void oplus_level(const OplusFields &F, const OplusConsts &C, double *scr, double *xiop2p,
+                                            double *xiop2d, double *Fe, double *Fn, int nk, long ld, long col, int j)
+{
+    const OplusLevel L = oplus_level_at(F, C, xiop2p, xiop2d, Fe, Fn, nk, ld, col, j, true);
+    auto S = [&](int e) -> double & { return scr[(long)e * nk * ld + (long)j * ld + col]; };
+    S(S_DJ) = L.dj;
+    S(S_HDZ) = L.hdz;
+    S(S_TP1) = L.tp1;
+    S(S_BDOTU) = L.bdotu;
+    S(S_OL) = L.ol;
+    S(S_PROD) = L.prod;
 }
 
 // Per-column constants of the rows: the top O+ flux (oplus_flux,
@@ -124,12 +144,14 @@ struct OplusCol {
 
 // Interface and half-level quantities of row j built from the level planes
 // (oplus_ng.F90:209-254), as the reference forms them.
+// (e, k) of the planes is at e*slab + k*sld + scol.
 struct OplusRowsAt {
     const double *scr;
-    long slab, ld, col;
+    long slab, sld, scol;
+    long ld, col;
     int nk;
-    double gmr, dvbz, bz2;
-    __device__ __forceinline__ double S(int e, int k) const { return scr[(long)e * slab + (long)k * ld + col]; }
+    double gmr;
+    __device__ __forceinline__ double S(int e, int k) const { return scr[(long)e * slab + (long)k * sld + scol]; }
     __device__ __forceinline__ double hdzi(int j) const
     {
         if (j == 0) return xs(xm(1.5, S(S_HDZ, 0)), xm(0.5, S(S_HDZ, 1)));
@@ -272,7 +294,7 @@ __device__ __forceinline__ void oplus_walk(const OplusFields &F, const OplusCons
                                            unsigned *status, const PostStep &post, int has_post, int pd)
 {
     const long slab = (long)nk * ld;
-    OplusRowsAt A{scr, slab, ld, col, nk, 0., 0., 0.};
+    OplusRowsAt A{scr, slab, ld, col, ld, col, nk, 0.};
     const OplusCol cc = oplus_col(F, C, A);
     A.gmr = cc.gmr;
     bool ok = true;
@@ -393,16 +415,17 @@ __global__ void __launch_bounds__(128) k_oplus_rows(OplusFields F, OplusConsts C
 }
 
 // oplus_row of a row that no boundary touches (0 < k < nk-2): the same
-// operations on level values read once; re by its reciprocal.
-__device__ __forceinline__ void oplus_row_mid(const OplusFields &F, const OplusConsts &C, const double *scr, long slab,
-                                              long o, long ld, const OplusCol &cc, double yre, double &p, double &q,
+// operations on each level value read once; re by its reciprocal.
+// S(e, d): quantity e of level k + d.
+template <class Level>
+__device__ __forceinline__ void oplus_row_mid(const OplusFields &F, const OplusConsts &C, Level S, long o, long ld,
+                                              const OplusCol &cc, double yre, bool rhs, double &p, double &q,
                                               double &r, double &ex)
 {
-    auto S = [&](int e, long d) { return __ldg(scr + (long)e * slab + o + d); };
-    const double djm = S(S_DJ, -ld), dj0 = S(S_DJ, 0), djp = S(S_DJ, ld);
-    const double hzm = S(S_HDZ, -ld), hz0 = S(S_HDZ, 0), hzp = S(S_HDZ, ld);
-    const double tpm = S(S_TP1, -ld), tp0 = S(S_TP1, 0), tpp = S(S_TP1, ld);
-    const double bum = S(S_BDOTU, -ld), bu0 = S(S_BDOTU, 0), bup = S(S_BDOTU, ld);
+    const double djm = S(S_DJ, -1), dj0 = S(S_DJ, 0), djp = S(S_DJ, 1);
+    const double hzm = S(S_HDZ, -1), hz0 = S(S_HDZ, 0), hzp = S(S_HDZ, 1);
+    const double tpm = S(S_TP1, -1), tp0 = S(S_TP1, 0), tpp = S(S_TP1, 1);
+    const double bum = S(S_BDOTU, -1), bu0 = S(S_BDOTU, 0), bup = S(S_BDOTU, 1);
     const double wii = xm(.5, xa(__ldg(F.wi + o), __ldg(F.wi + o + ld)));
     const double hi0 = xm(0.5, xa(hzm, hz0)), hi1 = xm(0.5, xa(hz0, hzp));
     const double dji_k = xm(0.5, xa(djm, dj0)), dji_1 = xm(0.5, xa(dj0, djp));
@@ -415,6 +438,8 @@ __device__ __forceinline__ void oplus_row_mid(const OplusFields &F, const OplusC
     q = xa(xa(q, qdiv1(xm(-wii, 6.), C.re, yre)), xm(xm(-bu0, cc.dvbz), cc.bz));
     q = xs(xs(q, cc.dtn), S(S_OL, 0));
     r = xa(xa(xm(xm(hdzp_k, dji_1), t11), xm(xm(-wii, 0.5), hz0)), xm(xm(xm(-cc.bz, bup), 0.5), hz0));
+    ex = 0.;
+    if (!rhs) return;
     ex = xs(__ldg(F.explicit_h + o), xm(xm(__ldg(F.optm1_smooth2 + o), C.dtx2inv), (double)C.nstep_sub));
     ex = xs(ex, S(S_PROD, 0));
 }
@@ -436,7 +461,7 @@ __global__ void __launch_bounds__(128, 8) k_oplus_coefs(OplusFields F, OplusCons
     if (col >= ncol) return;
     const int k = blockIdx.y;
     const long slab = (long)nk * ld, o = (long)k * ld + col;
-    OplusRowsAt A{scr, slab, ld, col, nk, 0., 0., 0.};
+    OplusRowsAt A{scr, slab, ld, col, ld, col, nk, 0.};
     // every line row k reads, requested into L1 at once: the loads below
     // sit between divisions and would otherwise wait one at a time
     {
@@ -455,7 +480,8 @@ __global__ void __launch_bounds__(128, 8) k_oplus_coefs(OplusFields F, OplusCons
     }
     double p, q, r, ex;
     if (k > 0 && k < nk - 2) {
-        oplus_row_mid(F, C, scr, slab, o, ld, oplus_col_rows(F, C, col, gmr), yre, p, q, r, ex);
+        oplus_row_mid(F, C, [&](int e, int d) { return __ldg(scr + (long)e * slab + o + d * ld); }, o, ld,
+                      oplus_col_rows(F, C, col, gmr), yre, true, p, q, r, ex);
     } else {
         const OplusCol cc = oplus_col(F, C, A);
         A.gmr = cc.gmr;
@@ -474,6 +500,96 @@ __global__ void __launch_bounds__(128, 8) k_oplus_coefs(OplusFields F, OplusCons
         sys_out[2 * slab + o] = r;
         sys_out[3 * slab + o] = ex;
     }
+}
+
+// Passes 1 and 2 in one kernel for launches of few blocks: 10 levels of 32
+// columns, one warp each, and the levels below and above them, which lend the
+// rows four of their quantities in shared memory; the level planes never leave
+// the SM.  It saves a launch and the planes' way through L2, and loses to the
+// two kernels where these stream at the memory's rate (see launch_oplus_rows).
+// 3 blocks per SM, 56 registers; other heights (4 to 14 levels) and 2 to 5
+// blocks are no faster.
+constexpr int kSysLevels = 10, kSysBlocks = 3;
+__global__ void __launch_bounds__(32 * (kSysLevels + 2), kSysBlocks)
+    k_oplus_system(OplusFields F, OplusConsts C, double gmr, double yre, double *xiop2p, double *xiop2d, double *Fe,
+                   double *Fn, double *scr, int nk, int ncol, long ld, bool rhs, double *sys_out)
+{
+    __shared__ double sh[S_P][kSysLevels + 2][32];
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const long col = (long)blockIdx.x * 32 + tx;
+    const int k = blockIdx.y * kSysLevels + ty - 1;
+    if (col >= ncol || k < 0 || k >= nk) return;   // a barrier counts the threads that are left
+    const long slab = (long)nk * ld, o = (long)k * ld + col;
+    // the levels below and above the group's lend the four quantities that its
+    // rows take from their neighbours; the top level, no row's own, is the
+    // group's below it
+    const bool own = (ty > 0 && ty <= kSysLevels) || k == nk - 1, row = ty > 0 && ty <= kSysLevels && k < nk - 1;
+    if (own) {
+        // the lines of the chemistry and the row, requested ahead
+        const double *lvl[] = {F.ne, F.rk19, F.rk20, F.rk25, F.rk1, F.rk2, F.n2d, F.qop2p, F.qop2d, F.qop, F.wi,
+                               F.bdotdh_djbz};
+#pragma unroll
+        for (int i = 0; i < 12; ++i) pf_l1(lvl[i] + o);
+        if (rhs) {
+            pf_l1(F.explicit_h + o);
+            pf_l1(F.optm1_smooth2 + o);
+        }
+    }
+    {
+        const OplusLevel L = oplus_level_at(F, C, xiop2p, xiop2d, Fe, Fn, nk, ld, col, k, own);
+        sh[S_DJ][ty][tx] = L.dj;
+        sh[S_HDZ][ty][tx] = L.hdz;
+        sh[S_TP1][ty][tx] = L.tp1;
+        sh[S_BDOTU][ty][tx] = L.bdotu;
+        sh[S_OL][ty][tx] = L.ol;
+        sh[S_PROD][ty][tx] = L.prod;
+        if (own) scr[S_PROD * slab + o] = L.prod;
+    }
+    __syncthreads();
+    if (!row) return;
+    double p, q, r, ex;
+    if (k > 0 && k < nk - 2) {
+        oplus_row_mid(F, C, [&](int e, int d) { return sh[e][ty + d][tx]; }, o, ld, oplus_col_rows(F, C, col, gmr), yre,
+                      rhs, p, q, r, ex);
+    } else {
+        // (e, j) of the block's levels, the first of which is level k - ty
+        OplusRowsAt A{&sh[0][0][0], (kSysLevels + 2) * 32, 32, tx - (long)(k - ty) * 32, ld, col, nk, gmr};
+        // the top row alone takes the upper-boundary ratios, of levels nk-3 and nk-2
+        const OplusCol cc = k == nk - 2 ? oplus_col(F, C, A) : oplus_col_rows(F, C, col, gmr);
+        double t_top = 0., t_bot = 0.;
+        oplus_row(F, C, A, cc, k, p, q, r, ex, &t_top, &t_bot);
+        if (k == nk - 2) scr[S_TB * slab + col] = t_top;
+        if (k == 0) scr[S_TB * slab + ld + col] = t_bot;
+    }
+    scr[S_P * slab + o] = p;
+    scr[S_Q * slab + o] = q;
+    scr[S_R * slab + o] = r;
+    if (rhs) scr[S_EX * slab + o] = ex;
+    if (sys_out) {
+        sys_out[o] = p;
+        sys_out[slab + o] = q;
+        sys_out[2 * slab + o] = r;
+        sys_out[3 * slab + o] = ex;
+    }
+}
+// Rows p, q, r (and with rhs the right-hand side) of every column.  One kernel
+// up to three rounds of its resident blocks: 2,072 columns x 57 levels 22.7 us
+// the routine against 28.6 with two, 2,816 x 29 18.0 and 20.7, 2,816 x 113 53.4
+// and 55.0, 6,969 x 57 49.1 and 51.4; past that two: 9,006 x 57 58.7 and 59.1,
+// 11,248 x 57 70.0 and 67.8, 43,216 x 57 237 and 202.
+static void launch_oplus_rows(const OplusFields &F, const OplusConsts &C, double *xiop2p, double *xiop2d, double *Fe,
+                              double *Fn, double *scr, int nk, int ncol, long ld, bool rhs, double *sys_out,
+                              cudaStream_t st)
+{
+    const double gmr = oplus_gmr(C), yre = 1.0 / C.re;
+    const dim3 sys((ncol + 31) / 32, (nk - 1 + kSysLevels - 1) / kSysLevels), full((ncol + 127) / 128, nk);
+    if ((long)sys.x * sys.y <= 3L * kSysBlocks * sm_count()) {
+        k_oplus_system<<<sys, dim3(32, kSysLevels + 2), 0, st>>>(F, C, gmr, yre, xiop2p, xiop2d, Fe, Fn, scr, nk, ncol,
+                                                                 ld, rhs, sys_out);
+        return;
+    }
+    k_oplus_levels<<<full, 128, 0, st>>>(F, C, xiop2p, xiop2d, Fe, Fn, scr, nk, ncol, ld);
+    k_oplus_coefs<<<dim3(full.x, nk - 1), 128, 0, st>>>(F, C, gmr, yre, scr, nk, ncol, ld, sys_out);
 }
 
 // ---- the O+ sub-cycle: factor once, solve every sub-step -------------------
@@ -993,7 +1109,7 @@ __global__ void __launch_bounds__(128) k_oplus_diag_ng(OplusFields F, OplusConst
         D(3) = D(4) = D(5) = 0.0;
         return;
     }
-    OplusRowsAt A{scr, slab, ld, col, nk, 0., 0., 0.};
+    OplusRowsAt A{scr, slab, ld, col, ld, col, nk, 0.};
     const OplusCol cc = oplus_col(F, C, A);
     A.gmr = cc.gmr;
     double pt[9];
@@ -1027,10 +1143,7 @@ cudaError_t launch_oplus_factor(const OplusFields &F, const OplusConsts &C, doub
 {
     if (ncol <= 0) return cudaSuccess;
     if (nk < 3) return cudaErrorInvalidValue;
-    k_oplus_levels<<<dim3((ncol + 127) / 128, nk), 128, 0, st>>>(F, C, xiop2p, xiop2d, nullptr, nullptr, factor, nk,
-                                                                 ncol, ld);
-    k_oplus_coefs<<<dim3((ncol + 127) / 128, nk - 1), 128, 0, st>>>(F, C, oplus_gmr(C), 1.0 / C.re, factor, nk, ncol,
-                                                                    ld, nullptr);
+    launch_oplus_rows(F, C, xiop2p, xiop2d, nullptr, nullptr, factor, nk, ncol, ld, false, nullptr, st);
     return launch_oplus_factor_pass(factor, nk, ncol, ld, status, st);
 }
 
@@ -1141,10 +1254,7 @@ cudaError_t launch_oplus_ng(const OplusFields &F, const OplusConsts &C, double *
     const int pd = walk_prefetch(ncol);
     if (assembly_mode() == 2) {
         const long slab = (long)nk * ld;
-        k_oplus_levels<<<dim3((ncol + 127) / 128, nk), 128, 0, st>>>(F, C, xiop2p, xiop2d, Fe, Fn, scratch, nk, ncol,
-                                                                     ld);
-        k_oplus_coefs<<<dim3((ncol + 127) / 128, nk - 1), 128, 0, st>>>(F, C, oplus_gmr(C), 1.0 / C.re, scratch, nk,
-                                                                        ncol, ld, sys_out);
+        launch_oplus_rows(F, C, xiop2p, xiop2d, Fe, Fn, scratch, nk, ncol, ld, true, sys_out, st);
         return launch_thomas_post(scratch + S_P * slab, scratch + S_Q * slab, scratch + S_R * slab,
                                   scratch + S_EX * slab, opout, nk, nk - 1, 1, ncol, ld, status, post, st);
     }
