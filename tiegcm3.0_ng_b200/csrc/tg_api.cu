@@ -2497,6 +2497,14 @@ __attribute__((visibility("default"))) int tg_plan_create(const tg_segment *segs
             if (g0.shape.blocks > half && half > 0) g0.shape.blocks = half;
         }
     }
+    // Scratch write-back that is too much for one kind's launch is too much for
+    // the plan: all kinds discard, or none (2.5 deg grid with 2x2 blocks 54.3 us,
+    // 56.6 with the scalar kind alone, 62.2 with the blocks alone, 64.7 with
+    // neither; with one nest 119.5, 125.4, 128.3, 134.1; with 3x3 blocks 95.9,
+    // 98.5 scalar alone, 101.4 neither).
+    int drop = 0;
+    for (const auto &g : p->groups) drop |= g.nseg > 0 && g.shape.drop;
+    for (auto &g : p->groups) g.shape.drop = drop;
     for (auto &g : p->groups) {
         if (!g.nseg) continue;
         const bool ring_refine = g.kind == TG_KIND_SCALAR && precision != TG_PREC_F64 && g.shape.stages > 0;

@@ -71,6 +71,7 @@ struct SegTable {
     int k2max;        // largest k2 of any segment (sizes per-thread scratch)
     Seg one;
     int hints;        // L2 policy hints: inputs evict-first, sweep scratch evict-last
+    int drop;         // a finished tile's scratch is discarded from L2
 };
 
 struct Refine {
@@ -93,6 +94,7 @@ struct Shape {
     int res;            // scalar FP64 chunked ring: 1 w2 in shared memory (w3 parked in x), 2 w2 and w3 in
                         // shared memory (k_scalar_f64_res); 0 L2 scratch (k_scalar_f64_chunk)
     int one_wave;       // the grid holds every tile at once (no grid-stride second pass)
+    int drop;           // warps discard a finished tile's scratch from L2
 };
 
 // Register-prefetch kernel shape of a kind/precision (tg_set_tile).

@@ -464,6 +464,16 @@ __device__ __forceinline__ void cp_async_own(void *dst, const void *src, unsigne
                  "l"(pol)
                  : "memory");
 }
+// The warp's scratch of a finished tile, bytes from p on (both multiples of 128),
+// after every lane's last read of it: dead, so its dirty lines need not be
+// written back.
+__device__ __forceinline__ void discard_slice(const void *p, long bytes, int lane)
+{
+    for (long o = (long)lane * 128; o < bytes; o += 32 * 128)
+        asm volatile("discard.global.L2 [%0], 128;" ::"l"(static_cast<const char *>(p) + o) : "memory");
+    __syncwarp();
+}
+
 // ---------------------------------------------------------------------------
 // Scalar Thomas, FP64, one warp per 32-column tile, the coefficients through a
 // shared-memory ring of C stages of L levels filled by 16-byte asynchronous
@@ -607,6 +617,7 @@ __global__ void __launch_bounds__(256) k_scalar_f64_chunk(SegTable tab, double *
         }
         cp_async_wait<0>();
         __syncwarp();
+        if (tab.drop) discard_slice(wz - lane * 2, (long)k2 * 512, lane);
         if (valid) report(status, s.status_idx, (ok ? 0u : FLAG_PIVOT) | (finite(xn) ? 0u : FLAG_NONFINITE));
     }
 }
@@ -1288,6 +1299,8 @@ __global__ void __launch_bounds__(256) k_scalar_refine_ring(SegTable tab, Refine
             }
             flags = FLAG_NOCONV | (okd ? 0u : FLAG_PIVOT) | (fin ? 0u : FLAG_NONFINITE);
         }
+        __syncwarp();
+        if (tab.drop) discard_slice(gwy - 2 * lane, (long)k2 * 384, lane);
         if (valid) report(status, s.status_idx, flags);
         const int bin = taken < kMaxSweepBins - 1 ? taken : kMaxSweepBins - 1;
 #pragma unroll
@@ -2105,6 +2118,7 @@ __global__ void __launch_bounds__(256, 1) k_block_f64_chunk(SegTable tab, double
         }
         cp_async_wait<0>();
         __syncwarp();
+        if (tab.drop) discard_slice(gz, (long)k2 * NB * 256, lane);
         if (!valid) continue;
         if (s.ubc_ratio) {
 #pragma unroll
@@ -3819,6 +3833,18 @@ cudaError_t plan_shape(int kind, int precision, int k2max, int ntiles, int cpb, 
     }
     if (blocks > units) blocks = units;
     sh->blocks = (int)(blocks > 0 ? blocks : 1);
+    // Whether the launch's warps discard the scratch of their finished tiles
+    // (discard_slice): where its write-back takes memory time that the launch
+    // lacks.  Scalar: from 8 tiles per SM (41,472 columns x 113 levels 43.5 us
+    // against 47.0, 82,944 x 57 41.4 and 43.2, 41,472 x 57 23.1 both ways;
+    // 30,000 x 113, 6.3 tiles, 34.0 and 33.4, 20,000 x 113 33.3 and 31.7).  2x2
+    // blocks: from 4 (20,000 x 57 33.8 and 36.1, 41,472 x 57 65.6 and 69.8;
+    // 15,000 x 57, 3.2 tiles, 28.1 and 27.1, 10,368 x 113 48.0 and 46.3).  3x3
+    // blocks, whose arithmetic hides more of it: from 8 and 48 levels (41,472 x
+    // 57 132 and 143, 82,944 x 57 258 and 281; 30,000 x 57 126.5 and 123.4,
+    // 82,944 x 29 142 and 140).
+    sh->drop = kind == TG_KIND_SCALAR ? ntiles >= 8 * nsm
+               : kind == 2            ? ntiles >= 4 * nsm : ntiles >= 8 * nsm && k2max >= 48;
     return cudaSuccess;
 }
 
@@ -3838,6 +3864,7 @@ cudaError_t launch_scalar(const SegTable &tab, int precision, const Shape &sh, R
     } else if (precision != TG_PREC_F64 && sh.stages > 0) {
         SegTable t = tab;
         t.hints = cache_hints();
+        t.drop = sh.drop;
         e = with_scalar_refine_ring(sh.stages, [&](auto k) {
             k<<<sh.blocks, sh.threads, sh.smem, st>>>(t, rf, reinterpret_cast<float *>(scratch), status, hist);
             return cudaSuccess;
@@ -3852,6 +3879,7 @@ cudaError_t launch_scalar(const SegTable &tab, int precision, const Shape &sh, R
     } else if (precision == TG_PREC_F64 && sh.stages > 0 && sh.lps > 1) {
         SegTable t = tab;
         t.hints = cache_hints();
+        t.drop = sh.drop;
         e = with_scalar_chunk(sh.stages, sh.lps, [&](auto k) {
             k<<<sh.blocks, sh.threads, sh.smem, st>>>(t, scratch, status);
             return cudaSuccess;
@@ -3914,6 +3942,7 @@ cudaError_t launch_block(const SegTable &tab, int B, int precision, const Shape 
     } else if (precision == TG_PREC_F64 && sh.stages > 0) {
         SegTable t = tab;
         t.hints = cache_hints();
+        t.drop = sh.drop;
         cudaError_t e = with_block_ring(B, sh.stages, sh.bw, [&](auto k) {
             k<<<sh.blocks, sh.threads, sh.smem, st>>>(t, scratch, status);
             return cudaSuccess;
