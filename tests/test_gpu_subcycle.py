@@ -47,3 +47,10 @@ def test_subcycle_is_its_parts(pkg, nk, nlon, nlat, ldpad, nsub, bnd):
     for got, ref in ((op[last], want[0]), (tm[last], want[1]), (x2p, y2p), (x2d, y2d)):
         assert torch.equal(got[:, :n].view(torch.int64), ref[:, :n].view(torch.int64))
     assert int(stat.item()) == pkg.TG_OK
+
+
+@pytest.mark.parametrize("nk,nlon,nlat", [(29, 60, 30), (30, 120, 90), (31, 40, 40), (57, 90, 60), (57, 120, 75), (57, 140, 74),
+                                          (57, 150, 84), (57, 156, 96), (61, 30, 20), (61, 60, 50)])
+def test_every_register_variant(pkg, nk, nlon, nlat):
+    """On each side of the rules that choose the sub-step's registers."""
+    test_subcycle_is_its_parts(pkg, nk, nlon, nlat, 0, 2, True)

@@ -852,7 +852,8 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_oplus_solve_tile(OplusField
 // solve as two kernels -> 107, 6,969 columns 297 -> 149, 11,248 columns 389 ->
 // 252 (there the solve's 130 KB tiles also left one block per SM; these take
 // 38 KB).
-// R: levels a thread holds (10 threads per column: nk <= 10 R).
+// R: levels a thread holds (10 threads per column: nk <= 10 R).  MB: blocks per
+// SM that its registers allow (0: the compiler's choice).
 // shapiro_at at a fixed index t of n points (stride s) over many levels: the
 // neighbours it does not use are read at the point itself, so that every read
 // can be in flight at once, and the edge forms are selected.
@@ -879,8 +880,8 @@ struct Shapiro3 {
     }
 };
 constexpr int kSubCols = 16, kSubThreads = 160;
-template <int R>
-__global__ void __launch_bounds__(kSubThreads) k_oplus_substep(OplusFields F, OplusConsts C, const double *scr,
+template <int R, int MB>
+__global__ void __launch_bounds__(kSubThreads, MB) k_oplus_substep(OplusFields F, OplusConsts C, const double *scr,
                                                                const double *op, const double *optm1, double *op_out,
                                                                double *optm1_out, double sh, int nlond, int nlatd,
                                                                int nk, int ncol, long ld, unsigned *status,
@@ -1197,9 +1198,26 @@ cudaError_t launch_oplus_subcycle(const OplusFields &F, const OplusConsts &C, do
     const bool wide = ld % 2 == 0 && ld >= (ncol + kSubCols - 1) / kSubCols * kSubCols && ((uintptr_t)factor & 15) == 0;
     if (fused)
         once_per_device([] {
-            cudaFuncSetAttribute(k_oplus_substep<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin());
-            cudaFuncSetAttribute(k_oplus_substep<13>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin());
+            for (auto k : {k_oplus_substep<3, 0>, k_oplus_substep<3, 4>, k_oplus_substep<6, 0>, k_oplus_substep<6, 4>,
+                           k_oplus_substep<6, 5>, k_oplus_substep<13, 0>, k_oplus_substep<13, 3>})
+                cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin());
         });
+    const int sms = sm_count(), per = ((ncol + kSubCols - 1) / kSubCols + sms - 1) / sms;   // blocks per SM, rounded up
+    // Registers against blocks per SM, chosen for a sub-cycle beside the step's
+    // other chains: up to 4 blocks per SM the variant whose registers allow 4,
+    // also where fewer are needed, since the SM is shared (57 levels, whole step:
+    // 130 blocks 158 us, 162 with 128 registers, 195 with 186, although alone the
+    // sub-cycle takes 105, 102 and 88; 229 blocks 259 and 271; 436 435 and 438;
+    // 563, two waves of 128 registers, 531 and 575), then 5 (703 blocks, step 673
+    // us and 695 with 128 registers, sub-cycle 200 and 239), then two waves of 3
+    // (888 blocks, sub-cycle 254, 264 at 4), then 4 again (1,018 blocks 278 and
+    // 344).  Up to 30 levels a thread holds 3 and needs 72 registers (703 blocks:
+    // step 360 us, 378 with room for 6 levels; 190 blocks 122 and 136).  Past 60
+    // levels 1 block per SM, else 3: 436 blocks of 113 levels 317 and 442.
+    auto k = nk <= 30   ? per <= 4 ? k_oplus_substep<3, 4> : k_oplus_substep<3, 0>
+             : nk > 60  ? per == 1 ? k_oplus_substep<13, 0> : k_oplus_substep<13, 3>
+             : per == 5 ? k_oplus_substep<6, 5>
+             : per == 6 ? k_oplus_substep<6, 0> : k_oplus_substep<6, 4>;
     const double *op = sc.op0, *optm1 = sc.optm10;
     for (int s = 0; s < C.nstep_sub && e == cudaSuccess; ++s) {
         double *op_out = sc.op[s % 2], *optm1_out = sc.optm1[s % 2];
@@ -1215,7 +1233,6 @@ cudaError_t launch_oplus_subcycle(const OplusFields &F, const OplusConsts &C, do
             attr[0].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = attr;
             cfg.numAttrs = s > 0 ? 1 : 0;
-            auto k = nk <= 60 ? k_oplus_substep<6> : k_oplus_substep<13>;
             e = cudaLaunchKernelEx(&cfg, k, F, C, (const double *)factor, op, optm1, op_out, optm1_out, sc.shapiro,
                                    nlond, nlatd, nk, ncol, ld, status, post, (int)wide);
         } else {
