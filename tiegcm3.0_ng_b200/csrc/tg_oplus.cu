@@ -255,10 +255,11 @@ __device__ __forceinline__ void oplus_parts(const OplusFields &F, const OplusCon
 // Row k (0..nk-2) of the O+ system: p, q, r and the right-hand side, with
 // both boundary folds (oplus_ng.F90:255-303).
 // t_top and t_bot receive the boundary terms the right-hand side takes at
-// k = nk-2 and k = 0 (when given).
+// k = nk-2 and k = 0 (when given).  Without rhs the right-hand side is not
+// formed, and explicit_h and optm1_smooth2 are not read.
 __device__ __forceinline__ void oplus_row(const OplusFields &F, const OplusConsts &C, const OplusRowsAt &A,
-                                          const OplusCol &cc, int k, double &p, double &q, double &r, double &ex,
-                                          double *t_top = nullptr, double *t_bot = nullptr)
+                                          const OplusCol &cc, int k, bool rhs, double &p, double &q, double &r,
+                                          double &ex, double *t_top = nullptr, double *t_bot = nullptr)
 {
     const int nk = A.nk;
     const long ld = A.ld, col = A.col;
@@ -268,7 +269,8 @@ __device__ __forceinline__ void oplus_row(const OplusFields &F, const OplusConst
     p = xa(xa(pt[0], pt[3]), pt[6]);
     q = xs(xa(xa(pt[1], pt[4]), pt[7]), cc.dtn);
     r = xa(xa(pt[2], pt[5]), pt[8]);
-    ex = xs(at(F.explicit_h, k), xm(xm(at(F.optm1_smooth2, k), C.dtx2inv), (double)C.nstep_sub));
+    ex = 0.;
+    if (rhs) ex = xs(at(F.explicit_h, k), xm(xm(at(F.optm1_smooth2, k), C.dtx2inv), (double)C.nstep_sub));
     if (k == nk - 2) {
         q = xa(q, xm(xd(cc.ubcb, cc.ubca), r));
         const double tt = xd(xm(cc.opflux, r), cc.ubca);
@@ -318,7 +320,7 @@ __device__ __forceinline__ void oplus_walk(const OplusFields &F, const OplusCons
     for (int k = 0; k < nk - 1; ++k) {
         if (k + pd < nk - 1) pf_row(k + pd);
         double p, q, r, ex;
-        oplus_row(F, C, A, cc, k, p, q, r, ex);
+        oplus_row(F, C, A, cc, k, true, p, q, r, ex);
         if (sys_out) {
             const long o = (long)k * ld + col;
             sys_out[o] = p;
@@ -455,7 +457,8 @@ __device__ __forceinline__ void oplus_row_mid(const OplusFields &F, const OplusC
 // lines are requested into L1 first (208 without); 8 blocks per SM, 64
 // registers without spills (10 blocks 208, 12 blocks 212).
 __global__ void __launch_bounds__(128, 8) k_oplus_coefs(OplusFields F, OplusConsts C, double gmr, double yre,
-                                                        double *scr, int nk, int ncol, long ld, double *sys_out)
+                                                        double *scr, int nk, int ncol, long ld, bool rhs,
+                                                        double *sys_out)
 {
     const long col = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= ncol) return;
@@ -471,29 +474,31 @@ __global__ void __launch_bounds__(128, 8) k_oplus_coefs(OplusFields F, OplusCons
 #pragma unroll
             for (int j = 0; j < 3; ++j) pf_l1(scr + (long)e * slab + (long)(km + j) * ld + col);
         pf_l1(scr + (long)S_OL * slab + o);
-        pf_l1(scr + (long)S_PROD * slab + o);
         pf_l1(F.bdotdh_djbz + o);
         pf_l1(F.wi + o);
         pf_l1(F.wi + o + ld);
-        pf_l1(F.explicit_h + o);
-        pf_l1(F.optm1_smooth2 + o);
+        if (rhs) {
+            pf_l1(scr + (long)S_PROD * slab + o);
+            pf_l1(F.explicit_h + o);
+            pf_l1(F.optm1_smooth2 + o);
+        }
     }
     double p, q, r, ex;
     if (k > 0 && k < nk - 2) {
         oplus_row_mid(F, C, [&](int e, int d) { return __ldg(scr + (long)e * slab + o + d * ld); }, o, ld,
-                      oplus_col_rows(F, C, col, gmr), yre, true, p, q, r, ex);
+                      oplus_col_rows(F, C, col, gmr), yre, rhs, p, q, r, ex);
     } else {
         const OplusCol cc = oplus_col(F, C, A);
         A.gmr = cc.gmr;
         double t_top = 0., t_bot = 0.;
-        oplus_row(F, C, A, cc, k, p, q, r, ex, &t_top, &t_bot);
+        oplus_row(F, C, A, cc, k, rhs, p, q, r, ex, &t_top, &t_bot);
         if (k == nk - 2) scr[S_TB * slab + col] = t_top;
         if (k == 0) scr[S_TB * slab + ld + col] = t_bot;
     }
     scr[S_P * slab + o] = p;
     scr[S_Q * slab + o] = q;
     scr[S_R * slab + o] = r;
-    scr[S_EX * slab + o] = ex;
+    if (rhs) scr[S_EX * slab + o] = ex;
     if (sys_out) {
         sys_out[o] = p;
         sys_out[slab + o] = q;
@@ -557,7 +562,7 @@ __global__ void __launch_bounds__(32 * (kSysLevels + 2), kSysBlocks)
         // the top row alone takes the upper-boundary ratios, of levels nk-3 and nk-2
         const OplusCol cc = k == nk - 2 ? oplus_col(F, C, A) : oplus_col_rows(F, C, col, gmr);
         double t_top = 0., t_bot = 0.;
-        oplus_row(F, C, A, cc, k, p, q, r, ex, &t_top, &t_bot);
+        oplus_row(F, C, A, cc, k, rhs, p, q, r, ex, &t_top, &t_bot);
         if (k == nk - 2) scr[S_TB * slab + col] = t_top;
         if (k == 0) scr[S_TB * slab + ld + col] = t_bot;
     }
@@ -589,7 +594,7 @@ static void launch_oplus_rows(const OplusFields &F, const OplusConsts &C, double
         return;
     }
     k_oplus_levels<<<full, 128, 0, st>>>(F, C, xiop2p, xiop2d, Fe, Fn, scr, nk, ncol, ld);
-    k_oplus_coefs<<<dim3(full.x, nk - 1), 128, 0, st>>>(F, C, gmr, yre, scr, nk, ncol, ld, sys_out);
+    k_oplus_coefs<<<dim3(full.x, nk - 1), 128, 0, st>>>(F, C, gmr, yre, scr, nk, ncol, ld, rhs, sys_out);
 }
 
 // ---- the O+ sub-cycle: factor once, solve every sub-step -------------------
