@@ -583,7 +583,13 @@ int tg_oplus_ng_solve_dev(const tg_oplus_fields *F, const tg_oplus_consts *C, co
  * when s is even and op_b, optm1_b when it is odd, and reads what s-1 wrote
  * (F->op and optm1 at s = 0).  explicit_h is the same in every sub-step;
  * F->optm1_smooth2 is not read.  optm1_smooth (nk planes) is work space;
- * bnd_mask and bnd as in tg_post_step (both or neither). */
+ * bnd_mask and bnd as in tg_post_step (both or neither).  As nm_upd may alias
+ * prev or cur there, optm1_a may be optm1 or F->op and optm1_b may be optm1_a:
+ * such calls smooth and solve in two kernels a sub-step, as do all whose
+ * buffers overlap.  op_a and op_b must differ from F->op, optm1, bnd, each
+ * other, optm1_a and optm1_b, and optm1_smooth from every field that a
+ * sub-step still reads; TG_EINVAL where a buffer that is written is one that
+ * is still read. */
 int tg_oplus_ng_subcycle_dev(const tg_oplus_fields *F, const tg_oplus_consts *C, double *xiop2p, double *xiop2d,
                              double *factor, const double *optm1, double *optm1_smooth, double shapiro, double *op_a,
                              double *optm1_a, double *op_b, double *optm1_b, int nk, int nlon, int nlat, long ld,

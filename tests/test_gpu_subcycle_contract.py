@@ -67,3 +67,31 @@ def test_subcycle_does_not_read_optm1_smooth2(pkg, nk, nlon, nlat):
         res.append((*op, *tm))
     for a, b in zip(*res):
         assert same(a, b, ncol) and bool(torch.isfinite(b[:, :ncol]).all())
+
+
+# (optm1_a, optm1_b) in place of a buffer that the sub-step filters
+@pytest.mark.parametrize("where", [("optm1", None), (None, "optm1_a"), ("optm1", "optm1_a"), ("op", None), ("op", "optm1_a"),
+                                   (None, "optm1")])
+@pytest.mark.parametrize("nk,nlon,nlat", [(29, 11, 9), (57, 52, 33), (57, 160, 100), (131, 12, 4)])
+def test_subcycle_filters_in_place(pkg, nk, nlon, nlat, where):
+    """optm1_a and optm1_b where the filter's nm_upd may lie: the bits of
+    separate buffers, on both sides of the fused sub-step's range."""
+    import torch
+    cs = pkg.colsolve
+    grid, F, C, optm1, bnd, mask = setup(pkg, nk, nlon, nlat, 3)
+    ld, ncol, st = grid.ld, grid.ncol, torch.cuda.current_stream()
+    z = lambda: torch.zeros((nk, ld), dtype=torch.float64, device="cuda")  # noqa: E731
+
+    def call(a, b):
+        G, prev = dict(F, op=F["op"].clone()), optm1.clone()
+        place = {"optm1": prev, "op": G["op"]}
+        tm_a = place[a] if a else z()
+        tm_b = tm_a if b == "optm1_a" else place[b] if b else z()
+        fac, op = torch.zeros(cs.oplus_ng_factor_doubles(nk, ld), dtype=torch.float64, device="cuda"), [z(), z()]
+        cs.oplus_ng_subcycle_dev(G, C, z(), z(), fac, prev, z(), 0.003, op, [tm_a, tm_b], nk, nlon, nlat, ld, 0.95, 0.025,
+                                 bnd_mask=mask, bnd=bnd, stream=st)
+        torch.cuda.synchronize()
+        return op[0], tm_a     # sub-step 2's, the last
+
+    for got, want in zip(call(*where), call(None, None)):
+        assert same(got, want, ncol)

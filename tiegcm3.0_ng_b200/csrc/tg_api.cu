@@ -2130,6 +2130,27 @@ __attribute__((visibility("default"))) int tg_oplus_ng_solve_dev(const tg_oplus_
     return TG_OK;
 }
 
+// Each sub-step keeps tg_post_step's rule (opout in no place that the sub-step
+// reads or filters into; nm_upd may alias prev or cur), and nothing that a
+// later sub-step reads is overwritten before it does.
+static bool subcycle_buffers_ok(const tg_oplus_fields *F, int nstep_sub, const double *xiop2p, const double *xiop2d,
+                                const double *factor, const double *optm1, const double *smooth,
+                                const double *const (&op)[2], const double *const (&nm)[2], const double *bnd)
+{
+    const double *cur = F->op, *prev = optm1;
+    for (int s = 0; s < nstep_sub && s < 3; ++s) {
+        const double *x = op[s % 2], *n = nm[s % 2];
+        if (x == cur || x == prev || x == n || x == bnd || smooth == cur || smooth == prev) return false;
+        if (s + 1 < nstep_sub && (x == F->explicit_h || n == F->explicit_h || n == bnd)) return false;
+        cur = x;
+        prev = n;
+    }
+    if (smooth == F->explicit_h || smooth == bnd) return false;
+    for (const double *p : {F->op, F->explicit_h, optm1, smooth, op[0], op[1], nm[0], nm[1], bnd, xiop2p, xiop2d})
+        if (p == factor) return false;
+    return true;
+}
+
 __attribute__((visibility("default"))) int tg_oplus_ng_subcycle_dev(
     const tg_oplus_fields *F, const tg_oplus_consts *C, double *xiop2p, double *xiop2d, double *factor,
     const double *optm1, double *optm1_smooth, double shapiro, double *op_a, double *optm1_a, double *op_b,
@@ -2141,6 +2162,11 @@ __attribute__((visibility("default"))) int tg_oplus_ng_subcycle_dev(
         !optm1_b || nk < 3 || ncol < 0 || ncol > 0x7fffffffL || ld < ncol || C->nstep_sub < 1 ||
         (!bnd_mask) != (!bnd) || !oplus_fields_ok(F)) {
         set_err("tg_oplus_ng_subcycle_dev: bad arguments (nk=%d nlon=%d nlat=%d ld=%ld)", nk, nlon, nlat, ld);
+        return TG_EINVAL;
+    }
+    if (!subcycle_buffers_ok(F, C->nstep_sub, xiop2p, xiop2d, factor, optm1, optm1_smooth, {op_a, op_b},
+                             {optm1_a, optm1_b}, bnd)) {
+        set_err("tg_oplus_ng_subcycle_dev: a buffer that is written is one that is still read");
         return TG_EINVAL;
     }
     DevCtx *cx = nullptr;

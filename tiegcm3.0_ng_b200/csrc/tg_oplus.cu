@@ -1199,7 +1199,24 @@ cudaError_t launch_oplus_subcycle(const OplusFields &F, const OplusConsts &C, do
     cudaError_t e = launch_oplus_factor(F, C, xiop2p, xiop2d, factor, nk, ncol, ld, status, st);
     const size_t smem = substep_smem(nk);
     const int nlond = sc.nlon + 4, nlatd = sc.nlat + 4;
-    const bool fused = ncol <= kSmallWalkColumns && nk <= 130 && smem <= (size_t)smem_optin();
+    // The fused sub-step reads optm1 beside its block's own columns while other
+    // blocks store, and explicit_h, bnd and the factor while the sub-step before
+    // still runs: where a buffer that a sub-step writes overlaps one that it
+    // reads (the filter in place, say), smoothing and solve run apart.
+    const uintptr_t field = sizeof(double) * ((uintptr_t)(nk - 1) * ld + ncol), all = sizeof(double) * S_N * (uintptr_t)nk * ld;
+    auto meet = [](const double *a, uintptr_t na, const double *b, uintptr_t nb) {
+        return b && (uintptr_t)a < (uintptr_t)b + nb && (uintptr_t)b < (uintptr_t)a + na;
+    };
+    bool apart = true;
+    for (int s = 0; s < C.nstep_sub && s < 2; ++s) {
+        for (const double *w : {sc.op[s], sc.optm1[s]}) {
+            for (const double *r : {s ? sc.op[0] : sc.op0, s ? sc.optm1[0] : sc.optm10, F.explicit_h, post.bnd})
+                apart = apart && !meet(w, field, r, field);
+            apart = apart && !meet(w, field, factor, all);
+        }
+        apart = apart && !meet(sc.op[s], field, sc.optm1[s], field);
+    }
+    const bool fused = apart && ncol <= kSmallWalkColumns && nk <= 130 && smem <= (size_t)smem_optin();
     const bool wide = ld % 2 == 0 && ld >= (ncol + kSubCols - 1) / kSubCols * kSubCols && ((uintptr_t)factor & 15) == 0;
     if (fused)
         once_per_device([] {
