@@ -2076,20 +2076,16 @@ size_t comp_scratch_doubles(int nk, long ld)
 
 // comp_ng post-solve steps (src/comp_ng.F90:394-457): the lateral-boundary
 // values of the columns flagged in bmask (when given), the time filter, the N2
-// extrapolation, floors and normalisation.  A block takes 16 columns with 32
-// threads each, so that two levels per thread cover a 57-level column and few
-// columns still spread over the chip; every phase runs over all levels at
-// once: the search for the first level with N2 < 0.01 (the least level any
-// thread finds), the extrapolation constants (one thread per column), then the
-// per-level steps.  Bound by the reads' latency: the search reads its levels
-// without leaving off at the first and requests the last phase's lines.
-// 2,072 columns x 57 levels 10.4 us with 32-column blocks that stopped at the
-// first such level, 6.3 now; 6,969 12.4 and 10.7; 11,248 17.7 and 16.5.
-// The N2 extrapolation uses the device log/exp, so it agrees with the CPU
+// extrapolation, floors and normalisation.  A block takes T columns with G
+// threads each; every phase runs over all levels at once: the search for the
+// first level with N2 < 0.01 (the least level any thread finds; it reads its
+// levels without leaving off at the first, so that all are in flight), the
+// extrapolation constants (one thread per column), then the per-level steps.
+// Bound by the reads' latency, past one round of blocks by the memory.  The
+// N2 extrapolation uses the device log/exp, so it agrees with the CPU
 // restatement to a tolerance in the extrapolated levels.
 namespace tg {
-constexpr int kPostCols = 16, kPostGroups = 32;
-
+template <int kPostCols, int kPostGroups>
 __global__ void __launch_bounds__(kPostCols * kPostGroups) k_comp_post_ng(
     const double *o2, const double *o1, const double *he, const double *o2_nm, const double *o1_nm,
     const double *he_nm, const double *xnmbar, const double *zpmid, double dz, double ds, double ds2, int nk, int ncol,
@@ -2114,15 +2110,7 @@ __global__ void __launch_bounds__(kPostCols * kPostGroups) k_comp_post_ng(
         int kt = nk;
 #pragma unroll 4
         for (int k = w; k < nk; k += kPostGroups) {
-            const long o = (long)k * ld + col;
-            pf_l1(o2_nm + o);
-            pf_l1(o1_nm + o);
-            pf_l1(he_nm + o);
-            pf_l1(o2 + o);
-            pf_l1(o1 + o);
-            pf_l1(he + o);
-            pf_l1(xnmbar + o);
-            if (n2_at(o) < 0.01) kt = min(kt, k);
+            if (n2_at((long)k * ld + col) < 0.01) kt = min(kt, k);
         }
         if (kt < nk) atomicMin(&ktop_s[c], kt);
     }
@@ -2178,10 +2166,29 @@ cudaError_t launch_comp_post_ng(const double *const *in7, const double *zpmid, d
                                 const unsigned char *bnd_mask, const double *const *bnd3)
 {
     if (ncol <= 0) return cudaSuccess;
-    k_comp_post_ng<<<(ncol + kPostCols - 1) / kPostCols, kPostCols * kPostGroups, 0, st>>>(
-        in7[0], in7[1], in7[2], in7[3], in7[4], in7[5], in7[6], zpmid, dz, dtsmooth, dtsmooth_div2, nk, ncol, ld,
-        upd6[0], upd6[1], upd6[2], upd6[3], upd6[4], upd6[5], bnd_mask, bnd_mask ? bnd3[0] : nullptr,
-        bnd_mask ? bnd3[1] : nullptr, bnd_mask ? bnd3[2] : nullptr);
+    auto go = [&](auto k, int T, int G) {
+        k<<<(ncol + T - 1) / T, T * G, 0, st>>>(
+            in7[0], in7[1], in7[2], in7[3], in7[4], in7[5], in7[6], zpmid, dz, dtsmooth, dtsmooth_div2, nk, ncol, ld,
+            upd6[0], upd6[1], upd6[2], upd6[3], upd6[4], upd6[5], bnd_mask, bnd_mask ? bnd3[0] : nullptr,
+            bnd_mask ? bnd3[1] : nullptr, bnd_mask ? bnd3[2] : nullptr);
+    };
+    // The most threads per column with which every column is resident at once
+    // (1,024 threads per SM at 56 registers); past that 8, or 16 for columns too
+    // tall for 8.  us without a lateral boundary, x 29 / 57 / 113 levels, the
+    // chosen shape against 32 columns with 16 threads each whose search stopped
+    // at the first level:
+    //   2,072 columns (16 x 32)  4.5 / 5.8 / 8.4 and 5.5 / 8.0 / 13.1
+    //   6,969 (16 x 16)          6.0 / 9.2 / 19.6 and 6.5 / 9.9 / 20.9
+    //   11,248 (32 x 8)          8.5 / 14.7 / 34.3 and 11.2 / 18.6 / 43.7
+    //   43,216 (32 x 8, 32 x 16) 37.8 / 61.5 / 115.4 and 42.4 / 67.2 / 120.7
+    // One shape of 16 x 32 for all, with the last phase's lines requested by
+    // the search, took 4.7 / 6.0 / 8.7, 8.8 / 11.7 / 25.6, 12.6 / 19.5 / 42.0 and
+    // 52.2 / 77.5 / 137.0.
+    const long wave = 1024L * sm_count();   // threads
+    if (ncol * 32L <= wave) go(k_comp_post_ng<16, 32>, 16, 32);
+    else if (ncol * 16L <= wave) go(k_comp_post_ng<16, 16>, 16, 16);
+    else if (ncol * 8L <= wave || nk <= 85) go(k_comp_post_ng<32, 8>, 32, 8);
+    else go(k_comp_post_ng<32, 16>, 32, 16);
     return cudaGetLastError();
 }
 
