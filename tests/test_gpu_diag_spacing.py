@@ -21,3 +21,15 @@ def test_minor_diag(pkg, orc, nk, dz, ncol):
             assert rel(got[name], want[name]) <= 1e-12, name
         else:
             assert np.array_equal(got[name], want[name]), name
+
+
+@pytest.mark.parametrize("nk,dz,ncol", [(57, 0.25, 200), (47, 0.3, 200), (15, 1.0 / 3.0, 33), (4, 0.7, 5)])
+def test_comp_diag(pkg, orc, nk, dz, ncol):
+    F, C = pkg.synth.comp_inputs(nk, ncol, dz, 22)
+    upd = orc.comp_ng(F, C)
+    got, want = pkg.comp_diag_ng(F, C, *[np.asfortranarray(u) for u in upd]), orc.comp_diag_ng(F, C, upd)
+    for name in pkg.colsolve.COMP_DIAG_NAMES:
+        if name.endswith("_MOLDIF") or name.endswith("_EDDYDIF"):
+            assert rel(got[name], want[name]) <= 1e-11, name
+        else:
+            assert np.array_equal(got[name], want[name]), name

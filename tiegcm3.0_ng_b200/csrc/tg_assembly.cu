@@ -2019,8 +2019,11 @@ cudaError_t launch_comp_diag_ng(const CompFields &F, const CompConsts &C, const 
     if (nk < 3) return cudaErrorInvalidValue;
     const int T = 128;
     double *lv = scratch + comp_gz_doubles(nk, ld);
-    k_comp_levels<false><<<dim3((ncol + T - 1) / T, nk), T, 0, st>>>(F, C, DivBy<false>{C.dz, 1.0 / C.dz}, lv, nk, ncol,
-                                                                     ld);
+    const dim3 grid((ncol + T - 1) / T, nk);
+    if (exact_reciprocal(C.dz))
+        k_comp_levels<true><<<grid, T, 0, st>>>(F, C, DivBy<true>{C.dz, 1.0 / C.dz}, lv, nk, ncol, ld);
+    else
+        k_comp_levels<false><<<grid, T, 0, st>>>(F, C, DivBy<false>{C.dz, 1.0 / C.dz}, lv, nk, ncol, ld);
     k_comp_diag_ng<<<dim3((ncol + T - 1) / T, nk), T, 0, st>>>(F, C, lv, x, nk, ncol, ld, diag);
     return cudaGetLastError();
 }
