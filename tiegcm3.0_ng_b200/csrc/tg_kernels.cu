@@ -3249,9 +3249,11 @@ struct TileCfg {
 const TileCfg kDefaultTile[3][2] = {{{256, 1, 3, 1, 4, 1, 0, 32, 4, 0}, {64, 1, 2, 0, 8, 1, 0, 32, 1, 0}},
                                      {{64, 1, 8, 0, 4, 1, 0, 32, 1, 0}, {64, 1, 4, 0, 4, 1, 0, 32, 1, 0}},
                                      {{128, 1, 8, 0, 4, 1, 0, 32, 1, 0}, {128, 1, 0, 0, 4, 4, 0, 32, 1, 0}}};
-TileCfg g_tile[3][2] = {{{256, 1, 3, 1, 4, 1, 0, 32, 4, 0}, {64, 1, 2, 0, 8, 1, 0, 32, 1, 0}},
-                        {{64, 1, 8, 0, 4, 1, 0, 32, 1, 0}, {64, 1, 4, 0, 4, 1, 0, 32, 1, 0}},
-                        {{128, 1, 8, 0, 4, 1, 0, 32, 1, 0}, {128, 1, 0, 0, 4, 4, 0, 32, 1, 0}}};
+// As set by the caller; a negative ring depth is the default of the kernel that
+// the other settings choose (ring_depth).
+TileCfg g_tile[3][2] = {{{256, 1, -1, 1, 4, 1, 0, 32, 4, 0}, {64, 1, -1, 0, 8, 1, 0, 32, 1, 0}},
+                        {{64, 1, -1, 0, 4, 1, 0, 32, 1, 0}, {64, 1, -1, 0, 4, 1, 0, 32, 1, 0}},
+                        {{128, 1, -1, 0, 4, 1, 0, 32, 1, 0}, {128, 1, -1, 0, 4, 4, 0, 32, 1, 0}}};
 int kind_index(int kind) { return kind == TG_KIND_SCALAR ? 0 : (kind == TG_KIND_BLOCK2 ? 1 : 2); }
 constexpr int kMaxDevIdx = 64;
 int g_num_sms[kMaxDevIdx] = {};
@@ -3551,14 +3553,30 @@ void set_prefetch(int kind, int precision, int pf)
     t.pf = pf > 0 ? pf : kDefaultTile[kind_index(kind)][precision ? 1 : 0].pf;
 }
 
+// The ring depth of a kind.  kDefaultTile's depths are the chunk kernels'.  The
+// scalar kernel with its scratch on chip keeps 2 stages: 41,472 columns x 57
+// levels 28.7 us, 46.7 with 3, which leave 8 warps per SM instead of 10.  The
+// block rings of 16 and 8 columns keep 4 levels, whose smaller rings leave more
+// warps resident: Gamma on chip, 2x2, 41,472 x 57 in 16 columns 171 us and 220
+// with 8 levels, 3x3 in 8 columns 803 and 862; Gamma in L2, 3x3, 87,000 x 57 in
+// 16 columns 576 and 649.
+static int ring_depth(int kind, int precision, const TileCfg &t)
+{
+    if (t.stages >= 0) return t.stages;
+    if (precision == TG_PREC_F64 && kind == TG_KIND_SCALAR && t.res > 0) return 2;
+    if (precision == TG_PREC_F64 && kind != TG_KIND_SCALAR && !t.rows && t.bw < 32) return 4;
+    return kDefaultTile[kind_index(kind)][precision ? 1 : 0].stages;
+}
+
 void tile_for(int kind, int precision, bool ring_ok, int *cpb, int *cpt, int *stages, int *w2g)
 {
     const TileCfg &t = g_tile[kind_index(kind)][precision ? 1 : 0];
+    const int depth = ring_depth(kind, precision, t);
     *w2g = 0;
-    if ((precision == TG_PREC_F64 || kind != TG_KIND_BLOCK3) && t.stages > 0 && ring_ok) {
+    if ((precision == TG_PREC_F64 || kind != TG_KIND_BLOCK3) && depth > 0 && ring_ok) {
         *cpb = 32;
         *cpt = 1;
-        *stages = t.stages;
+        *stages = depth;
         *w2g = kind == TG_KIND_SCALAR ? t.w2g : 0;
     } else {
         *cpb = t.cpb;
@@ -3596,7 +3614,7 @@ void set_stages(int kind, int precision, int stages, int wpb)
 {
     TileCfg &t = g_tile[kind_index(kind)][precision ? 1 : 0];
     const TileCfg &d = kDefaultTile[kind_index(kind)][precision ? 1 : 0];
-    t.stages = stages >= 0 ? stages : d.stages;
+    t.stages = stages >= 0 ? stages : -1;
     t.wpb = wpb > 0 ? wpb : d.wpb;
 }
 int ring_warps(int kind, int precision) { return g_tile[kind_index(kind)][precision ? 1 : 0].wpb; }
