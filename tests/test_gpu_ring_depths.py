@@ -54,3 +54,15 @@ def test_defaults(settings):
     pkg = settings
     assert kernel(pkg, 0) == "k_scalar_f64_chunk<3,4>"
     assert [kernel(pkg, k).startswith(f"k_block_f64_chunk<{k},") for k in (2, 3)] == [True, True]
+
+
+@pytest.mark.parametrize("kind", [2, 3])
+def test_columns_of_few_levels(settings, kind):
+    pkg = settings
+    depth = lambda nk: kernel(pkg, kind, nk, 4096)  # noqa: E731
+    four, eight = depth(10), depth(11)
+    assert four != eight and depth(1) == four and depth(57) == eight
+    pkg.set_pipeline(kind, pkg.TG_PREC_F64, 4, 0)
+    assert depth(57) == four
+    pkg.set_pipeline(kind, pkg.TG_PREC_F64, 8, 0)
+    assert depth(10) == eight

@@ -3737,6 +3737,14 @@ cudaError_t plan_shape(int kind, int precision, int k2max, int ntiles, int cpb, 
         if (!built(stages)) sh->res = 0;
     }
     if (sh->rows && stages > 8) stages = sh->stages = 8;
+    // Block columns of few levels: a ring of 4 levels, half the shared memory of
+    // one of 8, so that twice the warps are resident.  3x3, 169,360 columns x 4
+    // levels 38.5 us and 70.7 with 8, x 10 80.6 and 117; 2x2, x 3 12.7 and 20.5, x
+    // 10 42.4 and 45.3.  Taller columns have the deeper ring's latency to hide:
+    // 3x3, 10,368 x 12 11.8 and 11.4, x 57 44.8 and 41.9.
+    if (kind != TG_KIND_SCALAR && precision == TG_PREC_F64 && stages > 4 && k2max <= 10 && !sh->rows && !sh->res &&
+        sh->bw == 32 && g_tile[kind_index(kind)][0].stages < 0)
+        stages = sh->stages = 4;
     if (kind == TG_KIND_SCALAR && sh->cpt == 2 && sh->pf > 8) sh->pf = 8;
     if (stages > 0) {
         // a ring that does not fit in shared memory falls back to the
