@@ -735,16 +735,17 @@ int tg_set_assembly_mode(int mode);
  * waiting on memory otherwise, 1 above.  Same results. */
 int tg_set_walk_prefetch(int levels);
 
-/* Block kinds: the budget for the sweep scratch (FP64: Gamma and z;
- * refinement: the FP32 planes) of all resident warps, in MB (<= 0 restores
- * the kernels' own limits).  It caps how many columns are in flight at once
- * on large batches. */
+/* FP64 block kinds: the budget for the sweep scratch (Gamma and, in the
+ * default kernels, z) of all resident columns, in MB (<= 0 restores the
+ * kernels' own limits).  It caps how many columns are in flight at once on
+ * large batches; one thread block always is.  The refinement kernels take no
+ * budget. */
 int tg_set_block_scratch_budget(double megabytes);
 
-/* Scalar kind, ring kernels: the L2 budget for the sweep scratch of all
- * resident columns and what they stream, in MB (<= 0 restores the kernels'
- * own limits).  It caps how many columns are in flight at once on large
- * batches. */
+/* Scalar kind, ring kernels: the budget for the sweep scratch (w2 and w3;
+ * refinement: the FP32 planes and the iterate) of all resident columns, in MB
+ * (<= 0 restores the kernels' own limits).  It caps how many columns are in
+ * flight at once on large batches; one thread block always is. */
 int tg_set_scalar_scratch_budget(double megabytes);
 
 /* How the kinds of one plan share the GPU, read when a plan is created: 1 the

@@ -1090,7 +1090,7 @@ def set_walk_prefetch(levels):
 
 
 def set_scalar_scratch_budget(megabytes):
-    """L2 budget (MB) of the scalar ring kernels' w2 scratch and parked results (<= 0: default)."""
+    """Budget (MB) of the scalar ring kernels' sweep scratch in flight (<= 0: the kernels' own limits)."""
     return _check(lib().tg_set_scalar_scratch_budget(float(megabytes)), "tg_set_scalar_scratch_budget")
 
 
@@ -1105,7 +1105,7 @@ def set_host_pipeline(chunk_kb=0, streams=0):
 
 
 def set_block_scratch_budget(megabytes):
-    """Budget (MB) of the block kernels' Gamma scratch (<= 0: default 160)."""
+    """Budget (MB) of the FP64 block kernels' sweep scratch in flight (<= 0: the kernels' own limits)."""
     return _check(lib().tg_set_block_scratch_budget(float(megabytes)), "tg_set_block_scratch_budget")
 
 

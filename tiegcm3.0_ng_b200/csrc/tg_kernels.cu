@@ -11,6 +11,7 @@
 // __dsub_rn intrinsics and divisions are IEEE (__ddiv_rn), in the reference's
 // operation order (src/trsolv_ng.F90:14-26, src/comp_ng.F90:281-332,
 // src/matutil.F90:25-27,63-71,116).
+#include <algorithm>
 #include <cfloat>
 #include <cstdio>
 #include <atomic>
@@ -3535,12 +3536,9 @@ constexpr int kBlockRefineWarps = 7;
 constexpr double kBlockRegBudgetMB = 160.0, kRingBudgetMB = 128.0;
 constexpr double kMB = 1024.0 * 1024.0;
 double g_scalar_scratch_budget = 0.0, g_block_scratch_budget = 0.0;   // set by the caller; 0: the defaults
-double chunk_budget(int kind, bool refine)
-{
-    const int i = kind == TG_KIND_SCALAR ? 0 : 1;
-    const double set = i ? g_block_scratch_budget : g_scalar_scratch_budget;
-    return set > 0.0 ? set : (refine ? kRefineBudgetMB[i] : kChunkBudgetMB[i]) * kMB;
-}
+// The defaults keep three warps per SM in flight past their budget, while
+// those hold no more than this (columns of some thousand levels and more).
+constexpr double kTallScratchMB = 512.0;
 double block_reg_budget() { return g_block_scratch_budget > 0.0 ? g_block_scratch_budget : kBlockRegBudgetMB * kMB; }
 double ring_budget() { return g_scalar_scratch_budget > 0.0 ? g_scalar_scratch_budget : kRingBudgetMB * kMB; }
 std::atomic<int> g_kind_overlap{-1};
@@ -3829,18 +3827,27 @@ cudaError_t plan_shape(int kind, int precision, int k2max, int ntiles, int cpb, 
     const bool chunk = stages > 0 && !sh->res &&
                        (refine || (kind == TG_KIND_SCALAR ? sh->lps > 1 : !sh->rows && sh->bw == 32));
     if (chunk) {
-        // the chunk kernels and the refinement rings: the resident warps
-        // within the budget (at least three per SM), then the tiles dealt
-        // evenly over the nearest whole number of passes, so that none is
-        // nearly empty
+        // the chunk kernels and the refinement rings.  held: what a warp keeps
+        // between its sweeps, its scratch and, refining, its iterate.  Within
+        // a caller's budget, which the held bytes of all resident warps stay
+        // below (block refinement takes none); else the resident warps within
+        // the default one (at least three per SM), then the tiles dealt evenly
+        // over the nearest whole number of passes, so that none is nearly empty
         const int wpb = sh->threads / 32;
-        const double per_warp = kind == TG_KIND_SCALAR ? (refine ? 640.0 : 512.0) * k2max + kStreamKB * 1024.0
-                                                       : (refine ? 1792.0 : 256.0 * (kind * kind + kind)) * k2max;
-        const double budget = chunk_budget(kind, refine);
-        long cap = budget > 0.0 ? (long)(budget / (per_warp * wpb)) : (long)kBlockRefineWarps * nsm / wpb;
-        if (cap < 3L * nsm / wpb) cap = 3L * nsm / wpb;
-        if (cap < 1) cap = 1;
-        long passes = (2 * units + cap) / (2 * cap);
+        const double held = (kind == TG_KIND_SCALAR ? (refine ? 640.0 : 512.0)
+                                                    : (refine ? 1792.0 : 256.0 * (kind * kind + kind))) * k2max * wpb;
+        const double set = kind == TG_KIND_SCALAR ? g_scalar_scratch_budget : refine ? 0.0 : g_block_scratch_budget;
+        long passes;
+        if (set > 0.0) {
+            const long cap = std::max(1L, (long)(set / held));
+            passes = (units + cap - 1) / cap;
+        } else {
+            const double budget = (refine ? kRefineBudgetMB : kChunkBudgetMB)[kind != TG_KIND_SCALAR] * kMB;
+            const double per_block = held + (kind == TG_KIND_SCALAR ? kStreamKB * 1024.0 * wpb : 0.0);
+            const long least = std::min(3L * nsm / wpb, (long)(kTallScratchMB * kMB / held));
+            const long cap = std::max({1L, least, budget > 0.0 ? (long)(budget / per_block) : (long)kBlockRefineWarps * nsm / wpb});
+            passes = (2 * units + cap) / (2 * cap);
+        }
         if (passes < 1) passes = 1;
         if (passes * blocks < units) passes = (units + blocks - 1) / blocks;   // what fits on the SMs at all
         blocks = (units + passes - 1) / passes;
