@@ -2667,7 +2667,14 @@ __attribute__((visibility("default"))) int tg_selftest_walk(int which, double *b
     if ((rc = stream_ws(cx, st, &ws))) return rc;
     TG_CUDA(cudaMemsetAsync(ws->flags, 0, sizeof(unsigned), st));
     const long slab = (long)nk * ld;
-    cudaError_t e = which == 0 ? launch_thomas_post(buf, buf + slab, buf + 2 * slab, buf + 3 * slab, buf + 4 * slab,
+    double *pq = buf;
+    if (which == 0 && ncol > 0) {   // the walk may overwrite its p and q planes: it gets copies
+        const size_t bytes = 2 * sizeof(double) * (size_t)slab;
+        if ((rc = grow(ws->scratch, bytes))) return rc;
+        pq = (double *)ws->scratch.p;
+        TG_CUDA(cudaMemcpyAsync(pq, buf, bytes, cudaMemcpyDeviceToDevice, st));
+    }
+    cudaError_t e = which == 0 ? launch_thomas_post(pq, pq + slab, buf + 2 * slab, buf + 3 * slab, buf + 4 * slab,
                                                     nk, K, top, ncol, ld, ws->flags, nullptr, st)
                                : launch_oplus_factor_pass(buf, nk, ncol, ld, ws->flags, st);
     if (e == cudaErrorInvalidValue) {
