@@ -66,3 +66,12 @@ def test_columns_of_few_levels(settings, kind):
     assert depth(57) == four
     pkg.set_pipeline(kind, pkg.TG_PREC_F64, 8, 0)
     assert depth(10) == eight
+
+
+@pytest.mark.parametrize("kind,depth,name", [(2, 4, "2,2,2"), (2, 8, "2,4,2"), (2, 16, "2,8,2"), (3, 4, "3,4,1"), (3, 8, "3,4,2"),
+                                             (3, 16, "3,8,2")])
+def test_describe_names_the_kernel(settings, kind, depth, name):
+    """The template's arguments, as a profiler's kernel filter takes them."""
+    pkg = settings
+    pkg.set_pipeline(kind, pkg.TG_PREC_F64, depth, 0)
+    assert kernel(pkg, kind) == f"k_block_f64_chunk<{name}>"

@@ -2809,7 +2809,10 @@ __attribute__((visibility("default"))) int tg_plan_describe(const tg_plan *p, ch
             else if (!f64) snprintf(name, sizeof name, "k_block_refine<%d>", g.kind);
             else if (h.stages && h.rows) snprintf(name, sizeof name, "k_block_f64_rows<%d,%d>", g.kind, h.stages);
             else if (h.stages && h.res) snprintf(name, sizeof name, "k_block_f64_ring<%d,%d,%d,1>", g.kind, h.stages, h.bw);
-            else if (h.stages && h.bw == 32) snprintf(name, sizeof name, "k_block_f64_chunk<%d,%d>", g.kind, h.stages);
+            else if (h.stages && h.bw == 32) {   // a ring of h.stages levels in stages of L (with_block_ring)
+                const int L = g.kind == TG_KIND_BLOCK3 && h.stages == 4 ? 1 : 2;
+                snprintf(name, sizeof name, "k_block_f64_chunk<%d,%d,%d>", g.kind, h.stages / L, L);
+            }
             else if (h.stages) snprintf(name, sizeof name, "k_block_f64_ring<%d,%d,%d>", g.kind, h.stages, h.bw);
             else snprintf(name, sizeof name, "k_block_f64<%d>", g.kind);
         }
