@@ -632,7 +632,7 @@ int tg_plan_status(tg_plan *plan, int *per_segment_status);
 /* Number of kernel launches one tg_plan_execute issues. */
 int tg_plan_launches(const tg_plan *plan);
 /* The kernel each group of the plan launches, with its launch shape, as
- * "k_scalar_f64_ring<4,1> kind=0 threads=32 blocks=...; ..." (for logs and
+ * "k_scalar_f64_chunk<3,4> kind=0 threads=32 blocks=...; ..." (for logs and
  * profiler filters).  TG_EINVAL when n is too small (output truncated). */
 int tg_plan_describe(const tg_plan *plan, char *buf, int n);
 /* Refinement sweep histogram of the last execute: hist[s] = columns that
@@ -662,11 +662,13 @@ int tg_set_host_precision(int precision);
 int tg_set_tile(int kind, int precision, int cols_per_block, int cols_per_thread);
 /* Coefficient staging of the FP64 kernels of a kind: 0 = register-prefetch
  * kernel (shape from tg_set_tile); 4, 8 or 16 = depth in levels of the
- * shared-memory ring that bulk asynchronous copies fill ahead of the sweep
- * (one warp per 32 columns, `warps` independent warps per CTA, 1..8, 0 the
+ * shared-memory ring that asynchronous copies fill ahead of the sweep (16-byte
+ * copies in the default kernels, bulk copies in the narrow, row and on-chip
+ * forms; one warp per 32 columns, `warps` independent warps per CTA, 1..8, 0 the
  * default count; used when the level-major column stride is a multiple
  * of 32 and the arrays are 16-byte aligned, otherwise the register-prefetch
- * kernel runs); -1 restores the default.  Scalar kind, TG_PREC_F32_REFINE:
+ * kernel runs); -1 restores the default, the depth of the kernel that the
+ * other settings choose.  Scalar kind, TG_PREC_F32_REFINE:
  * 2..4 = stages of 4 levels of the refinement ring (x 16-byte aligned too),
  * 0 = register-prefetch refinement kernel. */
 int tg_set_pipeline(int kind, int precision, int stages, int warps);
@@ -681,36 +683,36 @@ int tg_set_prefetch(int kind, int precision, int levels);
  * (residency then limited only by registers); -1 restores the default.
  * Only kind TG_KIND_SCALAR with TG_PREC_F64. */
 int tg_set_scratch_global(int kind, int precision, int on);
-/* L2 eviction-priority hints of the bulk-copy (ring) kernels: coefficient
- * streams evict-first, the sweep's scratch and parked w3 evict-last.
+/* L2 eviction-priority hints of the ring kernels: coefficient streams
+ * evict-first, the sweep's scratch (and w3 where it is parked in x) evict-last.
  * on: 1 (default), 0 off, -1 back to the default; 2 and 3 as 1, except that
  * the refinement kernels' coefficient fills, which every sweep reads again,
  * are evict-normal (2) or evict-last (3). */
 int tg_set_cache_hints(int on);
 
-/* FP64 block kinds with a bulk-copy ring: one lane per block row (B lanes per
+/* FP64 block kinds with a ring: one lane per block row (B lanes per
  * column, whole blocks exchanged by warp shuffles) instead of one lane per
  * column.  Same arithmetic, bit-identical results.  on: 1, 0, -1 default. */
 int tg_set_block_rows(int kind, int on);
 
-/* FP64 block kinds with a bulk-copy ring: columns per warp, 32 (default), 16
+/* FP64 block kinds with a ring: columns per warp, 32 (default), 16
  * or 8 (other values restore the default).  Fewer columns per warp means more
  * warps for the same columns, which helps when a grid has too few columns to
  * hide the latency of the block recurrence.  Same arithmetic, same bits. */
 int tg_set_block_width(int kind, int width);
 
-/* Scalar FP64 bulk-copy ring with w2 in global scratch: levels per ring stage
- * (1, 2, 4 or 8; other values restore the default).  With L > 1 one mbarrier
- * wait and one round of copies serve L levels; the ring depth set by
- * tg_set_pipeline then counts stages of L levels (2, 3 or 4). */
+/* Scalar FP64 ring with its scratch in global memory: levels per ring stage
+ * (1, 2, 4 or 8; other values restore the default, 4).  With L > 1 one wait and
+ * one round of copies serve L levels, and the ring depth set by tg_set_pipeline
+ * counts stages of L levels (2, 3 or 4); with 1 the bulk-copy ring runs. */
 int tg_set_stage_levels(int kind, int precision, int levels);
 
-/* Where the FP64 bulk-copy ring kernels keep the forward sweep's quantities
- * until the back sweep reads them.  Scalar kind (chunked ring): 0 w2 in an L2
- * scratch slot per resident lane, w3 parked in x (k_scalar_f64_chunk); 1 w2
- * in the warp's shared memory, w3 parked in x; 2 both in shared memory
- * (k_scalar_f64_res).  Block kinds: 0 Gamma in an L2 scratch slot, 1 or 2
- * Gamma in the warp's shared memory (k_block_f64_ring<..., 1>).  Scalar
+/* Where the FP64 ring kernels keep the forward sweep's quantities until the
+ * back sweep reads them.  Scalar kind (chunked ring): 0 w2 and w3 in the
+ * warp's L2 scratch (k_scalar_f64_chunk); 1 w2 in the warp's shared memory, w3
+ * parked in x; 2 both in shared memory (k_scalar_f64_res).  Block kinds: 0
+ * Gamma (and z) in L2 scratch, 1 or 2 Gamma in the warp's shared memory
+ * (k_block_f64_ring<..., 1>; not built for 32 columns of 3x3).  Scalar
  * refinement (TG_PREC_F32_REFINE): 1 the warp's whole 32-column tile (FP64
  * a, b, c, f, x and the FP32 factors) in shared memory, so the coefficients
  * are read once for all sweeps (k_scalar_refine_tile).  On chip,
@@ -719,20 +721,19 @@ int tg_set_stage_levels(int kind, int precision, int levels);
  * Same arithmetic, same bits. */
 int tg_set_column_residency(int kind, int precision, int mode);
 
-/* Fused assembly routines: 2 (default) three passes where built (dt_ng,
- * minor_ng, oplus_ng, settei_ng, and comp_ng on launches of up to 16384
- * columns): the level quantities and then the rows with one thread per
- * (level, column), then a column walk that is the recurrence alone (and
- * settei_ng's Te, Ti level-parallel again); 1 two passes, the level
- * quantities then a walk that forms the rows as it goes (comp_ng above
- * 16384 columns in mode 2 too); 0 one fused column walk.  Same operations,
- * same results. */
+/* Fused assembly routines: 2 (default) level quantities and rows with one
+ * thread per (level, column), in one kernel or two, then a column walk that
+ * is the recurrence alone (comp_ng forms its rows beside its block recurrence,
+ * in one kernel) and settei_ng's Te, Ti level-parallel again; 1 two passes,
+ * the level quantities then a walk that forms the rows as it goes; 0 one
+ * fused column walk.  Same operations, same results. */
 int tg_set_assembly_mode(int mode);
 
-/* Fused assembly routines: how many levels ahead their column walks request
- * the reads of a level (n >= 1), or -1 (default) for automatic: 8 levels for
- * launches of up to 16384 columns, where few warps per SM leave every level
- * waiting on memory otherwise, 1 above.  Same results. */
+/* Fused assembly routines, modes 0 and 1 of tg_set_assembly_mode, and the O+
+ * factor and solve past their shared-memory tiles: how many levels ahead their
+ * column walks request the reads of a level (n >= 1), or -1 (default) for
+ * automatic: 8 levels for launches of up to 16384 columns, where few warps per
+ * SM leave every level waiting on memory otherwise, 1 above.  Same results. */
 int tg_set_walk_prefetch(int levels);
 
 /* FP64 block kinds: the budget for the sweep scratch (Gamma and, in the
@@ -749,10 +750,12 @@ int tg_set_block_scratch_budget(double megabytes);
 int tg_set_scalar_scratch_budget(double megabytes);
 
 /* How the kinds of one plan share the GPU, read when a plan is created: 1 the
- * block kinds run on a side stream beside the scalar kind (whose FP64 grid is
- * then halved, leaving the block warps, the long pole, more issue slots), 0
- * one kind after the other, any other value (default) side by side only when
- * every kind's tiles fit in one resident wave.  Same results either way. */
+ * block kinds run on a side stream beside the scalar kind (each warp of whose
+ * FP64 grid then takes at least two tiles, leaving the block warps, the long
+ * pole, more issue slots), 0 one kind after the other, any other value
+ * (default) side by side only when the GPU could hold every tile of each kind
+ * at once (a kind may still run in more passes, to keep its scratch in L2).
+ * Same results either way. */
 int tg_set_kind_overlap(int mode);
 
 /* Host-array entries (tg_solve_host and the per-routine drop-ins): the input
@@ -786,8 +789,9 @@ int tg_selftest_division(const double *a, const double *b, double *q, long n, vo
  *            (planes 6, 7, 8 of nk*ld; rows 0..nk-2) the caller filled; the
  *            pass writes w1 (plane 10), 1/w1 (plane 11) and w2 (plane 12,
  *            rows 0..nk-3).
- * Launches of up to 16384 columns take the shared-memory tile walks, larger
- * ones the walks that read global memory; both give the same bits.
+ * Launches of few columns take the shared-memory tile walks, larger ones the
+ * walks that stream from global memory; both give the same bits, and the rows
+ * that they read are left as they were.
  * *status_dev receives the walk's status (TG_EPIVOT, TG_ENONFINITE). */
 int tg_selftest_walk(int which, double *buf, int nk, int K, int top, int ncol, long ld, int *status_dev,
                      void *stream);

@@ -7,7 +7,7 @@ from a CUDA graph, CUDA-event timed) and keeps the fastest:
   FP64      register-prefetch kernel: columns per block x columns per thread x
             prefetch depth, w2 scratch in shared memory ("reg") or global
             memory ("regg")
-            bulk-copy ring kernel: staging depth 4, 8 or 16 levels, w2 in shared
+            ring kernel: staging depth 4, 8 or 16 levels, w2 in shared
             ("ring") or global ("ringg") memory; for block kinds also one lane
             per block row ("rows", depth 4 or 8) and 16 or 8 columns per warp
             ("ring16", "ring8"), and those rings with Gamma resident in shared
@@ -16,7 +16,7 @@ from a CUDA graph, CUDA-event timed) and keeps the fastest:
             the sweep's w2 ("res1cL") or w2 and w3 ("res2cL") resident in
             shared memory, L levels per stage
   FP32+ref  columns per block x prefetch depth; scalar kind also the
-            bulk-copy refinement ring of 2, 3 or 4 stages ("ring") and the
+            refinement ring of 2, 3 or 4 stages ("ring") and the
             whole tile held in shared memory ("tile")
 
 Results are cached in a JSON file keyed by GPU name, kind, precision, level

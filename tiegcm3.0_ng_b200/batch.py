@@ -235,7 +235,7 @@ def shard_segments(segments, world, rank, align=32):
     """Plan segments restricted to this rank's columns (views, no copies).
     Cuts inside a segment fall on multiples of `align` columns, so a share
     starts on a 32-column tile with 16-byte aligned rows and keeps the
-    bulk-copy kernels."""
+    ring kernels."""
     ncols = [s["ncol"] for s in segments]
     weights = [(1 if s["kind"] == TG_KIND_SCALAR else s["kind"]) * s["k2"] for s in segments]
     out = []

@@ -1018,8 +1018,8 @@ def set_tile(kind, precision, cols_per_block=0, cols_per_thread=0):
 
 
 def set_pipeline(kind, precision, stages=-1, warps=0):
-    """Ring depth of the bulk-copy staged FP64 kernels (0: register prefetch,
-    -1: default) and their warps per CTA (0: default)."""
+    """Ring depth of the staged kernels (0: register prefetch, -1: the default
+    of the kernel that runs) and their warps per CTA (0: default)."""
     return _check(lib().tg_set_pipeline(kind, precision, stages, warps), "tg_set_pipeline", numeric_ok=False)
 
 
@@ -1085,7 +1085,8 @@ def set_assembly_mode(mode):
 
 
 def set_walk_prefetch(levels):
-    """Levels the assembly walks read ahead: 1..32, or -1 automatic (8 up to 16384 columns, else 1)."""
+    """Levels that the column walks of assembly modes 0 and 1, and O+'s large factor and solve, read ahead: 1..32, or
+    -1 automatic (8 up to 16384 columns, else 1)."""
     return _check(lib().tg_set_walk_prefetch(int(levels)), "tg_set_walk_prefetch")
 
 

@@ -215,7 +215,7 @@ bool ring_ok_seg(const Seg &s)
 {
     return s.ld % 32 == 0 && aligned16(s.a) && aligned16(s.b) && aligned16(s.c) && aligned16(s.f);
 }
-// The refinement ring also reads x rows by bulk copies.
+// The refinement rings read x rows too.
 bool ring_ok_for(const Seg &s, int precision)
 {
     return ring_ok_seg(s) && (precision == TG_PREC_F64 || aligned16(s.x));

@@ -119,7 +119,7 @@ inline bool exact_reciprocal(double b)
 }
 
 // exp(z) of a small argument: for |z| <= 1/8 the Taylor polynomial of degree
-// 11 (the first dropped term is below 3e-20 of the result), else the device
+// 11 (the first dropped term is below 3.5e-20 of the result), else the device
 // exp.  Rounding: the last step adds 1 to less than 1/8 of an ulp's error.
 __device__ __forceinline__ double exp_small(double z)
 {

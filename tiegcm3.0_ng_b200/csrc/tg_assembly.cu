@@ -2055,9 +2055,12 @@ cudaError_t launch_comp_ng(const CompFields &F, const CompConsts &C, double *out
             };
             // while every tile is resident with four producers (three blocks
             // per SM) the tile's own time decides; past that, more tiles at
-            // once (two producers, five blocks per SM): 11,248 columns x 57
-            // levels 91 us with 4 and 108 with 2, 21,216 165 and 151, 43,216
-            // 292 and 279
+            // once (two producers, five blocks per SM).  us with 4 and 2, x 29,
+            // 57 and 113 levels: 11,248 columns 47 and 58, 86 and 105, 158 and 195;
+            // 14,400 73 and 64, 134 and 115, 245 and 213; 21,300 89 and 79, 161 and
+            // 148, 292 and 279; 43,216 160 and 148, 290 and 276, 556 and 535 (where
+            // the last round of five is nearly empty 4 win: 30,000 123 and 126, 216
+            // and 232, 408 and 445)
             auto pick = [&](auto dv) {
                 if (blocks <= 3 * sm_count()) go(dv, std::integral_constant<int, 4>{});
                 else go(dv, std::integral_constant<int, 2>{});

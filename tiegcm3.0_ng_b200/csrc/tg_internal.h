@@ -84,7 +84,7 @@ struct Shape {
     int threads;        // threads per block
     int cpt;            // columns per thread (1 or 2)
     int blocks;         // persistent grid size
-    int stages;         // bulk-copy ring depth (0: register-prefetch kernel)
+    int stages;         // ring depth (0: register-prefetch kernel)
     int w2g;            // scalar register kernel with w2 in global scratch
     int pf;             // scalar register kernels: prefetch depth in levels
     size_t smem;        // dynamic shared memory bytes
@@ -93,7 +93,7 @@ struct Shape {
     int lps;            // scalar FP64 ring: levels per stage (>1: chunked ring kernel)
     int res;            // scalar FP64 chunked ring: 1 w2 in shared memory (w3 parked in x), 2 w2 and w3 in
                         // shared memory (k_scalar_f64_res); 0 L2 scratch (k_scalar_f64_chunk)
-    int one_wave;       // the grid holds every tile at once (no grid-stride second pass)
+    int one_wave;       // the GPU could hold every tile at once (blocks may be fewer, to keep the scratch in L2)
     int drop;           // warps discard a finished tile's scratch from L2
 };
 
@@ -101,7 +101,8 @@ struct Shape {
 int cols_per_block(int kind, int precision);
 int cols_per_thread(int kind, int precision);
 void set_tile(int kind, int precision, int cpb, int cpt);
-// Bulk-copy ring depth of a kind/precision (tg_set_pipeline); 0 disables.
+// Ring depth of a kind/precision (tg_set_pipeline); 0 disables, a negative one
+// is the default of the kernel that runs.
 // wpb: independent warps per CTA of the ring kernels (0 keeps the default).
 void set_stages(int kind, int precision, int stages, int wpb);
 int ring_warps(int kind, int precision);
@@ -323,11 +324,11 @@ cudaError_t launch_selftest_wait(unsigned polls, unsigned *status, cudaStream_t 
 // (major*10 + minor of the SASS target: 100 for sm_100a).
 cudaError_t kernel_binary_version(int *v);
 
-// Block kinds: the bulk-copy ring kernel with one lane per block row
+// Block kinds: the (bulk-copy) ring kernel with one lane per block row
 // (tg_set_block_rows); 1 on, 0 off, -1 default.
 void set_block_rows(int kind, int on);
-// Block kinds: columns per warp of the bulk-copy ring kernel (32, 16 or 8;
-// other values restore the default).
+// Block kinds: columns per warp of the ring kernel (32; 16 and 8 by bulk
+// copies; other values restore the default).
 void set_block_width(int kind, int w);
 // Scalar FP64 ring with w2 in global scratch: levels per ring stage (1, 2, 4,
 // 8; other values restore the default).
@@ -337,16 +338,16 @@ void set_stage_levels(int kind, int precision, int l);
 // memory; other values restore the default).
 void set_column_residency(int kind, int precision, int mode);
 int column_residency();
-// L2 budget (MB) for the Gamma scratch of all resident block-kernel warps;
-// <= 0 restores the default.
+// Budget (MB) for the sweep scratch of all resident columns; <= 0 restores the
+// kernels' own limits.
 void set_block_scratch_budget(double mb);
 void set_scalar_scratch_budget(double mb);
 // Kinds of one plan: 1 concurrently (block kinds on a side stream), 0 one
-// after the other, -1 concurrently only when every kind fits in one wave.
+// after the other, -1 concurrently only when every kind could be resident at once.
 void set_kind_overlap(int mode);
 int kind_overlap();
 
-// L2 cache-policy hints of the bulk-copy ring kernels (tg_set_cache_hints).
+// L2 cache-policy hints of the ring kernels (tg_set_cache_hints).
 int cache_hints();
 void set_cache_hints(int on);
 

@@ -3513,13 +3513,15 @@ cudaError_t occupancy(K kernel, int threads, size_t smem, int *per_sm)
 // scratch (k_scalar_f64_chunk: w2 and w3, 16 B per level and column;
 // k_block_f64_chunk: Gamma and z) and, for the scalar kernel, kStreamKB for
 // what it streams (rows in flight, the x rows on their way out).  Past the
-// budget the scratch spills: scalar, 909,356 columns x 57 levels, 382 us at 10
-// warps per SM, 431 at 13, 469 at 16; 290,304 x 113, 283 us at 7, 310 at 9,
-// 332 at 10 (before finished scratch was discarded).  Block, 2x2, 130,000 x 57:
-// 200 us at 4 warps per SM, 208 at 5, 231 at 8, but 20,000 columns (4.2 tiles
-// per SM) 51 us at 4 and 38 at 5: 4.5, rounded.  Whole plans since: 2.5 deg grid
-// and 16 x 3 nests with 2x2 blocks 589 us at 120 and 57 MB, 570 at 130 and 57,
-// 580 at 120 and 64, 558 at 135 and 64; 1.25 deg grid 408 up to 130, 412 past it.
+// budget the scratch spills: before finished scratch was discarded, scalar,
+// 909,356 columns x 57 levels, 382 us at 10 warps per SM, 431 at 13, 469 at 16;
+// 290,304 x 113, 283 us at 7, 310 at 9, 332 at 10; block, 2x2, 130,000 x 57, 200
+// us at 4 warps per SM, 208 at 5, 231 at 8, but 20,000 columns (4.2 tiles per SM)
+// 51 us at 4 and 38 at 5: 4.5, rounded.  Whole plans with the discards, replayed
+// on the same inputs, at scalar and block MB: 2.5 deg grid and 16 x 3 nests with
+// 2x2 blocks 586 us at 120 and 57, 568 at 130 and 57, 575 at 120 and 64, 558 at 130
+// and 64, 555 at 135 and 64 (616 at 130 and 64 on inputs new to each pass); 1.25
+// deg grid x 113 levels 404 up to 130, 409 at 135; 2.5 deg grid 53 with all.
 constexpr double kChunkBudgetMB[2] = {130.0, 64.0};   // scalar, block
 constexpr double kStreamKB = 56.0;
 // Refinement rings.  Scalar (FP32 planes and the iterate, 20 B per level and

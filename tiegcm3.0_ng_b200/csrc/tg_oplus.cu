@@ -839,26 +839,6 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_oplus_solve_tile(OplusField
     }
 }
 
-// One sub-step of the O+ sub-cycle in one kernel: the Shapiro smoothing of
-// optm1, the right-hand side, the solve from the factor and the post-solve
-// steps.  A block of five warps takes kSubCols consecutive columns.  It copies
-// p, w1, 1/w1 and w2 of every level into shared memory and reads each thread's
-// explicit_h and op_prod values (none of which the sub-step before writes);
-// then waits for that sub-step (programmatic dependent launch), so those reads
-// and the launch overlap its tail.  The lat pass of the smoothing covers the
-// tile's columns and two on each side, straight from L2 (every column a value
-// is used from lies in the same grid row); the lon pass and the right-hand
-// side follow from shared memory, one thread per level and column, so that
-// the walk of warp 0 is the recurrence alone.  prev and cur stay in registers
-// from before the walk to the post-solve steps.
-// What bounds it: the walk (56 levels forward and back, one warp) and the L2
-// latency of the reads after the wait.  The step's O+ chain (factor pass and 10
-// sub-steps), as a graph: 2,072 columns x 57 levels 169 us with smoothing and
-// solve as two kernels -> 107, 6,969 columns 297 -> 149, 11,248 columns 389 ->
-// 252 (there the solve's 130 KB tiles also left one block per SM; these take
-// 38 KB).
-// R: levels a thread holds (10 threads per column: nk <= 10 R).  MB: blocks per
-// SM that its registers allow (0: the compiler's choice).
 // shapiro_at at a fixed index t of n points (stride s) over many levels: the
 // neighbours it does not use are read at the point itself, so that every read
 // can be in flight at once, and the edge forms are selected.
@@ -884,6 +864,26 @@ struct Shapiro3 {
         return edge ? x : near ? yn : yi;
     }
 };
+// One sub-step of the O+ sub-cycle in one kernel: the Shapiro smoothing of
+// optm1, the right-hand side, the solve from the factor and the post-solve
+// steps.  A block of five warps takes kSubCols consecutive columns.  It copies
+// p, w1, 1/w1 and w2 of every level into shared memory and reads each thread's
+// explicit_h and op_prod values (none of which the sub-step before writes);
+// then waits for that sub-step (programmatic dependent launch), so those reads
+// and the launch overlap its tail.  The lat pass of the smoothing covers the
+// tile's columns and two on each side, straight from L2 (every column a value
+// is used from lies in the same grid row); the lon pass and the right-hand
+// side follow from shared memory, one thread per level and column, so that
+// the walk of warp 0 is the recurrence alone.  prev and cur stay in registers
+// from before the walk to the post-solve steps.
+// What bounds it: the walk (56 levels forward and back, one warp) and the L2
+// latency of the reads after the wait.  The step's O+ chain (factor pass and 10
+// sub-steps), as a graph: 2,072 columns x 57 levels 169 us with smoothing and
+// solve as two kernels -> 107, 6,969 columns 297 -> 149, 11,248 columns 389 ->
+// 252 (there the solve's 130 KB tiles also left one block per SM; these take
+// 38 KB).
+// R: levels a thread holds (10 threads per column: nk <= 10 R).  MB: blocks per
+// SM that its registers allow (0: the compiler's choice).
 constexpr int kSubCols = 16, kSubThreads = 160;
 template <int R, int MB>
 __global__ void __launch_bounds__(kSubThreads, MB) k_oplus_substep(OplusFields F, OplusConsts C, const double *scr,
@@ -1216,6 +1216,10 @@ cudaError_t launch_oplus_subcycle(const OplusFields &F, const OplusConsts &C, do
         }
         apart = apart && !meet(sc.op[s], field, sc.optm1[s], field);
     }
+    // kSmallWalkColumns is the limit of the tile solve, which the fused sub-step
+    // took the place of; past it smoothing and solve run as they did.  The fused
+    // one would be the faster there too (17,688 columns x 57 levels 309 us and
+    // 1,143 for 10 sub-steps, 43,216 x 57 793 and 1,507).
     const bool fused = apart && ncol <= kSmallWalkColumns && nk <= 130 && smem <= (size_t)smem_optin();
     const bool wide = ld % 2 == 0 && ld >= (ncol + kSubCols - 1) / kSubCols * kSubCols && ((uintptr_t)factor & 15) == 0;
     if (fused)

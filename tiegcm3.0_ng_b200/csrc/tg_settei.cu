@@ -87,10 +87,10 @@ __device__ __forceinline__ double qsum(const SetteiFields &F, long o)
 
 namespace {
 // x^e of e = RN(2/7), the power that turns Te^3.5 back into Te, within 0.51
-// ulp.  y, the single-precision root, is off by a few 1e-6: its exact seventh
-// power against x*x (both as sums of two doubles) gives e7 = x^2/y^7 - 1, the
-// binomial series of (1 + e7)^(1/7) the correction (Newton's step and its next
-// two terms; the first dropped term is below 1e-20), and x^(e - 2/7) =
+// ulp.  y, the single-precision root, is off by at most some 5e-6: its exact
+// seventh power against x*x (both as sums of two doubles) gives e7 = x^2/y^7 - 1,
+// the binomial series of (1 + e7)^(1/7) the correction (Newton's step and its
+// next two terms; the first dropped term is below 1e-19), and x^(e - 2/7) =
 // 1 + (e - 2/7)*log(x) the difference of the exponents, e - 2/7 =
 // -2/7*2^-54.  About 40 operations for pow's two hundred.  Outside the range
 // that single precision holds with room to spare (zeros, negative values and

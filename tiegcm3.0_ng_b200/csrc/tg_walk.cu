@@ -89,10 +89,18 @@ __global__ void __launch_bounds__(kWalkTileThreads) k_thomas_post_tile(const dou
 // the walk took 107 us with w2 in shared memory, w3 parked in x and the stores
 // waiting on their inputs level by level (issue 20%, 6.6 long-scoreboard stalls
 // per issue); dt_ng there went from 203 to 130 us, minor_ng from 252 to 186.
-// The tile walk is taken while its blocks are resident all at once (16,576
-// columns at 57 levels, 7,104 at 113): dt_ng with its rows on 16,384 columns
-// took 66 us with the tiles and 68 on 16,770 with the ring; at 113 levels 142
-// us (16,384, tiles in three passes) against 126 (17,420, ring).
+// The tile walk is taken while shared memory alone would hold its blocks all at
+// once: 35,520 columns at 29 levels, 16,576 at 57, 7,104 at 113.  (Its registers
+// hold 5 blocks per SM, 11,840 columns, so that the upper part of the range runs
+// in two or three rounds.)  dt_ng with its rows, us with tile and ring:
+//   29 levels  11,760 columns 21.9, 27.2; 13,440 29.0, 29.1; 22,080 40.3, 40.1;
+//              29,000 52.7, 48.3; 36,000 64.8, 55.4
+//   57         11,760 40.5, 49.5; 13,440 51.5, 53.1; 16,320 57.7, 58.6; 22,080
+//              71.9, 71.0; 29,000 93.2, 87.1
+//   113        7,000 53.2, 72.3; 8,400 76.5, 77.5; 11,280 90.3, 88.3; 16,320 128,
+//              108
+// The limit lies where the two meet at 57 and 113 levels; at 29 they meet near
+// 14,000 columns, part by 1% up to 22,000 and by 9% at 29,000.
 constexpr int kRingLevels = 4, kRingStages = 3;
 constexpr int kRingDoubles = 5 * 32;   // a level of the back sweep: w2, w3, prev, cur, bnd
 template <bool WIDE>
