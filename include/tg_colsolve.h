@@ -24,8 +24,10 @@
  *     streams may run at the same time (up to 16 streams at once; a 17th
  *     stream drains the device and takes the least recently used stream's
  *     buffers).  A stream's first call, and a call that needs larger buffers
- *     than the stream had, allocate and synchronise: make those calls once
- *     before capturing the calls into a CUDA graph.
+ *     than the stream had, allocate and synchronise.  Calls captured into a
+ *     CUDA graph get buffers of that graph's own, which live as long as the
+ *     graph and its executables, so graphs may run side by side (make one
+ *     call outside a capture first, which sets up the device).
  *   - Every entry point returns a tg_status.  The reference has no error
  *     return (a zero pivot silently yields Inf/NaN); the solves here produce
  *     the same numbers in that case and additionally report TG_EPIVOT.

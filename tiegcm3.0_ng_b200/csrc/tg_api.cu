@@ -50,6 +50,7 @@ int g_host_precision = TG_PREC_F64;
 struct Buf {
     void *p = nullptr;
     size_t n = 0;
+    std::vector<void *> *outgrown = nullptr;   // set where a captured graph may hold p: see CaptureWs
 };
 
 // Per-device work buffers and streams, created on first use.  The host
@@ -73,6 +74,42 @@ struct StreamWs {
     unsigned *flags = nullptr;     // device status word
 };
 constexpr int kStreamWs = 16;
+// The workspace of one stream within one capture.  The captured graph's kernels
+// hold its addresses for as long as the graph can be launched, so it is the
+// graph's own: no later call on the stream grows, frees or uses it, and a buffer
+// outgrown within the capture stays.  The graph (and every executable made from
+// it) holds a user object whose destructor, after the last of them and its last
+// launch are done, marks the workspace unused; it then serves another capture,
+// and beyond kStreamWs unused ones it is freed.
+struct CaptureWs : StreamWs {
+    unsigned long long id = 0;   // of the capture
+    std::vector<void *> outgrown;
+    std::atomic<bool> unused{true};
+    CaptureWs()
+    {
+        for (Buf &b : lvl) b.outgrown = &outgrown;
+        scratch.outgrown = &outgrown;
+    }
+    void free_outgrown()
+    {
+        for (void *p : outgrown) cudaFree(p);
+        outgrown.clear();
+    }
+    ~CaptureWs()
+    {
+        free_outgrown();
+        for (Buf &b : lvl)
+            if (b.p) cudaFree(b.p);
+        if (scratch.p) cudaFree(scratch.p);
+        if (flags) cudaFree(flags);
+    }
+};
+// While one lives, this thread may allocate and free beside any stream capture.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
 
 struct DevCtx {
     int dev = -1;
@@ -91,6 +128,9 @@ struct DevCtx {
 
 constexpr int kMaxDev = 64;
 DevCtx *g_ctx[kMaxDev] = {};
+// Per device, see CaptureWs; under the context's lock.  They outlive a context
+// that tg_release_buffers ends: graphs hold them.
+std::vector<CaptureWs *> g_captures[kMaxDev];
 std::mutex g_ctx_mu;
 
 int get_ctx(DevCtx **out)
@@ -125,11 +165,22 @@ int get_ctx(DevCtx **out)
     return TG_OK;
 }
 
+cudaError_t capture_malloc(void **p, size_t bytes)
+{
+    RelaxedCapture relaxed;
+    return cudaMalloc(p, bytes);
+}
+
 // Grows a device buffer; the device is synchronised before an old buffer is
-// freed, since queued work may still use it.
+// freed, since queued work may still use it.  A capture's old buffer stays.
 int grow(Buf &b, size_t bytes)
 {
     if (bytes <= b.n) return TG_OK;
+    if (b.p && b.outgrown) {
+        b.outgrown->push_back(b.p);
+        b.p = nullptr;
+        b.n = 0;
+    }
     if (b.p) {
         TG_CUDA(cudaDeviceSynchronize());
         TG_CUDA(cudaFree(b.p));
@@ -137,9 +188,10 @@ int grow(Buf &b, size_t bytes)
         b.n = 0;
     }
     bytes = (bytes + 4095) & ~(size_t)4095;
-    cudaError_t e = cudaMalloc(&b.p, bytes);
+    cudaError_t e = b.outgrown ? capture_malloc(&b.p, bytes) : cudaMalloc(&b.p, bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
+        b.p = nullptr;
         set_err("cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
         return TG_ENOMEM;
     }
@@ -147,11 +199,74 @@ int grow(Buf &b, size_t bytes)
     return TG_OK;
 }
 
+// The workspace of stream st in the capture `id` into `graph`.
+int capture_ws(DevCtx *c, cudaStream_t st, unsigned long long id, cudaGraph_t graph, StreamWs **out)
+{
+    CaptureWs *w = nullptr;
+    for (CaptureWs *p : g_captures[c->dev]) {
+        if (p->unused.load(std::memory_order_acquire)) {
+            if (!w) w = p;
+        } else if (p->key == st && p->id == id) {
+            *out = p;
+            return TG_OK;
+        }
+    }
+    if (!w) {
+        w = new (std::nothrow) CaptureWs;
+        if (!w) return TG_ENOMEM;
+        g_captures[c->dev].push_back(w);
+    }
+    if (!w->flags) TG_CUDA(capture_malloc((void **)&w->flags, sizeof(unsigned)));
+    // the destructor, on a thread of the driver's, may call no CUDA function
+    cudaUserObject_t obj = nullptr;
+    TG_CUDA(cudaUserObjectCreate(
+        &obj, w, [](void *p) { static_cast<CaptureWs *>(p)->unused.store(true, std::memory_order_release); }, 1,
+        cudaUserObjectNoDestructorSync));
+    w->unused.store(false, std::memory_order_release);
+    cudaError_t e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
+    if (e != cudaSuccess) cudaUserObjectRelease(obj, 1);   // marks it unused
+    TG_CUDA(e);
+    w->key = st;
+    w->id = id;
+    *out = w;
+    return TG_OK;
+}
+
+// Gives back what captures whose graphs are gone leave: the buffers that they
+// outgrew, and the workspaces beyond `keep`.
+void trim_captures(DevCtx *c, size_t keep)
+{
+    std::vector<CaptureWs *> &all = g_captures[c->dev];
+    RelaxedCapture relaxed;
+    size_t n = 0;
+    for (size_t i = 0; i < all.size();) {
+        CaptureWs *w = all[i];
+        if (!w->unused.load(std::memory_order_acquire)) {
+            ++i;
+        } else if (n++ < keep) {
+            w->free_outgrown();
+            ++i;
+        } else {
+            delete w;
+            all.erase(all.begin() + i);
+        }
+    }
+}
+
 // The workspace of caller stream st (the caller holds c->mu).  A stream
 // seen for the first time takes a free entry; with all kStreamWs taken, the
-// least recently used one is drained (device synchronised) and reassigned.
+// least recently used one is drained (device synchronised) and reassigned.  A
+// stream that is being captured gets the capture's own.
 int stream_ws(DevCtx *c, cudaStream_t st, StreamWs **out)
 {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo(st, &capture, &id, &graph, nullptr, nullptr) != cudaSuccess)
+        cudaGetLastError();   // the legacy stream beside a capture: the launches report it
+    else if (capture == cudaStreamCaptureStatusActive)
+        return capture_ws(c, st, id, graph, out);
+    if (g_captures[c->dev].size() > kStreamWs) trim_captures(c, kStreamWs);
     StreamWs *hit = nullptr, *free_ws = nullptr, *lru = nullptr;
     for (StreamWs &w : c->ws) {
         if (w.used && w.key == st) {
@@ -2877,6 +2992,7 @@ __attribute__((visibility("default"))) int tg_release_buffers(void)
             if (w.scratch.p) cudaFree(w.scratch.p);
             if (w.flags) cudaFree(w.flags);
         }
+        trim_captures(c, 0);   // those of live graphs stay theirs
         if (c->flags) cudaFree(c->flags);
         if (c->flags_host) cudaFreeHost(c->flags_host);
         if (c->hist) cudaFree(c->hist);

@@ -269,7 +269,7 @@ class DynamicsStep:
 
     def capture(self, stream):
         """Records one step into a CUDA graph (after an eager step, which
-        sizes the library's per-stream buffers); replay() then runs it."""
+        loads the kernels); replay() then runs it."""
         import torch
         self.issue(stream)
         stream.synchronize()
