@@ -797,7 +797,17 @@ int tg_selftest_division(const double *a, const double *b, double *q, long n, vo
  * *status_dev receives the walk's status (TG_EPIVOT, TG_ENONFINITE). */
 int tg_selftest_walk(int which, double *buf, int nk, int K, int top, int ncol, long ld, int *status_dev,
                      void *stream);
-/* Frees the per-device mirrors, work buffers and streams. */
+/* Work buffers of captured calls.  By default the graph holds them through a
+ * CUDA user object, which costs each of its launches some microseconds.  A
+ * caller who knows when the graph is gone saves that: tg_capture_own, on a
+ * stream that is being captured and before the first captured call of this
+ * library, gives the capture's id; tg_capture_release, after the graph and its
+ * executables are destroyed (launches may still be running), gives the buffers
+ * back; owned buffers that are never released stay until the process exits. */
+int tg_capture_own(void *stream, unsigned long long *id);
+int tg_capture_release(unsigned long long id);
+/* Frees the per-device mirrors, work buffers and streams (not the buffers that
+ * captured graphs hold). */
 int tg_release_buffers(void);
 /* Library version, e.g. "tg_colsolve 0.1.0 sm_100a". */
 const char *tg_version(void);

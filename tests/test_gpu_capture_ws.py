@@ -122,3 +122,56 @@ def test_buffers_of_destroyed_graphs_are_used_again(cuda, pkg):
         torch.cuda.synchronize()
         free.append(torch.cuda.mem_get_info()[0])
     assert free[9] - free[-1] <= 20 * 37e6
+
+
+def test_owned_captures(cuda, pkg):
+    """60 graphs whose owner says when they are gone; the refusals."""
+    import torch
+    st, d = torch.cuda.Stream(), Dt(pkg, 57, 20000, 6)
+    want = d.result(st, lambda: d.issue(st))
+    with pytest.raises(pkg.TgError):          # no capture
+        pkg.capture_own(st)
+    with pytest.raises(pkg.TgError):          # nobody's
+        pkg.capture_release(1 << 60)
+    free = []
+    for i in range(60):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st, capture_error_mode="thread_local"):
+            own = pkg.capture_own(st)
+            d.issue(st)
+            with pytest.raises(pkg.TgError):  # too late
+                pkg.capture_own(st)
+        if i % 20 == 19:
+            assert bits(d.result(st, g.replay), want)
+        with torch.cuda.stream(st):
+            g.replay()                        # in flight while the graph goes
+        g.reset()
+        pkg.capture_release(own)
+        assert bits(d.result(st, lambda: d.issue(st)), want)
+        free.append(torch.cuda.mem_get_info()[0])
+    with pytest.raises(pkg.TgError):          # given back already
+        pkg.capture_release(own)
+    assert free[9] - free[-1] <= 8 * 37e6
+
+
+def test_steps_of_two_sizes(cuda, pkg):
+    """Steps captured one after another on one stream, the larger one later,
+    more of them than the library has workspaces; then each replayed."""
+    import torch
+    dyn, st, steps, want = pkg.dynamics, torch.cuda.Stream(), [], []
+    for i, (nlon, nlat) in enumerate([(9, 5), (30, 20), (12, 7), (40, 22), (9, 5)]):
+        grid = dyn.Grid(29, nlon, nlat, 0.5, lat0_deg=20.0, dlat_deg=0.3)
+        s = dyn.DynamicsStep(grid, dyn.synthetic_inputs(grid, 50 + i, nstep_sub=2))
+        s.issue(st)
+        torch.cuda.synchronize()
+        want.append({k: v[:, :grid.ncol].clone() for k, v in s.outputs().items()})
+        s.capture(st)
+        steps.append(s)
+    for s, w in zip(steps, want):
+        for v in s.outputs().values():
+            v.fill_(float("nan"))
+        torch.cuda.synchronize()
+        s.replay(st)
+        torch.cuda.synchronize()
+        for k, v in s.outputs().items():
+            assert bits(v[:, :s.grid.ncol].contiguous(), w[k].contiguous()), k

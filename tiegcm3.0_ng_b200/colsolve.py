@@ -43,7 +43,7 @@ EXPORTS = ("tg_solve_host", "tg_dt_ng", "tg_dt_ng_dev", "tg_minor_ng", "tg_minor
            "tg_oplus_ng_dev", "tg_trsolv", "tg_trsolv_ng", "tg_blktri", "tg_comp_blksolve_ng", "tg_blksolve", "tg_trsolv_dev",
            "tg_blksolve_dev", "tg_blksolve_dev_noalloc", "tg_plan_create", "tg_plan_execute", "tg_plan_capture_graph",
            "tg_plan_status", "tg_plan_launches", "tg_plan_describe", "tg_set_cache_hints", "tg_set_block_rows", "tg_set_block_width", "tg_set_stage_levels", "tg_set_column_residency", "tg_set_assembly_mode", "tg_set_walk_prefetch", "tg_set_block_scratch_budget", "tg_set_scalar_scratch_budget", "tg_set_kind_overlap", "tg_set_host_pipeline", "tg_selftest_wait", "tg_plan_sweep_histogram", "tg_plan_destroy",
-           "tg_set_refine", "tg_set_host_precision", "tg_set_tile", "tg_set_pipeline", "tg_set_prefetch", "tg_set_scratch_global", "tg_selftest_division", "tg_selftest_walk", "tg_release_buffers", "tg_version", "tg_kernel_arch", "tg_ringfilter", "tg_ringfilter_dev", "tg_filter_o2o", "tg_trsolv_defer", "tg_trsolv_flush", "tg_dt_diag_ng", "tg_dt_diag_ng_dev", "tg_minor_diag_ng", "tg_minor_diag_ng_dev", "tg_dt_ng_post_dev", "tg_minor_ng_post_dev", "tg_oplus_ng_post_dev", "tg_last_error")
+           "tg_set_refine", "tg_set_host_precision", "tg_set_tile", "tg_set_pipeline", "tg_set_prefetch", "tg_set_scratch_global", "tg_selftest_division", "tg_selftest_walk", "tg_capture_own", "tg_capture_release", "tg_release_buffers", "tg_version", "tg_kernel_arch", "tg_ringfilter", "tg_ringfilter_dev", "tg_filter_o2o", "tg_trsolv_defer", "tg_trsolv_flush", "tg_dt_diag_ng", "tg_dt_diag_ng_dev", "tg_minor_diag_ng", "tg_minor_diag_ng_dev", "tg_dt_ng_post_dev", "tg_minor_ng_post_dev", "tg_oplus_ng_post_dev", "tg_last_error")
 
 
 class PostStepArgs(ctypes.Structure):
@@ -285,6 +285,8 @@ def lib():
             "tg_set_prefetch": [I, I, I],
             "tg_selftest_division": [P, P, P, Lg, P],
             "tg_selftest_walk": [I, P, I, I, I, I, Lg, P, P],
+            "tg_capture_own": [P, ctypes.POINTER(ctypes.c_ulonglong)],
+            "tg_capture_release": [ctypes.c_ulonglong],
             "tg_release_buffers": [],
             "tg_version": [],
             "tg_last_error": [],
@@ -1115,6 +1117,20 @@ def selftest_wait(polls, status, stream=None):
     tensor) receives TG_ETIMEOUT."""
     return _check(lib().tg_selftest_wait(int(polls), _int_dptr(status), _stream(stream)), "tg_selftest_wait",
                   numeric_ok=False)
+
+
+def capture_own(stream=None):
+    """On a stream being captured, before the first captured call: the capture's
+    id, for capture_release once the graph is gone.  The graph's launches are
+    then spared the object that would otherwise tell the library so."""
+    n = ctypes.c_ulonglong()
+    _check(lib().tg_capture_own(_stream(stream), ctypes.byref(n)), "tg_capture_own", numeric_ok=False)
+    return n.value
+
+
+def capture_release(capture):
+    """Gives back the work buffers of a capture (capture_own) whose graph is destroyed."""
+    return _check(lib().tg_capture_release(capture), "tg_capture_release", numeric_ok=False)
 
 
 def release_buffers():

@@ -77,14 +77,9 @@ constexpr int kStreamWs = 16;
 // The workspace of one stream within one capture.  The captured graph's kernels
 // hold its addresses for as long as the graph can be launched, so it is the
 // graph's own: no later call on the stream grows, frees or uses it, and a buffer
-// outgrown within the capture stays.  The graph (and every executable made from
-// it) holds a user object whose destructor, after the last of them and its last
-// launch are done, marks the workspace unused; it then serves another capture,
-// and beyond kStreamWs unused ones it is freed.
+// outgrown within the capture stays.
 struct CaptureWs : StreamWs {
-    unsigned long long id = 0;   // of the capture
     std::vector<void *> outgrown;
-    std::atomic<bool> unused{true};
     CaptureWs()
     {
         for (Buf &b : lvl) b.outgrown = &outgrown;
@@ -104,6 +99,26 @@ struct CaptureWs : StreamWs {
         if (flags) cudaFree(flags);
     }
 };
+// Those of one capture, a stream each.  The graph (and every executable made from
+// it) holds a user object whose destructor, after the last of them and its last
+// launch are done, marks them unused; they then serve another capture, and beyond
+// kCaptures unused sets are freed.  The object costs every launch of the graph 2 to
+// 7 us (a dynamics step of 161 us takes 163 to 168), so a caller who says when the
+// graph is gone (tg_capture_own, tg_capture_release) gets none; what it releases is
+// unused once the device has been drained.
+struct Capture {
+    enum State { kUnused, kLive, kReleased };
+    unsigned long long id = 0;
+    std::vector<CaptureWs *> ws;
+    size_t used = 0;   // the first ws, in the order in which the capture's streams came
+    bool owned = false;
+    std::atomic<int> state{kUnused};
+    ~Capture()
+    {
+        for (CaptureWs *w : ws) delete w;
+    }
+};
+constexpr size_t kCaptures = 4;
 // While one lives, this thread may allocate and free beside any stream capture.
 struct RelaxedCapture {
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
@@ -128,9 +143,9 @@ struct DevCtx {
 
 constexpr int kMaxDev = 64;
 DevCtx *g_ctx[kMaxDev] = {};
-// Per device, see CaptureWs; under the context's lock.  They outlive a context
-// that tg_release_buffers ends: graphs hold them.
-std::vector<CaptureWs *> g_captures[kMaxDev];
+// Per device, see Capture; under the context's lock.  They outlive a context that
+// tg_release_buffers ends: graphs hold them.
+std::vector<Capture *> g_captures[kMaxDev];
 std::mutex g_ctx_mu;
 
 int get_ctx(DevCtx **out)
@@ -199,55 +214,99 @@ int grow(Buf &b, size_t bytes)
     return TG_OK;
 }
 
+// The live capture `id`, or nullptr.
+Capture *find_capture(DevCtx *c, unsigned long long id)
+{
+    for (Capture *p : g_captures[c->dev])
+        if (p->state.load(std::memory_order_acquire) == Capture::kLive && p->id == id) return p;
+    return nullptr;
+}
+
+// A set of workspaces for the capture `id` into `graph`.
+int new_capture(DevCtx *c, unsigned long long id, cudaGraph_t graph, bool owned, Capture **out)
+{
+    Capture *s = nullptr;
+    for (Capture *p : g_captures[c->dev])
+        if (p->state.load(std::memory_order_acquire) == Capture::kUnused) s = p;
+    if (!s) {
+        s = new (std::nothrow) Capture;
+        if (!s) return TG_ENOMEM;
+        g_captures[c->dev].push_back(s);
+    }
+    s->id = id;
+    s->used = 0;
+    s->owned = owned;
+    if (!owned) {
+        // the destructor, on a thread of the driver's, may call no CUDA function
+        cudaUserObject_t obj = nullptr;
+        TG_CUDA(cudaUserObjectCreate(
+            &obj, s,
+            [](void *p) { static_cast<Capture *>(p)->state.store(Capture::kUnused, std::memory_order_release); }, 1,
+            cudaUserObjectNoDestructorSync));
+        s->state.store(Capture::kLive, std::memory_order_release);
+        cudaError_t e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
+        if (e != cudaSuccess) cudaUserObjectRelease(obj, 1);   // marks it unused
+        TG_CUDA(e);
+    }
+    s->state.store(Capture::kLive, std::memory_order_release);
+    *out = s;
+    return TG_OK;
+}
+
 // The workspace of stream st in the capture `id` into `graph`.
 int capture_ws(DevCtx *c, cudaStream_t st, unsigned long long id, cudaGraph_t graph, StreamWs **out)
 {
-    CaptureWs *w = nullptr;
-    for (CaptureWs *p : g_captures[c->dev]) {
-        if (p->unused.load(std::memory_order_acquire)) {
-            if (!w) w = p;
-        } else if (p->key == st && p->id == id) {
-            *out = p;
+    Capture *s = find_capture(c, id);
+    int rc = TG_OK;
+    if (!s && (rc = new_capture(c, id, graph, false, &s))) return rc;
+    for (size_t i = 0; i < s->used; ++i)
+        if (s->ws[i]->key == st) {
+            *out = s->ws[i];
             return TG_OK;
         }
-    }
-    if (!w) {
-        w = new (std::nothrow) CaptureWs;
+    if (s->used == s->ws.size()) {
+        CaptureWs *w = new (std::nothrow) CaptureWs;
         if (!w) return TG_ENOMEM;
-        g_captures[c->dev].push_back(w);
+        s->ws.push_back(w);
     }
+    CaptureWs *w = s->ws[s->used];
     if (!w->flags) TG_CUDA(capture_malloc((void **)&w->flags, sizeof(unsigned)));
-    // the destructor, on a thread of the driver's, may call no CUDA function
-    cudaUserObject_t obj = nullptr;
-    TG_CUDA(cudaUserObjectCreate(
-        &obj, w, [](void *p) { static_cast<CaptureWs *>(p)->unused.store(true, std::memory_order_release); }, 1,
-        cudaUserObjectNoDestructorSync));
-    w->unused.store(false, std::memory_order_release);
-    cudaError_t e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
-    if (e != cudaSuccess) cudaUserObjectRelease(obj, 1);   // marks it unused
-    TG_CUDA(e);
     w->key = st;
-    w->id = id;
+    ++s->used;
     *out = w;
     return TG_OK;
 }
 
 // Gives back what captures whose graphs are gone leave: the buffers that they
-// outgrew, and the workspaces beyond `keep`.
+// outgrew, and the sets of workspaces beyond `keep`.
 void trim_captures(DevCtx *c, size_t keep)
 {
-    std::vector<CaptureWs *> &all = g_captures[c->dev];
+    std::vector<Capture *> &all = g_captures[c->dev];
+    bool released = false;
+    for (Capture *s : all) released = released || s->state.load(std::memory_order_acquire) == Capture::kReleased;
+    if (!released && all.size() <= keep) return;
     RelaxedCapture relaxed;
+    if (released) {
+        // launches of the graphs that held them may still run
+        if (cudaDeviceSynchronize() == cudaSuccess) {
+            for (Capture *s : all) {
+                int expect = Capture::kReleased;
+                s->state.compare_exchange_strong(expect, Capture::kUnused, std::memory_order_acq_rel);
+            }
+        } else {
+            cudaGetLastError();   // beside another capture: a later call does it
+        }
+    }
     size_t n = 0;
     for (size_t i = 0; i < all.size();) {
-        CaptureWs *w = all[i];
-        if (!w->unused.load(std::memory_order_acquire)) {
+        Capture *s = all[i];
+        if (s->state.load(std::memory_order_acquire) != Capture::kUnused) {
             ++i;
         } else if (n++ < keep) {
-            w->free_outgrown();
+            for (CaptureWs *w : s->ws) w->free_outgrown();
             ++i;
         } else {
-            delete w;
+            delete s;
             all.erase(all.begin() + i);
         }
     }
@@ -266,7 +325,7 @@ int stream_ws(DevCtx *c, cudaStream_t st, StreamWs **out)
         cudaGetLastError();   // the legacy stream beside a capture: the launches report it
     else if (capture == cudaStreamCaptureStatusActive)
         return capture_ws(c, st, id, graph, out);
-    if (g_captures[c->dev].size() > kStreamWs) trim_captures(c, kStreamWs);
+    trim_captures(c, kCaptures);
     StreamWs *hit = nullptr, *free_ws = nullptr, *lru = nullptr;
     for (StreamWs &w : c->ws) {
         if (w.used && w.key == st) {
@@ -2963,6 +3022,42 @@ __attribute__((visibility("default"))) int tg_plan_destroy(tg_plan *p)
     if (!p) return TG_OK;
     cudaDeviceSynchronize();
     plan_free(p);
+    return TG_OK;
+}
+
+__attribute__((visibility("default"))) int tg_capture_own(void *stream, unsigned long long *id)
+{
+    DevCtx *cx = nullptr;
+    if (!id) {
+        set_err("tg_capture_own: id is NULL");
+        return TG_EINVAL;
+    }
+    int rc = get_ctx(&cx);
+    if (rc) return rc;
+    std::lock_guard<std::mutex> lk(cx->mu);
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    cudaGraph_t graph = nullptr;
+    TG_CUDA(cudaStreamGetCaptureInfo((cudaStream_t)stream, &status, id, &graph, nullptr, nullptr));
+    if (status != cudaStreamCaptureStatusActive || find_capture(cx, *id)) {
+        set_err("tg_capture_own: the stream is not being captured, or a call was captured before this one");
+        return TG_EINVAL;
+    }
+    Capture *s = nullptr;
+    return new_capture(cx, *id, graph, true, &s);
+}
+
+__attribute__((visibility("default"))) int tg_capture_release(unsigned long long id)
+{
+    DevCtx *cx = nullptr;
+    int rc = get_ctx(&cx);
+    if (rc) return rc;
+    std::lock_guard<std::mutex> lk(cx->mu);
+    Capture *s = find_capture(cx, id);
+    if (!s || !s->owned) {
+        set_err("tg_capture_release: no capture %llu that a caller owns on this device", id);
+        return TG_EINVAL;
+    }
+    s->state.store(Capture::kReleased, std::memory_order_release);
     return TG_OK;
 }
 

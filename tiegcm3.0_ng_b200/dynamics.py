@@ -189,7 +189,7 @@ class DynamicsStep:
         # the O+ sub-cycle is the step's longest chain: its stream gets the higher priority
         self.streams = ([torch.cuda.Stream(device=device, priority=-1)] +
                         [torch.cuda.Stream(device=device) for _ in range(3)]) if fan_out else []
-        self.graph = None
+        self.graph = self._captured = None
 
     # ---- the routines, each on one stream --------------------------------
     def _horiz(self, f, hadvec, fin, fout, st):
@@ -271,12 +271,29 @@ class DynamicsStep:
         """Records one step into a CUDA graph (after an eager step, which
         loads the kernels); replay() then runs it."""
         import torch
+        self._drop_graph()
         self.issue(stream)
         stream.synchronize()
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph, stream=stream, capture_error_mode="thread_local"):
+            self._captured = cs.capture_own(stream)
             self.issue(stream)
         return self.graph
+
+    def _drop_graph(self):
+        # the graph's work buffers live as long as this object, whose fields its kernels use too
+        graph, self.graph = self.graph, None
+        if graph is not None:
+            graph.reset()
+        captured, self._captured = self._captured, None
+        if captured is not None:
+            cs.capture_release(captured)
+
+    def __del__(self):
+        try:
+            self._drop_graph()
+        except Exception:
+            pass
 
     def replay(self, stream):
         import torch
