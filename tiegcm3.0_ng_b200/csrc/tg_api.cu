@@ -214,10 +214,10 @@ int grow(Buf &b, size_t bytes)
     return TG_OK;
 }
 
-// The live capture `id`, or nullptr.
-Capture *find_capture(DevCtx *c, unsigned long long id)
+// The live capture `id` on a device, or nullptr.
+Capture *find_capture(int dev, unsigned long long id)
 {
-    for (Capture *p : g_captures[c->dev])
+    for (Capture *p : g_captures[dev])
         if (p->state.load(std::memory_order_acquire) == Capture::kLive && p->id == id) return p;
     return nullptr;
 }
@@ -256,7 +256,7 @@ int new_capture(DevCtx *c, unsigned long long id, cudaGraph_t graph, bool owned,
 // The workspace of stream st in the capture `id` into `graph`.
 int capture_ws(DevCtx *c, cudaStream_t st, unsigned long long id, cudaGraph_t graph, StreamWs **out)
 {
-    Capture *s = find_capture(c, id);
+    Capture *s = find_capture(c->dev, id);
     int rc = TG_OK;
     if (!s && (rc = new_capture(c, id, graph, false, &s))) return rc;
     for (size_t i = 0; i < s->used; ++i)
@@ -3038,7 +3038,7 @@ __attribute__((visibility("default"))) int tg_capture_own(void *stream, unsigned
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     cudaGraph_t graph = nullptr;
     TG_CUDA(cudaStreamGetCaptureInfo((cudaStream_t)stream, &status, id, &graph, nullptr, nullptr));
-    if (status != cudaStreamCaptureStatusActive || find_capture(cx, *id)) {
+    if (status != cudaStreamCaptureStatusActive || find_capture(cx->dev, *id)) {
         set_err("tg_capture_own: the stream is not being captured, or a call was captured before this one");
         return TG_EINVAL;
     }
@@ -3048,17 +3048,19 @@ __attribute__((visibility("default"))) int tg_capture_own(void *stream, unsigned
 
 __attribute__((visibility("default"))) int tg_capture_release(unsigned long long id)
 {
-    DevCtx *cx = nullptr;
-    int rc = get_ctx(&cx);
-    if (rc) return rc;
-    std::lock_guard<std::mutex> lk(cx->mu);
-    Capture *s = find_capture(cx, id);
-    if (!s || !s->owned) {
-        set_err("tg_capture_release: no capture %llu that a caller owns on this device", id);
-        return TG_EINVAL;
+    // on any device: the ids are the process's, and the current device need not
+    // be the capture's
+    std::lock_guard<std::mutex> lk(g_ctx_mu);
+    for (int d = 0; d < kMaxDev; ++d) {
+        std::unique_lock<std::mutex> lk2;
+        if (g_ctx[d]) lk2 = std::unique_lock<std::mutex>(g_ctx[d]->mu);
+        Capture *s = find_capture(d, id);
+        if (!s || !s->owned) continue;
+        s->state.store(Capture::kReleased, std::memory_order_release);
+        return TG_OK;
     }
-    s->state.store(Capture::kReleased, std::memory_order_release);
-    return TG_OK;
+    set_err("tg_capture_release: no capture %llu that a caller owns", id);
+    return TG_EINVAL;
 }
 
 __attribute__((visibility("default"))) int tg_release_buffers(void)
