@@ -803,7 +803,9 @@ int tg_selftest_walk(int which, double *buf, int nk, int K, int top, int ncol, l
  * stream that is being captured and before the first captured call of this
  * library, gives the capture's id; tg_capture_release, after the graph and its
  * executables are destroyed (launches may still be running), gives the buffers
- * back; owned buffers that are never released stay until the process exits. */
+ * back; owned buffers that are never released stay until the process exits.  An
+ * owned graph takes over the buffers that earlier calls on its streams used:
+ * those calls must be complete before it is launched. */
 int tg_capture_own(void *stream, unsigned long long *id);
 int tg_capture_release(unsigned long long id);
 /* Frees the per-device mirrors, work buffers and streams (not the buffers that

@@ -175,3 +175,42 @@ def test_steps_of_two_sizes(cuda, pkg):
         torch.cuda.synchronize()
         for k, v in s.outputs().items():
             assert bits(v[:, :s.grid.ncol].contiguous(), w[k].contiguous()), k
+
+
+def test_released_captures_without_eager_calls(cuda, pkg):
+    """A caller that only captures and releases, 40 times."""
+    import torch
+    st, d = torch.cuda.Stream(), Dt(pkg, 57, 20000, 7)
+    want, free = d.result(st, lambda: d.issue(st)), []
+    for i in range(40):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st, capture_error_mode="thread_local"):
+            own = pkg.capture_own(st)
+            d.issue(st)
+        assert bits(d.result(st, g.replay), want)
+        g.reset()
+        pkg.capture_release(own)
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[9] - free[-1] <= 8 * 37e6
+
+
+def test_an_owned_graph_and_eager_calls_after_it(cuda, pkg):
+    """The graph took over its stream's buffers: eager calls there get others."""
+    import torch
+    st = torch.cuda.Stream()
+    p, q = Dt(pkg, 57, 6000, 8), Dt(pkg, 57, 6000, 9)
+    want = [x.result(st, lambda: x.issue(st)) for x in (p, q)]
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st, capture_error_mode="thread_local"):
+        own = pkg.capture_own(st)
+        p.issue(st)
+    other = torch.cuda.Stream()
+    for _ in range(20):
+        with torch.cuda.stream(other):
+            g.replay()
+        q.issue(st)
+    torch.cuda.synchronize()
+    for x, w in zip((p, q), want):
+        assert bits(x.out[:, :x.ncol], w)
+    g.reset()
+    pkg.capture_release(own)

@@ -14,6 +14,7 @@
 #include <cstdio>
 #include <cstring>
 #include <atomic>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <new>
@@ -50,7 +51,7 @@ int g_host_precision = TG_PREC_F64;
 struct Buf {
     void *p = nullptr;
     size_t n = 0;
-    std::vector<void *> *outgrown = nullptr;   // set where a captured graph may hold p: see CaptureWs
+    std::vector<Buf> *outgrown = nullptr;   // set where a captured graph may hold p: see Capture
 };
 
 // Per-device work buffers and streams, created on first use.  The host
@@ -74,51 +75,31 @@ struct StreamWs {
     unsigned *flags = nullptr;     // device status word
 };
 constexpr int kStreamWs = 16;
-// The workspace of one stream within one capture.  The captured graph's kernels
-// hold its addresses for as long as the graph can be launched, so it is the
-// graph's own: no later call on the stream grows, frees or uses it, and a buffer
-// outgrown within the capture stays.
-struct CaptureWs : StreamWs {
-    std::vector<void *> outgrown;
-    CaptureWs()
-    {
-        for (Buf &b : lvl) b.outgrown = &outgrown;
-        scratch.outgrown = &outgrown;
-    }
-    void free_outgrown()
-    {
-        for (void *p : outgrown) cudaFree(p);
-        outgrown.clear();
-    }
-    ~CaptureWs()
-    {
-        free_outgrown();
-        for (Buf &b : lvl)
-            if (b.p) cudaFree(b.p);
-        if (scratch.p) cudaFree(scratch.p);
-        if (flags) cudaFree(flags);
-    }
-};
-// Those of one capture, a stream each.  The graph (and every executable made from
-// it) holds a user object whose destructor, after the last of them and its last
-// launch are done, marks them unused; they then serve another capture, and beyond
-// kCaptures unused sets are freed.  The object costs every launch of the graph 2 to
-// 7 us (a dynamics step of 161 us takes 163 to 168), so a caller who says when the
-// graph is gone (tg_capture_own, tg_capture_release) gets none; what it releases is
-// unused once the device has been drained.
+// The workspaces of one capture, a stream each.  The captured graph's kernels hold
+// their addresses for as long as the graph can be launched, so they are the
+// graph's own: no later call on its streams grows, frees or uses them, and a
+// buffer outgrown within the capture stays.  The graph (and every executable made
+// from it) holds a user object whose destructor, after the last of them and its
+// last launch are done, marks them unused.  The object costs every launch of the
+// graph 2 to 7 us (a dynamics step of 161 us takes 163 to 168), so a caller who
+// says when the graph is gone (tg_capture_own, tg_capture_release) gets none; what
+// it releases is unused once the device has been drained.
 struct Capture {
+    struct Ws : StreamWs {
+        Buf flagbuf;
+    };
     enum State { kUnused, kLive, kReleased };
-    unsigned long long id = 0;
-    std::vector<CaptureWs *> ws;
-    size_t used = 0;   // the first ws, in the order in which the capture's streams came
-    bool owned = false;
-    std::atomic<int> state{kUnused};
-    ~Capture()
-    {
-        for (CaptureWs *w : ws) delete w;
-    }
+    unsigned long long id;
+    bool owned;
+    std::vector<std::unique_ptr<Ws>> ws;
+    std::vector<Buf> outgrown;
+    std::atomic<int> state{kLive};
+    Capture(unsigned long long id_, bool owned_) : id(id_), owned(owned_) {}
 };
-constexpr size_t kCaptures = 4;
+// Buffers that captures left, for the next need of about their size; past this
+// many the oldest are freed.
+constexpr size_t kPooled = 32;
+constexpr size_t kReleasedMost = 4;   // captures that owners released and no call has taken back
 // While one lives, this thread may allocate and free beside any stream capture.
 struct RelaxedCapture {
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
@@ -143,9 +124,10 @@ struct DevCtx {
 
 constexpr int kMaxDev = 64;
 DevCtx *g_ctx[kMaxDev] = {};
-// Per device, see Capture; under the context's lock.  They outlive a context that
+// Per device, see Capture and kPooled; under the context's lock.  They outlive a context that
 // tg_release_buffers ends: graphs hold them.
 std::vector<Capture *> g_captures[kMaxDev];
+std::vector<Buf> g_pool[kMaxDev];
 std::mutex g_ctx_mu;
 
 int get_ctx(DevCtx **out)
@@ -186,13 +168,30 @@ cudaError_t capture_malloc(void **p, size_t bytes)
     return cudaMalloc(p, bytes);
 }
 
+// The smallest buffer of the current device's pool that holds `bytes` and at most
+// twice as many.
+bool take_pooled(Buf &b, size_t bytes)
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return false;
+    std::vector<Buf> &pool = g_pool[dev];
+    size_t best = pool.size();
+    for (size_t i = 0; i < pool.size(); ++i)
+        if (pool[i].n >= bytes && pool[i].n <= 2 * bytes && (best == pool.size() || pool[i].n < pool[best].n)) best = i;
+    if (best == pool.size()) return false;
+    b.p = pool[best].p;
+    b.n = pool[best].n;
+    pool.erase(pool.begin() + best);
+    return true;
+}
+
 // Grows a device buffer; the device is synchronised before an old buffer is
 // freed, since queued work may still use it.  A capture's old buffer stays.
 int grow(Buf &b, size_t bytes)
 {
     if (bytes <= b.n) return TG_OK;
     if (b.p && b.outgrown) {
-        b.outgrown->push_back(b.p);
+        b.outgrown->push_back(Buf{b.p, b.n});
         b.p = nullptr;
         b.n = 0;
     }
@@ -203,6 +202,7 @@ int grow(Buf &b, size_t bytes)
         b.n = 0;
     }
     bytes = (bytes + 4095) & ~(size_t)4095;
+    if (take_pooled(b, bytes)) return TG_OK;
     cudaError_t e = b.outgrown ? capture_malloc(&b.p, bytes) : cudaMalloc(&b.p, bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -222,33 +222,71 @@ Capture *find_capture(int dev, unsigned long long id)
     return nullptr;
 }
 
-// A set of workspaces for the capture `id` into `graph`.
+// Takes the buffers of captures whose graphs are gone into the pool and, outside a
+// capture, waits for those that owners released and keeps the pool within `keep`.
+void recycle_captures(int dev, size_t keep, bool capturing)
+{
+    std::vector<Capture *> &all = g_captures[dev];
+    std::vector<Buf> &pool = g_pool[dev];
+    bool released = false, unused = false;
+    for (Capture *s : all) {
+        const int state = s->state.load(std::memory_order_acquire);
+        released = released || state == Capture::kReleased;
+        unused = unused || state == Capture::kUnused;
+    }
+    if (capturing ? !unused : !released && !unused && pool.size() <= keep) return;
+    RelaxedCapture relaxed;
+    // launches of the graphs whose owners released their buffers may still run
+    // (beside another capture the wait is refused: a later call does it)
+    const bool drained = released && !capturing && cudaDeviceSynchronize() == cudaSuccess;
+    if (released && !capturing && !drained) cudaGetLastError();
+    for (size_t i = 0; i < all.size();) {
+        Capture *s = all[i];
+        const int state = s->state.load(std::memory_order_acquire);
+        if (state == Capture::kLive || (state == Capture::kReleased && !drained)) {
+            ++i;
+            continue;
+        }
+        auto give = [&](const Buf &b) {
+            if (b.p) pool.push_back(Buf{b.p, b.n});
+        };
+        for (const Buf &b : s->outgrown) give(b);
+        for (auto &w : s->ws) {
+            give(w->scratch);
+            give(w->flagbuf);
+            for (const Buf &b : w->lvl) give(b);
+        }
+        delete s;
+        all.erase(all.begin() + i);
+    }
+    while (!capturing && pool.size() > keep) {
+        cudaFree(pool.front().p);
+        pool.erase(pool.begin());
+    }
+}
+
+// The workspaces of the capture `id` into `graph`, none yet.
 int new_capture(DevCtx *c, unsigned long long id, cudaGraph_t graph, bool owned, Capture **out)
 {
-    Capture *s = nullptr;
-    for (Capture *p : g_captures[c->dev])
-        if (p->state.load(std::memory_order_acquire) == Capture::kUnused) s = p;
-    if (!s) {
-        s = new (std::nothrow) Capture;
-        if (!s) return TG_ENOMEM;
-        g_captures[c->dev].push_back(s);
-    }
-    s->id = id;
-    s->used = 0;
-    s->owned = owned;
+    recycle_captures(c->dev, kPooled, true);
+    Capture *s = new (std::nothrow) Capture(id, owned);
+    if (!s) return TG_ENOMEM;
     if (!owned) {
         // the destructor, on a thread of the driver's, may call no CUDA function
         cudaUserObject_t obj = nullptr;
-        TG_CUDA(cudaUserObjectCreate(
+        cudaError_t e = cudaUserObjectCreate(
             &obj, s,
             [](void *p) { static_cast<Capture *>(p)->state.store(Capture::kUnused, std::memory_order_release); }, 1,
-            cudaUserObjectNoDestructorSync));
-        s->state.store(Capture::kLive, std::memory_order_release);
-        cudaError_t e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
+            cudaUserObjectNoDestructorSync);
+        if (e != cudaSuccess) delete s;
+        TG_CUDA(e);
+        g_captures[c->dev].push_back(s);
+        e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
         if (e != cudaSuccess) cudaUserObjectRelease(obj, 1);   // marks it unused
         TG_CUDA(e);
+    } else {
+        g_captures[c->dev].push_back(s);
     }
-    s->state.store(Capture::kLive, std::memory_order_release);
     *out = s;
     return TG_OK;
 }
@@ -259,57 +297,30 @@ int capture_ws(DevCtx *c, cudaStream_t st, unsigned long long id, cudaGraph_t gr
     Capture *s = find_capture(c->dev, id);
     int rc = TG_OK;
     if (!s && (rc = new_capture(c, id, graph, false, &s))) return rc;
-    for (size_t i = 0; i < s->used; ++i)
-        if (s->ws[i]->key == st) {
-            *out = s->ws[i];
+    for (auto &w : s->ws)
+        if (w->key == st) {
+            *out = w.get();
             return TG_OK;
         }
-    if (s->used == s->ws.size()) {
-        CaptureWs *w = new (std::nothrow) CaptureWs;
-        if (!w) return TG_ENOMEM;
-        s->ws.push_back(w);
-    }
-    CaptureWs *w = s->ws[s->used];
-    if (!w->flags) TG_CUDA(capture_malloc((void **)&w->flags, sizeof(unsigned)));
+    std::unique_ptr<Capture::Ws> w(new (std::nothrow) Capture::Ws);
+    if (!w) return TG_ENOMEM;
     w->key = st;
-    ++s->used;
-    *out = w;
-    return TG_OK;
-}
-
-// Gives back what captures whose graphs are gone leave: the buffers that they
-// outgrew, and the sets of workspaces beyond `keep`.
-void trim_captures(DevCtx *c, size_t keep)
-{
-    std::vector<Capture *> &all = g_captures[c->dev];
-    bool released = false;
-    for (Capture *s : all) released = released || s->state.load(std::memory_order_acquire) == Capture::kReleased;
-    if (!released && all.size() <= keep) return;
-    RelaxedCapture relaxed;
-    if (released) {
-        // launches of the graphs that held them may still run
-        if (cudaDeviceSynchronize() == cudaSuccess) {
-            for (Capture *s : all) {
-                int expect = Capture::kReleased;
-                s->state.compare_exchange_strong(expect, Capture::kUnused, std::memory_order_acq_rel);
+    w->flagbuf.outgrown = &s->outgrown;
+    if ((rc = grow(w->flagbuf, sizeof(unsigned)))) return rc;
+    w->flags = (unsigned *)w->flagbuf.p;
+    // an owner's graph takes over the stream's own buffers: the eager calls that
+    // used them are done before its first launch
+    if (s->owned)
+        for (StreamWs &e : c->ws)
+            if (e.used && e.key == st) {
+                std::swap(w->scratch, e.scratch);
+                for (int i = 0; i < 7; ++i) std::swap(w->lvl[i], e.lvl[i]);
             }
-        } else {
-            cudaGetLastError();   // beside another capture: a later call does it
-        }
-    }
-    size_t n = 0;
-    for (size_t i = 0; i < all.size();) {
-        Capture *s = all[i];
-        if (s->state.load(std::memory_order_acquire) != Capture::kUnused) {
-            ++i;
-        } else if (n++ < keep) {
-            for (CaptureWs *w : s->ws) w->free_outgrown();
-            ++i;
-        } else {
-            delete s;
-            all.erase(all.begin() + i);
-        }
-    }
+    w->scratch.outgrown = &s->outgrown;
+    for (Buf &b : w->lvl) b.outgrown = &s->outgrown;
+    *out = w.get();
+    s->ws.push_back(std::move(w));
+    return TG_OK;
 }
 
 // The workspace of caller stream st (the caller holds c->mu).  A stream
@@ -325,7 +336,7 @@ int stream_ws(DevCtx *c, cudaStream_t st, StreamWs **out)
         cudaGetLastError();   // the legacy stream beside a capture: the launches report it
     else if (capture == cudaStreamCaptureStatusActive)
         return capture_ws(c, st, id, graph, out);
-    trim_captures(c, kCaptures);
+    recycle_captures(c->dev, kPooled, false);
     StreamWs *hit = nullptr, *free_ws = nullptr, *lru = nullptr;
     for (StreamWs &w : c->ws) {
         if (w.used && w.key == st) {
@@ -3057,6 +3068,16 @@ __attribute__((visibility("default"))) int tg_capture_release(unsigned long long
         Capture *s = find_capture(d, id);
         if (!s || !s->owned) continue;
         s->state.store(Capture::kReleased, std::memory_order_release);
+        // the next eager call takes them back; a caller who makes none waits here
+        size_t n = 0;
+        for (Capture *p : g_captures[d]) n += p->state.load(std::memory_order_acquire) == Capture::kReleased;
+        if (n > kReleasedMost) {
+            int cur = 0;
+            cudaGetDevice(&cur);
+            cudaSetDevice(d);
+            recycle_captures(d, kPooled, false);
+            cudaSetDevice(cur);
+        }
         return TG_OK;
     }
     set_err("tg_capture_release: no capture %llu that a caller owns", id);
@@ -3089,7 +3110,7 @@ __attribute__((visibility("default"))) int tg_release_buffers(void)
             if (w.scratch.p) cudaFree(w.scratch.p);
             if (w.flags) cudaFree(w.flags);
         }
-        trim_captures(c, 0);   // those of live graphs stay theirs
+        recycle_captures(d, 0, false);   // those of live graphs stay theirs
         if (c->flags) cudaFree(c->flags);
         if (c->flags_host) cudaFreeHost(c->flags_host);
         if (c->hist) cudaFree(c->hist);
