@@ -27,7 +27,9 @@
  *     than the stream had, allocate and synchronise.  Calls captured into a
  *     CUDA graph get buffers of that graph's own, which live as long as the
  *     graph and its executables, so graphs may run side by side (make one
- *     call outside a capture first, which sets up the device).
+ *     call outside a capture first, which sets up the device).  A capture in
+ *     another thread does not survive a synchronisation: no first call, no
+ *     growing one and no seventeenth stream beside it.
  *   - Every entry point returns a tg_status.  The reference has no error
  *     return (a zero pivot silently yields Inf/NaN); the solves here produce
  *     the same numbers in that case and additionally report TG_EPIVOT.
@@ -801,11 +803,11 @@ int tg_selftest_walk(int which, double *buf, int nk, int K, int top, int ncol, l
  * CUDA user object, which costs each of its launches some microseconds.  A
  * caller who knows when the graph is gone saves that: tg_capture_own, on a
  * stream that is being captured and before the first captured call of this
- * library, gives the capture's id; tg_capture_release, after the graph and its
- * executables are destroyed (launches may still be running), gives the buffers
- * back; owned buffers that are never released stay until the process exits.  An
- * owned graph takes over the buffers that earlier calls on its streams used:
- * those calls must be complete before it is launched. */
+ * library, gives the capture's id; tg_capture_release, when the graph's launches
+ * are done and it will not be launched again, gives the buffers back; owned
+ * buffers that are never released stay until the process exits.  An owned graph
+ * takes over the buffers that earlier calls on its streams used: those calls
+ * must be complete before it is launched. */
 int tg_capture_own(void *stream, unsigned long long *id);
 int tg_capture_release(unsigned long long id);
 /* Frees the per-device mirrors, work buffers and streams (not the buffers that

@@ -1129,7 +1129,8 @@ def capture_own(stream=None):
 
 
 def capture_release(capture):
-    """Gives back the work buffers of a capture (capture_own) whose graph is destroyed."""
+    """Gives back the work buffers of a capture (capture_own) whose graph's launches are done and that will
+    not be launched again."""
     return _check(lib().tg_capture_release(capture), "tg_capture_release", numeric_ok=False)
 
 

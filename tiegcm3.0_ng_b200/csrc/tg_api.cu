@@ -82,24 +82,20 @@ constexpr int kStreamWs = 16;
 // from it) holds a user object whose destructor, after the last of them and its
 // last launch are done, marks them unused.  The object costs every launch of the
 // graph 2 to 7 us (a dynamics step of 161 us takes 163 to 168), so a caller who
-// says when the graph is gone (tg_capture_own, tg_capture_release) gets none; what
-// it releases is unused once the device has been drained.
+// says when the graph is gone (tg_capture_own, tg_capture_release) gets none.
 struct Capture {
-    struct Ws : StreamWs {
-        Buf flagbuf;
-    };
-    enum State { kUnused, kLive, kReleased };
     unsigned long long id;
     bool owned;
-    std::vector<std::unique_ptr<Ws>> ws;
+    std::vector<std::unique_ptr<StreamWs>> ws;
+    Buf flags;   // the workspaces' status words, kFlagStride apart
     std::vector<Buf> outgrown;
-    std::atomic<int> state{kLive};
+    std::atomic<bool> unused{false};
     Capture(unsigned long long id_, bool owned_) : id(id_), owned(owned_) {}
 };
-// Buffers that captures left, for the next need of about their size; past this
-// many the oldest are freed.
-constexpr size_t kPooled = 32;
-constexpr size_t kReleasedMost = 4;   // captures that owners released and no call has taken back
+constexpr size_t kFlagStride = 32, kFlagBytes = 4096;
+// What captures left, for the next need of about its size: the oldest buffers
+// past either limit are freed (with the device's synchronisation that brings).
+constexpr size_t kPooled = 64, kPooledBytes = (size_t)512 << 20;
 // While one lives, this thread may allocate and free beside any stream capture.
 struct RelaxedCapture {
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
@@ -218,57 +214,48 @@ int grow(Buf &b, size_t bytes)
 Capture *find_capture(int dev, unsigned long long id)
 {
     for (Capture *p : g_captures[dev])
-        if (p->state.load(std::memory_order_acquire) == Capture::kLive && p->id == id) return p;
+        if (!p->unused.load(std::memory_order_acquire) && p->id == id) return p;
     return nullptr;
 }
 
 // Takes the buffers of captures whose graphs are gone into the pool and, outside a
-// capture, waits for those that owners released and keeps the pool within `keep`.
-void recycle_captures(int dev, size_t keep, bool capturing)
+// capture, keeps that within its limits.
+void recycle_captures(int dev, size_t keep, size_t keep_bytes, bool capturing)
 {
     std::vector<Capture *> &all = g_captures[dev];
     std::vector<Buf> &pool = g_pool[dev];
-    bool released = false, unused = false;
-    for (Capture *s : all) {
-        const int state = s->state.load(std::memory_order_acquire);
-        released = released || state == Capture::kReleased;
-        unused = unused || state == Capture::kUnused;
-    }
-    if (capturing ? !unused : !released && !unused && pool.size() <= keep) return;
-    RelaxedCapture relaxed;
-    // launches of the graphs whose owners released their buffers may still run
-    // (beside another capture the wait is refused: a later call does it)
-    const bool drained = released && !capturing && cudaDeviceSynchronize() == cudaSuccess;
-    if (released && !capturing && !drained) cudaGetLastError();
     for (size_t i = 0; i < all.size();) {
         Capture *s = all[i];
-        const int state = s->state.load(std::memory_order_acquire);
-        if (state == Capture::kLive || (state == Capture::kReleased && !drained)) {
+        if (!s->unused.load(std::memory_order_acquire)) {
             ++i;
             continue;
         }
         auto give = [&](const Buf &b) {
             if (b.p) pool.push_back(Buf{b.p, b.n});
         };
+        give(s->flags);
         for (const Buf &b : s->outgrown) give(b);
         for (auto &w : s->ws) {
             give(w->scratch);
-            give(w->flagbuf);
             for (const Buf &b : w->lvl) give(b);
         }
         delete s;
         all.erase(all.begin() + i);
     }
-    while (!capturing && pool.size() > keep) {
+    if (capturing || pool.empty()) return;
+    size_t bytes = 0;
+    for (const Buf &b : pool) bytes += b.n;
+    while (pool.size() > keep || bytes > keep_bytes) {
+        RelaxedCapture relaxed;
+        bytes -= pool.front().n;
         cudaFree(pool.front().p);
         pool.erase(pool.begin());
     }
 }
-
 // The workspaces of the capture `id` into `graph`, none yet.
 int new_capture(DevCtx *c, unsigned long long id, cudaGraph_t graph, bool owned, Capture **out)
 {
-    recycle_captures(c->dev, kPooled, true);
+    recycle_captures(c->dev, kPooled, kPooledBytes, true);
     Capture *s = new (std::nothrow) Capture(id, owned);
     if (!s) return TG_ENOMEM;
     if (!owned) {
@@ -276,7 +263,7 @@ int new_capture(DevCtx *c, unsigned long long id, cudaGraph_t graph, bool owned,
         cudaUserObject_t obj = nullptr;
         cudaError_t e = cudaUserObjectCreate(
             &obj, s,
-            [](void *p) { static_cast<Capture *>(p)->state.store(Capture::kUnused, std::memory_order_release); }, 1,
+            [](void *p) { static_cast<Capture *>(p)->unused.store(true, std::memory_order_release); }, 1,
             cudaUserObjectNoDestructorSync);
         if (e != cudaSuccess) delete s;
         TG_CUDA(e);
@@ -302,12 +289,17 @@ int capture_ws(DevCtx *c, cudaStream_t st, unsigned long long id, cudaGraph_t gr
             *out = w.get();
             return TG_OK;
         }
-    std::unique_ptr<Capture::Ws> w(new (std::nothrow) Capture::Ws);
+    std::unique_ptr<StreamWs> w(new (std::nothrow) StreamWs);
     if (!w) return TG_ENOMEM;
     w->key = st;
-    w->flagbuf.outgrown = &s->outgrown;
-    if ((rc = grow(w->flagbuf, sizeof(unsigned)))) return rc;
-    w->flags = (unsigned *)w->flagbuf.p;
+    // one buffer of status words for as many streams as it has room for, then another
+    const size_t slot = s->ws.size() % (kFlagBytes / (kFlagStride * sizeof(unsigned)));
+    if (slot == 0) {
+        if (s->flags.p) s->outgrown.push_back(Buf{s->flags.p, s->flags.n});
+        s->flags = Buf{nullptr, 0, &s->outgrown};
+        if ((rc = grow(s->flags, kFlagBytes))) return rc;
+    }
+    w->flags = (unsigned *)s->flags.p + slot * kFlagStride;
     // an owner's graph takes over the stream's own buffers: the eager calls that
     // used them are done before its first launch
     if (s->owned)
@@ -336,7 +328,7 @@ int stream_ws(DevCtx *c, cudaStream_t st, StreamWs **out)
         cudaGetLastError();   // the legacy stream beside a capture: the launches report it
     else if (capture == cudaStreamCaptureStatusActive)
         return capture_ws(c, st, id, graph, out);
-    recycle_captures(c->dev, kPooled, false);
+    recycle_captures(c->dev, kPooled, kPooledBytes, false);
     StreamWs *hit = nullptr, *free_ws = nullptr, *lru = nullptr;
     for (StreamWs &w : c->ws) {
         if (w.used && w.key == st) {
@@ -3067,17 +3059,7 @@ __attribute__((visibility("default"))) int tg_capture_release(unsigned long long
         if (g_ctx[d]) lk2 = std::unique_lock<std::mutex>(g_ctx[d]->mu);
         Capture *s = find_capture(d, id);
         if (!s || !s->owned) continue;
-        s->state.store(Capture::kReleased, std::memory_order_release);
-        // the next eager call takes them back; a caller who makes none waits here
-        size_t n = 0;
-        for (Capture *p : g_captures[d]) n += p->state.load(std::memory_order_acquire) == Capture::kReleased;
-        if (n > kReleasedMost) {
-            int cur = 0;
-            cudaGetDevice(&cur);
-            cudaSetDevice(d);
-            recycle_captures(d, kPooled, false);
-            cudaSetDevice(cur);
-        }
+        s->unused.store(true, std::memory_order_release);
         return TG_OK;
     }
     set_err("tg_capture_release: no capture %llu that a caller owns", id);
@@ -3110,7 +3092,7 @@ __attribute__((visibility("default"))) int tg_release_buffers(void)
             if (w.scratch.p) cudaFree(w.scratch.p);
             if (w.flags) cudaFree(w.flags);
         }
-        recycle_captures(d, 0, false);   // those of live graphs stay theirs
+        recycle_captures(d, 0, 0, false);   // those of live graphs stay theirs
         if (c->flags) cudaFree(c->flags);
         if (c->flags_host) cudaFreeHost(c->flags_host);
         if (c->hist) cudaFree(c->hist);

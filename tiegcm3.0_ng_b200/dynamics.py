@@ -281,7 +281,8 @@ class DynamicsStep:
         return self.graph
 
     def _drop_graph(self):
-        # the graph's work buffers live as long as this object, whose fields its kernels use too
+        # the graph's work buffers live as long as this object, whose fields its kernels use too:
+        # neither may go while a replay runs
         graph, self.graph = self.graph, None
         if graph is not None:
             graph.reset()
