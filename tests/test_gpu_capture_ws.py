@@ -212,3 +212,51 @@ def test_an_owned_graph_and_eager_calls_after_it(cuda, pkg):
         assert bits(x.out[:, :x.ncol], w)
     g.reset()
     pkg.capture_release(own)
+
+
+def test_captures_beside_other_threads(cuda, pkg):
+    """Three threads, each on its stream: eager calls, captures (owned and not),
+    replays, releases.  What one thread's graphs leave, the others' calls take."""
+    import threading
+    import torch
+    sizes, errs, lock, start = (700, 3000, 1500), [], threading.Lock(), threading.Barrier(3)
+    work = [[Dt(pkg, 57, n, 20 + i) for i, n in enumerate(sizes)] for _ in range(3)]
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    want = [d.result(streams[0], lambda: d.issue(streams[0])) for d in work[0]]
+    for st, ds in zip(streams, work):          # a growing call synchronises, which another thread's capture does not survive
+        ds[1].result(st, lambda: ds[1].issue(st))
+
+    def run(t):
+        try:
+            st = streams[t]
+            start.wait()
+            for it in range(9):
+                d, w = work[t][(t + it) % 3], want[(t + it) % 3]
+                with torch.cuda.stream(st):
+                    for _ in range(3):
+                        d.issue(st)
+                g, own = torch.cuda.CUDAGraph(), None
+                with lock:                     # torch's own bookkeeping of captures
+                    with torch.cuda.graph(g, stream=st, capture_error_mode="thread_local"):
+                        own = pkg.capture_own(st) if it % 2 else None
+                        d.issue(st)
+                with torch.cuda.stream(st):
+                    d.out.fill_(float("nan"))
+                    g.replay()
+                    r = d.out[:, :d.ncol].clone()
+                st.synchronize()
+                if not bits(r, w):
+                    errs.append((t, it))
+                with lock:
+                    g.reset()
+                if own is not None:
+                    pkg.capture_release(own)
+        except Exception as e:                 # reported below, with the thread's number
+            errs.append((t, repr(e)))
+
+    threads = [threading.Thread(target=run, args=(t,)) for t in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert errs == []
